@@ -13,6 +13,26 @@
 
 namespace pn {
 
+// 2: only the C11..C33 block and the shear diagonal; 1: monoclinic about z;
+// 0: general (see c_used in rsg_grid.cu and rsg_fast.cu)
+int symmetry_class(const MaterialTables &mt) {
+  bool ortho = true, mono = true;
+  for (int32_t m = 0; m < mt.n_mat; m++) {
+    const double *c = &mt.c36[(size_t)m * 36];
+    for (int k = 0; k < 6; k++)
+      for (int j = 0; j < 6; j++) {
+        const double v = c[k * 6 + j];
+        if (v == 0.0) continue;
+        const bool in_ortho = (k < 3 && j < 3) || k == j;
+        const bool in_mono = in_ortho || (k == 5 && j < 3) || (j == 5 && k < 3) || (k == 3 && j == 4) ||
+                             (k == 4 && j == 3);
+        ortho = ortho && in_ortho;
+        mono = mono && in_mono;
+      }
+  }
+  return ortho ? 2 : mono ? 1 : 0;
+}
+
 namespace {
 
 struct Tiles {
@@ -68,26 +88,6 @@ void cell_ijk(const GridMap &g, int64_t q, int64_t &i, int64_t &j, int64_t &k) {
   i = q % g.pcx;
   j = (q / g.pcx) % g.ny;
   k = q / ((int64_t)g.pcx * g.ny);
-}
-
-// 2: only the C11..C33 block and the shear diagonal; 1: monoclinic about z;
-// 0: general (see c_used in rsg_grid.cu)
-int symmetry_class(const MaterialTables &mt) {
-  bool ortho = true, mono = true;
-  for (int32_t m = 0; m < mt.n_mat; m++) {
-    const double *c = &mt.c36[(size_t)m * 36];
-    for (int k = 0; k < 6; k++)
-      for (int j = 0; j < 6; j++) {
-        const double v = c[k * 6 + j];
-        if (v == 0.0) continue;
-        const bool in_ortho = (k < 3 && j < 3) || k == j;
-        const bool in_mono = in_ortho || (k == 5 && j < 3) || (j == 5 && k < 3) || (k == 3 && j == 4) ||
-                             (k == 4 && j == 3);
-        ortho = ortho && in_ortho;
-        mono = mono && in_mono;
-      }
-  }
-  return ortho ? 2 : mono ? 1 : 0;
 }
 
 // (block, layer, local, payload) rows sorted by (block, layer) with the

@@ -82,7 +82,7 @@ struct pn_solver {
 
   // grid form
   pn::GridMap grid;
-  int sym = 0;             // material symmetry class of the stiffness table
+  int sym = 0;             // material symmetry class of the stiffness table (both forms)
   uint8_t *d_gmat = nullptr;
   void *d_tmaps = nullptr;   // tensor maps [2 input parities] (null: classic kernel)
   int32_t *d_ktop = nullptr; // [tiles] cell layers the tensor-copy kernel marches per tile
@@ -301,6 +301,10 @@ namespace pn {
 // (may_alloc false: refill the resident table in place, never grow it)
 void ensure_signal_rows(pn_solver *s, int64_t nsteps, bool may_alloc = true);
 int64_t sig_row(const pn_solver *s, int64_t step_in_call);  // row of this step
+
+// symmetry class of a stiffness table (pn_grid.cpp): 2 orthotropic in the
+// axes, 1 monoclinic about z, 0 general
+int symmetry_class(const MaterialTables &mt);
 
 // table form (pn_table.cpp)
 int64_t table_footprint(const MeshTables &m, const MaterialTables &mt, int precision);

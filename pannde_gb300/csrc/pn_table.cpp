@@ -35,6 +35,7 @@ void table_create(pn_solver *s) {
   s->upload_raw(s->d_ncc, s->mesh.ncc.data(), (size_t)nn * 32);
   s->upload_real(s->d_coef, s->mat.coef.data(), nn);
   s->upload_raw(s->d_mat, s->mat.cell_mat.data(), (size_t)nc * 4);
+  s->sym = symmetry_class(s->mat);
   std::vector<double> ct(s->mat.c36);
   if (!exact)
     for (double &v : ct) v *= s->dt;  // fast forms fold dt into C
@@ -179,6 +180,7 @@ void table_args(pn_solver *s, VelArgs<T> &va, StressArgs<T> &sa) {
   sa.sig_stride = 0;
   sa.sig_rows = 1;
   sa.has_moments = s->has_moments ? 1 : 0;
+  sa.sym = s->sym;
 }
 template void table_args<double>(pn_solver *, VelArgs<double> &, StressArgs<double> &);
 template void table_args<float>(pn_solver *, VelArgs<float> &, StressArgs<float> &);

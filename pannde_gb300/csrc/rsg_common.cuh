@@ -86,6 +86,8 @@ struct StressArgs {
   int32_t sig_stride;
   int32_t sig_rows;
   int32_t has_moments;
+  int32_t sym;  // symmetry class of the whole stiffness table (symmetry_class): 0 general, 1 monoclinic
+                // about z, 2 orthotropic
 };
 
 #ifdef __CUDACC__

@@ -13,10 +13,20 @@
 //   S_k += dt*(C_k0 exx + C_k1 eyy + C_k2 ezz + C_k3 gyz + C_k4 gxz + C_k5 gxy [+ moment_k])
 // with the 3x3 velocity gradient from the 8 corners (RightHex.hpp:100-141).
 //
-// Both differences use one butterfly over the 8 values (corner / slot order
-// 0=(0,0,0) 1=(1,0,0) 2=(1,1,0) 3=(0,1,0) 4..7 the same at +z):
-//   a=f1-f0 b=f2-f3 c=f5-f4 d=f6-f7, p=f1+f0 q=f2+f3 r=f5+f4 s=f6+f7
-//   Dx=(a+b)+(c+d)  Dy=(q-p)+(s-r)  Dz=(r+s)-(p+q)
+// The differences over the 8 values (corner / slot order 0=(0,0,0) 1=(1,0,0)
+// 2=(1,1,0) 3=(0,1,0) 4..7 the same at +z) are formed with as few operations
+// as each field needs: FP64 and double-float are bound by them (GB300's FP64
+// pipe is 80-85% busy in both kernels).
+//   all three   the four space diagonals f6-f0, f7-f1, f2-f4, f3-f5, then
+//               Dx=(d06+d24)-(d17+d35) Dy=(d06+d24)+(d17+d35)
+//               Dz=(d06-d24)+(d17-d35)                       11 operations
+//   two axes    pair sums along the third axis leave a square whose two
+//               diagonals u, w give u+w and u-w                8 operations
+//   one axis    four differences and their sum                 7 operations
+// Measured on a graded aluminium plate of 131 x 97 x 21 cells, FP64 (with the
+// stiffness terms of the material's symmetry class, see c_used): 20 steps and
+// the state's read-back 2.21 -> 1.58 ms; FP32 on a graded plate of 200 x 200 x
+// 40 cells, 20 steps 1.76 -> 1.56 ms.
 // Constants are folded on the host: g = 0.25/h, coef = dt/rho_n, ctab = dt*C,
 // moment weights carry dt.  This changes rounding only.
 #include <type_traits>
@@ -60,13 +70,38 @@ template <> struct Num<df64> {
   static __device__ __forceinline__ double dbl(df64 v) { return (double)v.hi + (double)v.lo; }
 };
 
+// all three differences
 template <typename R>
 __device__ __forceinline__ void diff3(const R f[8], R &dx, R &dy, R &dz) {
-  const R a = f[1] - f[0], b = f[2] - f[3], c = f[5] - f[4], d = f[6] - f[7];
-  const R p = f[1] + f[0], q = f[2] + f[3], r = f[5] + f[4], s = f[6] + f[7];
-  dx = (a + b) + (c + d);
-  dy = (q - p) + (s - r);
-  dz = (r + s) - (p + q);
+  const R d06 = f[6] - f[0], d17 = f[7] - f[1], d24 = f[2] - f[4], d35 = f[3] - f[5];
+  const R a = d06 + d24, b = d17 + d35;
+  dx = a - b;
+  dy = a + b;
+  dz = (d06 - d24) + (d17 - d35);
+}
+template <typename R> __device__ __forceinline__ R diff_x(const R f[8]) {
+  return ((f[1] - f[0]) + (f[2] - f[3])) + ((f[5] - f[4]) + (f[6] - f[7]));
+}
+template <typename R> __device__ __forceinline__ R diff_y(const R f[8]) {
+  return ((f[3] - f[0]) + (f[2] - f[1])) + ((f[7] - f[4]) + (f[6] - f[5]));
+}
+template <typename R> __device__ __forceinline__ R diff_z(const R f[8]) {
+  return ((f[4] - f[0]) + (f[5] - f[1])) + ((f[6] - f[2]) + (f[7] - f[3]));
+}
+template <typename R> __device__ __forceinline__ void diff_xy(const R f[8], R &dx, R &dy) {
+  const R u = (f[2] + f[6]) - (f[0] + f[4]), w = (f[1] + f[5]) - (f[3] + f[7]);
+  dx = u + w;
+  dy = u - w;
+}
+template <typename R> __device__ __forceinline__ void diff_xz(const R f[8], R &dx, R &dz) {
+  const R u = (f[5] + f[6]) - (f[0] + f[3]), w = (f[1] + f[2]) - (f[4] + f[7]);
+  dx = u + w;
+  dz = u - w;
+}
+template <typename R> __device__ __forceinline__ void diff_yz(const R f[8], R &dy, R &dz) {
+  const R u = (f[6] + f[7]) - (f[0] + f[1]), w = (f[2] + f[3]) - (f[4] + f[5]);
+  dy = u + w;
+  dz = u - w;
 }
 
 template <typename R>
@@ -107,44 +142,44 @@ __device__ __forceinline__ void velocity_node(const VelArgs<typename Num<R>::S> 
       R h[8];
       gather_slots<R>(a.S0, s, f);
       gather_slots<R>(a.S5, s, h);
-      diff3(f, dx, dy, dz);
-      ax = gx * dx;
-      diff3(h, dx, dy, dz);
-      ax = ax + gy * dy;
+      ax = gx * diff_x(f);
+      diff_xy(h, dx, dy);
+      ax = madd(gy, dy, ax);
       ay = gx * dx;
       gather_slots<R>(a.S4, s, f);
       gather_slots<R>(a.S1, s, h);
-      diff3(f, dx, dy, dz);
-      ax = ax + gz * dz;
+      diff_xz(f, dx, dz);
+      ax = madd(gz, dz, ax);
       az = gx * dx;
-      diff3(h, dx, dy, dz);
-      ay = ay + gy * dy;
+      ay = madd(gy, diff_y(h), ay);
       gather_slots<R>(a.S3, s, f);
       gather_slots<R>(a.S2, s, h);
-      diff3(f, dx, dy, dz);
-      ay = ay + gz * dz;
-      az = az + gy * dy;
-      diff3(h, dx, dy, dz);
-      az = az + gz * dz;
+      diff_yz(f, dy, dz);
+      ay = madd(gz, dz, ay);
+      az = madd(gy, dy, az);
+      az = madd(gz, diff_z(h), az);
     } else {
       // one field's 8 gathers at a time: grouping three fields' gathers raised
       // the registers (FP32 32 -> 40, double-float 48 -> 78) and the kernel ran
       // 8-10% slower at the lower occupancy
-      gather_slots<R>(a.S0, s, f); diff3(f, dx, dy, dz);
-      ax = gx * dx;
-      gather_slots<R>(a.S5, s, f); diff3(f, dx, dy, dz);
-      ax = ax + gy * dy;
+      gather_slots<R>(a.S0, s, f);
+      ax = gx * diff_x(f);
+      gather_slots<R>(a.S5, s, f);
+      diff_xy(f, dx, dy);
+      ax = madd(gy, dy, ax);
       ay = gx * dx;
-      gather_slots<R>(a.S4, s, f); diff3(f, dx, dy, dz);
-      ax = ax + gz * dz;
+      gather_slots<R>(a.S4, s, f);
+      diff_xz(f, dx, dz);
+      ax = madd(gz, dz, ax);
       az = gx * dx;
-      gather_slots<R>(a.S1, s, f); diff3(f, dx, dy, dz);
-      ay = ay + gy * dy;
-      gather_slots<R>(a.S3, s, f); diff3(f, dx, dy, dz);
-      ay = ay + gz * dz;
-      az = az + gy * dy;
-      gather_slots<R>(a.S2, s, f); diff3(f, dx, dy, dz);
-      az = az + gz * dz;
+      gather_slots<R>(a.S1, s, f);
+      ay = madd(gy, diff_y(f), ay);
+      gather_slots<R>(a.S3, s, f);
+      diff_yz(f, dy, dz);
+      ay = madd(gz, dz, ay);
+      az = madd(gy, dy, az);
+      gather_slots<R>(a.S2, s, f);
+      az = madd(gz, diff_z(f), az);
     }
     if (a.tile_src) {
       const int2 r = a.tile_src[tile];
@@ -159,9 +194,9 @@ __device__ __forceinline__ void velocity_node(const VelArgs<typename Num<R>::S> 
         else az = az + v;
       }
     }
-    v0 = v0 + cf * ax;
-    v1 = v1 + cf * ay;
-    v2 = v2 + cf * az;
+    v0 = madd(cf, ax, v0);
+    v1 = madd(cf, ay, v1);
+    v2 = madd(cf, az, v2);
     N::put(a.V0, n, v0);
     N::put(a.V1, n, v1);
     N::put(a.V2, n, v2);
@@ -181,8 +216,18 @@ __device__ __forceinline__ void velocity_node(const VelArgs<typename Num<R>::S> 
   }
 }
 
+// entries of the stiffness product by the material table's symmetry class (0
+// general, 1 monoclinic about z, 2 orthotropic in the axes): the others are
+// zero, 36 / 20 / 12 terms
+__host__ __device__ constexpr bool c_used(int sym, int k, int j) {
+  return sym == 0 ? true
+       : sym == 2 ? ((k < 3 && j < 3) || k == j)
+                  : ((k < 3 && j < 3) || k == j || (k == 5 && j < 3) || (j == 5 && k < 3) ||
+                     (k == 3 && j == 4) || (k == 4 && j == 3));
+}
+
 // stress update of cell c
-template <typename R, bool UNIFORM>
+template <typename R, bool UNIFORM, int SYM>
 __device__ __forceinline__ void stress_cell(const StressArgs<typename Num<R>::S> &a, int c, int tile,
                                             int step) {
   using N = Num<R>;
@@ -208,14 +253,15 @@ __device__ __forceinline__ void stress_cell(const StressArgs<typename Num<R>::S>
   e[0] = gx * d00;
   e[1] = gy * d11;
   e[2] = gz * d22;
-  e[3] = gy * d12 + gz * d21;
-  e[4] = gx * d02 + gz * d20;
-  e[5] = gx * d01 + gy * d10;
+  e[3] = madd(gz, d21, gy * d12);
+  e[4] = madd(gz, d20, gx * d02);
+  e[5] = madd(gy, d10, gx * d01);
 
   const typename N::S *C = a.ctab + 36 * a.mat[c];
-  R m[6];
+  typename N::S *S[6] = {a.S0, a.S1, a.S2, a.S3, a.S4, a.S5};
+  R acc[6];
 #pragma unroll
-  for (int q = 0; q < 6; q++) m[q] = R();
+  for (int k = 0; k < 6; k++) acc[k] = N::get(S[k], c);
   if (a.tile_src) {
     const int2 r = a.tile_src[tile];
     const typename N::S *sig = signal_row(a.sigval, step, a.sig_stride, a.sig_rows);
@@ -226,16 +272,15 @@ __device__ __forceinline__ void stress_cell(const StressArgs<typename Num<R>::S>
       const int k = code & 7;
 #pragma unroll
       for (int q = 0; q < 6; q++)
-        if (q == k) m[q] = m[q] + v;
+        if (q == k) acc[q] = acc[q] + v;
     }
   }
-  typename N::S *S[6] = {a.S0, a.S1, a.S2, a.S3, a.S4, a.S5};
 #pragma unroll
   for (int k = 0; k < 6; k++) {
-    R acc = N::get(S[k], c) + m[k];
 #pragma unroll
-    for (int j = 0; j < 6; j++) acc = acc + N::ld(C, 6 * k + j) * e[j];
-    N::put(S[k], c, acc);
+    for (int j = 0; j < 6; j++)
+      if (c_used(SYM, k, j)) acc[k] = madd(N::ld(C, 6 * k + j), e[j], acc[k]);
+    N::put(S[k], c, acc[k]);
   }
 }
 
@@ -245,10 +290,10 @@ __global__ void __launch_bounds__(kTile) k_velocity(const VelArgs<typename Num<R
   if (n < a.n_nodes) velocity_node<R, UNIFORM>(a, n, blockIdx.x, step);
 }
 
-template <typename R, bool UNIFORM>
+template <typename R, bool UNIFORM, int SYM>
 __global__ void __launch_bounds__(kTile) k_stress(const StressArgs<typename Num<R>::S> a, int step) {
   const int c = blockIdx.x * kTile + threadIdx.x;
-  if (c < a.n_cells) stress_cell<R, UNIFORM>(a, c, blockIdx.x, step);
+  if (c < a.n_cells) stress_cell<R, UNIFORM, SYM>(a, c, blockIdx.x, step);
 }
 
 // member owning work tile t: tile_start is the members' prefix of tile counts
@@ -327,8 +372,14 @@ __global__ void __launch_bounds__(kTile) k_stress_batch(const StressArgs<typenam
     const int tl = t - m_begin;
     const int c = tl * kTile + threadIdx.x;
     if (c >= a.n_cells) continue;
-    if (a.gcell) stress_cell<R, false>(a, c, tl, step);
-    else stress_cell<R, true>(a, c, tl, step);
+    // (the class of each member's own table; monoclinic ones take the general product)
+    if (a.sym == 2) {
+      if (a.gcell) stress_cell<R, false, 2>(a, c, tl, step);
+      else stress_cell<R, true, 2>(a, c, tl, step);
+    } else {
+      if (a.gcell) stress_cell<R, false, 0>(a, c, tl, step);
+      else stress_cell<R, true, 0>(a, c, tl, step);
+    }
   }
 }
 
@@ -341,13 +392,20 @@ cudaError_t launch_vel(const VelArgs<typename Num<R>::S> &a, int step, bool unif
   return cudaGetLastError();
 }
 
+template <typename R, int SYM>
+cudaError_t launch_str_sym(const StressArgs<typename Num<R>::S> &a, int step, bool uniform, cudaStream_t st) {
+  const unsigned grid = (unsigned)((a.n_cells + kTile - 1) / kTile);
+  if (uniform) k_stress<R, true, SYM><<<grid, kTile, 0, st>>>(a, step);
+  else k_stress<R, false, SYM><<<grid, kTile, 0, st>>>(a, step);
+  return cudaGetLastError();
+}
+
 template <typename R>
 cudaError_t launch_str(const StressArgs<typename Num<R>::S> &a, int step, bool uniform, cudaStream_t st) {
   if (a.n_cells <= 0) return cudaSuccess;
-  const unsigned grid = (unsigned)((a.n_cells + kTile - 1) / kTile);
-  if (uniform) k_stress<R, true><<<grid, kTile, 0, st>>>(a, step);
-  else k_stress<R, false><<<grid, kTile, 0, st>>>(a, step);
-  return cudaGetLastError();
+  if (a.sym == 2) return launch_str_sym<R, 2>(a, step, uniform, st);
+  if (a.sym == 1) return launch_str_sym<R, 1>(a, step, uniform, st);
+  return launch_str_sym<R, 0>(a, step, uniform, st);
 }
 
 // blocks of the batch kernels that are resident at once on the current
