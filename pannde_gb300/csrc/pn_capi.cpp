@@ -150,7 +150,7 @@ int create_common(const pn_mesh *mesh, double dt, int32_t mode, pn_solver **out,
     s->form = choose_form(s->mesh, s->mat, precision, form, s->grid);
     // size everything first so that a budget failure allocates nothing
     const int64_t need = s->form == PN_FORM_GRID ? pn::grid_footprint(s->grid, s->mat, precision)
-                                                 : pn::table_footprint(s->mesh, s->mat, precision);
+                                                 : pn::table_footprint(s->mesh, s->mat, precision, false);
     const int64_t budget = pn::hbm_budget();
     if (budget >= 0 && need > budget)
       return set_err(PN_ERR_ALLOC, "solver needs " + std::to_string(need) +

@@ -78,6 +78,7 @@ struct pn_solver {
   // table form
   int4 *d_hex = nullptr, *d_ncc = nullptr;
   void *d_gnode = nullptr, *d_gcell = nullptr;
+  void *d_rnode = nullptr, *d_rcell = nullptr;  // exact form: reciprocals of the spacings, or null
   int32_t *d_mat = nullptr;
 
   // grid form
@@ -307,7 +308,9 @@ int64_t sig_row(const pn_solver *s, int64_t step_in_call);  // row of this step
 int symmetry_class(const MaterialTables &mt);
 
 // table form (pn_table.cpp)
-int64_t table_footprint(const MeshTables &m, const MaterialTables &mt, int precision);
+// (reciprocals: with the exact form's reciprocal spacings, which it can do without)
+int64_t table_footprint(const MeshTables &m, const MaterialTables &mt, int precision, bool reciprocals = true);
+double exact_reciprocal(double d);  // of a spacing, as the exact form's kernels take it
 void table_create(pn_solver *s);
 void table_sources(pn_solver *s);
 void table_sensors(pn_solver *s, const std::vector<std::pair<int32_t, int32_t>> &sorted);

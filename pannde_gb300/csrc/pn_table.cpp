@@ -1,5 +1,6 @@
 // pn_table.cpp -- table form of the solver: any hex mesh, connectivity tables
 // on the device, two kernels per step (velocity then stress).
+#include <cmath>
 #include <cstring>
 #include <type_traits>
 
@@ -7,14 +8,26 @@
 
 namespace pn {
 
-int64_t table_footprint(const MeshTables &m, const MaterialTables &mt, int precision) {
+int64_t table_footprint(const MeshTables &m, const MaterialTables &mt, int precision, bool reciprocals) {
   const int64_t nn = m.n_nodes, nc = m.n_cells;
   const int64_t e = precision == PN_PREC_F32 ? 4 : 8;
   const bool per_elem = precision == PN_PREC_F64_EXACT || !m.uniform;
   int64_t need = nn * 3 * e + nc * 6 * e + nc * 32 + nn * 32 + nn * e + nc * 4 +
                  (int64_t)mt.n_mat * 36 * e;
   if (per_elem) need += nn * 3 * e + nc * 3 * e;
+  if (precision == PN_PREC_F64_EXACT && reciprocals) need += nn * 3 * e + nc * 3 * e;
   return need;
+}
+
+// The exact form's reciprocal of a spacing d: r = RN(1 / (4 d)), negated when
+// the short quotient of rsg_exact.cu does not hold for it (2^53 |4 d r - 1| >
+// 1/2; the remainder 1 - 4 d r is exact in one FMA), 0 when 4 d is outside
+// [2^-100, 2^100].
+double exact_reciprocal(double d) {
+  const double c = 4. * d;
+  if (!(c >= 0x1p-100 && c <= 0x1p100)) return 0.;
+  const double r = 1. / c;
+  return std::fabs(std::fma(-c, r, 1.)) <= 0x1p-54 ? r : -r;
 }
 
 void table_create(pn_solver *s) {
@@ -54,6 +67,26 @@ void table_create(pn_solver *s) {
     s->d_gcell = s->alloc<void>(h.size() * e);
     s->upload_real(s->d_gnode, g.data(), g.size());
     s->upload_real(s->d_gcell, h.data(), h.size());
+    if (exact) {
+      ck(cudaStreamSynchronize(s->stream), "create sync");  // the arrays are reused
+      const int64_t ng = (int64_t)g.size(), nh = (int64_t)h.size();
+#pragma omp parallel for schedule(static)
+      for (int64_t q = 0; q < ng; q++) g[q] = exact_reciprocal(g[q]);
+#pragma omp parallel for schedule(static)
+      for (int64_t q = 0; q < nh; q++) h[q] = exact_reciprocal(h[q]);
+      try {
+        s->d_rnode = s->alloc<void>(g.size() * e);
+        s->d_rcell = s->alloc<void>(h.size() * e);
+      } catch (const SetupError &) {  // no room: the kernels form the reciprocals themselves
+        s->release(s->d_rnode);
+        s->release(s->d_rcell);
+      }
+      if (s->d_rcell) {
+        s->upload_real(s->d_rnode, g.data(), g.size());
+        s->upload_real(s->d_rcell, h.data(), h.size());
+      }
+      ck(cudaStreamSynchronize(s->stream), "create sync");  // before the arrays go
+    }
   }
   ck(cudaStreamSynchronize(s->stream), "create sync");
 }
@@ -152,6 +185,7 @@ void table_args(pn_solver *s, VelArgs<T> &va, StressArgs<T> &sa) {
   va.gy = to_store<T>(0.25 / s->mesh.hy);
   va.gz = to_store<T>(0.25 / s->mesh.hz);
   va.gnode = (const T *)s->d_gnode;
+  va.rnode = (const T *)s->d_rnode;
   if (s->n_force > 0) {
     va.tile_src = s->d_ftile; va.src_elem = s->d_felem; va.src_code = s->d_fcode;
     va.src_w = (const T *)s->d_fw;
@@ -171,6 +205,7 @@ void table_args(pn_solver *s, VelArgs<T> &va, StressArgs<T> &sa) {
   sa.ctab = (const T *)s->d_ctab;
   sa.gx = va.gx; sa.gy = va.gy; sa.gz = va.gz;
   sa.gcell = (const T *)s->d_gcell;
+  sa.rcell = (const T *)s->d_rcell;
   sa.dt = to_store<T>(s->dt);
   if (s->n_moment > 0) {
     sa.tile_src = s->d_mtile; sa.src_elem = s->d_melem; sa.src_code = s->d_mcode;

@@ -39,6 +39,7 @@ struct VelArgs {
   // (fast forms: 0.25/d; exact form: d)
   T gx, gy, gz;
   const T *__restrict__ gnode;
+  const T *__restrict__ rnode;  // exact form only: reciprocal spacings [3][n_nodes] (exact_reciprocal)
   // force sources
   const int2 *__restrict__ tile_src;  // [n_tiles] or null
   const int32_t *__restrict__ src_elem;
@@ -75,6 +76,7 @@ struct StressArgs {
   const T *__restrict__ ctab;
   T gx, gy, gz;
   const T *__restrict__ gcell;  // per cell [3][n_cells] or null
+  const T *__restrict__ rcell;  // exact form only: reciprocal spacings [3][n_cells]
   T dt;                          // exact form only (fast forms fold dt into ctab)
   // moment sources
   const int2 *__restrict__ tile_src;
