@@ -99,8 +99,9 @@ struct Keyed {
 };
 
 // entries sorted by (slot, local index), stably: a thread finds its own
-// entries of a slot by a binary search (first_local), and one node's entries
-// keep their order (the order their terms are added in)
+// entries of a slot by its place in it (SlotIndex) or a binary search
+// (first_local, the classic kernel), and one node's entries keep their order
+// (the order their terms are added in)
 void ranges_of(std::vector<Keyed> &L, int64_t n_slots, std::vector<int32_t> &rng) {
   std::stable_sort(L.begin(), L.end(), [](const Keyed &a, const Keyed &b) {
     return a.slot != b.slot ? a.slot < b.slot : (a.key & 0xffff) < (b.key & 0xffff);
@@ -113,6 +114,47 @@ void ranges_of(std::vector<Keyed> &L, int64_t n_slots, std::vector<int32_t> &rng
     rng[(size_t)sl * 2 + 1] = (int32_t)e;
   }
 }
+
+// the slots' index (SlotIndex, rsg_grid.cuh) over sorted entries and their
+// ranges, on the device; empty lists have none
+void upload_index(pn_solver *s, const std::vector<Keyed> &L, const std::vector<int32_t> &rng, int tile_rows,
+                  pn_solver::SlotTables &out) {
+  const size_t n_slots = rng.size() / 2;
+  std::vector<int32_t> id(n_slots, -1), node;
+  std::vector<uint32_t> rows;
+  int32_t slots = 0;
+  for (size_t sl = 0; sl < n_slots; sl++) {
+    const int32_t e0 = rng[2 * sl], e1 = rng[2 * sl + 1];
+    if (e0 == e1) continue;
+    id[sl] = slots++;
+    bool several = false;  // entries at one node of the slot
+    for (int32_t e = e0 + 1; e < e1; e++) several = several || (L[e].key & 0xffff) == (L[e - 1].key & 0xffff);
+    const size_t at = rows.size();
+    rows.resize(at + 2 * (size_t)tile_rows, 0);
+    std::vector<bool> begun((size_t)tile_rows, false);
+    for (int32_t e = e0; e < e1; e++) {
+      if (e > e0 && (L[e].key & 0xffff) == (L[e - 1].key & 0xffff)) continue;
+      const int t = L[e].key & 0xffff, ty = t / kGridTileX, tx = t % kGridTileX;
+      uint32_t *r = &rows[at + 2 * (size_t)ty];
+      if (!begun[(size_t)ty]) {
+        begun[(size_t)ty] = true;
+        r[1] = several ? (uint32_t)node.size() | 0x80000000u : (uint32_t)e;
+      }
+      r[0] |= 1u << tx;
+      if (several) node.push_back(e);
+    }
+    if (several) node.push_back(e1);
+  }
+  out.id = s->alloc<int32_t>(id.size() * 4);
+  out.rows = s->alloc<uint2>(rows.size() * 4);
+  out.node = s->alloc<int32_t>(node.size() * 4);
+  s->upload_raw(out.id, id.data(), id.size() * 4);
+  s->upload_raw(out.rows, rows.data(), rows.size() * 4);
+  s->upload_raw(out.node, node.data(), node.size() * 4);
+  ck(cudaStreamSynchronize(s->stream), "slot index upload");  // before the host lists go
+}
+
+SlotIndex index_of(const pn_solver::SlotTables &t) { return SlotIndex{t.id, t.rows, t.node}; }
 
 }  // namespace
 
@@ -277,6 +319,7 @@ bool grid_set_tile_rows(pn_solver *s, int rows) {
   if (!s->src.empty() && !s->src_dirty) grid_sources(s);
   if (s->n_sens > 0) {
     s->release(s->d_srng); s->release(s->d_skey); s->release(s->d_sidx);
+    s->release(s->s_slots);
     grid_sensors(s, s->sensor_pairs);
   }
   ck(cudaStreamSynchronize(s->stream), "retile upload");
@@ -565,16 +608,19 @@ void grid_sources(pn_solver *s) {
   ck(cudaStreamSynchronize(s->stream), "sources sync");
   s->release(s->d_frng); s->release(s->d_fkey); s->release(s->d_fsig); s->release(s->d_fw);
   s->release(s->d_mrng); s->release(s->d_mkey); s->release(s->d_msig); s->release(s->d_mw);
+  s->release(s->f_slots);
+  s->release(s->m_slots);
   const GridMap &g = s->grid;
   const Tiles T = tiles_of(g, s->tile_rows);
   s->n_force = (int32_t)fe.size();
   s->n_moment = (int32_t)me.size();
   s->n_src_nodes = s->n_src_cells = 0;
   auto upload = [&](std::vector<Keyed> &L, int64_t layers, int2 *&rng, int32_t *&key, int32_t *&sig,
-                    void *&w) {
+                    void *&w, pn_solver::SlotTables &index) {
     if (L.empty()) return;
     std::vector<int32_t> r;
     ranges_of(L, T.blocks() * layers, r);
+    if (s->d_tmaps) upload_index(s, L, r, s->tile_rows, index);
     std::vector<int32_t> k(L.size()), sg(L.size());
     std::vector<double> wt(L.size());
     for (size_t q = 0; q < L.size(); q++) {
@@ -620,8 +666,8 @@ void grid_sources(pn_solver *s) {
     const int32_t fx = g.fix_of_cell.empty() ? -1 : g.fix_of_cell[(size_t)me[q].elem];
     if (fx >= 0) s->fix_moments.push_back({fx, me[q].comp, me[q].sig, s->dt * me[q].w});
   }
-  upload(F, g.nz + 1, s->d_frng, s->d_fkey, s->d_fsig, s->d_fw);
-  upload(M, g.nz, s->d_mrng, s->d_mkey, s->d_msig, s->d_mw);
+  upload(F, g.nz + 1, s->d_frng, s->d_fkey, s->d_fsig, s->d_fw, s->f_slots);
+  upload(M, g.nz, s->d_mrng, s->d_mkey, s->d_msig, s->d_mw, s->m_slots);
   if (s->d_rflags) {  // the stresses' double-float range also covers the source weights
     double cmin = s->r_cmin_s, cmax = s->r_cmax_s;
     for (const std::vector<Keyed> *L : {&F, &M})
@@ -660,6 +706,7 @@ void grid_sensors(pn_solver *s, const std::vector<std::pair<int32_t, int32_t>> &
   }
   std::vector<int32_t> r;
   ranges_of(L, T.blocks() * (g.nz + 1), r);
+  if (s->d_tmaps) upload_index(s, L, r, s->tile_rows, s->s_slots);
   std::vector<int32_t> key(L.size()), idx(L.size());
   for (size_t q = 0; q < L.size(); q++) {
     key[q] = L[q].key;
@@ -692,14 +739,17 @@ void grid_args(pn_solver *s, GridArgs<T> &a) {
   a.g[2] = to_store<T>(folded ? 1.0 : 0.25 / s->mesh.hz);
   if (s->n_force > 0) {
     a.f_rng = s->d_frng; a.f_key = s->d_fkey; a.f_sig = s->d_fsig; a.f_w = (const T *)s->d_fw;
+    a.f_ix = index_of(s->f_slots);
   }
   if (s->n_moment > 0) {
     a.m_rng = s->d_mrng; a.m_key = s->d_mkey; a.m_sig = s->d_msig; a.m_w = (const T *)s->d_mw;
+    a.m_ix = index_of(s->m_slots);
   }
   a.n_sens = s->n_sens;
   a.traces = s->d_traces;
   a.rec_cap = s->rec_cap;
   a.s_rng = s->n_sens > 0 ? s->d_srng : nullptr;
+  if (s->n_sens > 0) a.s_ix = index_of(s->s_slots);
   a.s_key = s->d_skey;
   a.s_idx = s->d_sidx;
   a.sig_stride = 0;

@@ -151,6 +151,13 @@ struct pn_solver {
   int2 *d_frng = nullptr, *d_mrng = nullptr;
   int32_t *d_fkey = nullptr, *d_fsig = nullptr, *d_mkey = nullptr, *d_msig = nullptr;
   void *d_fw = nullptr, *d_mw = nullptr;
+  // ... and how a thread finds its own entries of a slot (SlotIndex)
+  struct SlotTables {
+    int32_t *id = nullptr;
+    uint2 *rows = nullptr;
+    int32_t *node = nullptr;
+  };
+  SlotTables f_slots, m_slots, s_slots;
   // signal table: rows [sig_step0, sig_step0 + sig_rows) of [n_sig] values;
   // sig_hold: the last row holds for every later step
   void *d_sig = nullptr;
@@ -198,6 +205,12 @@ struct pn_solver {
     if (it != allocs.end()) allocs.erase(it);
     cudaFree((void *)p);
     p = nullptr;
+  }
+
+  void release(SlotTables &t) {
+    release(t.id);
+    release(t.rows);
+    release(t.node);
   }
 
   // upload a double host array in the storage type (double, float, or the

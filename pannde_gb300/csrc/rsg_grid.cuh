@@ -29,6 +29,21 @@ struct FixCell {
   int32_t m0, m1;     // its moment entries [m0, m1)
 };
 
+// A thread's own entries of its (block, layer) slot without a search
+// (tensor-copy kernel): id gives a non-empty slot its number (-1: empty); rows
+// holds per slot and tile row one bit per lane with entries and where the
+// row's first entry lies, so a lane's own is found by counting bits.  With
+// more than one entry at some node of the slot (bit 31 of the second word)
+// that place counts the slot's nodes instead, and node[] holds where each
+// one's entries begin (and the slot's end).  Every lane reading through a
+// slot of a few hundred entries, or searching it, was the longest serial
+// chain of a small lattice's step: a dependent load per probe.
+struct SlotIndex {
+  const int32_t *id;    // [blocks][layers]
+  const uint2 *rows;    // [slots][tile rows]
+  const int32_t *node;
+};
+
 template <typename T>
 struct GridArgs {
   int32_t nx, ny, nz;  // cells per axis
@@ -47,11 +62,13 @@ struct GridArgs {
   const int32_t *f_key;  // local node | direction << 16
   const int32_t *f_sig;
   const T *f_w;
+  SlotIndex f_ix;
   // moment sources, ranges per (block, cell layer): [blocks][nz]
   const int2 *m_rng;
   const int32_t *m_key;  // local cell | Voigt component << 16
   const int32_t *m_sig;
   const T *m_w;          // weights carry dt
+  SlotIndex m_ix;
   const T *sigval;       // signal rows: row min(step, sig_rows-1) at stride sig_stride
   int32_t sig_stride;    // 0 when sigval already points at the step's row
   int32_t sig_rows;
@@ -59,6 +76,7 @@ struct GridArgs {
   const int2 *s_rng;
   const int32_t *s_key;  // local node
   const int32_t *s_idx;  // sensor number
+  SlotIndex s_ix;
   double *traces;        // [records][n_sens][3]
   int32_t n_sens;
   int64_t rec;           // record written by step 0 of the launch (rec + step later)
@@ -100,7 +118,7 @@ struct GridArgs {
   int32_t tail_from, tail_chunk;
 };
 
-// where a thread's scan of its (block, layer) slot starts: the entries are
+// where a thread's scan of its (block, layer) slot starts (classic kernel): the entries are
 // sorted by local index (key & 0xffff), so in a long slot (a transducer patch
 // puts a few hundred entries in one) a binary search finds the first entry of
 // local index t, or the first past them, in log2(hi - lo) loads; a short slot
@@ -115,6 +133,17 @@ __device__ __forceinline__ int first_local(const int32_t *__restrict__ key, int 
     else hi = mid;
   }
   return lo;
+}
+
+// entries [x, y) of lane tx of tile row ty (TY rows) in slot `id`
+template <int TY>
+__device__ __forceinline__ int2 slot_entries(const SlotIndex &ix, int id, int tx, int ty) {
+  if (id < 0) return make_int2(0, 0);
+  const uint2 r = __ldg(ix.rows + (int64_t)id * TY + ty);
+  if (!((r.x >> tx) & 1u)) return make_int2(0, 0);
+  const int n = (int)(r.y & 0x7fffffffu) + __popc(r.x & ((1u << tx) - 1u));
+  if (r.y >> 31) return make_int2(__ldg(ix.node + n), __ldg(ix.node + n + 1));
+  return make_int2(n, n + 1);
 }
 #endif
 

@@ -30,7 +30,7 @@
 // when whole columns leave a last partial wave of resident blocks, a 1D grid
 // whose last wave's columns are cut into shorter chunks (block_coords).  The
 // sparse sources and sensors of a (tile, layer) slot are sorted by node: a
-// thread finds its own by a binary search in a long slot.
+// thread finds its own through a bit per lane and row (slot_entries).
 //
 // Every wait is bounded (about one second of %globaltimer); a wait that gives
 // up records an error word for the host, the block drains its own copies in
@@ -75,7 +75,7 @@ struct GridMaps {
 #define PN_GRID_F32_OWN_STRESS 1  // FP32: old stress from the tile (four stress slots)
 #endif
 #ifndef PN_GRID_F32_MIN_BLOCKS
-#define PN_GRID_F32_MIN_BLOCKS 0  // FP32: resident blocks per SM the kernel is compiled for
+#define PN_GRID_F32_MIN_BLOCKS 4  // FP32: resident blocks per SM the kernel is compiled for
 #endif
 template <int ESZ, int TY>
 struct Geo {
@@ -101,8 +101,8 @@ struct Geo {
   static constexpr int OFF_M = OFF_V + NV * VSLOT;             // material ring [NM]
   static constexpr int OFF_VT = OFF_M + NM * MBOX;             // computed velocity [2][3][NT]
   static constexpr int OFF_C = OFF_VT + 2 * 3 * NT * ESZ;      // dt*C rows [ROWS_MAX][36]
-  static constexpr int OFF_R = OFF_C + ROWS_MAX * 36 * ESZ;    // ranges f, s [KC_MAX+2], m [KC_MAX]
-  static constexpr int OFF_B = OFF_R + (3 * KC_MAX + 4) * 8;   // mbarriers [NS]
+  static constexpr int OFF_R = OFF_C + ROWS_MAX * 36 * ESZ;    // slot numbers f, s [KC_MAX+2], m [KC_MAX]
+  static constexpr int OFF_B = OFF_R + (3 * KC_MAX + 4) * 4;   // mbarriers [NS]
   static constexpr int BYTES = OFF_B + NS * 8;
   static constexpr size_t SMEM = BYTES + 128;                  // + base alignment
   static_assert(SLOT % 128 == 0 && VBOX % 128 == 0 && OFF_V % 128 == 0 && OFF_M % 128 == 0 && OFF_B % 8 == 0,
@@ -272,12 +272,115 @@ __device__ __forceinline__ int floor_to(int v, int m) {  // largest multiple of 
 // error word codes
 constexpr int32_t kErrWait = 1;
 
+// Programmatic dependent launch: a step's kernel may start while the one
+// before it drains (the launches carry the stream-serialization attribute); it
+// loads the tables no step writes, then waits here for the previous kernel's
+// end and its memory before it touches states, path flags or traces.  A block
+// lets the next kernel start when it reaches its last node layer: let at its
+// start, the next kernel's waiting blocks slowed the ones still marching
+// (laminate 400 x 400 x 40, FP32: 103.3 us per step without the overlap, 106.7
+// let at the start, 100.1 here; aluminium plate 64 x 64 x 8, FP32, one layer
+// per chunk: 8.2 / 5.6 / 5.2).
+__device__ __forceinline__ void wait_previous_step() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_step_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// The block's tile copies: ring slots, barriers and the issue of one layer's
+// copies (layers [k0 - 1, k1] of tile (bx, by)).
+template <typename St, int TY, bool BATCH>
+struct Copies {
+  using G = Geo<(int)sizeof(St), TY>;
+  const GridMaps *M;
+  unsigned char *base;
+  uint32_t bars;
+  int xs_c, xs_n, xs_m, j0, k0, k1, skip;
+  // the copies are issued (and, on failure, drained) by the first thread of
+  // the last warp: its row is the tile's apron, which has no stress half
+  static constexpr int ISSUER = (TY - 1) * TX;
+  __device__ __forceinline__ Copies(const GridArgs<St> &a, unsigned char *smem, int bx, int by, int k0_, int k1_)
+      : M(reinterpret_cast<const GridMaps *>(a.tmaps)), k0(k0_), k1(k1_), skip(a.test_skip_layer) {
+    // 128-byte aligned base.  A single launch derives it from the shared array
+    // by an offset, so that every tile pointer stays in the shared state space (shared
+    // loads and stores, 32-bit addressing: FP32 45.4 -> 47.8, double-float 18.0
+    // -> 19.3 Gcell-steps/s on the laminate).  The batch kernel, which reads its
+    // arguments through global memory, spilled with that and ran slower; it keeps
+    // the generic pointer.
+    base = BATCH ? (unsigned char *)(((uintptr_t)smem + 127) & ~(uintptr_t)127)
+                 : smem + ((128u - (smem_u32(smem) & 127u)) & 127u);
+    bars = smem_u32(base + G::OFF_B);
+    // tile origins of the copies (x on the 16-byte boundary)
+    const int i0 = bx * (TX - 1);
+    j0 = by * (TY - 1);
+    xs_c = floor_to(i0 - 1, G::A);
+    xs_n = floor_to(i0, G::A);
+    xs_m = floor_to(i0, 16);
+  }
+  // layer L is copy number u = L - k0 + 1 of the block: stress slot and
+  // mbarrier u % NS (phase (u / NS) & 1), velocity slot u % NV, material slot u % NM
+  __device__ __forceinline__ uint32_t ucount(int L) const { return (uint32_t)(L - k0 + 1); }
+  __device__ __forceinline__ unsigned char *sslot(int L) const { return base + (ucount(L) % G::NS) * G::SLOT; }
+  __device__ __forceinline__ unsigned char *vslot(int L) const {
+    return base + G::OFF_V + (ucount(L) % G::NV) * G::VSLOT;
+  }
+  __device__ __forceinline__ unsigned char *mslot(int L) const {
+    return base + G::OFF_M + (ucount(L) % G::NM) * G::MBOX;
+  }
+  __device__ __forceinline__ uint32_t bar_of(int L) const { return bars + 8u * (ucount(L) % G::NS); }
+  __device__ __forceinline__ uint32_t parity(int L) const { return (ucount(L) / G::NS) & 1u; }
+  // The chunk's first layer k0 - 1 gives only the partial sums of its cell
+  // layer (stress boxes); no node velocity or cell stress of it is computed
+  // here, so its velocity, dt/rho and material boxes are not copied.  The top
+  // layer k1 gives the velocity of node layer k1 but no cell stress: no
+  // material box.  (A chunk above the lattice's first layer re-reads two
+  // layers; these are the bytes of them it does not need.)
+  __device__ __forceinline__ void issue(int L) const {
+    if (L == skip) return;  // failure-path test: this layer's wait runs out
+    const uint32_t bar = bar_of(L);
+    unsigned char *sl = sslot(L), *vl = vslot(L);
+    const bool first = L == k0 - 1, top = L == k1;
+    mbar_expect_tx(bar, first ? 6u * G::SBOX_BYTES : top ? G::TX_BYTES - G::MBOX_BYTES : G::TX_BYTES);
+#pragma unroll
+    for (int f = 0; f < 6; f++) tma_load_3d(smem_u32(sl + f * G::SBOX), &M->S[f], xs_c, j0 - 1, L, bar);
+    if (first) return;
+#pragma unroll
+    for (int c = 0; c < 3; c++) tma_load_3d(smem_u32(vl + c * G::VBOX), &M->V[c], xs_n, j0, L, bar);
+    tma_load_3d(smem_u32(vl + 3 * G::VBOX), &M->coef, xs_n, j0, L, bar);
+    if (!top) tma_load_3d(smem_u32(mslot(L)), &M->mat, xs_m, j0, L, bar);
+  }
+  // the issuing thread alone: barriers, then the first layers' copies as soon
+  // as the previous step is done (they need nothing of the block's tables);
+  // the block's next barrier shows the mbarriers to the other threads
+  __device__ __forceinline__ void start() const {
+#pragma unroll
+    for (int f = 0; f < 6; f++) tma_prefetch_map(&M->S[f]);
+#pragma unroll
+    for (int c = 0; c < 3; c++) tma_prefetch_map(&M->V[c]);
+    tma_prefetch_map(&M->coef);
+    tma_prefetch_map(&M->mat);
+#pragma unroll
+    for (int s = 0; s < G::NS; s++) mbar_init(bars + 8u * s, 1);
+    mbar_init_fence();
+    proxy_fence_async_smem();
+    wait_previous_step();
+#pragma unroll
+    for (int d = 0; d <= G::PD; d++)
+      if (k0 - 1 + d <= k1) issue(k0 - 1 + d);
+  }
+};
+
+// the tile's columns (and their apron) hold no solid cell at or above its top:
+// the march ends there, and a chunk above it has nothing to do
+template <typename T>
+__device__ __forceinline__ int tile_top(const GridArgs<T> &a, int blk) {
+  return a.ktop ? min(a.nz, __ldg(a.ktop + blk)) : a.nz;
+}
+
 // RANGE (the FP64 form's kernel): every V and S value the block stores is
 // tested against the double-float range, and a block that stored one outside
 // it marks its tile for the FP64 path in the next step (range_flags_write).
 template <typename K, int SYM, int TY, bool BATCH = false, bool RANGE = false>
-__device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::S> &a, const GridMaps *M,
-                                               int bx, int by, int k0, int kc, int gxc, int step) {
+__device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::S> &a,
+                                               const Copies<typename GNum<K>::S, TY, BATCH> &cp, int bx, int by,
+                                               bool last_chunk, int gxc, int step) {
   using N = GNum<K>;
   using R = typename N::R;
   using St = typename N::S;
@@ -290,27 +393,19 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
   constexpr bool CUBIC = (SYM & 4) != 0;
   constexpr int SB = G::SBOX / (int)sizeof(St);  // field stride in a slot (elements)
   constexpr int VB = G::VBOX / (int)sizeof(St);
-  extern __shared__ unsigned char smem_raw[];
-  // 128-byte aligned base.  A single launch derives it from smem_raw by an
-  // offset, so that every tile pointer stays in the shared state space (shared
-  // loads and stores, 32-bit addressing: FP32 45.4 -> 47.8, double-float 18.0
-  // -> 19.3 Gcell-steps/s on the laminate).  The batch kernel, which reads its
-  // arguments through global memory, spilled with that and ran slower; it keeps
-  // the generic pointer.
-  unsigned char *base = BATCH ? (unsigned char *)(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127)
-                              : smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
+  unsigned char *base = cp.base;
   Sm *sVt = reinterpret_cast<Sm *>(base + G::OFF_VT);
   Sm *sC = reinterpret_cast<Sm *>(base + G::OFF_C);
-  int2 *sRf = reinterpret_cast<int2 *>(base + G::OFF_R);
-  int2 *sRs = sRf + (KC_MAX + 2);
-  int2 *sRm = sRs + (KC_MAX + 2);
-  const uint32_t bars = smem_u32(base + G::OFF_B);
+  int *sRf = reinterpret_cast<int *>(base + G::OFF_R);
+  int *sRs = sRf + (KC_MAX + 2);
+  int *sRm = sRs + (KC_MAX + 2);
 
   const int t = threadIdx.x;
   const int tx = t % TX, ty = t / TX;
   const int i0 = bx * (TX - 1), j0 = by * (TY - 1);
   const int blk = by * gxc + bx;
   const int nx = a.nx, ny = a.ny, nz = a.nz;
+  const int k0 = cp.k0, k1 = cp.k1;
   const int i = i0 + tx, j = j0 + ty;
   const bool node_own = (i <= nx) && (j <= ny) && tx < TX - 1 && ty < TY - 1;
   const bool cell_own = tx < TX - 1 && ty < TY - 1 && i < nx && j < ny;
@@ -320,77 +415,26 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
   const R gx = N::val(a.g[0]), gy = N::val(a.g[1]), gz = N::val(a.g[2]);
   const St *sigrow = a.sigval ? a.sigval + (int64_t)min(step, a.sig_rows - 1) * a.sig_stride : nullptr;
   const int64_t rec = a.rec + step;
-  // columns of the tile (and its apron) hold no solid cell at or above ktop:
-  // the march ends there, and a chunk above it has nothing to do
-  const int ktop = a.ktop ? min(nz, __ldg(a.ktop + blk)) : nz;
-  const int k1 = min(ktop, k0 + kc);
-  if (k0 >= ktop) return;
-  const bool last_chunk = k1 == ktop;
+  const int oc = i0 - 1 - cp.xs_c, on = i0 - cp.xs_n, om = i0 - cp.xs_m;  // offsets in the copies
+  constexpr int ISSUER = Copies<St, TY, BATCH>::ISSUER;
+  auto sslot = [&](int L) { return cp.sslot(L); };
+  auto vslot = [&](int L) { return cp.vslot(L); };
+  auto mslot = [&](int L) { return cp.mslot(L); };
+  auto bar_of = [&](int L) { return cp.bar_of(L); };
+  auto parity = [&](int L) { return cp.parity(L); };
 
-  // tile origins of the copies (x on the 16-byte boundary) and offsets in them
-  const int xs_c = floor_to(i0 - 1, G::A), oc = i0 - 1 - xs_c;
-  const int xs_n = floor_to(i0, G::A), on = i0 - xs_n;
-  const int xs_m = floor_to(i0, 16), om = i0 - xs_m;
-
-  // layer L is copy number u = L - k0 + 1 of the block: stress slot and
-  // mbarrier u % NS (phase (u / NS) & 1), velocity slot u % NV, material slot u % NM
-  auto ucount = [&](int L) { return (uint32_t)(L - k0 + 1); };
-  auto sslot = [&](int L) { return base + (ucount(L) % G::NS) * G::SLOT; };
-  auto vslot = [&](int L) { return base + G::OFF_V + (ucount(L) % G::NV) * G::VSLOT; };
-  auto mslot = [&](int L) { return base + G::OFF_M + (ucount(L) % G::NM) * G::MBOX; };
-  auto bar_of = [&](int L) { return bars + 8u * (ucount(L) % G::NS); };
-  auto parity = [&](int L) { return (ucount(L) / G::NS) & 1u; };
-  // The chunk's first layer k0 - 1 gives only the partial sums of its cell
-  // layer (stress boxes); no node velocity or cell stress of it is computed
-  // here, so its velocity, dt/rho and material boxes are not copied.  The top
-  // layer k1 gives the velocity of node layer k1 but no cell stress: no
-  // material box.  (A chunk above the lattice's first layer re-reads two
-  // layers; these are the bytes of them it does not need.)
-  auto issue = [&](int L) {  // the issuing thread: copies of layer L
-    if (L == a.test_skip_layer) return;  // failure-path test: this layer's wait runs out
-    const uint32_t bar = bar_of(L);
-    unsigned char *sl = sslot(L), *vl = vslot(L);
-    const bool first = L == k0 - 1, top = L == k1;
-    mbar_expect_tx(bar, first ? 6u * G::SBOX_BYTES : top ? G::TX_BYTES - G::MBOX_BYTES : G::TX_BYTES);
-#pragma unroll
-    for (int f = 0; f < 6; f++) tma_load_3d(smem_u32(sl + f * G::SBOX), &M->S[f], xs_c, j0 - 1, L, bar);
-    if (first) return;
-#pragma unroll
-    for (int c = 0; c < 3; c++) tma_load_3d(smem_u32(vl + c * G::VBOX), &M->V[c], xs_n, j0, L, bar);
-    tma_load_3d(smem_u32(vl + 3 * G::VBOX), &M->coef, xs_n, j0, L, bar);
-    if (!top) tma_load_3d(smem_u32(mslot(L)), &M->mat, xs_m, j0, L, bar);
-  };
-
-  if (t == 0) {
-#pragma unroll
-    for (int f = 0; f < 6; f++) tma_prefetch_map(&M->S[f]);
-#pragma unroll
-    for (int c = 0; c < 3; c++) tma_prefetch_map(&M->V[c]);
-    tma_prefetch_map(&M->coef);
-    tma_prefetch_map(&M->mat);
-#pragma unroll
-    for (int s = 0; s < G::NS; s++) mbar_init(bars + 8u * s, 1);
-    mbar_init_fence();
-  }
   // per-chunk tables: stiffness rows, source and sensor ranges
   for (int q = t; q < a.n_rows * 36; q += NT) sC[q] = N::tsto(N::val(a.ctab[q]));
   const int nL = k1 - k0 + 2;  // node layers k0-1 .. k1
   for (int q = t; q < nL; q += NT) {
     const int k = k0 - 1 + q;
     const bool ok = k >= 0 && k <= nz;
-    sRf[q] = (a.f_rng && ok) ? a.f_rng[(int64_t)blk * (nz + 1) + k] : make_int2(0, 0);
-    sRs[q] = (a.s_rng && ok) ? a.s_rng[(int64_t)blk * (nz + 1) + k] : make_int2(0, 0);
+    sRf[q] = (a.f_ix.id && ok) ? __ldg(a.f_ix.id + (int64_t)blk * (nz + 1) + k) : -1;
+    sRs[q] = (a.s_ix.id && ok) ? __ldg(a.s_ix.id + (int64_t)blk * (nz + 1) + k) : -1;
   }
-  for (int q = t; q < k1 - k0; q += NT) sRm[q] = a.m_rng ? a.m_rng[(int64_t)blk * nz + k0 + q] : make_int2(0, 0);
+  for (int q = t; q < k1 - k0; q += NT) sRm[q] = a.m_ix.id ? __ldg(a.m_ix.id + (int64_t)blk * nz + k0 + q) : -1;
+  if (!RANGE) wait_previous_step();  // (the FP64 form's blocks have waited to choose their path)
   __syncthreads();
-  // the copies are issued (and, on failure, drained) by the first thread of
-  // the last warp: its row is the tile's apron, which has no stress half
-  constexpr int ISSUER = (TY - 1) * TX;
-  if (t == ISSUER) {
-#pragma unroll
-    for (int d = 0; d <= G::PD; d++)
-      if (k0 - 1 + d <= k1) issue(k0 - 1 + d);
-  }
   // split the stress slot of layer L in place (df64d): each stored double
   // becomes its double-float pair, so the velocity half reads pairs; the
   // slot is waited for first (false: the wait gave up).  Two elements per
@@ -456,9 +500,10 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
   // one layer to the next alternate registers instead of moving
 #pragma unroll(sizeof(St) == 4 ? 2 : 1)
   for (int k = k0 - 1; k <= k1 + 1; k++) {
+    if (k == k1) let_next_step_start();
     if (t == ISSUER && k >= k0 && k + G::PD <= k1) {
       proxy_fence_async_smem();
-      issue(k + G::PD);
+      cp.issue(k + G::PD);
     }
     // ---- B: velocity of node layer k
     if (k <= k1) {
@@ -484,43 +529,37 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
       L px5, py5;
       diffdiff22_u(A, B, C, D, px5, py5);
       // x: Sxx along x, Sxy along y, Sxz along z; y: Sxy, Syy, Syz; z: Sxz, Syz, Szz
-      R tx, ty, tz, ax, ay, az, nbx, nby, nbz;
+      R dx, dy, dz, ax, ay, az, nbx, nby, nbz;
       L axu, ayu, azu;  // A of this layer (renormalised when B of the layer below joins)
       if constexpr (CUBIC) {  // 0.25/h folded into dt/rho and the force weights
-        tx = add_uu(px0, py5);
-        ty = add_uu(px5, py1);
-        tz = add_uu(px4, py3);
-        axu = add_unnorm(to_u(tx), s4);
-        ayu = add_unnorm(to_u(ty), s3);
-        azu = add_unnorm(to_u(tz), s2);
-        nbx = sub_uu(to_u(tx), s4);
-        nby = sub_uu(to_u(ty), s3);
-        nbz = sub_uu(to_u(tz), s2);
+        dx = add_uu(px0, py5);
+        dy = add_uu(px5, py1);
+        dz = add_uu(px4, py3);
+        axu = add_unnorm(to_u(dx), s4);
+        ayu = add_unnorm(to_u(dy), s3);
+        azu = add_unnorm(to_u(dz), s2);
+        nbx = sub_uu(to_u(dx), s4);
+        nby = sub_uu(to_u(dy), s3);
+        nbz = sub_uu(to_u(dz), s2);
       } else {
-        tx = madd(gy, norm_u(py5), gx * norm_u(px0));
-        ty = madd(gy, norm_u(py1), gx * norm_u(px5));
-        tz = madd(gy, norm_u(py3), gx * norm_u(px4));
+        dx = madd(gy, norm_u(py5), gx * norm_u(px0));
+        dy = madd(gy, norm_u(py1), gx * norm_u(px5));
+        dz = madd(gy, norm_u(py3), gx * norm_u(px4));
         const R n4 = norm_u(s4), n3 = norm_u(s3), n2 = norm_u(s2);
-        axu = to_u(madd(gz, n4, tx));
-        ayu = to_u(madd(gz, n3, ty));
-        azu = to_u(madd(gz, n2, tz));
-        nbx = madd(-gz, n4, tx);
-        nby = madd(-gz, n3, ty);
-        nbz = madd(-gz, n2, tz);
+        axu = to_u(madd(gz, n4, dx));
+        ayu = to_u(madd(gz, n3, dy));
+        azu = to_u(madd(gz, n2, dz));
+        nbx = madd(-gz, n4, dx);
+        nby = madd(-gz, n3, dy);
+        nbz = madd(-gz, n2, dz);
       }
       if (k >= k0) {
         ax = add_uu(axu, to_u(blx));
         ay = add_uu(ayu, to_u(bly));
         az = add_uu(azu, to_u(blz));
-        const int2 fr = sRf[k - k0 + 1];
-        // this node's force sources (the batch kernel scans its slots whole:
-        // the searches cost it registers for a fourth block per SM)
-        for (int e = BATCH ? fr.x : first_local(a.f_key, fr.x, fr.y, t); e < fr.y; e++) {
+        const int2 fr = slot_entries<TY>(a.f_ix, sRf[k - k0 + 1], tx, ty);  // this node's force sources
+        for (int e = fr.x; e < fr.y; e++) {
           const int key = __ldg(a.f_key + e);
-          if ((key & 0xffff) != t) {
-            if (!BATCH && (key & 0xffff) > t) break;
-            continue;
-          }
           const R w = N::val(a.f_w[e]), sg = N::val(sigrow[__ldg(a.f_sig + e)]);
           const int d = key >> 16;
           if (d == 0) ax = madd(w, sg, ax);
@@ -568,14 +607,9 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
 #pragma unroll
             for (int c = 0; c < 3; c++) store(a.V_out[c], n, vn[c], 0);
           }
-          const int2 sr = sRs[k - k0 + 1];
           if (rec < a.rec_cap) {
-            for (int e = BATCH ? sr.x : first_local(a.s_key, sr.x, sr.y, t); e < sr.y; e++) {  // sensor traces
-              const int lk = __ldg(a.s_key + e);
-              if (lk != t) {
-                if (!BATCH && lk > t) break;
-                continue;
-              }
+            const int2 sr = slot_entries<TY>(a.s_ix, sRs[k - k0 + 1], tx, ty);
+            for (int e = sr.x; e < sr.y; e++) {  // sensor traces
               double *tr = a.traces + (rec * a.n_sens + __ldg(a.s_idx + e)) * 3;
               tr[0] = out(0);
               tr[1] = out(1);
@@ -639,13 +673,9 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
 #pragma unroll
           for (int f = 0; f < 6; f++) acc[f] = N::ld(a.S_in[f], cg);
         }
-        const int2 mr = sRm[kc - k0];
-        for (int ee = BATCH ? mr.x : first_local(a.m_key, mr.x, mr.y, t); ee < mr.y; ee++) {  // this cell's moments
+        const int2 mr = slot_entries<TY>(a.m_ix, sRm[kc - k0], tx, ty);  // this cell's moments
+        for (int ee = mr.x; ee < mr.y; ee++) {
           const int key = __ldg(a.m_key + ee);
-          if ((key & 0xffff) != t) {
-            if (!BATCH && (key & 0xffff) > t) break;
-            continue;
-          }
           const R w = N::val(a.m_w[ee]), sg = N::val(sigrow[__ldg(a.m_sig + ee)]);
           const int kk = key >> 16;
 #pragma unroll
@@ -729,7 +759,7 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
 // (flag_phase + step) % 3, or-ed by this step's blocks (+1), cleared for the
 // step after next by each tile's first chunk (+2).  Block-uniform.
 template <int TY>
-__device__ __forceinline__ bool fp64_path(const GridArgs<double> &a, int bx, int by, int k0, int kc, int gxc,
+__device__ __forceinline__ bool fp64_path(const GridArgs<double> &a, int bx, int by, int k0, int k1, int gxc,
                                           int step) {
   constexpr int NT = TX * TY;
   const int t = threadIdx.x;
@@ -746,9 +776,7 @@ __device__ __forceinline__ bool fp64_path(const GridArgs<double> &a, int bx, int
     }
   }
   const int nz = a.nz;
-  const int ktop = a.ktop ? min(nz, __ldg(a.ktop + blk)) : nz;
-  const int k1 = min(ktop, k0 + kc);
-  if (k0 < ktop && a.sigval) {
+  if (k0 < k1 && a.sigval) {
     const double *sigrow = a.sigval + (int64_t)min(step, a.sig_rows - 1) * a.sig_stride;
     const uint32_t lo = (uint32_t)a.r_elo_s, hi = (uint32_t)a.r_ehi_s;
     auto bad = [&](double w, double sg) { return !in_df64_range(sg, lo, hi) || !in_df64_range(w * sg, lo, hi); };
@@ -807,26 +835,27 @@ __device__ __forceinline__ void block_coords(const GridArgs<T> &a, int &bx, int 
 #ifndef PN_F64H_TWO_LAUNCHES
 #define PN_F64H_TWO_LAUNCHES 0
 #endif
-template <typename K, int SYM, bool BATCH>
-__device__ __forceinline__ void f64h_path(const GridArgs<double> &a, const GridMaps *M, int bx, int by, int k0,
-                                          int kc, int gxc, int step) {
-  grid_block_tma<K, SYM, 8, BATCH, true>(a, M, bx, by, k0, kc, gxc, step);
-}
-
 template <int SYM, bool BATCH, int MODE>
-__device__ __forceinline__ void f64h_block(const GridArgs<double> &a, int bx, int by, int k0, int kc, int gxc,
-                                           int step) {
-  const GridMaps *M = reinterpret_cast<const GridMaps *>(a.tmaps);
-  const bool fp64 = fp64_path<8>(a, bx, by, k0, kc, gxc, step);
+__device__ __forceinline__ void f64h_block(const GridArgs<double> &a, unsigned char *smem, int bx, int by, int k0,
+                                           int kc, int gxc, int step) {
+  const int ktop = tile_top(a, by * gxc + bx), k1 = min(ktop, k0 + kc);
+  const Copies<double, 8, BATCH> cp(a, smem, bx, by, k0, k1);
+  // both paths read the same tiles: the copies start before the path is chosen
+  const bool work = k0 < k1;
+  if (MODE == 0 && work && threadIdx.x == cp.ISSUER) cp.start();
+  wait_previous_step();
+  const bool fp64 = fp64_path<8>(a, bx, by, k0, k1, gxc, step);
   if ((MODE == 1 && fp64) || (MODE == 2 && !fp64)) return;
   if (threadIdx.x == 0 && a.path_count) atomicAdd(a.path_count + (fp64 ? 0 : 1), 1ull);
+  if (!work) return;
+  if (MODE != 0 && threadIdx.x == cp.ISSUER) cp.start();
   if constexpr (MODE != 1) {
     if (fp64) {
-      f64h_path<double, SYM, BATCH>(a, M, bx, by, k0, kc, gxc, step);
+      grid_block_tma<double, SYM, 8, BATCH, true>(a, cp, bx, by, k1 == ktop, gxc, step);
       return;
     }
   }
-  if constexpr (MODE != 2) f64h_path<df64d, SYM, BATCH>(a, M, bx, by, k0, kc, gxc, step);
+  if constexpr (MODE != 2) grid_block_tma<df64d, SYM, 8, BATCH, true>(a, cp, bx, by, k1 == ktop, gxc, step);
 }
 
 // resident blocks per SM the FP64 form's kernel is compiled for (its register
@@ -838,15 +867,17 @@ __device__ __forceinline__ void f64h_block(const GridArgs<double> &a, int bx, in
 template <int SYM, int MODE>
 __global__ void __launch_bounds__(TX * 8, PN_F64H_MIN_BLOCKS)
     k_grid_tma_f64h(const __grid_constant__ GridArgs<double> a, int step) {
+  extern __shared__ unsigned char smem_raw[];
   int bx, by, k0, kc, gxc;
   block_coords<8>(a, bx, by, k0, kc, gxc);
-  f64h_block<SYM, false, MODE>(a, bx, by, k0, kc, gxc, step);
+  f64h_block<SYM, false, MODE>(a, smem_raw, bx, by, k0, kc, gxc, step);
 }
 
 template <int SYM, int MODE>
 __global__ void __launch_bounds__(TX * 8, PN_F64H_MIN_BLOCKS)
     k_grid_tma_f64h_batch(const GridArgs<double> *__restrict__ args, const int *__restrict__ block_start,
                           const int *__restrict__ order, int n_members, int step) {
+  extern __shared__ unsigned char smem_raw[];
   const int id = order ? __ldg(order + blockIdx.x) : (int)blockIdx.x;
   int lo = 0, hi = n_members;
   while (hi - lo > 1) {
@@ -857,31 +888,42 @@ __global__ void __launch_bounds__(TX * 8, PN_F64H_MIN_BLOCKS)
   const GridArgs<double> &a = args[lo];
   const int local = id - __ldg(block_start + lo);
   const int gxc = a.nx / (TX - 1) + 1, gyc = a.ny / 7 + 1;
-  f64h_block<SYM, true, MODE>(a, local % gxc, (local / gxc) % gyc, local / (gxc * gyc) * a.kchunk, a.kchunk, gxc,
+  f64h_block<SYM, true, MODE>(a, smem_raw, local % gxc, (local / gxc) % gyc, local / (gxc * gyc) * a.kchunk, a.kchunk, gxc,
                               step);
 }
 
 // minimum blocks per SM each storage type is compiled for (the register cap
 // follows): 3 for 8-byte storage (80 registers; shared memory holds 3 blocks);
-// none for 4-byte storage (the compiler's 62-64 registers give 4 blocks, and a
-// cap of 4 blocks measured 6% slower)
+// 4 for 4-byte storage (56-64 registers; left to itself the compiler takes 80
+// and 3 blocks fit: laminate FP32 107.8 us per step against 105.8)
 // (32 x 16 tiles with 8-byte storage: shared memory holds one block per SM)
 template <typename R, int TY> struct GMinBlocks { static constexpr int v = TY == 8 ? 3 : 1; };
 template <int TY> struct GMinBlocks<float, TY> { static constexpr int v = PN_GRID_F32_MIN_BLOCKS; };
 
+template <typename R, int SYM, int TY, bool BATCH>
+__device__ __forceinline__ void run_block(const GridArgs<typename GNum<R>::S> &a, unsigned char *smem, int bx, int by,
+                                          int k0, int kc, int gxc, int step) {
+  const int ktop = tile_top(a, by * gxc + bx), k1 = min(ktop, k0 + kc);
+  if (k0 >= k1) return;
+  const Copies<typename GNum<R>::S, TY, BATCH> cp(a, smem, bx, by, k0, k1);
+  if (threadIdx.x == cp.ISSUER) cp.start();
+  grid_block_tma<R, SYM, TY, BATCH>(a, cp, bx, by, k1 == ktop, gxc, step);
+}
+
 template <typename R, int SYM, int TY>
 __global__ void __launch_bounds__(TX *TY, GMinBlocks<R, TY>::v)
     k_grid_tma(const GridArgs<typename GNum<R>::S> a, int step) {
-  const GridMaps *M = reinterpret_cast<const GridMaps *>(a.tmaps);
+  extern __shared__ unsigned char smem_raw[];
   int bx, by, k0, kc, gxc;
   block_coords<TY>(a, bx, by, k0, kc, gxc);
-  grid_block_tma<R, SYM, TY>(a, M, bx, by, k0, kc, gxc, step);
+  run_block<R, SYM, TY, false>(a, smem_raw, bx, by, k0, kc, gxc, step);
 }
 
 template <typename R, int SYM, int TY>
 __global__ void __launch_bounds__(TX *TY, GMinBlocks<R, TY>::v)
     k_grid_tma_batch(const GridArgs<typename GNum<R>::S> *__restrict__ args, const int *__restrict__ block_start,
                      const int *__restrict__ order, int n_members, int step) {
+  extern __shared__ unsigned char smem_raw[];
   const int id = order ? __ldg(order + blockIdx.x) : (int)blockIdx.x;
   int lo = 0, hi = n_members;
   while (hi - lo > 1) {
@@ -890,11 +932,27 @@ __global__ void __launch_bounds__(TX *TY, GMinBlocks<R, TY>::v)
     else hi = mid;
   }
   const GridArgs<typename GNum<R>::S> &a = args[lo];
-  const GridMaps *M = reinterpret_cast<const GridMaps *>(a.tmaps);
   const int local = id - __ldg(block_start + lo);
   const int gxc = a.nx / (TX - 1) + 1, gyc = a.ny / (TY - 1) + 1;
-  grid_block_tma<R, SYM, TY, true>(a, M, local % gxc, (local / gxc) % gyc, local / (gxc * gyc) * a.kchunk, a.kchunk,
-                                   gxc, step);
+  run_block<R, SYM, TY, true>(a, smem_raw, local % gxc, (local / gxc) % gyc, local / (gxc * gyc) * a.kchunk, a.kchunk,
+                              gxc, step);
+}
+
+// a step launch that may start while the previous step drains
+// (wait_previous_step)
+template <typename F, typename... A>
+cudaError_t launch_step(F f, dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, f, args...);
 }
 
 template <typename R, int SYM, int TY>
@@ -950,8 +1008,7 @@ cudaError_t launch_t(const GridArgs<typename GNum<R>::S> &a, cudaStream_t st) {
   GridArgs<typename GNum<R>::S> b = a;
   const dim3 grid = single_grid<TY>(b, sms, per_sm);
   if (grid.x == 0) return cudaErrorInvalidValue;
-  k_grid_tma<R, SYM, TY><<<grid, TX * TY, S::smem, st>>>(b, 0);
-  return cudaGetLastError();
+  return launch_step(k_grid_tma<R, SYM, TY>, grid, TX * TY, S::smem, st, b, 0);
 }
 
 template <typename R, int SYM, int TY>
@@ -961,9 +1018,8 @@ cudaError_t launch_batch_t(const GridBatchLaunch &b, int step, cudaStream_t st) 
   cudaError_t e = S::ensure(sms, per_sm);
   if (e != cudaSuccess) return e;
   if (b.total_blocks <= 0) return cudaSuccess;
-  k_grid_tma_batch<R, SYM, TY><<<b.total_blocks, TX * TY, S::smem, st>>>(
-      (const GridArgs<typename GNum<R>::S> *)b.args, b.block_start, b.order, b.n_members, step);
-  return cudaGetLastError();
+  return launch_step(k_grid_tma_batch<R, SYM, TY>, dim3((unsigned)b.total_blocks), TX * TY, S::smem, st,
+                     (const GridArgs<typename GNum<R>::S> *)b.args, b.block_start, b.order, b.n_members, step);
 }
 
 // the FP64 form's kernels (k_grid_tma_f64h*): the FP64 path's shared-memory geometry
@@ -992,8 +1048,7 @@ template <int SYM, int MODE>
 cudaError_t launch_h_mode(const GridArgs<double> &b, const dim3 &grid, cudaStream_t st) {
   cudaError_t e = SetupH<SYM, MODE>::ensure();
   if (e != cudaSuccess) return e;
-  k_grid_tma_f64h<SYM, MODE><<<grid, TX * 8, SetupH<SYM, MODE>::smem, st>>>(b, 0);
-  return cudaGetLastError();
+  return launch_step(k_grid_tma_f64h<SYM, MODE>, grid, TX * 8, SetupH<SYM, MODE>::smem, st, b, 0);
 }
 
 template <int SYM>
@@ -1016,9 +1071,9 @@ template <int SYM, int MODE>
 cudaError_t launch_batch_h_mode(const GridBatchLaunch &b, int step, cudaStream_t st) {
   cudaError_t e = SetupH<SYM, MODE>::ensure();
   if (e != cudaSuccess) return e;
-  k_grid_tma_f64h_batch<SYM, MODE><<<b.total_blocks, TX * 8, SetupH<SYM, MODE>::smem, st>>>(
-      (const GridArgs<double> *)b.args, b.block_start, b.order, b.n_members, step);
-  return cudaGetLastError();
+  return launch_step(k_grid_tma_f64h_batch<SYM, MODE>, dim3((unsigned)b.total_blocks), TX * 8,
+                     SetupH<SYM, MODE>::smem, st, (const GridArgs<double> *)b.args, b.block_start, b.order, b.n_members,
+                     step);
 }
 
 template <int SYM>
