@@ -10,7 +10,7 @@ from pannde_gb300 import _native as N
 from pannde_gb300 import cases
 from pannde_gb300.solver import Batch, Solver
 
-from .test_parity_gpu import TOL, compare
+from tests.test_parity_gpu import TOL, compare
 
 pytestmark = pytest.mark.gpu
 
