@@ -22,213 +22,154 @@
 
 namespace pn {
 
-// Two floats worked on by one instruction (Blackwell's packed add, multiply
-// and fused multiply-add): the pipe does the same number of operations a
-// second as with single ones (measured 3.8e13 elements/s for both) but the
-// pair takes one issue slot instead of two.  Each half is rounded as the
-// scalar operation rounds it.
-struct f32x2 {
-  unsigned long long v;
-  __device__ __forceinline__ f32x2() : v(0ull) {}
-  __device__ __forceinline__ f32x2(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
-  __device__ __forceinline__ float half(int h) const {
-    float a, b;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-    return h ? b : a;
-  }
+struct df64 {
+  float hi, lo;
+  __device__ __forceinline__ df64() : hi(0.f), lo(0.f) {}
+  __device__ __forceinline__ df64(float h, float l) : hi(h), lo(l) {}
+  __device__ __forceinline__ explicit df64(float h) : hi(h), lo(0.f) {}
 };
 
-// the operations the algorithms below are written in: one float, or two
-__device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float ffma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ float fneg(float a) { return -a; }
-__device__ __forceinline__ f32x2 fadd(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ f32x2 fsub(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ f32x2 fmul(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ f32x2 ffma(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-  return r;
-}
-__device__ __forceinline__ f32x2 fneg(f32x2 a) {
-  a.v ^= 0x8000000080000000ull;
-  return a;
-}
-__device__ __forceinline__ f32x2 operator+(f32x2 a, f32x2 b) { return fadd(a, b); }
-__device__ __forceinline__ f32x2 operator-(f32x2 a, f32x2 b) { return fsub(a, b); }
-__device__ __forceinline__ f32x2 operator*(f32x2 a, f32x2 b) { return fmul(a, b); }
-__device__ __forceinline__ f32x2 operator-(f32x2 a) { return fneg(a); }
-__device__ __forceinline__ f32x2 madd(f32x2 a, f32x2 b, f32x2 c) { return ffma(a, b, c); }
-
-// native types: the compiler contracts a*b + c into one FMA
-__device__ __forceinline__ float madd(float a, float b, float c) { return a * b + c; }
-__device__ __forceinline__ double madd(double a, double b, double c) { return a * b + c; }
-
-// two doubles (no packed instructions: each half on its own)
-struct f64x2 {
-  double a, b;
-  __device__ __forceinline__ f64x2() : a(0.), b(0.) {}
-  __device__ __forceinline__ f64x2(double x, double y) : a(x), b(y) {}
-};
-__device__ __forceinline__ f64x2 operator+(f64x2 x, f64x2 y) { return f64x2(x.a + y.a, x.b + y.b); }
-__device__ __forceinline__ f64x2 operator-(f64x2 x, f64x2 y) { return f64x2(x.a - y.a, x.b - y.b); }
-__device__ __forceinline__ f64x2 operator*(f64x2 x, f64x2 y) { return f64x2(x.a * y.a, x.b * y.b); }
-__device__ __forceinline__ f64x2 operator-(f64x2 x) { return f64x2(-x.a, -x.b); }
-__device__ __forceinline__ f64x2 madd(f64x2 x, f64x2 y, f64x2 z) { return f64x2(x.a * y.a + z.a, x.b * y.b + z.b); }
-
-// a double-float (F = float), or two side by side (F = f32x2)
-template <typename F> struct ddf {
-  F hi, lo;
-  __device__ __forceinline__ ddf() : hi(), lo() {}
-  __device__ __forceinline__ ddf(F h, F l) : hi(h), lo(l) {}
-};
-using df64 = ddf<float>;
-using df64x2 = ddf<f32x2>;
-
-template <typename F> __device__ __forceinline__ ddf<F> two_sum(F a, F b) {
-  const F s = fadd(a, b);
-  const F bb = fsub(s, a);
-  const F e = fadd(fsub(a, fsub(s, bb)), fsub(b, bb));
-  return ddf<F>(s, e);
-}
-// two_sum(a, -b) without forming -b
-template <typename F> __device__ __forceinline__ ddf<F> two_diff(F a, F b) {
-  const F s = fsub(a, b);
-  const F bb = fsub(s, a);
-  const F e = fsub(fsub(a, fsub(s, bb)), fadd(b, bb));
-  return ddf<F>(s, e);
+__device__ __forceinline__ df64 two_sum(float a, float b) {
+  const float s = __fadd_rn(a, b);
+  const float bb = __fsub_rn(s, a);
+  const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+  return df64(s, e);
 }
 
-template <typename F> __device__ __forceinline__ ddf<F> quick_two_sum(F a, F b) {
-  const F s = fadd(a, b);
-  return ddf<F>(s, fsub(b, fsub(s, a)));
+__device__ __forceinline__ df64 quick_two_sum(float a, float b) {
+  const float s = __fadd_rn(a, b);
+  return df64(s, __fsub_rn(b, __fsub_rn(s, a)));
 }
 
-template <typename F> __device__ __forceinline__ ddf<F> operator+(ddf<F> a, ddf<F> b) {
-  ddf<F> s = two_sum(a.hi, b.hi);
-  s.lo = fadd(s.lo, fadd(a.lo, b.lo));
+__device__ __forceinline__ df64 operator+(df64 a, df64 b) {
+  df64 s = two_sum(a.hi, b.hi);
+  s.lo = __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo));
   return quick_two_sum(s.hi, s.lo);
 }
 
-template <typename F> __device__ __forceinline__ ddf<F> operator-(ddf<F> a) { return ddf<F>(fneg(a.hi), fneg(a.lo)); }
+__device__ __forceinline__ df64 operator-(df64 a) { return df64(-a.hi, -a.lo); }
 
-template <typename F> __device__ __forceinline__ ddf<F> operator-(ddf<F> a, ddf<F> b) {
-  ddf<F> s = two_diff(a.hi, b.hi);
-  s.lo = fadd(s.lo, fsub(a.lo, b.lo));
-  return quick_two_sum(s.hi, s.lo);
-}
+__device__ __forceinline__ df64 operator-(df64 a, df64 b) { return a + (-b); }
 
-template <typename F> __device__ __forceinline__ ddf<F> operator*(ddf<F> a, ddf<F> b) {
-  const F p = fmul(a.hi, b.hi);
-  F e = ffma(a.hi, b.hi, fneg(p));
-  e = ffma(a.hi, b.lo, e);
-  e = ffma(a.lo, b.hi, e);
+__device__ __forceinline__ df64 operator*(df64 a, df64 b) {
+  const float p = __fmul_rn(a.hi, b.hi);
+  float e = __fmaf_rn(a.hi, b.hi, -p);
+  e = __fmaf_rn(a.hi, b.lo, e);
+  e = __fmaf_rn(a.lo, b.hi, e);
   return quick_two_sum(p, e);
 }
+
+__device__ __forceinline__ df64 &operator+=(df64 &a, df64 b) { return a = a + b; }
 
 // a*b + c without renormalising the product first: the two_prod error terms
 // join c's low word before the one renormalisation (15 flops against 18 for
 // a separate mul and add; the same "sloppy" error bound)
-template <typename F> __device__ __forceinline__ ddf<F> madd(ddf<F> a, ddf<F> b, ddf<F> c) {
-  const F p = fmul(a.hi, b.hi);
-  F e = ffma(a.hi, b.hi, fneg(p));
-  e = ffma(a.hi, b.lo, e);
-  e = ffma(a.lo, b.hi, e);
-  ddf<F> s = two_sum(p, c.hi);
-  s.lo = fadd(s.lo, fadd(e, c.lo));
+__device__ __forceinline__ df64 madd(df64 a, df64 b, df64 c) {
+  const float p = __fmul_rn(a.hi, b.hi);
+  float e = __fmaf_rn(a.hi, b.hi, -p);
+  e = __fmaf_rn(a.hi, b.lo, e);
+  e = __fmaf_rn(a.lo, b.hi, e);
+  df64 s = two_sum(p, c.hi);
+  s.lo = __fadd_rn(s.lo, __fadd_rn(e, c.lo));
   return quick_two_sum(s.hi, s.lo);
 }
 // Four-term sums of the stencil with one renormalisation at the end: the
 // high words go through error-free two_sums, the low words and the errors
 // are summed as floats ("lazy" double-float accumulation; 27 flops for
-// (b+c)-(a+d) against 33 for three renormalised adds).  The sums stay
-// unnormalised (lo not yet bounded by ulp(hi) / 2) until the add that consumes
-// them renormalises anyway (3 flops fewer per value); Lazy<T> is T itself for
-// the native types.
-template <typename F> struct ddf_unnorm {
-  F hi, lo;  // hi + lo, |lo| not yet bounded by ulp(hi)/2
+// (b+c)-(a+d) against 33 for three renormalised adds).
+struct df64_unnorm {
+  float hi, lo;  // hi + lo, |lo| not yet bounded by ulp(hi)/2
 };
-template <typename T> struct Lazy { using type = T; };
-template <typename F> struct Lazy<ddf<F>> { using type = ddf_unnorm<F>; };
-template <typename F> __device__ __forceinline__ ddf_unnorm<F> add_lazy(ddf<F> a, ddf<F> b) {
-  const ddf<F> s = two_sum(a.hi, b.hi);
-  return {s.hi, fadd(s.lo, fadd(a.lo, b.lo))};
+__device__ __forceinline__ df64_unnorm add_lazy(df64 a, df64 b) {
+  const df64 s = two_sum(a.hi, b.hi);
+  return {s.hi, __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo))};
 }
-template <typename F> __device__ __forceinline__ ddf_unnorm<F> sub_lazy(ddf<F> a, ddf<F> b) {
-  const ddf<F> s = two_diff(a.hi, b.hi);
-  return {s.hi, fadd(s.lo, fsub(a.lo, b.lo))};
+__device__ __forceinline__ df64 sub_norm(df64_unnorm a, df64_unnorm b) {
+  const df64 s = two_sum(a.hi, -b.hi);
+  return quick_two_sum(s.hi, __fadd_rn(s.lo, __fsub_rn(a.lo, b.lo)));
 }
-template <typename F> __device__ __forceinline__ ddf_unnorm<F> add_unnorm(ddf_unnorm<F> a, ddf_unnorm<F> b) {
-  const ddf<F> s = two_sum(a.hi, b.hi);
-  return {s.hi, fadd(s.lo, fadd(a.lo, b.lo))};
+__device__ __forceinline__ df64 add_norm(df64_unnorm a, df64_unnorm b) {
+  const df64 s = two_sum(a.hi, b.hi);
+  return quick_two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo)));
 }
-template <typename F> __device__ __forceinline__ ddf_unnorm<F> sub_unnorm(ddf_unnorm<F> a, ddf_unnorm<F> b) {
-  const ddf<F> s = two_diff(a.hi, b.hi);
-  return {s.hi, fadd(s.lo, fsub(a.lo, b.lo))};
-}
-template <typename F> __device__ __forceinline__ ddf<F> add_uu(ddf_unnorm<F> a, ddf_unnorm<F> b) {
-  const ddf<F> s = two_sum(a.hi, b.hi);
-  return quick_two_sum(s.hi, fadd(s.lo, fadd(a.lo, b.lo)));
-}
-template <typename F> __device__ __forceinline__ ddf<F> sub_uu(ddf_unnorm<F> a, ddf_unnorm<F> b) {
-  const ddf<F> s = two_diff(a.hi, b.hi);
-  return quick_two_sum(s.hi, fadd(s.lo, fsub(a.lo, b.lo)));
-}
-template <typename F> __device__ __forceinline__ ddf_unnorm<F> to_u(ddf<F> a) { return {a.hi, a.lo}; }
-template <typename F> __device__ __forceinline__ ddf<F> norm_u(ddf_unnorm<F> a) { return quick_two_sum(a.hi, a.lo); }
 // (b + c) - (a + d)
-template <typename F>
-__device__ __forceinline__ ddf_unnorm<F> diff22_u(ddf<F> b, ddf<F> c, ddf<F> a, ddf<F> d) {
-  return sub_unnorm(add_lazy(b, c), add_lazy(a, d));
+__device__ __forceinline__ df64 diff22(df64 b, df64 c, df64 a, df64 d) {
+  return sub_norm(add_lazy(b, c), add_lazy(a, d));
 }
 // (a + b) + (c + d)
-template <typename F>
-__device__ __forceinline__ ddf_unnorm<F> sum22_u(ddf<F> a, ddf<F> b, ddf<F> c, ddf<F> d) {
-  return add_unnorm(add_lazy(a, b), add_lazy(c, d));
+__device__ __forceinline__ df64 sum22(df64 a, df64 b, df64 c, df64 d) {
+  return add_norm(add_lazy(a, b), add_lazy(c, d));
 }
 // (c + d) - (a + b) and (a + b) + (c + d) sharing the pair sums
-template <typename F>
-__device__ __forceinline__ void diffsum22_u(ddf<F> a, ddf<F> b, ddf<F> c, ddf<F> d, ddf_unnorm<F> &diff,
-                                            ddf_unnorm<F> &sum) {
-  const ddf_unnorm<F> ab = add_lazy(a, b), cd = add_lazy(c, d);
-  diff = sub_unnorm(cd, ab);
-  sum = add_unnorm(ab, cd);
+__device__ __forceinline__ void diffsum22(df64 a, df64 b, df64 c, df64 d, df64 &diff, df64 &sum) {
+  const df64_unnorm ab = add_lazy(a, b), cd = add_lazy(c, d);
+  diff = sub_norm(cd, ab);
+  sum = add_norm(ab, cd);
 }
 // (b + c) - (a + d) and (c + d) - (a + b) as (c - a) + (b - d) and
 // (c - a) - (b - d): two pair differences shared (38 flops against 54)
-template <typename F>
-__device__ __forceinline__ void diffdiff22_u(ddf<F> a, ddf<F> b, ddf<F> c, ddf<F> d, ddf_unnorm<F> &dx,
-                                             ddf_unnorm<F> &dy) {
-  const ddf_unnorm<F> u = sub_lazy(c, a), w = sub_lazy(b, d);
-  dx = add_unnorm(u, w);
-  dy = sub_unnorm(u, w);
+__device__ __forceinline__ df64_unnorm sub_lazy(df64 a, df64 b) {
+  const df64 s = two_sum(a.hi, -b.hi);
+  return {s.hi, __fadd_rn(s.lo, __fsub_rn(a.lo, b.lo))};
 }
-// the same for the native types
-template <typename T> __device__ __forceinline__ T diff22_u(T b, T c, T a, T d) { return (b + c) - (a + d); }
-template <typename T> __device__ __forceinline__ T sum22_u(T a, T b, T c, T d) { return (a + b) + (c + d); }
-template <typename T> __device__ __forceinline__ void diffsum22_u(T a, T b, T c, T d, T &diff, T &sum) {
+__device__ __forceinline__ void diffdiff22(df64 a, df64 b, df64 c, df64 d, df64 &dx, df64 &dy) {
+  const df64_unnorm u = sub_lazy(c, a), w = sub_lazy(b, d);
+  dx = add_norm(u, w);
+  dy = sub_norm(u, w);
+}
+template <typename T> __device__ __forceinline__ void diffdiff22(T a, T b, T c, T d, T &dx, T &dy) {
+  const T u = c - a, w = b - d;
+  dx = u + w;
+  dy = u - w;
+}
+template <typename T> __device__ __forceinline__ T diff22(T b, T c, T a, T d) { return (b + c) - (a + d); }
+template <typename T> __device__ __forceinline__ T sum22(T a, T b, T c, T d) { return (a + b) + (c + d); }
+template <typename T> __device__ __forceinline__ void diffsum22(T a, T b, T c, T d, T &diff, T &sum) {
   const T ab = a + b, cd = c + d;
   diff = cd - ab;
   sum = ab + cd;
 }
+
+// The stencil's pair differences kept unnormalised (lo not yet bounded by
+// ulp(hi) / 2) until the add that consumes them renormalises anyway (3 flops
+// fewer per value); Lazy<T> is T itself for the native types.
+template <typename T> struct Lazy { using type = T; };
+template <> struct Lazy<df64> { using type = df64_unnorm; };
+__device__ __forceinline__ df64_unnorm sub_unnorm(df64_unnorm a, df64_unnorm b) {
+  const df64 s = two_sum(a.hi, -b.hi);
+  return {s.hi, __fadd_rn(s.lo, __fsub_rn(a.lo, b.lo))};
+}
+__device__ __forceinline__ df64_unnorm add_unnorm(df64_unnorm a, df64_unnorm b) {
+  const df64 s = two_sum(a.hi, b.hi);
+  return {s.hi, __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo))};
+}
+__device__ __forceinline__ df64_unnorm diff22_u(df64 b, df64 c, df64 a, df64 d) {
+  return sub_unnorm(add_lazy(b, c), add_lazy(a, d));
+}
+__device__ __forceinline__ df64_unnorm sum22_u(df64 a, df64 b, df64 c, df64 d) {
+  return add_unnorm(add_lazy(a, b), add_lazy(c, d));
+}
+__device__ __forceinline__ void diffsum22_u(df64 a, df64 b, df64 c, df64 d, df64_unnorm &diff, df64_unnorm &sum) {
+  const df64_unnorm ab = add_lazy(a, b), cd = add_lazy(c, d);
+  diff = sub_unnorm(cd, ab);
+  sum = add_unnorm(ab, cd);
+}
+__device__ __forceinline__ void diffdiff22_u(df64 a, df64 b, df64 c, df64 d, df64_unnorm &dx, df64_unnorm &dy) {
+  const df64_unnorm u = sub_lazy(c, a), w = sub_lazy(b, d);
+  dx = add_unnorm(u, w);
+  dy = sub_unnorm(u, w);
+}
+__device__ __forceinline__ df64 add_uu(df64_unnorm a, df64_unnorm b) { return add_norm(a, b); }
+__device__ __forceinline__ df64 sub_uu(df64_unnorm a, df64_unnorm b) { return sub_norm(a, b); }
+__device__ __forceinline__ df64_unnorm to_u(df64 a) { return {a.hi, a.lo}; }
+__device__ __forceinline__ df64 norm_u(df64_unnorm a) { return quick_two_sum(a.hi, a.lo); }
+template <typename T> __device__ __forceinline__ T diff22_u(T b, T c, T a, T d) { return diff22(b, c, a, d); }
+template <typename T> __device__ __forceinline__ T sum22_u(T a, T b, T c, T d) { return sum22(a, b, c, d); }
+template <typename T> __device__ __forceinline__ void diffsum22_u(T a, T b, T c, T d, T &diff, T &sum) {
+  diffsum22(a, b, c, d, diff, sum);
+}
 template <typename T> __device__ __forceinline__ void diffdiff22_u(T a, T b, T c, T d, T &dx, T &dy) {
-  const T u = c - a, w = b - d;
-  dx = u + w;
-  dy = u - w;
+  diffdiff22(a, b, c, d, dx, dy);
 }
 template <typename T> __device__ __forceinline__ T add_unnorm(T a, T b) { return a + b; }
 template <typename T> __device__ __forceinline__ T sub_unnorm(T a, T b) { return a - b; }
@@ -241,21 +182,24 @@ template <typename T> __device__ __forceinline__ T norm_u(T a) { return a; }
 // stiffness product): each product's high part joins the running sum through
 // an error-free two_sum, its error terms and the low words are summed as
 // floats (12 flops per term against madd's 15, the same "sloppy" bound)
-template <typename F> __device__ __forceinline__ ddf_unnorm<F> acc_start(ddf<F> c) { return {c.hi, c.lo}; }
-template <typename F> __device__ __forceinline__ void acc_madd(ddf_unnorm<F> &s, ddf<F> a, ddf<F> b) {
-  const F p = fmul(a.hi, b.hi);
-  F e = ffma(a.hi, b.hi, fneg(p));
-  e = ffma(a.hi, b.lo, e);
-  e = ffma(a.lo, b.hi, e);
-  const ddf<F> t = two_sum(s.hi, p);
+struct df64_acc {
+  float hi, lo;
+};
+__device__ __forceinline__ df64_acc acc_start(df64 c) { return {c.hi, c.lo}; }
+__device__ __forceinline__ void acc_madd(df64_acc &s, df64 a, df64 b) {
+  const float p = __fmul_rn(a.hi, b.hi);
+  float e = __fmaf_rn(a.hi, b.hi, -p);
+  e = __fmaf_rn(a.hi, b.lo, e);
+  e = __fmaf_rn(a.lo, b.hi, e);
+  const df64 t = two_sum(s.hi, p);
   s.hi = t.hi;
-  s.lo = fadd(s.lo, fadd(t.lo, e));
+  s.lo = __fadd_rn(s.lo, __fadd_rn(t.lo, e));
 }
-template <typename F> __device__ __forceinline__ ddf<F> acc_end(ddf_unnorm<F> s) { return quick_two_sum(s.hi, s.lo); }
-// ... and for the native types: one FMA per term
-template <typename T> __device__ __forceinline__ T acc_start(T c) { return c; }
-template <typename T> __device__ __forceinline__ void acc_madd(T &s, T a, T b) { s = madd(a, b, s); }
-template <typename T> __device__ __forceinline__ T acc_end(T s) { return s; }
+__device__ __forceinline__ df64 acc_end(df64_acc s) { return quick_two_sum(s.hi, s.lo); }
+
+// the same for the native types: the compiler contracts a*b + c into one FMA
+__device__ __forceinline__ float madd(float a, float b, float c) { return a * b + c; }
+__device__ __forceinline__ double madd(double a, double b, double c) { return a * b + c; }
 
 __device__ __forceinline__ bool operator==(df64 a, df64 b) { return a.hi == b.hi && a.lo == b.lo; }
 
