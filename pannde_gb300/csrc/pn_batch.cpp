@@ -387,16 +387,31 @@ void solve_grid(pn_batch *b, int32_t nsteps, int precision, const Stage &stage, 
     std::vector<int> order;
     int listed = 0;  // blocks launched
     size_t start_ints = 2 * (n + 1);
+    // chunk length of shape c for a member: the batch's own choice over all
+    // members' columns (0), or so many chunks per column
+    std::map<int, int> own_len;  // by tile rows
+    auto chunk_layers = [&](int c, const pn_solver *s) {
+      const int rows = shapes[c].first, per = shapes[c].second, nz = s->grid.nz;
+      if (per != 0) return std::min(pn::kGridChunkMax, std::max(1, (nz + per - 1) / per));
+      auto it = own_len.find(rows);
+      if (it == own_len.end()) {
+        std::map<int, long long> tops;
+        for (pn_solver *q : b->members)
+          if (tma)
+            for (int32_t top : pn::grid_tile_tops(q->grid, rows)) tops[std::min(top, q->grid.nz)]++;
+          else tops[q->grid.nz] += (long long)(q->grid.nx / (tx - 1) + 1) * (q->grid.ny / (rows - 1) + 1);
+        tops.erase(0);
+        it = own_len.emplace(rows, pn::grid_chunk_layers(precision, tops, tma, rows)).first;
+      }
+      return std::max(1, std::min(it->second, nz));
+    };
     if (ordered) {
       size_t most = 0;
-      for (auto &sh : shapes) {
+      for (int c = 0; c < (int)shapes.size(); c++) {
         size_t blocks = 0;
         for (pn_solver *s : b->members) {
-          const int kc = sh.second == 0 ? pn::grid_chunk_layers(precision, s->grid.nx, s->grid.ny, s->grid.nz, tma,
-                                                                sh.first)
-                                        : std::min(pn::kGridChunkMax, std::max(1, (s->grid.nz + sh.second - 1) /
-                                                                                       sh.second));
-          blocks += (size_t)(s->grid.nx / (tx - 1) + 1) * (s->grid.ny / (sh.first - 1) + 1) *
+          const int kc = chunk_layers(c, s);
+          blocks += (size_t)(s->grid.nx / (tx - 1) + 1) * (s->grid.ny / (shapes[c].first - 1) + 1) *
                     ((s->grid.nz + kc - 1) / kc);
         }
         most = std::max(most, blocks);
@@ -427,9 +442,7 @@ void solve_grid(pn_batch *b, int32_t nsteps, int precision, const Stage &stage, 
           a.sig_rows = (int32_t)(s->sig_rows - row0);
         }
         a.rec = s->rec_count;
-        const int per = shapes[c].second;
-        a.kchunk = per == 0 ? pn::grid_chunk_layers(precision, a.nx, a.ny, a.nz, tma, rows)
-                            : std::min(pn::kGridChunkMax, std::max(1, (a.nz + per - 1) / per));
+        a.kchunk = chunk_layers(c, s);
         for (int p = 0; p < 2; p++) {  // step parity: buffers swap every step
           pn::GridArgs<T> q = a;
           const int in = s->cur ^ p, out = in ^ 1;

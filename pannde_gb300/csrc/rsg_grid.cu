@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstdint>
+#include <map>
 
 #include "df64.cuh"
 #include "rsg_common.cuh"
@@ -405,21 +406,76 @@ cudaError_t launch_batch_sym(const GridBatchLaunch &b, int step, cudaStream_t st
 }  // namespace
 
 
-int grid_chunk_for(int nz, long long xy_blocks, int sms, int per_sm) {
+// Modelled time of a step whose tile columns (tops: number of columns per
+// height in cell layers) are cut into chunks of `len` layers, in units of one
+// block's share of a full SM's time per layer.  A block takes its layers and
+// about 1.5 more (the re-marched ones, the start); while few blocks share an SM
+// a layer takes its latency, 2.6 units, and the throughput of the SM counts
+// from three blocks on.  Blocks beyond the resident ones run as others end and
+// leave 0.4 of a last block's time uncovered.
+// Fitted to sweeps of every chunk length on eleven lattices from 40 x 40 x 8 to
+// 300 x 280 x 24 cells (12 to 410 columns), each in FP32, double-float and FP64:
+// the length chosen is 3% slower than the best on average (at most 11 / 18 /
+// 9%), where the rule before (as many chunks as one wave of resident blocks
+// needs, of four layers at least) was 17% slower.
+static double chunk_time(const std::map<int, long long> &tops, int len, int sms, int per_sm) {
+  constexpr double o = 1.5, latency = 2.6, uncovered = 0.4;
+  long long blocks = 0, layers = 0;
+  int longest = 0;
+  for (const auto &t : tops) {
+    const long long per = (t.first + len - 1) / len;
+    blocks += t.second * per;
+    layers += t.second * t.first;
+    longest = std::max(longest, std::min(t.first, len));
+  }
+  const double share = ((double)layers + o * (double)blocks) / sms, last = longest + o;
+  const long long slots = (long long)sms * per_sm;
+  if (blocks <= slots) return std::max(last * std::max(latency, (double)((blocks + sms - 1) / sms)), share);
+  return std::max(share + uncovered * last * latency, last * std::max(latency, (double)per_sm));
+}
+
+int grid_chunk_for(const std::map<int, long long> &tops, int sms, int per_sm) {
+  const int nz = tops.empty() ? 0 : tops.rbegin()->first;
   if (nz <= 0) return 1;
   // tuning override: PN_GRID_KCHUNK cell layers per chunk
   if (const char *v = std::getenv("PN_GRID_KCHUNK")) {
     const int k = std::atoi(v);
     if (k > 0) return std::min(std::min(k, kGridChunkMax), nz);
   }
-  // Each chunk re-marches two layers (the partial sums below it, the node
-  // layer above it), which costs more than a partly empty last wave: split
-  // columns only as far as one wave of resident blocks needs.
-  const long long want = (long long)sms * per_sm;
-  long long chunks = (want + xy_blocks - 1) / xy_blocks;
-  chunks = std::max(1LL, std::min(chunks, (long long)std::max(1, nz / 4)));
-  chunks = std::max(chunks, (long long)((nz + kGridChunkMax - 1) / kGridChunkMax));
-  return (int)((nz + chunks - 1) / chunks);
+  int best = 0;
+  double best_t = 0.0;
+  for (int chunks = (nz + kGridChunkMax - 1) / kGridChunkMax, last = 0; chunks <= nz; chunks++) {
+    const int len = (nz + chunks - 1) / chunks;
+    if (len == last) continue;
+    last = len;
+    const double t = chunk_time(tops, len, sms, per_sm);
+    if (best == 0 || t < best_t * (1.0 - 1e-9)) {
+      best = len;
+      best_t = t;
+    }
+  }
+  return best;
+}
+
+int grid_chunk_for(int nz, long long xy_blocks, int sms, int per_sm) {
+  if (nz <= 0) return 1;
+  // as many columns as resident blocks or more: whole columns (each cut costs
+  // two re-marched layers), the last wave's cut by grid_tail_split
+  if (xy_blocks >= (long long)sms * per_sm && !std::getenv("PN_GRID_KCHUNK")) {
+    const int chunks = (nz + kGridChunkMax - 1) / kGridChunkMax;
+    return (nz + chunks - 1) / chunks;
+  }
+  // (called once per launch: the last answer of the thread is kept with what it depends on)
+  struct Last {
+    int nz, sms, per_sm, len;
+    long long xy;
+  };
+  static thread_local Last last{0, 0, 0, 0, 0};
+  const bool fixed = std::getenv("PN_GRID_KCHUNK") != nullptr;
+  if (!fixed && last.nz == nz && last.xy == xy_blocks && last.sms == sms && last.per_sm == per_sm) return last.len;
+  const int len = grid_chunk_for(std::map<int, long long>{{nz, xy_blocks}}, sms, per_sm);
+  if (!fixed) last = Last{nz, sms, per_sm, len, xy_blocks};
+  return len;
 }
 
 // The blocks of a one-chunk launch run in waves of `slots`; whole columns in
@@ -457,19 +513,17 @@ void grid_tail_split(int nz, int kchunk, long long tiles, long long slots, int &
   tail_chunk = (nz + best - 1) / best;
 }
 
-int grid_chunk_layers(int precision, int nx, int ny, int nz, bool tma, int tile_rows) {
+int grid_chunk_layers(int precision, const std::map<int, long long> &tops, bool tma, int tile_rows) {
   int sms = 0, per_sm = 0;
   cudaError_t e = precision == 2 ? Setup<float, 32, 8, 0>::ensure(sms, per_sm)
                 : precision == 3 ? Setup<df64, 32, 8, 0>::ensure(sms, per_sm)
                                  : Setup<double, 32, 8, 0>::ensure(sms, per_sm);
-  if (e != cudaSuccess || nz <= 0) return std::min(std::max(nz, 1), kGridChunkMax);
-  if (!tma) tile_rows = kGridTileRows;
+  if (e != cudaSuccess) return kGridChunkMax;
   if (tma) {
     const int p = grid_tma_blocks_per_sm(precision, tile_rows);
     if (p > 0) per_sm = p;
   }
-  const long long xy = (long long)(nx / (kGridTileX - 1) + 1) * (ny / (tile_rows - 1) + 1);
-  return grid_chunk_for(nz, xy, sms, per_sm);
+  return grid_chunk_for(tops, sms, per_sm);
 }
 
 cudaError_t launch_grid_f32(const GridArgs<float> &a, int sym, cudaStream_t st) {

@@ -10,6 +10,7 @@
 #pragma once
 #include <climits>
 #include <cstdint>
+#include <map>
 #include <cuda_runtime.h>
 
 namespace pn {
@@ -161,12 +162,14 @@ constexpr int kGridTmaRowsMax = 32;   // stiffness rows the tensor-copy kernel s
 // well for the tensor-copy kernel with FP32 storage
 constexpr int kGridTileX = 32;
 constexpr int kGridTileRows = 8;  // the classic kernel's, and the default
-// cell layers per z chunk: about one wave of blocks, at least four layers,
-// at most kGridChunkMax
+// cell layers per z chunk (at most kGridChunkMax) by a cost model of the step:
+// for one solver's xy_blocks columns of nz layers, or for columns of the given
+// heights (number of columns per height; a batch's, all members together)
 int grid_chunk_for(int nz, long long xy_blocks, int sms, int per_sm);
-// cell layers per z chunk the launcher picks for this lattice, precision and
-// kernel (tma: the tensor-copy kernel of rsg_grid_tma.cu)
-int grid_chunk_layers(int precision, int nx, int ny, int nz, bool tma, int tile_rows = kGridTileRows);
+int grid_chunk_for(const std::map<int, long long> &tops, int sms, int per_sm);
+// ... with the resident blocks of this precision's kernel (tma: the
+// tensor-copy kernel of rsg_grid_tma.cu)
+int grid_chunk_layers(int precision, const std::map<int, long long> &tops, bool tma, int tile_rows = kGridTileRows);
 
 // a batch of grid-form members: argument blocks (kchunk set) and the prefix
 // of their block counts ((nx/(TX-1)+1) * (ny/(TY-1)+1) * chunks each)
