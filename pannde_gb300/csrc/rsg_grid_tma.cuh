@@ -246,11 +246,6 @@ __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity) {
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return mbar_try_wait(bar, parity) || mbar_wait_slow(bar, parity);
 }
-// the whole wait out of line (fewer registers live across it: the batch
-// kernel, which reads its arguments through global memory)
-__device__ __noinline__ bool mbar_wait_call(uint32_t bar, uint32_t parity) {
-  return mbar_try_wait(bar, parity) || mbar_wait_slow(bar, parity);
-}
 __device__ __forceinline__ void proxy_fence_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
@@ -298,14 +293,11 @@ struct Copies {
   static constexpr int ISSUER = (TY - 1) * TX;
   __device__ __forceinline__ Copies(const GridArgs<St> &a, unsigned char *smem, int bx, int by, int k0_, int k1_)
       : M(reinterpret_cast<const GridMaps *>(a.tmaps)), k0(k0_), k1(k1_), skip(a.test_skip_layer) {
-    // 128-byte aligned base.  A single launch derives it from the shared array
-    // by an offset, so that every tile pointer stays in the shared state space (shared
-    // loads and stores, 32-bit addressing: FP32 45.4 -> 47.8, double-float 18.0
-    // -> 19.3 Gcell-steps/s on the laminate).  The batch kernel, which reads its
-    // arguments through global memory, spilled with that and ran slower; it keeps
-    // the generic pointer.
-    base = BATCH ? (unsigned char *)(((uintptr_t)smem + 127) & ~(uintptr_t)127)
-                 : smem + ((128u - (smem_u32(smem) & 127u)) & 127u);
+    // 128-byte aligned base, by an offset from the shared array, so that every
+    // tile pointer stays in the shared state space (shared loads and stores,
+    // 32-bit addressing: FP32 45.4 -> 47.8, double-float 18.0 -> 19.3
+    // Gcell-steps/s on the laminate)
+    base = smem + ((128u - (smem_u32(smem) & 127u)) & 127u);
     bars = smem_u32(base + G::OFF_B);
     // tile origins of the copies (x on the 16-byte boundary)
     const int i0 = bx * (TX - 1);
@@ -507,7 +499,7 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
     }
     // ---- B: velocity of node layer k
     if (k <= k1) {
-      if (BATCH ? mbar_wait_call(bar_of(k), parity(k)) : mbar_wait(bar_of(k), parity(k))) waited = k;
+      if (mbar_wait(bar_of(k), parity(k))) waited = k;
       else fail = true;
       const Sm *Sk = reinterpret_cast<const Sm *>(sslot(k));
       auto cellv = [&](int f, int q) { return N::tval(Sk[f * SB + q]); };
@@ -858,6 +850,15 @@ __device__ __forceinline__ void f64h_block(const GridArgs<double> &a, unsigned c
   if constexpr (MODE != 2) grid_block_tma<df64d, SYM, 8, BATCH, true>(a, cp, bx, by, k1 == ktop, gxc, step);
 }
 
+// an argument block copied to shared memory by the whole block
+template <typename A>
+__device__ __forceinline__ void load_block(unsigned char *dst, const A *src) {
+  static_assert(sizeof(A) % 8 == 0, "argument blocks are copied in 8-byte words");
+  for (int w = threadIdx.x; w < (int)(sizeof(A) / 8); w += blockDim.x)
+    reinterpret_cast<unsigned long long *>(dst)[w] = __ldg(reinterpret_cast<const unsigned long long *>(src) + w);
+  __syncthreads();
+}
+
 // resident blocks per SM the FP64 form's kernel is compiled for (its register
 // cap: 3 -> 80 registers, 2 -> 128)
 #ifndef PN_F64H_MIN_BLOCKS
@@ -885,7 +886,9 @@ __global__ void __launch_bounds__(TX * 8, PN_F64H_MIN_BLOCKS)
     if (__ldg(block_start + mid) <= id) lo = mid;
     else hi = mid;
   }
-  const GridArgs<double> &a = args[lo];
+  __shared__ __align__(16) unsigned char sargs[sizeof(GridArgs<double>)];
+  load_block(sargs, args + lo);
+  const GridArgs<double> &a = *reinterpret_cast<const GridArgs<double> *>(sargs);
   const int local = id - __ldg(block_start + lo);
   const int gxc = a.nx / (TX - 1) + 1, gyc = a.ny / 7 + 1;
   f64h_block<SYM, true, MODE>(a, smem_raw, local % gxc, (local / gxc) % gyc, local / (gxc * gyc) * a.kchunk, a.kchunk, gxc,
@@ -931,7 +934,12 @@ __global__ void __launch_bounds__(TX *TY, GMinBlocks<R, TY>::v)
     if (__ldg(block_start + mid) <= id) lo = mid;
     else hi = mid;
   }
-  const GridArgs<typename GNum<R>::S> &a = args[lo];
+  // the member's argument block in shared memory: its pointers are read every
+  // layer, from global memory a load each (six brackets, FP32: 95 -> 85 us per
+  // step, with the tile pointers in the shared state space)
+  __shared__ __align__(16) unsigned char sargs[sizeof(GridArgs<typename GNum<R>::S>)];
+  load_block(sargs, args + lo);
+  const GridArgs<typename GNum<R>::S> &a = *reinterpret_cast<const GridArgs<typename GNum<R>::S> *>(sargs);
   const int local = id - __ldg(block_start + lo);
   const int gxc = a.nx / (TX - 1) + 1, gyc = a.ny / (TY - 1) + 1;
   run_block<R, SYM, TY, true>(a, smem_raw, local % gxc, (local / gxc) % gyc, local / (gxc * gyc) * a.kchunk, a.kchunk,
