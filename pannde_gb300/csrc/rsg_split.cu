@@ -44,6 +44,16 @@ template <> struct SN<float2> {
 
 constexpr int TPB = 128;
 
+// The three kernels of a step follow one another by programmatic dependent
+// launch: each may start while the one before it ends, finds its item and reads
+// the tables no step writes, and waits for the kernel before it ahead of the
+// first state value.  Both are a few thousand threads of a few memory
+// latencies each, so the launch gap and the chain of loads were all of their
+// time.  Measured with the argument blocks of the batch kernel in shared memory
+// (rsg_grid_tma.cuh): six brackets, FP32, 85 -> 77 us per step.
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // FP64 form (a.rflags set): a stored value outside the double-float range
 // puts the tile of lattice column (i, j) on the FP64 path for the next step
 // (the tensor-copy kernel's flags, rsg_grid_tma.cuh fp64_path)
@@ -71,13 +81,30 @@ __device__ void copy_velocity(const GridArgs<S> &a, int q, int step) {
   using R = typename N::R;
   const SplitCopy cp = a.copies[q];
   const int64_t cplane = (int64_t)a.pcx * a.ny;
+  wait_previous();
+  // every load of the copy is issued before its sums: a cell at a time was
+  // eight memory latencies in a row
+  S sv[8][6], vold[3];
+  const S *in[6] = {a.S_in[0], a.S_in[1], a.S_in[2], a.S_in[3], a.S_in[4], a.S_in[5]};
+#pragma unroll
+  for (int c = 0; c < 8; c++) {
+    const int64_t cell = (int64_t)(cp.k - 1 + (c >> 2)) * cplane + (int64_t)(cp.j - 1 + ((c >> 1) & 1)) * a.pcx +
+                         (cp.i - 1 + (c & 1));
+    if ((cp.mask >> c) & 1u) {
+#pragma unroll
+      for (int f = 0; f < 6; f++) sv[c][f] = in[f][cell];
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 3; c++) vold[c] = a.V_in[c][cp.v];
+  const S cfs = a.coef[cp.v];
   R x0 = R(), x5 = R(), x4 = R(), y5 = R(), y1 = R(), y3 = R(), z4 = R(), z3 = R(), z2 = R();
+#pragma unroll
   for (int c = 0; c < 8; c++) {
     if (!((cp.mask >> c) & 1u)) continue;
     const int ca = c & 1, cb = (c >> 1) & 1, cc = c >> 2;
-    const int64_t cell = (int64_t)(cp.k - 1 + cc) * cplane + (int64_t)(cp.j - 1 + cb) * a.pcx + (cp.i - 1 + ca);
-    const R s0 = N::val(a.S_in[0][cell]), s1 = N::val(a.S_in[1][cell]), s2 = N::val(a.S_in[2][cell]);
-    const R s3 = N::val(a.S_in[3][cell]), s4 = N::val(a.S_in[4][cell]), s5 = N::val(a.S_in[5][cell]);
+    const R s0 = N::val(sv[c][0]), s1 = N::val(sv[c][1]), s2 = N::val(sv[c][2]);
+    const R s3 = N::val(sv[c][3]), s4 = N::val(sv[c][4]), s5 = N::val(sv[c][5]);
     if (ca) { x0 = x0 + s0; x5 = x5 + s5; x4 = x4 + s4; } else { x0 = x0 - s0; x5 = x5 - s5; x4 = x4 - s4; }
     if (cb) { y5 = y5 + s5; y1 = y1 + s1; y3 = y3 + s3; } else { y5 = y5 - s5; y1 = y1 - s1; y3 = y3 - s3; }
     if (cc) { z4 = z4 + s4; z3 = z3 + s3; z2 = z2 + s2; } else { z4 = z4 - s4; z3 = z3 - s3; z2 = z2 - s2; }
@@ -95,11 +122,11 @@ __device__ void copy_velocity(const GridArgs<S> &a, int q, int step) {
     else if (d == 1) acc[1] = madd(w, sg, acc[1]);
     else acc[2] = madd(w, sg, acc[2]);
   }
-  const R cf = N::val(a.coef[cp.v]);
+  const R cf = N::val(cfs);
   R vn[3];
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    vn[c] = N::val(a.V_in[c][cp.v]);
+    vn[c] = N::val(vold[c]);
     if (!(cf == R())) vn[c] = madd(cf, acc[c], vn[c]);
     a.V_out[c][cp.v] = N::sto(vn[c]);
     flag_range(a, N::dbl(vn[c]), cp.i, cp.j, step, false);
@@ -120,6 +147,17 @@ __device__ void fix_stress(const GridArgs<S> &a, int q, int step) {
   using N = SN<S>;
   using R = typename N::R;
   const FixCell fc = a.fix[q];
+  const S *Cm = a.ctab + 36 * (int)a.mat[fc.cell];
+  S *vo[3] = {a.V_out[0], a.V_out[1], a.V_out[2]};
+  wait_previous();
+  R acc[6];
+#pragma unroll
+  for (int k = 0; k < 6; k++) acc[k] = N::val(a.S_in[k][fc.cell]);
+  S v8[8][3];  // (as above: every load first)
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) v8[k][c] = vo[c][fc.v[k]];
   R d[3][3];  // d[axis][component]: differences of the corner velocities
 #pragma unroll
   for (int m = 0; m < 3; m++)
@@ -130,7 +168,7 @@ __device__ void fix_stress(const GridArgs<S> &a, int q, int step) {
     const int bx = (k == 1 || k == 2 || k == 5 || k == 6), by = (k == 2 || k == 3 || k == 6 || k == 7), bz = k >= 4;
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      const R v = N::val(a.V_out[c][fc.v[k]]);
+      const R v = N::val(v8[k][c]);
       d[0][c] = bx ? d[0][c] + v : d[0][c] - v;
       d[1][c] = by ? d[1][c] + v : d[1][c] - v;
       d[2][c] = bz ? d[2][c] + v : d[2][c] - v;
@@ -144,10 +182,6 @@ __device__ void fix_stress(const GridArgs<S> &a, int q, int step) {
   e[3] = madd(gz, d[2][1], gy * d[1][2]);
   e[4] = madd(gz, d[2][0], gx * d[0][2]);
   e[5] = madd(gy, d[1][0], gx * d[0][1]);
-  const S *Cm = a.ctab + 36 * (int)a.mat[fc.cell];
-  R acc[6];
-#pragma unroll
-  for (int k = 0; k < 6; k++) acc[k] = N::val(a.S_in[k][fc.cell]);
   const S *sigrow = signal_row(a, step);
   for (int ee = fc.m0; ee < fc.m1; ee++) {
     const int comp = a.cm_comp[ee];
@@ -166,13 +200,15 @@ __device__ void fix_stress(const GridArgs<S> &a, int q, int step) {
 }
 
 template <typename S>
-__global__ void __launch_bounds__(TPB) k_split_copies(const GridArgs<S> a) {
+__global__ void __launch_bounds__(TPB) k_split_copies(const __grid_constant__ GridArgs<S> a) {
+  let_next_start();
   const int q = blockIdx.x * TPB + threadIdx.x;
   if (q < a.n_copies) copy_velocity(a, q, 0);
 }
 
 template <typename S>
-__global__ void __launch_bounds__(TPB) k_split_cells(const GridArgs<S> a) {
+__global__ void __launch_bounds__(TPB) k_split_cells(const __grid_constant__ GridArgs<S> a) {
+  let_next_start();
   const int q = blockIdx.x * TPB + threadIdx.x;
   if (q < a.n_fix) fix_stress(a, q, 0);
 }
@@ -192,6 +228,7 @@ template <typename S>
 __global__ void __launch_bounds__(TPB)
     k_split_copies_batch(const GridArgs<S> *__restrict__ args, const int *__restrict__ start, int n, int total,
                          int step) {
+  let_next_start();
   const int id = blockIdx.x * TPB + threadIdx.x;
   if (id >= total) return;
   const int m = member_of(start, n, id);
@@ -202,29 +239,44 @@ template <typename S>
 __global__ void __launch_bounds__(TPB)
     k_split_cells_batch(const GridArgs<S> *__restrict__ args, const int *__restrict__ start, int n, int total,
                         int step) {
+  let_next_start();
   const int id = blockIdx.x * TPB + threadIdx.x;
   if (id >= total) return;
   const int m = member_of(start, n, id);
   fix_stress(args[m], id - __ldg(start + m), step);
 }
 
+template <typename F, typename... A>
+cudaError_t launch(F f, int items, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)((items + TPB - 1) / TPB));
+  cfg.blockDim = dim3(TPB);
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, f, args...);
+}
+
 template <typename S>
 cudaError_t split_one(const GridArgs<S> &a, cudaStream_t st) {
-  if (a.n_copies > 0) k_split_copies<S><<<(a.n_copies + TPB - 1) / TPB, TPB, 0, st>>>(a);
-  if (a.n_fix > 0) k_split_cells<S><<<(a.n_fix + TPB - 1) / TPB, TPB, 0, st>>>(a);
-  return cudaGetLastError();
+  cudaError_t e = cudaSuccess;
+  if (a.n_copies > 0) e = launch(k_split_copies<S>, a.n_copies, st, a);
+  if (e == cudaSuccess && a.n_fix > 0) e = launch(k_split_cells<S>, a.n_fix, st, a);
+  return e;
 }
 
 template <typename S>
 cudaError_t split_batch(const GridSplitBatch &b, int step, cudaStream_t st) {
   const GridArgs<S> *args = (const GridArgs<S> *)b.args;
-  if (b.total_copies > 0)
-    k_split_copies_batch<S><<<(b.total_copies + TPB - 1) / TPB, TPB, 0, st>>>(args, b.copy_start, b.n_members,
-                                                                              b.total_copies, step);
-  if (b.total_fix > 0)
-    k_split_cells_batch<S><<<(b.total_fix + TPB - 1) / TPB, TPB, 0, st>>>(args, b.fix_start, b.n_members,
-                                                                         b.total_fix, step);
-  return cudaGetLastError();
+  cudaError_t e = cudaSuccess;
+  if (b.total_copies > 0) e = launch(k_split_copies_batch<S>, b.total_copies, st, args, b.copy_start, b.n_members,
+                                     b.total_copies, step);
+  if (e == cudaSuccess && b.total_fix > 0)
+    e = launch(k_split_cells_batch<S>, b.total_fix, st, args, b.fix_start, b.n_members, b.total_fix, step);
+  return e;
 }
 
 }  // namespace
