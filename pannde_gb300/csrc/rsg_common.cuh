@@ -10,6 +10,8 @@
 //   mat      cell -> material row                      [n_cells]  int32
 //   ctab     per material: 36 stiffness entries         [n_mat][36]    T
 //            (fast forms: dt*C; exact form: C)
+// The state is never read through the read-only path (__ldg, const
+// __restrict__): a launch overlaps the kernel that writes it.
 // Sources and sensors are sparse lists sorted by element, with one [begin,end)
 // range per tile of kTile consecutive elements, so tiles without sources or
 // sensors pay nothing.
@@ -25,15 +27,15 @@ template <typename T>
 struct VelArgs {
   int32_t n_nodes;
   const int4 *__restrict__ ncc;  // [n_nodes*2]
-  T *__restrict__ V0;
-  T *__restrict__ V1;
-  T *__restrict__ V2;
-  const T *__restrict__ S0;
-  const T *__restrict__ S1;
-  const T *__restrict__ S2;
-  const T *__restrict__ S3;
-  const T *__restrict__ S4;
-  const T *__restrict__ S5;
+  T *V0;
+  T *V1;
+  T *V2;
+  const T *S0;
+  const T *S1;
+  const T *S2;
+  const T *S3;
+  const T *S4;
+  const T *S5;
   const T *__restrict__ coef;
   // spacing factors: uniform (gx,gy,gz = 0.25/h) or per node [3][n_nodes]
   // (fast forms: 0.25/d; exact form: d)
@@ -63,15 +65,15 @@ template <typename T>
 struct StressArgs {
   int32_t n_cells;
   const int4 *__restrict__ hex;  // [n_cells*2]
-  const T *__restrict__ V0;
-  const T *__restrict__ V1;
-  const T *__restrict__ V2;
-  T *__restrict__ S0;
-  T *__restrict__ S1;
-  T *__restrict__ S2;
-  T *__restrict__ S3;
-  T *__restrict__ S4;
-  T *__restrict__ S5;
+  const T *V0;
+  const T *V1;
+  const T *V2;
+  T *S0;
+  T *S1;
+  T *S2;
+  T *S3;
+  T *S4;
+  T *S5;
   const int32_t *__restrict__ mat;
   const T *__restrict__ ctab;
   T gx, gy, gz;
@@ -93,6 +95,29 @@ struct StressArgs {
 };
 
 #ifdef __CUDACC__
+// Programmatic dependent launch between the kernels of consecutive half
+// steps: launch_overlapped marks a launch that may start while the kernel
+// before it ends; such a kernel reads only tables that no step writes until
+// wait_previous, which waits for that kernel's end and its memory.
+// let_next_start: the next one may start once every block has come here.
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename F, typename... A>
+inline cudaError_t launch_overlapped(F f, dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, f, args...);
+}
+
 // signal row of a step: sigval + min(step, sig_rows-1) * sig_stride
 template <typename T>
 __device__ __forceinline__ const T *signal_row(const T *sigval, int step, int stride, int rows) {

@@ -54,7 +54,7 @@ __host__ __device__ constexpr int bwd_of(int a, int k) {
 // 0 + x is x except for x = -0: the sum of four differences is -0 only when
 // all four are, and div_spacing returns +0 for it.
 template <int A>
-__device__ __forceinline__ double sum_nc(const double *__restrict__ f, const int s[8]) {
+__device__ __forceinline__ double sum_nc(const double *f, const int s[8]) {
   double v[4];
 #pragma unroll
   for (int k = 0; k < 4; k++) {
@@ -67,7 +67,7 @@ __device__ __forceinline__ double sum_nc(const double *__restrict__ f, const int
 }
 
 template <int A>
-__device__ __forceinline__ double sum_cc(const double *__restrict__ f, const int s[8]) {
+__device__ __forceinline__ double sum_cc(const double *f, const int s[8]) {
   double v[4];
 #pragma unroll
   for (int k = 0; k < 4; k++) v[k] = f[s[fwd_of(A, k)]] - f[s[bwd_of(A, k)]];
@@ -188,15 +188,17 @@ __device__ __forceinline__ void record(const VelArgs<double> &a, int n, int step
   }
 }
 
-__global__ void __launch_bounds__(kTile) k_velocity_exact(const VelArgs<double> a, int step) {
+__global__ void __launch_bounds__(kTile) k_velocity_exact(const __grid_constant__ VelArgs<double> a, int step) {
+  let_next_start();
   const int n = blockIdx.x * kTile + threadIdx.x;
   if (n >= a.n_nodes) return;
   const double cf = a.coef[n];
+  const int4 lo = a.ncc[2 * n], hi = a.ncc[2 * n + 1];
+  wait_previous();  // (tables only so far)
   if (cf == 0.) {  // node owned by another partition: not updated, still recorded
     record(a, n, step, a.V0[n], a.V1[n], a.V2[n]);
     return;
   }
-  const int4 lo = a.ncc[2 * n], hi = a.ncc[2 * n + 1];
   const int s[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
   const int64_t ny = (int64_t)a.n_nodes + n, nz = 2 * (int64_t)a.n_nodes + n;
   Divisor dx(a.gnode[n], a.rnode, n), dy(a.gnode[ny], a.rnode, ny), dz(a.gnode[nz], a.rnode, nz);
@@ -243,7 +245,8 @@ __global__ void __launch_bounds__(kTile) k_velocity_exact(const VelArgs<double> 
 }
 
 template <int SYM, bool MOMENTS>
-__global__ void __launch_bounds__(kTile) k_stress_exact(const StressArgs<double> a, int step) {
+__global__ void __launch_bounds__(kTile) k_stress_exact(const __grid_constant__ StressArgs<double> a, int step) {
+  let_next_start();
   const int c = blockIdx.x * kTile + threadIdx.x;
   if (c >= a.n_cells) return;
   const int4 lo = a.hex[2 * c], hi = a.hex[2 * c + 1];
@@ -251,6 +254,7 @@ __global__ void __launch_bounds__(kTile) k_stress_exact(const StressArgs<double>
   const int64_t cy = (int64_t)a.n_cells + c, cz = 2 * (int64_t)a.n_cells + c;
   Divisor dx(a.gcell[c], a.rcell, c), dy(a.gcell[cy], a.rcell, cy), dz(a.gcell[cz], a.rcell, cz);
   const double *V[3] = {a.V0, a.V1, a.V2};
+  wait_previous();  // (tables only so far)
   // v[j][i], d[j][i]: velocity component j along axis i
   double v[3][3], d[3][3];
 #pragma unroll
@@ -318,23 +322,16 @@ __global__ void __launch_bounds__(kTile) k_stress_exact(const StressArgs<double>
 cudaError_t launch_velocity_exact(const VelArgs<double> &a, int step, cudaStream_t st) {
   if (a.n_nodes <= 0) return cudaSuccess;
   const unsigned grid = (unsigned)((a.n_nodes + kTile - 1) / kTile);
-  k_velocity_exact<<<grid, kTile, 0, st>>>(a, step);
-  return cudaGetLastError();
+  return launch_overlapped(k_velocity_exact, dim3(grid), kTile, 0, st, a, step);
 }
 
 cudaError_t launch_stress_exact(const StressArgs<double> &a, int step, cudaStream_t st) {
   if (a.n_cells <= 0) return cudaSuccess;
   const unsigned grid = (unsigned)((a.n_cells + kTile - 1) / kTile);
-  if (a.has_moments) {
-    if (a.sym == 2) k_stress_exact<2, true><<<grid, kTile, 0, st>>>(a, step);
-    else if (a.sym == 1) k_stress_exact<1, true><<<grid, kTile, 0, st>>>(a, step);
-    else k_stress_exact<0, true><<<grid, kTile, 0, st>>>(a, step);
-  } else {
-    if (a.sym == 2) k_stress_exact<2, false><<<grid, kTile, 0, st>>>(a, step);
-    else if (a.sym == 1) k_stress_exact<1, false><<<grid, kTile, 0, st>>>(a, step);
-    else k_stress_exact<0, false><<<grid, kTile, 0, st>>>(a, step);
-  }
-  return cudaGetLastError();
+  auto run = [&](auto kernel) { return launch_overlapped(kernel, dim3(grid), kTile, 0, st, a, step); };
+  if (a.has_moments)
+    return a.sym == 2 ? run(k_stress_exact<2, true>) : a.sym == 1 ? run(k_stress_exact<1, true>) : run(k_stress_exact<0, true>);
+  return a.sym == 2 ? run(k_stress_exact<2, false>) : a.sym == 1 ? run(k_stress_exact<1, false>) : run(k_stress_exact<0, false>);
 }
 
 }  // namespace pn

@@ -105,28 +105,29 @@ template <typename R> __device__ __forceinline__ void diff_yz(const R f[8], R &d
 }
 
 template <typename R>
-__device__ __forceinline__ void gather_slots(const typename Num<R>::S *__restrict__ f, const int s[8],
+__device__ __forceinline__ void gather_slots(const typename Num<R>::S *f, const int s[8],
                                              R out[8]) {
 #pragma unroll
-  for (int k = 0; k < 8; k++) out[k] = (s[k] >= 0) ? Num<R>::ld(f, s[k]) : R();
+  for (int k = 0; k < 8; k++) out[k] = (s[k] >= 0) ? Num<R>::get(f, s[k]) : R();
 }
 
 template <typename R>
-__device__ __forceinline__ void gather_nodes(const typename Num<R>::S *__restrict__ f, const int s[8],
+__device__ __forceinline__ void gather_nodes(const typename Num<R>::S *f, const int s[8],
                                              R out[8]) {
 #pragma unroll
-  for (int k = 0; k < 8; k++) out[k] = Num<R>::ld(f, s[k]);
+  for (int k = 0; k < 8; k++) out[k] = Num<R>::get(f, s[k]);
 }
 
 // velocity update of node n (tile = n / kTile, step within the call)
-template <typename R, bool UNIFORM>
+template <typename R, bool UNIFORM, bool OVERLAP = false>
 __device__ __forceinline__ void velocity_node(const VelArgs<typename Num<R>::S> &a, int n, int tile,
                                               int step) {
   using N = Num<R>;
   const R cf = N::get(a.coef, n);
+  const int4 lo = a.ncc[2 * n], hi = a.ncc[2 * n + 1];
+  if (OVERLAP) wait_previous();  // (tables only so far)
   R v0 = N::get(a.V0, n), v1 = N::get(a.V1, n), v2 = N::get(a.V2, n);
   if (!(cf == R())) {  // a zero coefficient marks a node owned by another partition
-    const int4 lo = a.ncc[2 * n], hi = a.ncc[2 * n + 1];
     const int s[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
     R gx = N::val(a.gx), gy = N::val(a.gy), gz = N::val(a.gz);
     if (!UNIFORM) {
@@ -227,7 +228,7 @@ __host__ __device__ constexpr bool c_used(int sym, int k, int j) {
 }
 
 // stress update of cell c
-template <typename R, bool UNIFORM, int SYM>
+template <typename R, bool UNIFORM, int SYM, bool OVERLAP = false>
 __device__ __forceinline__ void stress_cell(const StressArgs<typename Num<R>::S> &a, int c, int tile,
                                             int step) {
   using N = Num<R>;
@@ -239,6 +240,8 @@ __device__ __forceinline__ void stress_cell(const StressArgs<typename Num<R>::S>
     gy = N::get(a.gcell, a.n_cells + c);
     gz = N::get(a.gcell, 2 * a.n_cells + c);
   }
+  const typename N::S *C = a.ctab + 36 * a.mat[c];
+  if (OVERLAP) wait_previous();  // (tables only so far)
   // the 24 corner gathers are issued together, before their arithmetic (FP32
   // stress step 0.153 -> 0.136 ms on the 400 x 400 x 40 laminate)
   R f0[8], f1[8], f2[8];
@@ -257,7 +260,6 @@ __device__ __forceinline__ void stress_cell(const StressArgs<typename Num<R>::S>
   e[4] = madd(gz, d20, gx * d02);
   e[5] = madd(gy, d10, gx * d01);
 
-  const typename N::S *C = a.ctab + 36 * a.mat[c];
   typename N::S *S[6] = {a.S0, a.S1, a.S2, a.S3, a.S4, a.S5};
   R acc[6];
 #pragma unroll
@@ -285,15 +287,17 @@ __device__ __forceinline__ void stress_cell(const StressArgs<typename Num<R>::S>
 }
 
 template <typename R, bool UNIFORM>
-__global__ void __launch_bounds__(kTile) k_velocity(const VelArgs<typename Num<R>::S> a, int step) {
+__global__ void __launch_bounds__(kTile) k_velocity(const __grid_constant__ VelArgs<typename Num<R>::S> a, int step) {
+  let_next_start();
   const int n = blockIdx.x * kTile + threadIdx.x;
-  if (n < a.n_nodes) velocity_node<R, UNIFORM>(a, n, blockIdx.x, step);
+  if (n < a.n_nodes) velocity_node<R, UNIFORM, true>(a, n, blockIdx.x, step);
 }
 
 template <typename R, bool UNIFORM, int SYM>
-__global__ void __launch_bounds__(kTile) k_stress(const StressArgs<typename Num<R>::S> a, int step) {
+__global__ void __launch_bounds__(kTile) k_stress(const __grid_constant__ StressArgs<typename Num<R>::S> a, int step) {
+  let_next_start();
   const int c = blockIdx.x * kTile + threadIdx.x;
-  if (c < a.n_cells) stress_cell<R, UNIFORM, SYM>(a, c, blockIdx.x, step);
+  if (c < a.n_cells) stress_cell<R, UNIFORM, SYM, true>(a, c, blockIdx.x, step);
 }
 
 // member owning work tile t: tile_start is the members' prefix of tile counts
@@ -387,17 +391,15 @@ template <typename R>
 cudaError_t launch_vel(const VelArgs<typename Num<R>::S> &a, int step, bool uniform, cudaStream_t st) {
   if (a.n_nodes <= 0) return cudaSuccess;
   const unsigned grid = (unsigned)((a.n_nodes + kTile - 1) / kTile);
-  if (uniform) k_velocity<R, true><<<grid, kTile, 0, st>>>(a, step);
-  else k_velocity<R, false><<<grid, kTile, 0, st>>>(a, step);
-  return cudaGetLastError();
+  return uniform ? launch_overlapped(k_velocity<R, true>, dim3(grid), kTile, 0, st, a, step)
+                 : launch_overlapped(k_velocity<R, false>, dim3(grid), kTile, 0, st, a, step);
 }
 
 template <typename R, int SYM>
 cudaError_t launch_str_sym(const StressArgs<typename Num<R>::S> &a, int step, bool uniform, cudaStream_t st) {
   const unsigned grid = (unsigned)((a.n_cells + kTile - 1) / kTile);
-  if (uniform) k_stress<R, true, SYM><<<grid, kTile, 0, st>>>(a, step);
-  else k_stress<R, false, SYM><<<grid, kTile, 0, st>>>(a, step);
-  return cudaGetLastError();
+  return uniform ? launch_overlapped(k_stress<R, true, SYM>, dim3(grid), kTile, 0, st, a, step)
+                 : launch_overlapped(k_stress<R, false, SYM>, dim3(grid), kTile, 0, st, a, step);
 }
 
 template <typename R>

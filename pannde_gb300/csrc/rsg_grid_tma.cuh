@@ -119,6 +119,8 @@ struct Geo {
 //                           df64, T float2 -- loads split doubles exactly
 //                           (split_double), stores join them (join_double),
 //                           stress tiles are split in place once per layer
+// (ld reads a state value from L2: a launch overlaps the kernel that wrote it,
+// so neither a read-only load nor a line of L1 may serve it)
 struct df64d {};
 template <typename K> struct GNum;
 template <> struct GNum<float> {
@@ -126,7 +128,7 @@ template <> struct GNum<float> {
   using T = float;
   using R = float;
   static constexpr bool SPLIT = false;
-  static __device__ __forceinline__ float ld(const float *p, int64_t i) { return __ldg(p + i); }
+  static __device__ __forceinline__ float ld(const float *p, int64_t i) { return __ldcg(p + i); }
   static __device__ __forceinline__ float val(float v) { return v; }
   static __device__ __forceinline__ float tval(float v) { return v; }
   static __device__ __forceinline__ float tsto(float v) { return v; }
@@ -138,7 +140,7 @@ template <> struct GNum<double> {
   using T = double;
   using R = double;
   static constexpr bool SPLIT = false;
-  static __device__ __forceinline__ double ld(const double *p, int64_t i) { return __ldg(p + i); }
+  static __device__ __forceinline__ double ld(const double *p, int64_t i) { return __ldcg(p + i); }
   static __device__ __forceinline__ double val(double v) { return v; }
   static __device__ __forceinline__ double tval(double v) { return v; }
   static __device__ __forceinline__ double tsto(double v) { return v; }
@@ -151,7 +153,7 @@ template <> struct GNum<df64> {
   using R = df64;
   static constexpr bool SPLIT = false;
   static __device__ __forceinline__ df64 ld(const float2 *p, int64_t i) {
-    const float2 v = __ldg(p + i);
+    const float2 v = __ldcg(p + i);
     return df64(v.x, v.y);
   }
   static __device__ __forceinline__ df64 val(float2 v) { return df64(v.x, v.y); }
@@ -191,7 +193,7 @@ template <> struct GNum<df64d> {
   static __device__ __forceinline__ double join(df64 v) {
     return PN_F64H_JOIN_INT ? join_double_int(v) : join_double(v);
   }
-  static __device__ __forceinline__ df64 ld(const double *p, int64_t i) { return split_double(__ldg(p + i)); }
+  static __device__ __forceinline__ df64 ld(const double *p, int64_t i) { return split_double(__ldcg(p + i)); }
   static __device__ __forceinline__ df64 val(double v) { return split_double(v); }
   static __device__ __forceinline__ df64 tval(float2 v) { return df64(v.x, v.y); }
   static __device__ __forceinline__ float2 tsto(df64 v) { return make_float2(v.hi, v.lo); }
@@ -267,17 +269,13 @@ __device__ __forceinline__ int floor_to(int v, int m) {  // largest multiple of 
 // error word codes
 constexpr int32_t kErrWait = 1;
 
-// Programmatic dependent launch: a step's kernel may start while the one
-// before it drains (the launches carry the stream-serialization attribute); it
-// loads the tables no step writes, then waits here for the previous kernel's
-// end and its memory before it touches states, path flags or traces.  A block
-// lets the next kernel start when it reaches its last node layer: let at its
+// A step's kernel may start while the one before it drains (launch_overlapped):
+// it loads the tables no step writes, then waits before it touches states,
+// path flags or traces.  A block lets the next kernel start when it reaches its last node layer: let at its
 // start, the next kernel's waiting blocks slowed the ones still marching
 // (laminate 400 x 400 x 40, FP32: 103.3 us per step without the overlap, 106.7
 // let at the start, 100.1 here; aluminium plate 64 x 64 x 8, FP32, one layer
 // per chunk: 8.2 / 5.6 / 5.2).
-__device__ __forceinline__ void wait_previous_step() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void let_next_step_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // The block's tile copies: ring slots, barriers and the issue of one layer's
 // copies (layers [k0 - 1, k1] of tile (bx, by)).
@@ -352,7 +350,7 @@ struct Copies {
     for (int s = 0; s < G::NS; s++) mbar_init(bars + 8u * s, 1);
     mbar_init_fence();
     proxy_fence_async_smem();
-    wait_previous_step();
+    wait_previous();
 #pragma unroll
     for (int d = 0; d <= G::PD; d++)
       if (k0 - 1 + d <= k1) issue(k0 - 1 + d);
@@ -425,7 +423,7 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
     sRs[q] = (a.s_ix.id && ok) ? __ldg(a.s_ix.id + (int64_t)blk * (nz + 1) + k) : -1;
   }
   for (int q = t; q < k1 - k0; q += NT) sRm[q] = a.m_ix.id ? __ldg(a.m_ix.id + (int64_t)blk * nz + k0 + q) : -1;
-  if (!RANGE) wait_previous_step();  // (the FP64 form's blocks have waited to choose their path)
+  if (!RANGE) wait_previous();  // (the FP64 form's blocks have waited to choose their path)
   __syncthreads();
   // split the stress slot of layer L in place (df64d): each stored double
   // becomes its double-float pair, so the velocity half reads pairs; the
@@ -492,7 +490,7 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
   // one layer to the next alternate registers instead of moving
 #pragma unroll(sizeof(St) == 4 ? 2 : 1)
   for (int k = k0 - 1; k <= k1 + 1; k++) {
-    if (k == k1) let_next_step_start();
+    if (k == k1) let_next_start();
     if (t == ISSUER && k >= k0 && k + G::PD <= k1) {
       proxy_fence_async_smem();
       cp.issue(k + G::PD);
@@ -696,7 +694,7 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
               if (c_used(cls, kk, jj)) acc[kk] = madd(N::tval(Cm[6 * kk + jj]), e[jj], acc[kk]);
           }
           if constexpr (N::SPLIT)
-            store_d(a.S_out[kk], cg, add_increment(__ldg(a.S_in[kk] + cg), acc[kk]), 1);
+            store_d(a.S_out[kk], cg, add_increment(__ldcg(a.S_in[kk] + cg), acc[kk]), 1);
           else store(a.S_out[kk], cg, acc[kk], 1);
         };
         if (ortho) {
@@ -835,7 +833,7 @@ __device__ __forceinline__ void f64h_block(const GridArgs<double> &a, unsigned c
   // both paths read the same tiles: the copies start before the path is chosen
   const bool work = k0 < k1;
   if (MODE == 0 && work && threadIdx.x == cp.ISSUER) cp.start();
-  wait_previous_step();
+  wait_previous();
   const bool fp64 = fp64_path<8>(a, bx, by, k0, k1, gxc, step);
   if ((MODE == 1 && fp64) || (MODE == 2 && !fp64)) return;
   if (threadIdx.x == 0 && a.path_count) atomicAdd(a.path_count + (fp64 ? 0 : 1), 1ull);
@@ -946,23 +944,6 @@ __global__ void __launch_bounds__(TX *TY, GMinBlocks<R, TY>::v)
                               gxc, step);
 }
 
-// a step launch that may start while the previous step drains
-// (wait_previous_step)
-template <typename F, typename... A>
-cudaError_t launch_step(F f, dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, f, args...);
-}
-
 template <typename R, int SYM, int TY>
 struct SetupT {
   using St = typename GNum<R>::S;
@@ -1016,7 +997,7 @@ cudaError_t launch_t(const GridArgs<typename GNum<R>::S> &a, cudaStream_t st) {
   GridArgs<typename GNum<R>::S> b = a;
   const dim3 grid = single_grid<TY>(b, sms, per_sm);
   if (grid.x == 0) return cudaErrorInvalidValue;
-  return launch_step(k_grid_tma<R, SYM, TY>, grid, TX * TY, S::smem, st, b, 0);
+  return launch_overlapped(k_grid_tma<R, SYM, TY>, grid, TX * TY, S::smem, st, b, 0);
 }
 
 template <typename R, int SYM, int TY>
@@ -1026,7 +1007,7 @@ cudaError_t launch_batch_t(const GridBatchLaunch &b, int step, cudaStream_t st) 
   cudaError_t e = S::ensure(sms, per_sm);
   if (e != cudaSuccess) return e;
   if (b.total_blocks <= 0) return cudaSuccess;
-  return launch_step(k_grid_tma_batch<R, SYM, TY>, dim3((unsigned)b.total_blocks), TX * TY, S::smem, st,
+  return launch_overlapped(k_grid_tma_batch<R, SYM, TY>, dim3((unsigned)b.total_blocks), TX * TY, S::smem, st,
                      (const GridArgs<typename GNum<R>::S> *)b.args, b.block_start, b.order, b.n_members, step);
 }
 
@@ -1056,7 +1037,7 @@ template <int SYM, int MODE>
 cudaError_t launch_h_mode(const GridArgs<double> &b, const dim3 &grid, cudaStream_t st) {
   cudaError_t e = SetupH<SYM, MODE>::ensure();
   if (e != cudaSuccess) return e;
-  return launch_step(k_grid_tma_f64h<SYM, MODE>, grid, TX * 8, SetupH<SYM, MODE>::smem, st, b, 0);
+  return launch_overlapped(k_grid_tma_f64h<SYM, MODE>, grid, TX * 8, SetupH<SYM, MODE>::smem, st, b, 0);
 }
 
 template <int SYM>
@@ -1079,7 +1060,7 @@ template <int SYM, int MODE>
 cudaError_t launch_batch_h_mode(const GridBatchLaunch &b, int step, cudaStream_t st) {
   cudaError_t e = SetupH<SYM, MODE>::ensure();
   if (e != cudaSuccess) return e;
-  return launch_step(k_grid_tma_f64h_batch<SYM, MODE>, dim3((unsigned)b.total_blocks), TX * 8,
+  return launch_overlapped(k_grid_tma_f64h_batch<SYM, MODE>, dim3((unsigned)b.total_blocks), TX * 8,
                      SetupH<SYM, MODE>::smem, st, (const GridArgs<double> *)b.args, b.block_start, b.order, b.n_members,
                      step);
 }

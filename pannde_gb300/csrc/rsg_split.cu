@@ -17,6 +17,7 @@
 #include <cstdint>
 
 #include "df64.cuh"
+#include "rsg_common.cuh"
 #include "rsg_grid.cuh"
 
 namespace pn {
@@ -51,8 +52,6 @@ constexpr int TPB = 128;
 // latencies each, so the launch gap and the chain of loads were all of their
 // time.  Measured with the argument blocks of the batch kernel in shared memory
 // (rsg_grid_tma.cuh): six brackets, FP32, 85 -> 77 us per step.
-__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // FP64 form (a.rflags set): a stored value outside the double-float range
 // puts the tile of lattice column (i, j) on the FP64 path for the next step
@@ -248,16 +247,7 @@ __global__ void __launch_bounds__(TPB)
 
 template <typename F, typename... A>
 cudaError_t launch(F f, int items, cudaStream_t st, A... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)((items + TPB - 1) / TPB));
-  cfg.blockDim = dim3(TPB);
-  cfg.stream = st;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, f, args...);
+  return launch_overlapped(f, dim3((unsigned)((items + TPB - 1) / TPB)), TPB, 0, st, args...);
 }
 
 template <typename S>
