@@ -836,7 +836,10 @@ __device__ __forceinline__ void f64h_block(const GridArgs<double> &a, unsigned c
   wait_previous();
   const bool fp64 = fp64_path<8>(a, bx, by, k0, k1, gxc, step);
   if ((MODE == 1 && fp64) || (MODE == 2 && !fp64)) return;
-  if (threadIdx.x == 0 && a.path_count) atomicAdd(a.path_count + (fp64 ? 0 : 1), 1ull);
+  // a column cut into equal chunks counts once, the pieces of a launch's last
+  // wave (tail split) each
+  if (threadIdx.x == 0 && (k0 == 0 || a.tail_chunk > 0) && a.path_count)
+    atomicAdd(a.path_count + (fp64 ? 0 : 1), 1ull);
   if (!work) return;
   if (MODE != 0 && threadIdx.x == cp.ISSUER) cp.start();
   if constexpr (MODE != 1) {
