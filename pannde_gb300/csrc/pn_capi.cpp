@@ -448,14 +448,18 @@ int pn_solver_solve_signals(pn_solver *s, int32_t nsteps, const double *values, 
       return set_err(PN_ERR_NOT_FINITE, "non-finite signal value");
     refresh_sources(s);
     if (nsig > 0 && nsteps > 0) {
-      pn::ck(cudaStreamSynchronize(s->stream), "signal sync");
-      if (nsteps > s->sig_alloc_rows) {
-        s->release(s->d_sig);
-        s->d_sig = s->alloc<void>((size_t)nsteps * nsig * s->esz);
-        s->sig_alloc_rows = nsteps;
+      if (nsig <= pn::kSignalsHere) {  // few sources: each launch carries its step's values
+        s->call_values = values;
+      } else {
+        pn::ck(cudaStreamSynchronize(s->stream), "signal sync");
+        if (nsteps > s->sig_alloc_rows) {
+          s->release(s->d_sig);
+          s->d_sig = s->alloc<void>((size_t)nsteps * nsig * s->esz);
+          s->sig_alloc_rows = nsteps;
+        }
+        s->upload_real(s->d_sig, values, (size_t)nsteps * nsig);
+        pn::ck(cudaStreamSynchronize(s->stream), "signal upload");
       }
-      s->upload_real(s->d_sig, values, (size_t)nsteps * nsig);
-      pn::ck(cudaStreamSynchronize(s->stream), "signal upload");
       s->sig_step0 = s->step;
       s->sig_rows = nsteps;
       s->sig_hold = false;
@@ -466,10 +470,12 @@ int pn_solver_solve_signals(pn_solver *s, int32_t nsteps, const double *values, 
       run_any(s, nsteps);
     } catch (...) {
       s->caller_signals = false;
+      s->call_values = nullptr;
       s->sig_valid = false;
       throw;
     }
     s->caller_signals = false;
+    s->call_values = nullptr;
     s->sig_valid = false;  // the next plain solve evaluates the sources' own signals
     if (time_out) *time_out = s->time;
     return PN_OK;

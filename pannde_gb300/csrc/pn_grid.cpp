@@ -823,7 +823,10 @@ void run(pn_solver *s, int32_t nsteps) {
       }
       a.tmaps = grid_maps_for(s, in);
       a.flag_phase = (int32_t)((s->step + k) % 3);
-      a.sigval = nsig > 0 ? (const T *)s->d_sig + sig_row(s, k) * nsig : nullptr;
+      a.sig_here = s->call_values ? 1 : 0;
+      if (s->call_values)
+        for (int64_t q = 0; q < nsig; q++) a.sig_vals[q] = to_store<T>(s->call_values[(done + k) * nsig + q]);
+      else a.sigval = nsig > 0 ? (const T *)s->d_sig + sig_row(s, k) * nsig : nullptr;
       a.rec = s->rec_count + k;  // sigval points at this step's row (stride 0)
       pn_solver::Mark m{};
       if (s->timing) {

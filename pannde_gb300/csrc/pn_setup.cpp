@@ -92,7 +92,8 @@ void pinv_sym6(const double *a, double *out) {
 
 bool all_finite(const double *p, int64_t n) {
   bool ok = true;
-#pragma omp parallel for reduction(&& : ok) schedule(static)
+  // (waking the team costs more than a few thousand values)
+#pragma omp parallel for reduction(&& : ok) schedule(static) if (n > 16384)
   for (int64_t i = 0; i < n; i++) ok = ok && std::isfinite(p[i]);
   return ok;
 }

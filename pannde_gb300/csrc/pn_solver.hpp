@@ -131,6 +131,9 @@ struct pn_solver {
   std::vector<std::vector<uint8_t>> src_mask;  // non-empty: window given by a caller's mask
   bool src_dirty = false;
   bool caller_signals = false;  // inside pn_solver_solve_signals
+  // ... whose values each launch carries itself ([step of the call][source];
+  // null: they are in the table)
+  const double *call_values = nullptr;
 
   bool has_mask_sources() const {
     for (auto &m : src_mask)

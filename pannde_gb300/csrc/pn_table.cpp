@@ -238,8 +238,11 @@ void run(pn_solver *s, int32_t nsteps) {
     va.rec_base = s->rec_count;
     for (int32_t k = 0; k < chunk; k++) {
       if (nsig > 0) {
-        va.sigval = (const T *)s->d_sig + sig_row(s, k) * nsig;
-        sa.sigval = va.sigval;
+        va.sig_here = sa.sig_here = s->call_values ? 1 : 0;
+        if (s->call_values)
+          for (int64_t q = 0; q < nsig; q++)
+            va.sig_vals[q] = sa.sig_vals[q] = to_store<T>(s->call_values[(done + k) * nsig + q]);
+        else va.sigval = sa.sigval = (const T *)s->d_sig + sig_row(s, k) * nsig;
       }
       cudaError_t e1, e2;
       pn_solver::Mark mv{}, ms{};

@@ -23,6 +23,11 @@ namespace pn {
 
 constexpr int kTile = 256;  // elements per tile == threads per block
 
+// signal values a launch carries in its own arguments (sig_here; at most so
+// many sources): a caller's values of one step need no table on the device, and
+// so neither a copy nor a wait for the steps in flight
+constexpr int kSignalsHere = 8;
+
 template <typename T>
 struct VelArgs {
   int32_t n_nodes;
@@ -51,6 +56,8 @@ struct VelArgs {
   int32_t n_sig;
   int32_t sig_stride;            // 0 when sigval already points at this step's row
   int32_t sig_rows;
+  int32_t sig_here;              // 1: this step's values are sig_vals
+  T sig_vals[kSignalsHere];
   // sensors
   const int2 *__restrict__ tile_sens;  // [n_tiles] or null
   const int32_t *__restrict__ sens_node;
@@ -89,6 +96,8 @@ struct StressArgs {
   int32_t n_sig;
   int32_t sig_stride;
   int32_t sig_rows;
+  int32_t sig_here;
+  T sig_vals[kSignalsHere];
   int32_t has_moments;
   int32_t sym;  // symmetry class of the whole stiffness table (symmetry_class): 0 general, 1 monoclinic
                 // about z, 2 orthotropic
@@ -118,10 +127,12 @@ inline cudaError_t launch_overlapped(F f, dim3 grid, unsigned threads, size_t sm
   return cudaLaunchKernelEx(&cfg, f, args...);
 }
 
-// signal row of a step: sigval + min(step, sig_rows-1) * sig_stride
-template <typename T>
-__device__ __forceinline__ const T *signal_row(const T *sigval, int step, int stride, int rows) {
-  return sigval + (int64_t)min(step, rows - 1) * stride;
+// signal values of a step: the launch's own, or row min(step, sig_rows-1) of
+// the table (null: no sources)
+template <typename A>
+__device__ __forceinline__ auto signal_row(const A &a, int step) -> decltype(a.sigval) {
+  if (a.sig_here) return a.sig_vals;
+  return a.sigval ? a.sigval + (int64_t)min(step, a.sig_rows - 1) * a.sig_stride : nullptr;
 }
 #endif
 

@@ -206,10 +206,11 @@ __global__ void __launch_bounds__(kTile) k_velocity_exact(const __grid_constant_
   bool sourced = false;
   if (a.tile_src) {
     const int2 r = a.tile_src[blockIdx.x];
+    const double *sig = signal_row(a, 0);  // (the table's pointer is already at the step's row)
     for (int i = r.x; i < r.y; i++) {
       if (a.src_elem[i] != n) continue;
       const int code = a.src_code[i];
-      const double v = a.src_w[i] * a.sigval[code >> 2];
+      const double v = a.src_w[i] * sig[code >> 2];
       const int d = code & 3;
       if (d == 0) xd[0] = xd[0] + v;
       else if (d == 1) xd[1] = xd[1] + v;
@@ -268,10 +269,11 @@ __global__ void __launch_bounds__(kTile) k_stress_exact(const __grid_constant__ 
   double mom[6] = {0., 0., 0., 0., 0., 0.};
   if (MOMENTS && a.tile_src) {
     const int2 r = a.tile_src[blockIdx.x];
+    const double *sig = signal_row(a, 0);
     for (int i = r.x; i < r.y; i++) {
       if (a.src_elem[i] != c) continue;
       const int code = a.src_code[i];
-      const double w = a.src_w[i] * a.sigval[code >> 3];
+      const double w = a.src_w[i] * sig[code >> 3];
       const int k = code & 7;
 #pragma unroll
       for (int q = 0; q < 6; q++) if (q == k) mom[q] = mom[q] + w;

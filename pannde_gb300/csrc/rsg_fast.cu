@@ -184,7 +184,7 @@ __device__ __forceinline__ void velocity_node(const VelArgs<typename Num<R>::S> 
     }
     if (a.tile_src) {
       const int2 r = a.tile_src[tile];
-      const typename N::S *sig = signal_row(a.sigval, step, a.sig_stride, a.sig_rows);
+      const typename N::S *sig = signal_row(a, step);
       for (int i = r.x; i < r.y; i++) {
         if (a.src_elem[i] != n) continue;
         const int code = a.src_code[i];
@@ -266,7 +266,7 @@ __device__ __forceinline__ void stress_cell(const StressArgs<typename Num<R>::S>
   for (int k = 0; k < 6; k++) acc[k] = N::get(S[k], c);
   if (a.tile_src) {
     const int2 r = a.tile_src[tile];
-    const typename N::S *sig = signal_row(a.sigval, step, a.sig_stride, a.sig_rows);
+    const typename N::S *sig = signal_row(a, step);
     for (int i = r.x; i < r.y; i++) {
       if (a.src_elem[i] != c) continue;
       const int code = a.src_code[i];

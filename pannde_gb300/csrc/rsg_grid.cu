@@ -103,7 +103,7 @@ __device__ __forceinline__ void grid_block(const GridArgs<typename GNum<R>::S> &
   const int64_t nidx0 = (int64_t)j * a.pnx + i;  // node index in its layer
   const int64_t cidx0 = (int64_t)j * a.pcx + i;  // cell index in its layer
   const R gx = N::val(a.g[0]), gy = N::val(a.g[1]), gz = N::val(a.g[2]);
-  const St *sigrow = a.sigval ? a.sigval + (int64_t)min(step, a.sig_rows - 1) * a.sig_stride : nullptr;
+  const St *sigrow = signal_row(a, step);
   const int64_t rec = a.rec + step;
 
   // staged cells of this thread: tile position and validity per layer
@@ -306,7 +306,8 @@ __device__ __forceinline__ void grid_block(const GridArgs<typename GNum<R>::S> &
 }
 
 template <typename R, int TX, int TY, int SYM>
-__global__ void __launch_bounds__(TX *TY) k_grid_step(const GridArgs<typename GNum<R>::S> a, int step) {
+__global__ void __launch_bounds__(TX *TY) k_grid_step(const __grid_constant__ GridArgs<typename GNum<R>::S> a,
+                                                        int step) {
   grid_block<R, TX, TY, SYM>(a, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x, step);
 }
 

@@ -13,6 +13,8 @@
 #include <map>
 #include <cuda_runtime.h>
 
+#include "rsg_common.cuh"
+
 namespace pn {
 
 // split lattice sites (rsg_split.cu): a copy is one mesh node of a site that
@@ -73,6 +75,8 @@ struct GridArgs {
   const T *sigval;       // signal rows: row min(step, sig_rows-1) at stride sig_stride
   int32_t sig_stride;    // 0 when sigval already points at the step's row
   int32_t sig_rows;
+  int32_t sig_here;      // 1: this step's values are sig_vals
+  T sig_vals[kSignalsHere];
   // sensors, ranges per (block, node layer)
   const int2 *s_rng;
   const int32_t *s_key;  // local node

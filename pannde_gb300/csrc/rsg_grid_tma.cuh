@@ -403,7 +403,7 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
   const int64_t nidx0 = (int64_t)j * a.pnx + i;
   const int64_t cidx0 = (int64_t)j * a.pcx + i;
   const R gx = N::val(a.g[0]), gy = N::val(a.g[1]), gz = N::val(a.g[2]);
-  const St *sigrow = a.sigval ? a.sigval + (int64_t)min(step, a.sig_rows - 1) * a.sig_stride : nullptr;
+  const St *sigrow = signal_row(a, step);
   const int64_t rec = a.rec + step;
   const int oc = i0 - 1 - cp.xs_c, on = i0 - cp.xs_n, om = i0 - cp.xs_m;  // offsets in the copies
   constexpr int ISSUER = Copies<St, TY, BATCH>::ISSUER;
@@ -766,8 +766,8 @@ __device__ __forceinline__ bool fp64_path(const GridArgs<double> &a, int bx, int
     }
   }
   const int nz = a.nz;
-  if (k0 < k1 && a.sigval) {
-    const double *sigrow = a.sigval + (int64_t)min(step, a.sig_rows - 1) * a.sig_stride;
+  const double *sigrow = signal_row(a, step);
+  if (k0 < k1 && sigrow) {
     const uint32_t lo = (uint32_t)a.r_elo_s, hi = (uint32_t)a.r_ehi_s;
     auto bad = [&](double w, double sg) { return !in_df64_range(sg, lo, hi) || !in_df64_range(w * sg, lo, hi); };
     if (a.f_rng) {  // force entries of node layers k0-1 .. k1 (contiguous per block)
@@ -916,7 +916,7 @@ __device__ __forceinline__ void run_block(const GridArgs<typename GNum<R>::S> &a
 
 template <typename R, int SYM, int TY>
 __global__ void __launch_bounds__(TX *TY, GMinBlocks<R, TY>::v)
-    k_grid_tma(const GridArgs<typename GNum<R>::S> a, int step) {
+    k_grid_tma(const __grid_constant__ GridArgs<typename GNum<R>::S> a, int step) {
   extern __shared__ unsigned char smem_raw[];
   int bx, by, k0, kc, gxc;
   block_coords<TY>(a, bx, by, k0, kc, gxc);

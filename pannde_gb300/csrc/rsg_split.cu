@@ -66,11 +66,6 @@ __device__ __forceinline__ void flag_range(const GridArgs<S> &a, double v, int64
   atomicOr(a.rflags + ((a.flag_phase + step + 1) % 3) * (int64_t)gxc * gyc + blk, 0x1fu);  // the tile, every edge
 }
 
-template <typename S>
-__device__ __forceinline__ const S *signal_row(const GridArgs<S> &a, int step) {
-  return a.sigval ? a.sigval + (int64_t)min(step, a.sig_rows - 1) * a.sig_stride : nullptr;
-}
-
 // velocity of copy q: x differences of Sxx, Sxy, Sxz; y of Sxy, Syy, Syz; z of
 // Sxz, Syz, Szz over the cells the copy joins (a cell's sign along an axis is
 // + on the site's upper side)
