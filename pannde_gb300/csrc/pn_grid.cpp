@@ -423,7 +423,7 @@ void grid_create(pn_solver *s) {
                        std::max(s->r_cmax, s->r_cmax_s) > std::ldexp(1.0, 90);
   if (s->precision == PN_PREC_F64 && s->d_tmaps && s->r_elo <= s->r_ehi && s->r_elo_s <= s->r_ehi_s && !extreme) {
     const int64_t tiles = (int64_t)(g.nx / (kGridTileX - 1) + 1) * (g.ny / (kGridTileRows - 1) + 1);
-    s->d_rflags = s->alloc<uint32_t>((size_t)(3 * tiles) * sizeof(uint32_t));
+    s->d_rflags = s->alloc<uint32_t>((size_t)(kFlagPhases * tiles) * sizeof(uint32_t));
     s->d_pathcnt = s->alloc<unsigned long long>(2 * sizeof(unsigned long long));
     ck(cudaMemsetAsync(s->d_pathcnt, 0, 2 * sizeof(unsigned long long), s->stream), "memset");
     grid_reset_range_flags(s);
@@ -436,9 +436,12 @@ void grid_reset_range_flags(pn_solver *s) {
   if (!s->d_rflags) return;
   const GridMap &g = s->grid;
   const int64_t tiles = (int64_t)(g.nx / (kGridTileX - 1) + 1) * (g.ny / (kGridTileRows - 1) + 1);
-  ck(cudaMemsetAsync(s->d_rflags, 0, (size_t)(3 * tiles) * sizeof(uint32_t), s->stream), "memset");
-  ck(cudaMemsetAsync(s->d_rflags + (s->step % 3) * tiles, 0xff, (size_t)tiles * sizeof(uint32_t), s->stream),
-     "memset");  // every bit: every tile on the FP64 path
+  ck(cudaMemsetAsync(s->d_rflags, 0, (size_t)(kFlagPhases * tiles) * sizeof(uint32_t), s->stream), "memset");
+  // every bit: every tile on the FP64 path, and none taken for quiet for two
+  // steps (nothing is known of either buffer half)
+  for (int64_t p : {s->step, s->step + kFlagPhases - 1})
+    ck(cudaMemsetAsync(s->d_rflags + (p % kFlagPhases) * tiles, 0xff, (size_t)tiles * sizeof(uint32_t), s->stream),
+       "memset");
 }
 
 void grid_split_upload(pn_solver *s) {
@@ -545,7 +548,8 @@ int grid_put_state(pn_solver *s, const double *const *V, const double *const *S)
   StateRangeFlags rv{}, rs{};
   if (s->d_rflags) {  // staged: a refused state leaves the solver's flags as they were
     if (!s->d_rflags_stage) s->d_rflags_stage = s->alloc<uint32_t>((size_t)tiles * sizeof(uint32_t));
-    ck(cudaMemsetAsync(s->d_rflags_stage, 0, (size_t)tiles * sizeof(uint32_t), s->stream), "memset");
+    // (no tile is taken for quiet for two steps: kFlagNonzero in every byte)
+    ck(cudaMemsetAsync(s->d_rflags_stage, (int)kFlagNonzero, (size_t)tiles * sizeof(uint32_t), s->stream), "memset");
     rv.flags = s->d_rflags_stage;
     rv.unplaced = s->d_nonfinite + 2;
     rv.gxc = g.nx / (kGridTileX - 1) + 1;
@@ -583,8 +587,11 @@ int grid_put_state(pn_solver *s, const double *const *V, const double *const *S)
     if (bad[2]) {
       grid_reset_range_flags(s);  // a split-site copy out of range: FP64 for one step
     } else {
-      ck(cudaMemsetAsync(s->d_rflags, 0, (size_t)(3 * tiles) * sizeof(uint32_t), s->stream), "memset");
-      ck(cudaMemcpyAsync(s->d_rflags + (s->step % 3) * tiles, s->d_rflags_stage, (size_t)tiles * sizeof(uint32_t),
+      ck(cudaMemsetAsync(s->d_rflags, 0, (size_t)(kFlagPhases * tiles) * sizeof(uint32_t), s->stream), "memset");
+      ck(cudaMemsetAsync(s->d_rflags + ((s->step + kFlagPhases - 1) % kFlagPhases) * tiles, (int)kFlagNonzero,
+                         (size_t)tiles * sizeof(uint32_t), s->stream),
+         "memset");
+      ck(cudaMemcpyAsync(s->d_rflags + (s->step % kFlagPhases) * tiles, s->d_rflags_stage, (size_t)tiles * sizeof(uint32_t),
                          cudaMemcpyDeviceToDevice, s->stream),
          "range flags");
     }
@@ -782,7 +789,7 @@ void grid_args(pn_solver *s, GridArgs<T> &a) {
   a.test_skip_layer = skip && *skip ? std::atoi(skip) : kNoLayer;
   a.tile_rows = s->tile_rows;
   a.rflags = s->d_rflags;
-  a.flag_phase = (int32_t)(s->step % 3);
+  a.flag_phase = (int32_t)(s->step % kFlagPhases);
   a.r_elo = s->r_elo;
   a.r_ehi = s->r_ehi;
   a.r_elo_s = s->r_elo_s;
@@ -822,7 +829,7 @@ void run(pn_solver *s, int32_t nsteps) {
         a.S_out[c] = (T *)s->S[out][c];
       }
       a.tmaps = grid_maps_for(s, in);
-      a.flag_phase = (int32_t)((s->step + k) % 3);
+      a.flag_phase = (int32_t)((s->step + k) % kFlagPhases);
       a.sig_here = s->call_values ? 1 : 0;
       if (s->call_values)
         for (int64_t q = 0; q < nsig; q++) a.sig_vals[q] = to_store<T>(s->call_values[(done + k) * nsig + q]);

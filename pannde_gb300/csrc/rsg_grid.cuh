@@ -106,12 +106,12 @@ struct GridArgs {
   const T *cm_w;
   int32_t test_skip_layer;  // failure-path test: the layer whose copies are never issued (kNoLayer: none)
   int32_t tile_rows;        // rows TY of the 32 x TY block tile (8, or 16 with the tensor-copy kernel)
-  // FP64 form with the tensor-copy kernel: per-tile path flag words [3][tiles]
+  // FP64 form with the tensor-copy kernel: per-tile path flag words [kFlagPhases][tiles]
   // (rsg_grid_tma.cuh fp64_path) and the double-float ranges as biased double
   // exponents, [r_elo, r_ehi] for velocities and [r_elo_s, r_ehi_s] for
   // stresses and source terms; rflags null: no path choice (the other forms)
   uint32_t *rflags;
-  int32_t flag_phase;       // (step of this launch's step 0) % 3
+  int32_t flag_phase;       // (step of this launch's step 0) % kFlagPhases
   int32_t r_elo, r_ehi;
   int32_t r_elo_s, r_ehi_s;
   unsigned long long *path_count;  // [2] blocks that took the FP64 / double-float path, or null
@@ -121,6 +121,7 @@ struct GridArgs {
   // column into chunks of tail_chunk layers, chunk-major (the last partial wave
   // of whole columns would leave most SMs idle); 0: the 3D grid of kchunk chunks
   int32_t tail_from, tail_chunk;
+  int32_t fp64_chunk;  // FP64 form: layers per piece of a column on the FP64 path (0: not cut)
 };
 
 // where a thread's scan of its (block, layer) slot starts (classic kernel): the entries are
@@ -151,6 +152,11 @@ __device__ __forceinline__ int2 slot_entries(const SlotIndex &ix, int id, int tx
   return make_int2(n, n + 1);
 }
 #endif
+
+// the FP64 form's flag words rotate: read (the previous step's), written by this
+// step, being cleared for the next, and the step before the previous one's
+constexpr int kFlagPhases = 4;
+constexpr uint32_t kFlagNonzero = 0x20u;  // the tile stored a value other than zero
 
 constexpr int32_t kNoLayer = INT32_MIN;  // no layer index (layers run from -1 to nz)
 
@@ -209,9 +215,6 @@ int grid_tma_blocks_per_sm(int precision, int tile_rows = kGridTileRows);
 cudaError_t launch_grid_tma(const void *args /* GridArgs<storage type> */, int precision, int sym,
                             cudaStream_t st);
 cudaError_t launch_grid_tma_batch(const GridBatchLaunch &b, int precision, int step, cudaStream_t st);
-// kernel launches of one FP64-form step (the double-float and the FP64 blocks
-// in one launch or in two)
-int grid_tma_f64_launches();
 
 // fix-up of split sites after a step launch (rsg_split.cu): the copies'
 // velocities, then the fix cells' stresses, from the step's input buffers

@@ -403,8 +403,6 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
   const int64_t nidx0 = (int64_t)j * a.pnx + i;
   const int64_t cidx0 = (int64_t)j * a.pcx + i;
   const R gx = N::val(a.g[0]), gy = N::val(a.g[1]), gz = N::val(a.g[2]);
-  const St *sigrow = signal_row(a, step);
-  const int64_t rec = a.rec + step;
   const int oc = i0 - 1 - cp.xs_c, on = i0 - cp.xs_n, om = i0 - cp.xs_m;  // offsets in the copies
   constexpr int ISSUER = Copies<St, TY, BATCH>::ISSUER;
   auto sslot = [&](int L) { return cp.sslot(L); };
@@ -457,16 +455,20 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
   // the bits its neighbours read (1 any; 2 / 4 the first / last owned column,
   // 8 / 16 the first / last owned row -- the edges inside another tile's
   // boxes: nodes are read at the first column and row, cells at all four)
-  uint32_t oorb = 0;
+  uint32_t oorb = 0, nonzero = 0;
   const uint32_t vbits = 1u | (tx == 0 ? 2u : 0u) | (ty == 0 ? 8u : 0u);
   const uint32_t sbits = vbits | (tx == TX - 2 ? 4u : 0u) | (ty == TY - 2 ? 16u : 0u);
   // a double value into double storage (RANGE: tested against the velocity
   // range, field 0, or the stress range, field 1); generic, so that it is
   // instantiated only where called (double storage)
   auto store_d = [&](auto *p, int64_t i, double d, int field) {
-    if constexpr (RANGE)
+    if constexpr (RANGE) {
+      // (a double-float path's value other than zero is far from the subnormals: its
+      // high word shows it; -0 counts as a value)
+      nonzero |= (uint32_t)__double2hiint(d) | (N::SPLIT ? 0u : (uint32_t)__double2loint(d));
       if (!in_df64_range(d, (uint32_t)(field ? a.r_elo_s : a.r_elo), (uint32_t)(field ? a.r_ehi_s : a.r_ehi)))
         oorb |= field ? sbits : vbits;
+    }
     p[i] = d;
   };
   auto store = [&](St *p, int64_t i, R v, int field) {
@@ -550,7 +552,7 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
         const int2 fr = slot_entries<TY>(a.f_ix, sRf[k - k0 + 1], tx, ty);  // this node's force sources
         for (int e = fr.x; e < fr.y; e++) {
           const int key = __ldg(a.f_key + e);
-          const R w = N::val(a.f_w[e]), sg = N::val(sigrow[__ldg(a.f_sig + e)]);
+          const R w = N::val(a.f_w[e]), sg = N::val(signal_row(a, step)[__ldg(a.f_sig + e)]);
           const int d = key >> 16;
           if (d == 0) ax = madd(w, sg, ax);
           else if (d == 1) ay = madd(w, sg, ay);
@@ -597,6 +599,7 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
 #pragma unroll
             for (int c = 0; c < 3; c++) store(a.V_out[c], n, vn[c], 0);
           }
+          const int64_t rec = a.rec + step;
           if (rec < a.rec_cap) {
             const int2 sr = slot_entries<TY>(a.s_ix, sRs[k - k0 + 1], tx, ty);
             for (int e = sr.x; e < sr.y; e++) {  // sensor traces
@@ -666,7 +669,7 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
         const int2 mr = slot_entries<TY>(a.m_ix, sRm[kc - k0], tx, ty);  // this cell's moments
         for (int ee = mr.x; ee < mr.y; ee++) {
           const int key = __ldg(a.m_key + ee);
-          const R w = N::val(a.m_w[ee]), sg = N::val(sigrow[__ldg(a.m_sig + ee)]);
+          const R w = N::val(a.m_w[ee]), sg = N::val(signal_row(a, step)[__ldg(a.m_sig + ee)]);
           const int kk = key >> 16;
 #pragma unroll
           for (int f = 0; f < 6; f++)
@@ -731,9 +734,13 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
     }
   }
   if constexpr (RANGE) {  // values left the double-float range: mark the tile (and its edges)
+    if (a.fp64_chunk > 0) {  // values other than zero are told from zeros (fp64_path)
+      oorb = __reduce_or_sync(0xffffffffu, oorb | (nonzero ? kFlagNonzero : 0u));
+      if (tx != 0) oorb = 0;
+    }
     if (oorb) {
       const int nt = gxc * (a.ny / (TY - 1) + 1);
-      atomicOr(a.rflags + ((a.flag_phase + step + 1) % 3) * nt + blk, oorb);
+      atomicOr(a.rflags + ((a.flag_phase + step + 1) % kFlagPhases) * nt + blk, oorb);
     }
   }
 }
@@ -745,25 +752,48 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
 // its first node and cell column for the tile on its left, rows likewise, and
 // a corner for a diagonal neighbour: both edge bits), or when one of this
 // step's source terms of its layers lies outside the range; the double-float
-// path (df64d) otherwise.  Flags rotate through three per-tile words: read
-// (flag_phase + step) % 3, or-ed by this step's blocks (+1), cleared for the
-// step after next by each tile's first chunk (+2).  Block-uniform.
+// path (df64d) otherwise.  Flags rotate through four per-tile words: read
+// (flag_phase + step) % 4, or-ed by this step's blocks (+1), cleared for the
+// step after next by each tile's first chunk (+2), and the step before the
+// previous one's (+3).  Block-uniform.
+//
+// quiet: the chunk has nothing to do.  Neither its tile nor a neighbour stored
+// a value other than zero in the previous step, so every value the chunk reads
+// is zero; its tile stored none in the step before either, whose output buffer
+// this step writes, so what it would write (zeros) is there already; and it
+// has no source, no sensor to record and no split site (whose fix-up writes
+// outside the tiles' blocks).  Only launches of whole tall columns tell zeros
+// from values (a.fp64_chunk > 0); others mark every tile as holding values:
+// on small lattices the telling cost more (3%) than there is to save.  From rest a wave leaves most of a plate so for
+// the first hundreds of steps: laminate 400 x 400 x 40, an initial pulse of 80
+// cells' diameter, 20 steps with the state up- and downloaded 15.4 -> 14.3 ms.
 template <int TY>
 __device__ __forceinline__ bool fp64_path(const GridArgs<double> &a, int bx, int by, int k0, int k1, int gxc,
-                                          int step) {
+                                          int step, bool clear, bool &quiet) {
   constexpr int NT = TX * TY;
   const int t = threadIdx.x;
   const int gyc = a.ny / (TY - 1) + 1, nt = gxc * gyc;
   const int blk = by * gxc + bx;
-  const int phase = (a.flag_phase + step) % 3;
-  if (k0 == 0 && t == 0) a.rflags[((phase + 2) % 3) * nt + blk] = 0;
-  bool f = false;
+  const int phase = (a.flag_phase + step) % kFlagPhases;
+  const bool track = a.fp64_chunk > 0;
+  if (clear && t == 0) {
+    a.rflags[((phase + 2) % kFlagPhases) * nt + blk] = 0;
+    if (!track) atomicOr(a.rflags + ((phase + 1) % kFlagPhases) * nt + blk, kFlagNonzero);
+  }
+  bool f = false, active = !track || a.n_copies > 0 || a.n_fix > 0;
   if (t < 9) {
     const int dx = t % 3 - 1, dy = t / 3 - 1, x = bx + dx, y = by + dy;
     if (x >= 0 && x < gxc && y >= 0 && y < gyc) {
       const uint32_t m = (dx == 0 && dy == 0) ? 1u : ((dx < 0 ? 4u : dx > 0 ? 2u : 0u) | (dy < 0 ? 16u : dy > 0 ? 8u : 0u));
-      f = (a.rflags[phase * nt + y * gxc + x] & m) == m;
+      const uint32_t word = a.rflags[phase * nt + y * gxc + x];
+      f = (word & m) == m;
+      active = active || (word & kFlagNonzero) != 0;
     }
+  } else if (t == 9) {
+    active = active || (a.rflags[((phase + 3) % kFlagPhases) * nt + blk] & kFlagNonzero) != 0;
+  } else if (t == 10 && a.s_rng && k0 < k1 && a.rec + step < a.rec_cap) {
+    const int64_t r0 = (int64_t)blk * (a.nz + 1);
+    active = active || a.s_rng[r0 + k0].x < a.s_rng[r0 + k1].y;
   }
   const int nz = a.nz;
   const double *sigrow = signal_row(a, step);
@@ -773,15 +803,25 @@ __device__ __forceinline__ bool fp64_path(const GridArgs<double> &a, int bx, int
     if (a.f_rng) {  // force entries of node layers k0-1 .. k1 (contiguous per block)
       const int64_t r0 = (int64_t)blk * (nz + 1);
       const int e0 = a.f_rng[r0 + max(k0 - 1, 0)].x, e1 = a.f_rng[r0 + k1].y;
+      active = active || e0 < e1;
       for (int e = e0 + t; e < e1; e += NT) f = f || bad(a.f_w[e], sigrow[a.f_sig[e]]);
     }
     if (a.m_rng) {  // moment entries of cell layers k0 .. k1-1
       const int64_t r0 = (int64_t)blk * nz;
       const int e0 = a.m_rng[r0 + k0].x, e1 = a.m_rng[r0 + k1 - 1].y;
+      active = active || e0 < e1;
       for (int e = e0 + t; e < e1; e += NT) f = f || bad(a.m_w[e], sigrow[a.m_sig[e]]);
     }
   }
-  return __syncthreads_or(f) != 0;
+  // (what makes the chunk active is known to the first warp)
+  __shared__ int any_active;
+  if (t < TX) {
+    active = __any_sync(0xffffffffu, active);
+    if (t == 0) any_active = active;
+  }
+  const bool fp64 = __syncthreads_or(f) != 0;
+  quiet = any_active == 0;
+  return fp64;
 }
 
 // tile (bx, by) and layer range [k0, k0 + kc) of this block of a single
@@ -814,42 +854,62 @@ __device__ __forceinline__ void block_coords(const GridArgs<T> &a, int &bx, int 
   }
 }
 
-// The FP64 form's kernels: MODE 0 runs each block on its path; with the two
-// paths as two launches (PN_F64H_TWO_LAUNCHES), MODE 1 runs the double-float
-// blocks and MODE 2 the FP64 ones (the other blocks return at once), so each
-// kernel gets registers for one path only.  Both launches decide alike.
-// Measured on the laminate bench step (15% FP64 blocks): one launch 0.663 ms,
-// two launches 1.049 ms -- in one launch the FP64 blocks share the SMs with
-// double-float ones and the two pipes work at once; alone, the FP64 blocks
-// are a serial tail on a few SMs.  One launch is the default.
-#ifndef PN_F64H_TWO_LAUNCHES
-#define PN_F64H_TWO_LAUNCHES 0
-#endif
-template <int SYM, bool BATCH, int MODE>
+// The FP64 form's blocks, on the path each takes.  Both paths run in one launch:
+// FP64 blocks share the SMs with double-float ones and the two pipes work at
+// once (as two launches, one per path, the FP64 blocks were a serial tail: 1.049
+// against 0.663 ms on the laminate's first steps).
+//
+// An FP64 column is still the step's longest block: it has an SM's FP64 pipe for
+// 290 us when the laminate's 40 layers take it alone, against about 100 us of a
+// double-float one.  piece >= 0: the block belongs to a whole column that is cut
+// only if it takes the FP64 path, into pieces of a.fp64_chunk layers, one block
+// each; on the double-float path piece 0 marches the column and the other
+// pieces' blocks end.  Every piece's block decides alike, over the column.
+// piece < 0: a chunk [k0, k0 + kc) of its own.
+template <int SYM, bool BATCH>
 __device__ __forceinline__ void f64h_block(const GridArgs<double> &a, unsigned char *smem, int bx, int by, int k0,
-                                           int kc, int gxc, int step) {
-  const int ktop = tile_top(a, by * gxc + bx), k1 = min(ktop, k0 + kc);
-  const Copies<double, 8, BATCH> cp(a, smem, bx, by, k0, k1);
+                                           int kc, int piece, int gxc, int step) {
+  const int ktop = tile_top(a, by * gxc + bx);
+  const bool column = piece >= 0;
+  Copies<double, 8, BATCH> cp(a, smem, bx, by, column ? 0 : k0, column ? ktop : min(ktop, k0 + kc));
   // both paths read the same tiles: the copies start before the path is chosen
-  const bool work = k0 < k1;
-  if (MODE == 0 && work && threadIdx.x == cp.ISSUER) cp.start();
+  const bool work = cp.k0 < cp.k1, first = piece <= 0;
+  if (work && first && threadIdx.x == cp.ISSUER) cp.start();
   wait_previous();
-  const bool fp64 = fp64_path<8>(a, bx, by, k0, k1, gxc, step);
-  if ((MODE == 1 && fp64) || (MODE == 2 && !fp64)) return;
-  // a column cut into equal chunks counts once, the pieces of a launch's last
-  // wave (tail split) each
-  if (threadIdx.x == 0 && (k0 == 0 || a.tail_chunk > 0) && a.path_count)
+  bool quiet;
+  const bool fp64 = fp64_path<8>(a, bx, by, cp.k0, cp.k1, gxc, step, first && k0 == 0, quiet);
+  // a column cut into equal chunks or FP64 pieces counts once, the chunks of a
+  // launch's last wave (tail split) each
+  if (threadIdx.x == 0 && first && (k0 == 0 || a.tail_chunk > 0) && a.path_count)
     atomicAdd(a.path_count + (fp64 ? 0 : 1), 1ull);
   if (!work) return;
-  if (MODE != 0 && threadIdx.x == cp.ISSUER) cp.start();
-  if constexpr (MODE != 1) {
-    if (fp64) {
-      grid_block_tma<double, SYM, 8, BATCH, true>(a, cp, bx, by, k1 == ktop, gxc, step);
-      return;
+  if (quiet) {  // (the copies already under way land before the block ends)
+    if (first && threadIdx.x == cp.ISSUER) {
+      bool ok = true;
+      for (int L = cp.k0 - 1; L <= min(cp.k1, cp.k0 - 1 + Geo<8, 8>::PD); L++)
+        ok = mbar_wait(cp.bar_of(L), cp.parity(L)) && ok;
+      if (!ok && a.err) atomicExch(a.err, kErrWait);
     }
+    return;
   }
-  if constexpr (MODE != 2) grid_block_tma<df64d, SYM, 8, BATCH, true>(a, cp, bx, by, k1 == ktop, gxc, step);
+  if (column) {
+    if (!fp64 && !first) return;
+    if (fp64) {
+      cp.k0 = piece * a.fp64_chunk;
+      cp.k1 = min(ktop, cp.k0 + a.fp64_chunk);
+      if (cp.k0 >= ktop) return;
+    }
+    if (!first && threadIdx.x == cp.ISSUER) cp.start();
+  }
+  if (fp64) grid_block_tma<double, SYM, 8, BATCH, true>(a, cp, bx, by, cp.k1 == ktop, gxc, step);
+  else grid_block_tma<df64d, SYM, 8, BATCH, true>(a, cp, bx, by, cp.k1 == ktop, gxc, step);
 }
+
+// resident blocks per SM the FP64 form's kernel is compiled for (its register
+// cap: 3 -> 80 registers, 2 -> 128)
+#ifndef PN_F64H_MIN_BLOCKS
+#define PN_F64H_MIN_BLOCKS 3
+#endif
 
 // an argument block copied to shared memory by the whole block
 template <typename A>
@@ -860,22 +920,38 @@ __device__ __forceinline__ void load_block(unsigned char *dst, const A *src) {
   __syncthreads();
 }
 
-// resident blocks per SM the FP64 form's kernel is compiled for (its register
-// cap: 3 -> 80 registers, 2 -> 128)
-#ifndef PN_F64H_MIN_BLOCKS
-#define PN_F64H_MIN_BLOCKS 3
-#endif
-
-template <int SYM, int MODE>
+template <int SYM>
 __global__ void __launch_bounds__(TX * 8, PN_F64H_MIN_BLOCKS)
     k_grid_tma_f64h(const __grid_constant__ GridArgs<double> a, int step) {
   extern __shared__ unsigned char smem_raw[];
-  int bx, by, k0, kc, gxc;
-  block_coords<8>(a, bx, by, k0, kc, gxc);
-  f64h_block<SYM, false, MODE>(a, smem_raw, bx, by, k0, kc, gxc, step);
+  int bx, by, k0, kc, piece = -1, gxc;
+  if (a.fp64_chunk > 0) {
+    // whole columns (of all tiles, or of those before the tail split's), their
+    // further pieces, then the tail's chunks
+    gxc = a.nx / (TX - 1) + 1;
+    const int tiles = gxc * (a.ny / 7 + 1), cols = a.tail_chunk > 0 ? a.tail_from : tiles;
+    const int id = blockIdx.x, pieces = (a.nz + a.fp64_chunk - 1) / a.fp64_chunk;
+    int tile;
+    k0 = 0;
+    kc = a.kchunk;
+    if (id < cols * pieces) {
+      piece = id / cols;
+      tile = id % cols;
+    } else {
+      const int rest = tiles - cols, j = id - cols * pieces;
+      tile = cols + j % rest;
+      k0 = (j / rest) * a.tail_chunk;
+      kc = a.tail_chunk;
+    }
+    bx = tile % gxc;
+    by = tile / gxc;
+  } else {
+    block_coords<8>(a, bx, by, k0, kc, gxc);
+  }
+  f64h_block<SYM, false>(a, smem_raw, bx, by, k0, kc, piece, gxc, step);
 }
 
-template <int SYM, int MODE>
+template <int SYM>
 __global__ void __launch_bounds__(TX * 8, PN_F64H_MIN_BLOCKS)
     k_grid_tma_f64h_batch(const GridArgs<double> *__restrict__ args, const int *__restrict__ block_start,
                           const int *__restrict__ order, int n_members, int step) {
@@ -892,8 +968,8 @@ __global__ void __launch_bounds__(TX * 8, PN_F64H_MIN_BLOCKS)
   const GridArgs<double> &a = *reinterpret_cast<const GridArgs<double> *>(sargs);
   const int local = id - __ldg(block_start + lo);
   const int gxc = a.nx / (TX - 1) + 1, gyc = a.ny / 7 + 1;
-  f64h_block<SYM, true, MODE>(a, smem_raw, local % gxc, (local / gxc) % gyc, local / (gxc * gyc) * a.kchunk, a.kchunk, gxc,
-                              step);
+  f64h_block<SYM, true>(a, smem_raw, local % gxc, (local / gxc) % gyc, local / (gxc * gyc) * a.kchunk, a.kchunk, -1, gxc,
+                        step);
 }
 
 // minimum blocks per SM each storage type is compiled for (the register cap
@@ -1015,7 +1091,7 @@ cudaError_t launch_batch_t(const GridBatchLaunch &b, int step, cudaStream_t st) 
 }
 
 // the FP64 form's kernels (k_grid_tma_f64h*): the FP64 path's shared-memory geometry
-template <int SYM, int MODE>
+template <int SYM>
 struct SetupH {
   static constexpr size_t smem = Geo<8, 8>::SMEM;
   static cudaError_t ensure() {
@@ -1025,9 +1101,9 @@ struct SetupH {
     if (e != cudaSuccess) return e;
     const int d = dev & 63;
     if (!(done & (1ull << d))) {
-      e = cudaFuncSetAttribute(k_grid_tma_f64h<SYM, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      e = cudaFuncSetAttribute(k_grid_tma_f64h<SYM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_grid_tma_f64h_batch<SYM, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        e = cudaFuncSetAttribute(k_grid_tma_f64h_batch<SYM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem);
       if (e != cudaSuccess) return e;
       done |= 1ull << d;
@@ -1036,47 +1112,38 @@ struct SetupH {
   }
 };
 
-template <int SYM, int MODE>
-cudaError_t launch_h_mode(const GridArgs<double> &b, const dim3 &grid, cudaStream_t st) {
-  cudaError_t e = SetupH<SYM, MODE>::ensure();
-  if (e != cudaSuccess) return e;
-  return launch_overlapped(k_grid_tma_f64h<SYM, MODE>, grid, TX * 8, SetupH<SYM, MODE>::smem, st, b, 0);
-}
-
+// FP64 pieces (f64h_block): columns of 16 layers and more, cut into three
+// pieces of at least eight layers (a piece re-marches two layers and starts its
+// own copies), where the launch has whole columns.  Laminate 400 x 400 x 40,
+// an initial pulse and a transducer, 20 steps with the state up- and
+// downloaded: 14.0 ms uncut, 12.5 / 11.4 / 11.8 in 2 / 3 / 5 pieces; a state that
+// is all double-float pays 1% for the further pieces' blocks.
 template <int SYM>
 cudaError_t launch_h(const GridArgs<double> &a, cudaStream_t st) {
   int sms = 0, per_sm = 0;
   cudaError_t e = SetupT<double, SYM, 8>::ensure(sms, per_sm);
+  if (e == cudaSuccess) e = SetupH<SYM>::ensure();
   if (e != cudaSuccess) return e;
   GridArgs<double> b = a;
-  const dim3 grid = single_grid<8>(b, sms, per_sm);
+  dim3 grid = single_grid<8>(b, sms, per_sm);
   if (grid.x == 0) return cudaErrorInvalidValue;
-  if constexpr (PN_F64H_TWO_LAUNCHES != 0) {
-    e = launch_h_mode<SYM, 1>(b, grid, st);
-    return e == cudaSuccess ? launch_h_mode<SYM, 2>(b, grid, st) : e;
-  } else {
-    return launch_h_mode<SYM, 0>(b, grid, st);
+  b.fp64_chunk = 0;
+  if (b.kchunk >= b.nz && b.nz >= 16) {
+    b.fp64_chunk = std::max(8, (b.nz + 2) / 3);
+    const unsigned pieces = (unsigned)((b.nz + b.fp64_chunk - 1) / b.fp64_chunk);
+    const unsigned cols = b.tail_chunk > 0 ? (unsigned)b.tail_from : grid.x * grid.y;
+    grid = dim3((b.tail_chunk > 0 ? grid.x : cols) + cols * (pieces - 1));
   }
-}
-
-template <int SYM, int MODE>
-cudaError_t launch_batch_h_mode(const GridBatchLaunch &b, int step, cudaStream_t st) {
-  cudaError_t e = SetupH<SYM, MODE>::ensure();
-  if (e != cudaSuccess) return e;
-  return launch_overlapped(k_grid_tma_f64h_batch<SYM, MODE>, dim3((unsigned)b.total_blocks), TX * 8,
-                     SetupH<SYM, MODE>::smem, st, (const GridArgs<double> *)b.args, b.block_start, b.order, b.n_members,
-                     step);
+  return launch_overlapped(k_grid_tma_f64h<SYM>, grid, TX * 8, SetupH<SYM>::smem, st, b, 0);
 }
 
 template <int SYM>
 cudaError_t launch_batch_h(const GridBatchLaunch &b, int step, cudaStream_t st) {
   if (b.total_blocks <= 0) return cudaSuccess;
-  if constexpr (PN_F64H_TWO_LAUNCHES != 0) {
-    const cudaError_t e = launch_batch_h_mode<SYM, 1>(b, step, st);
-    return e == cudaSuccess ? launch_batch_h_mode<SYM, 2>(b, step, st) : e;
-  } else {
-    return launch_batch_h_mode<SYM, 0>(b, step, st);
-  }
+  const cudaError_t e = SetupH<SYM>::ensure();
+  if (e != cudaSuccess) return e;
+  return launch_overlapped(k_grid_tma_f64h_batch<SYM>, dim3((unsigned)b.total_blocks), TX * 8, SetupH<SYM>::smem, st,
+                           (const GridArgs<double> *)b.args, b.block_start, b.order, b.n_members, step);
 }
 
 template <typename T> inline bool is_one(T v) { return v == T(1); }
