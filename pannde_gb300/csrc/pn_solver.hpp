@@ -326,7 +326,6 @@ int symmetry_class(const MaterialTables &mt);
 // table form (pn_table.cpp)
 // (reciprocals: with the exact form's reciprocal spacings, which it can do without)
 int64_t table_footprint(const MeshTables &m, const MaterialTables &mt, int precision, bool reciprocals = true);
-double exact_reciprocal(double d);  // of a spacing, as the exact form's kernels take it
 void table_create(pn_solver *s);
 void table_sources(pn_solver *s);
 void table_sensors(pn_solver *s, const std::vector<std::pair<int32_t, int32_t>> &sorted);

@@ -1,6 +1,5 @@
 // pn_table.cpp -- table form of the solver: any hex mesh, connectivity tables
 // on the device, two kernels per step (velocity then stress).
-#include <cmath>
 #include <cstring>
 #include <type_traits>
 
@@ -15,19 +14,8 @@ int64_t table_footprint(const MeshTables &m, const MaterialTables &mt, int preci
   int64_t need = nn * 3 * e + nc * 6 * e + nc * 32 + nn * 32 + nn * e + nc * 4 +
                  (int64_t)mt.n_mat * 36 * e;
   if (per_elem) need += nn * 3 * e + nc * 3 * e;
-  if (precision == PN_PREC_F64_EXACT && reciprocals) need += nn * 3 * e + nc * 3 * e;
+  if (precision == PN_PREC_F64_EXACT && reciprocals) need += nn * 6 * e + nc * 6 * e;
   return need;
-}
-
-// The exact form's reciprocal of a spacing d: r = RN(1 / (4 d)), negated when
-// the short quotient of rsg_exact.cu does not hold for it (2^53 |4 d r - 1| >
-// 1/2; the remainder 1 - 4 d r is exact in one FMA), 0 when 4 d is outside
-// [2^-100, 2^100].
-double exact_reciprocal(double d) {
-  const double c = 4. * d;
-  if (!(c >= 0x1p-100 && c <= 0x1p100)) return 0.;
-  const double r = 1. / c;
-  return std::fabs(std::fma(-c, r, 1.)) <= 0x1p-54 ? r : -r;
 }
 
 void table_create(pn_solver *s) {
@@ -68,25 +56,21 @@ void table_create(pn_solver *s) {
     s->upload_real(s->d_gnode, g.data(), g.size());
     s->upload_real(s->d_gcell, h.data(), h.size());
     if (exact) {
-      ck(cudaStreamSynchronize(s->stream), "create sync");  // the arrays are reused
-      const int64_t ng = (int64_t)g.size(), nh = (int64_t)h.size();
-#pragma omp parallel for schedule(static)
-      for (int64_t q = 0; q < ng; q++) g[q] = exact_reciprocal(g[q]);
-#pragma omp parallel for schedule(static)
-      for (int64_t q = 0; q < nh; q++) h[q] = exact_reciprocal(h[q]);
-      try {
-        s->d_rnode = s->alloc<void>(g.size() * e);
-        s->d_rcell = s->alloc<void>(h.size() * e);
+      try {  // two words of every element's reciprocals
+        s->d_rnode = s->alloc<void>(2 * g.size() * e);
+        s->d_rcell = s->alloc<void>(2 * h.size() * e);
       } catch (const SetupError &) {  // no room: the kernels form the reciprocals themselves
         s->release(s->d_rnode);
         s->release(s->d_rcell);
       }
       if (s->d_rcell) {
-        s->upload_real(s->d_rnode, g.data(), g.size());
-        s->upload_real(s->d_rcell, h.data(), h.size());
+        ck(launch_exact_reciprocals((const double *)s->d_gnode, (int64_t)g.size(), (double *)s->d_rnode, s->stream),
+           "reciprocals");
+        ck(launch_exact_reciprocals((const double *)s->d_gcell, (int64_t)h.size(), (double *)s->d_rcell, s->stream),
+           "reciprocals");
       }
-      ck(cudaStreamSynchronize(s->stream), "create sync");  // before the arrays go
     }
+    ck(cudaStreamSynchronize(s->stream), "create sync");  // before the arrays go
   }
   ck(cudaStreamSynchronize(s->stream), "create sync");
 }

@@ -160,6 +160,9 @@ cudaError_t launch_table_batch(const BatchLaunch &b, int precision, int step, cu
 // one or both half steps of a batch step: halves bit 0 velocity, bit 1 stress
 cudaError_t launch_table_batch_halves(const BatchLaunch &b, int precision, int step, int halves, cudaStream_t st);
 
+// rec[i], rec[i + n]: the two words of the reciprocal of spacing d[i] as the
+// exact kernels take it (rsg_exact.cu)
+cudaError_t launch_exact_reciprocals(const double *d, int64_t n, double *rec, cudaStream_t st);
 cudaError_t launch_velocity_exact(const VelArgs<double> &a, int step, cudaStream_t st);
 cudaError_t launch_stress_exact(const StressArgs<double> &a, int step, cudaStream_t st);
 

@@ -22,16 +22,17 @@
 // FP64 operations per SM per clock), so what counts is the FP64 operations per
 // element.  Three groups of them are left out where the bits allow it, and the
 // integer and FP32 pipes, idle otherwise, check that they do:
-//   divisions   (value*0.25)/d = value/(4d): three or four operations with the
-//               stored reciprocal of 4d instead of about nine (div_spacing)
+//   divisions   (value*0.25)/d = value/(4d): two operations with the stored
+//               reciprocal of 4d instead of about nine (div_spacing)
 //   zeros       0 + x and x + 0 only turn -0 into +0: done on the bits
 //   products    with entries that are zero by the material's symmetry class:
 //               each adds +0 or -0, which changes a sum only when it is -0
 //               (then, and for strains that are not finite, the cell takes the
 //               full sum)
-// 168 -> 123 and 210 -> 150 FP64-pipe instructions per node and cell
+// 168 -> 118 and 210 -> 135 FP64-pipe instructions per node and cell
 // (orthotropic rows).  Measured on an aluminium plate of 128 x 128 x 16 cells: velocity
-// step 105.5 -> 82.4 us, stress step 123.2 -> 83.4 us (FP64 pipe 82% busy).
+// step 105.5 -> 76.5 us, stress step 123.2 -> 78.6 us (FP64 pipe 80% busy; with
+// Markstein's three or four operations per quotient throughout 82.4 and 83.4).
 #include "rsg_common.cuh"
 
 namespace pn {
@@ -81,50 +82,102 @@ __device__ __forceinline__ double no_negative_zero(double x) {  // x + 0.0
 // sign and zero tests on the bits: a comparison of doubles is an FP64-pipe operation
 __device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) & 0x7fffffffffffffffll) == 0; }
 
-// One axis' divisor c = 4d with its reciprocal r = RN(1/c) (exact_reciprocal,
-// pn_table.cpp): stored negated when the divisor needs the longer quotient, 0
-// when it is outside the range below.  Without stored reciprocals (rec null: no
-// memory for them) they are formed here, at one division per axis.
+// One axis' divisor c = 4d with its reciprocal in two words, r = RN(1/c) and
+// rl = RN(1/c - r) (k_reciprocals; element i's at rec[i] and
+// rec[i + n3], n3 = 3 elements' count): r is stored negated when the divisor
+// needs the longer quotient, 0 when it is outside the range below.  Without
+// stored reciprocals (rec null: no memory for them) they are formed here, at
+// one division per axis, for the longer quotient.
 struct Divisor {
   double d, c, r, rl;
   bool lng;
-  __device__ __forceinline__ Divisor(double dd, const double *__restrict__ rec, int64_t i) : d(dd), rl(0.) {
+  __device__ __forceinline__ Divisor(double dd, const double *__restrict__ rec, int64_t i, int64_t n3) : d(dd) {
     c = __hiloint2double(__double2hiint(d) + (2 << 20), __double2loint(d));
     if (rec) {
       r = rec[i];
+      rl = rec[i + n3];
     } else {
-      r = 0.;
+      r = rl = 0.;
       if (d >= 0x1p-102 && d <= 0x1p98) {
-        r = 1. / c;
-        if (!(fabs(fma(-c, r, 1.)) <= 0x1p-54)) r = -r;
+        r = -1. / c;
+        rl = fma(c, r, 1.) * -r;
       }
     }
     lng = __double2hiint(r) < 0;
     r = fabs(r);
   }
-  __device__ __forceinline__ void low_word() {
-    if (lng) rl = fma(-c, r, 1.) * r;  // 1/c - r to about 53 bits
-  }
 };
 
-// RN(v / c) by Markstein's correction ("Computation of elementary functions on
-// the IBM RISC System/6000 processor", 1990): with r = RN(1/c), q0 an
-// approximate quotient and the exact remainder v - q0 c (one FMA), q0 + r
-// times the remainder rounds to RN(v / c) when q0 is near enough.  With E =
-// 2^53 |c r - 1| <= 1/2, q0 = RN(v r) is: |q0 - v/c| <= (1/2 + E) ulp, so the
-// remainder is exact and the value before the last rounding is off by at most
-// (1/2 + E) E 2^-53 ulp, less than the least distance ulp/2 * ulp(c)/c of v/c
-// from a rounding boundary.  For larger E (the host decides per divisor) q0
-// takes the reciprocal's low word too (LONG: |q0 - v/c| is half an ulp and a
-// term of 2^-52 ulp).  The proof needs every intermediate to be a normal
-// number: |v| in [2^-850, 2^850] and c in [2^-100, 2^100] (or r = 0); ok says
-// so.  A zero v gives +0 whatever its sign, as (0 + v) * 0.25 / d does.
+// RN(v / c) for a divisor known in advance.  q = v r + RN(v rl), rounded once by
+// the FMA, is RN(v / c) unless v / c lies within 2^-105 of itself of a rounding
+// boundary (Brisebarre, Muller and Raina, "Accelerating correctly rounded
+// floating-point division when the divisor is known in advance", 2004);
+// k_reciprocals has tried every v for which it does, and marks the divisors one
+// of them fails for (LONG).  For those the exact remainder v - q c (one FMA) times r is
+// added (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990): q is within half an ulp and a term of 2^-52
+// ulp, so the value before the last rounding is off by less than 2^-53 times
+// that, below the least distance ulp/2 * ulp(c)/c of v / c from a boundary.  Both
+// need every intermediate to be a normal number: |v| in [2^-850, 2^850] and c in
+// [2^-100, 2^100] (or r = 0); ok says so.  A zero v gives +0 whatever its sign,
+// as (0 + v) * 0.25 / d does.
 template <bool LONG>
 __device__ __forceinline__ double div_spacing(double v, const Divisor &d, bool &ok) {
   const uint32_t e = ((uint32_t)__double2hiint(v) >> 20) & 0x7ffu;
-  ok = ok && (is_zero(v) || (e - 173u) <= 1700u);
-  const double q0 = LONG ? fma(v, d.r, v * d.rl) : v * d.r;
-  return fma(fma(-q0, d.c, v), d.r, q0);
+  const bool zero = is_zero(v);
+  ok = ok && (zero || (e - 173u) <= 1700u);
+  double q = fma(v, d.r, v * d.rl);
+  if (LONG) q = fma(fma(-q, d.c, v), d.r, q);
+  return zero ? 0. : q;
+}
+
+// Whether fma(v, r, v * rl) is RN(v / c) for every v.  With V, C the 53-bit
+// integer significands of v and c, and M the odd 54-bit one of a midpoint of two
+// doubles, v / c lies within 2^-105 of itself of that midpoint only for
+// |V 2^s - M C| < 4, s = 53 for V >= C and 54 below; the difference k is not 0 (a
+// quotient is never a midpoint), and for each k M = -k / C modulo 2^s leaves a few
+// values of M to try.  (Of 200,000 random divisors 1% failed, all at |k| = 1, and
+// none at 5 <= |k| <= 200.)
+__device__ bool short_quotient(double c, double r, double rl) {
+  int ec = 0;
+  const double f = frexp(c, &ec);  // c = f 2^ec, f in [1/2, 1)
+  const uint64_t C = (uint64_t)ldexp(f, 53);
+  const double cd = (double)C, rd = ldexp(r, ec - 53), rld = ldexp(rl, ec - 53);
+  const int z = __ffsll((long long)C) - 1;
+  if (z > 2) return true;  // k would have to be a multiple of 2^z
+  const uint64_t Co = C >> z;
+  uint64_t inv = Co;  // Co^-1 modulo 2^64, by Newton's iteration
+  for (int i = 0; i < 6; i++) inv *= 2 - Co * inv;
+  for (int s = 53; s <= 54; s++)
+    for (int k = -4; k <= 4; k++) {
+      if (k == 0 || (k & ((1 << z) - 1)) != 0) continue;
+      const uint64_t step = 1ull << (s - z);  // M Co = -(k / 2^z) modulo 2^(s - z)
+      uint64_t M = (0 - (uint64_t)(int64_t)(k / (1 << z))) * inv & (step - 1);
+      for (; M < (1ull << 54); M += step) {
+        if (M < (1ull << 53) || !(M & 1)) continue;
+        const __int128 n = (__int128)M * (__int128)C + k;
+        if ((n & (((__int128)1 << s) - 1)) != 0) continue;
+        const uint64_t V = (uint64_t)(n >> s);
+        if (V < (1ull << 52) || V >= (1ull << 53)) continue;
+        const double v = (double)V;
+        if (fma(v, rd, v * rld) != v / cd) return false;
+      }
+    }
+  return true;
+}
+
+__global__ void __launch_bounds__(256) k_reciprocals(const double *__restrict__ d, int64_t n, double *__restrict__ rec) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  const double c = 4. * d[i];
+  double r = 0., rl = 0.;
+  if (c >= 0x1p-100 && c <= 0x1p100) {
+    r = 1. / c;
+    rl = fma(-c, r, 1.) / c;  // (the remainder is exact)
+    if (!short_quotient(c, r, rl)) r = -r;
+  }
+  rec[i] = r;
+  rec[i + n] = rl;
 }
 
 // q[i][a] = RN(v[i][a] / (4 d_a)): by the short quotient when every divisor of
@@ -133,9 +186,6 @@ __device__ __forceinline__ double div_spacing(double v, const Divisor &d, bool &
 __device__ __forceinline__ void divide9(const double v[3][3], Divisor &dx, Divisor &dy, Divisor &dz, double q[3][3]) {
   bool ok = !is_zero(dx.r) && !is_zero(dy.r) && !is_zero(dz.r);
   if (__any_sync(__activemask(), dx.lng || dy.lng || dz.lng)) {
-    dx.low_word();
-    dy.low_word();
-    dz.low_word();
 #pragma unroll
     for (int i = 0; i < 3; i++) {
       q[i][0] = div_spacing<true>(v[i][0], dx, ok);
@@ -200,8 +250,8 @@ __global__ void __launch_bounds__(kTile) k_velocity_exact(const __grid_constant_
     return;
   }
   const int s[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-  const int64_t ny = (int64_t)a.n_nodes + n, nz = 2 * (int64_t)a.n_nodes + n;
-  Divisor dx(a.gnode[n], a.rnode, n), dy(a.gnode[ny], a.rnode, ny), dz(a.gnode[nz], a.rnode, nz);
+  const int64_t ny = (int64_t)a.n_nodes + n, nz = 2 * (int64_t)a.n_nodes + n, n3 = 3 * (int64_t)a.n_nodes;
+  Divisor dx(a.gnode[n], a.rnode, n, n3), dy(a.gnode[ny], a.rnode, ny, n3), dz(a.gnode[nz], a.rnode, nz, n3);
   double xd[3] = {0., 0., 0.};
   bool sourced = false;
   if (a.tile_src) {
@@ -252,8 +302,8 @@ __global__ void __launch_bounds__(kTile) k_stress_exact(const __grid_constant__ 
   if (c >= a.n_cells) return;
   const int4 lo = a.hex[2 * c], hi = a.hex[2 * c + 1];
   const int s[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-  const int64_t cy = (int64_t)a.n_cells + c, cz = 2 * (int64_t)a.n_cells + c;
-  Divisor dx(a.gcell[c], a.rcell, c), dy(a.gcell[cy], a.rcell, cy), dz(a.gcell[cz], a.rcell, cz);
+  const int64_t cy = (int64_t)a.n_cells + c, cz = 2 * (int64_t)a.n_cells + c, n3 = 3 * (int64_t)a.n_cells;
+  Divisor dx(a.gcell[c], a.rcell, c, n3), dy(a.gcell[cy], a.rcell, cy, n3), dz(a.gcell[cz], a.rcell, cz, n3);
   const double *V[3] = {a.V0, a.V1, a.V2};
   wait_previous();  // (tables only so far)
   // v[j][i], d[j][i]: velocity component j along axis i
@@ -320,6 +370,12 @@ __global__ void __launch_bounds__(kTile) k_stress_exact(const __grid_constant__ 
 }
 
 }  // namespace
+
+cudaError_t launch_exact_reciprocals(const double *d, int64_t n, double *rec, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  k_reciprocals<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d, n, rec);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_velocity_exact(const VelArgs<double> &a, int step, cudaStream_t st) {
   if (a.n_nodes <= 0) return cudaSuccess;

@@ -60,10 +60,10 @@ def test_bits(cuda_device, monkeypatch, mat, values, budget):
     if budget:  # the least the form needs: no reciprocals
         with Solver(m, c, c.dt, "f64_exact", "table") as s:
             full = s.info()["device_bytes"]
-        monkeypatch.setenv("PN_HBM_BUDGET_BYTES", str(full - 24 * (m.n_nodes + m.n_cells)))
+        monkeypatch.setenv("PN_HBM_BUDGET_BYTES", str(full - 48 * (m.n_nodes + m.n_cells)))
     with Solver(m, c, c.dt, "f64_exact", "table") as s:
         if budget:
-            assert s.info()["device_bytes"] == full - 24 * (m.n_nodes + m.n_cells)
+            assert s.info()["device_bytes"] == full - 48 * (m.n_nodes + m.n_cells)
         s.set_state(V0, S0)
         s.solve(steps)
         V, S = s.get_state()
