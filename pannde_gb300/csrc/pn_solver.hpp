@@ -77,6 +77,13 @@ struct pn_solver {
 
   // table form
   int4 *d_hex = nullptr, *d_ncc = nullptr;
+  // ... or the same as patterns (Connectivity): of the nodes' cells, of the cells' nodes
+  struct Patterns {
+    int32_t *base = nullptr;
+    uint8_t *pattern = nullptr;
+    int4 *offset = nullptr;
+  };
+  Patterns n_con, c_con;
   void *d_gnode = nullptr, *d_gcell = nullptr;
   void *d_rnode = nullptr, *d_rcell = nullptr;  // exact form: reciprocals of the spacings, or null
   int32_t *d_mat = nullptr;

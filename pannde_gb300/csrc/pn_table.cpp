@@ -1,7 +1,11 @@
 // pn_table.cpp -- table form of the solver: any hex mesh, connectivity tables
 // on the device, two kernels per step (velocity then stress).
+#include <algorithm>
+#include <array>
 #include <cstring>
 #include <type_traits>
+
+#include <omp.h>
 
 #include "pn_solver.hpp"
 
@@ -18,6 +22,92 @@ int64_t table_footprint(const MeshTables &m, const MaterialTables &mt, int preci
   return need;
 }
 
+namespace {
+
+// Connectivity lists [n][8] (missing: -1) as patterns: false when there are more
+// than 256.  Runs of elements find their patterns in parallel; merged in order,
+// the numbering does not depend on the threads.
+bool find_patterns(const int32_t *list, int32_t n, hvec<int32_t> &base, hvec<uint8_t> &id, std::vector<int32_t> &offsets) {
+  constexpr int kMost = 256;
+  using Row = std::array<int32_t, 8>;
+  base.resize(n);
+  id.resize(n);
+  const int team = std::max(1, std::min(omp_get_max_threads(), (int)(n / 4096) + 1));
+  std::vector<std::vector<Row>> found((size_t)team);
+  for (auto &rows : found) rows.reserve(kMost);  // nothing is allocated inside the region
+  std::vector<char> many((size_t)team, 0);
+#pragma omp parallel for schedule(static) num_threads(team)
+  for (int r = 0; r < team; r++) {
+    const int32_t e0 = (int32_t)((int64_t)n * r / team), e1 = (int32_t)((int64_t)n * (r + 1) / team);
+    std::vector<Row> &rows = found[(size_t)r];
+    size_t last = 0;
+    for (int32_t e = e0; e < e1; e++) {
+      const int32_t *q = list + (size_t)e * 8;
+      int32_t b = -1;
+      for (int k = 0; k < 8 && b < 0; k++) b = q[k];
+      b = std::max(b, 0);
+      Row row;
+      for (int k = 0; k < 8; k++) row[k] = q[k] < 0 ? INT32_MIN : q[k] - b;
+      if (rows.empty() || rows[last] != row) {
+        last = (size_t)(std::find(rows.begin(), rows.end(), row) - rows.begin());
+        if (last == rows.size()) {
+          if (rows.size() == kMost) {
+            many[(size_t)r] = 1;
+            break;
+          }
+          rows.push_back(row);
+        }
+      }
+      base[e] = b;
+      id[e] = (uint8_t)last;
+    }
+  }
+  std::vector<Row> all;
+  std::vector<std::vector<uint8_t>> to((size_t)team);
+  for (int r = 0; r < team; r++) {
+    if (many[(size_t)r]) return false;
+    for (const Row &row : found[(size_t)r]) {
+      const size_t at = (size_t)(std::find(all.begin(), all.end(), row) - all.begin());
+      if (at == all.size()) {
+        if (all.size() == kMost) return false;
+        all.push_back(row);
+      }
+      to[(size_t)r].push_back((uint8_t)at);
+    }
+  }
+#pragma omp parallel for schedule(static) num_threads(team)
+  for (int r = 0; r < team; r++)
+    for (int32_t e = (int32_t)((int64_t)n * r / team); e < (int32_t)((int64_t)n * (r + 1) / team); e++)
+      id[e] = to[(size_t)r][id[e]];
+  offsets.clear();
+  for (const Row &row : all) offsets.insert(offsets.end(), row.begin(), row.end());
+  return true;
+}
+
+// the device's connectivity of one kind: patterns for the fast forms where they
+// suffice, else the table
+void upload_connectivity(pn_solver *s, const int32_t *list, int32_t n, int4 *&table, pn_solver::Patterns &con) {
+  hvec<int32_t> base;
+  hvec<uint8_t> id;
+  std::vector<int32_t> offsets;
+  if (s->precision != PN_PREC_F64_EXACT && n > 0 && find_patterns(list, n, base, id, offsets)) {
+    con.base = s->alloc<int32_t>((size_t)n * 4);
+    con.pattern = s->alloc<uint8_t>((size_t)n);
+    con.offset = s->alloc<int4>(offsets.size() * 4);
+    s->upload_raw(con.base, base.data(), (size_t)n * 4);
+    s->upload_raw(con.pattern, id.data(), (size_t)n);
+    s->upload_raw(con.offset, offsets.data(), offsets.size() * 4);
+    ck(cudaStreamSynchronize(s->stream), "connectivity upload");  // before the host lists go
+    return;
+  }
+  table = s->alloc<int4>((size_t)n * 32);
+  s->upload_raw(table, list, (size_t)n * 32);
+}
+
+Connectivity connectivity(const pn_solver::Patterns &p) { return Connectivity{p.base, p.pattern, p.offset}; }
+
+}  // namespace
+
 void table_create(pn_solver *s) {
   const int32_t nn = s->mesh.n_nodes, nc = s->mesh.n_cells;
   const size_t e = s->esz;
@@ -25,15 +115,13 @@ void table_create(pn_solver *s) {
   const bool per_elem = exact || !s->mesh.uniform;
   for (int k = 0; k < 3; k++) s->V[0][k] = s->alloc<void>((size_t)nn * e);
   for (int k = 0; k < 6; k++) s->S[0][k] = s->alloc<void>((size_t)nc * e);
-  s->d_hex = s->alloc<int4>((size_t)nc * 32);
-  s->d_ncc = s->alloc<int4>((size_t)nn * 32);
   s->d_coef = s->alloc<void>((size_t)nn * e);
   s->d_mat = s->alloc<int32_t>((size_t)nc * 4);
   s->d_ctab = s->alloc<void>((size_t)s->mat.n_mat * 36 * e);
   for (int k = 0; k < 3; k++) ck(cudaMemsetAsync(s->V[0][k], 0, (size_t)nn * e, s->stream), "memset");
   for (int k = 0; k < 6; k++) ck(cudaMemsetAsync(s->S[0][k], 0, (size_t)nc * e, s->stream), "memset");
-  s->upload_raw(s->d_hex, s->mesh.hex.data(), (size_t)nc * 32);
-  s->upload_raw(s->d_ncc, s->mesh.ncc.data(), (size_t)nn * 32);
+  upload_connectivity(s, s->mesh.hex.data(), nc, s->d_hex, s->c_con);
+  upload_connectivity(s, s->mesh.ncc.data(), nn, s->d_ncc, s->n_con);
   s->upload_real(s->d_coef, s->mat.coef.data(), nn);
   s->upload_raw(s->d_mat, s->mat.cell_mat.data(), (size_t)nc * 4);
   s->sym = symmetry_class(s->mat);
@@ -160,6 +248,7 @@ void table_args(pn_solver *s, VelArgs<T> &va, StressArgs<T> &sa) {
   std::memset(&sa, 0, sizeof(sa));
   va.n_nodes = s->mesh.n_nodes;
   va.ncc = s->d_ncc;
+  va.con = connectivity(s->n_con);
   T *const *V = (T *const *)s->V[0];
   T *const *S = (T *const *)s->S[0];
   va.V0 = V[0]; va.V1 = V[1]; va.V2 = V[2];
@@ -183,6 +272,7 @@ void table_args(pn_solver *s, VelArgs<T> &va, StressArgs<T> &sa) {
   }
   sa.n_cells = s->mesh.n_cells;
   sa.hex = s->d_hex;
+  sa.con = connectivity(s->c_con);
   sa.V0 = V[0]; sa.V1 = V[1]; sa.V2 = V[2];
   sa.S0 = S[0]; sa.S1 = S[1]; sa.S2 = S[2]; sa.S3 = S[3]; sa.S4 = S[4]; sa.S5 = S[5];
   sa.mat = s->d_mat;

@@ -28,10 +28,22 @@ constexpr int kTile = 256;  // elements per tile == threads per block
 // so neither a copy nor a wait for the steps in flight
 constexpr int kSignalsHere = 8;
 
+// Connectivity as patterns (fast forms): an element's eight neighbours are its
+// base plus the offsets of its pattern.  Meshes numbered along lattice lines,
+// graded, holed or cracked ones too, have a few dozen patterns (interior, faces,
+// edges, rims), so an element takes 5 bytes instead of 32; a mesh with more than
+// 256 keeps the tables.  A missing cell's offset is INT32_MIN (base + it < 0).
+struct Connectivity {
+  const int32_t *__restrict__ base;     // [elements]
+  const uint8_t *__restrict__ pattern;  // [elements], null: the table
+  const int4 *__restrict__ offset;      // [patterns * 2]
+};
+
 template <typename T>
 struct VelArgs {
   int32_t n_nodes;
   const int4 *__restrict__ ncc;  // [n_nodes*2]
+  Connectivity con;              // ... or, when con.pattern is set, as patterns
   T *V0;
   T *V1;
   T *V2;
@@ -72,6 +84,7 @@ template <typename T>
 struct StressArgs {
   int32_t n_cells;
   const int4 *__restrict__ hex;  // [n_cells*2]
+  Connectivity con;              // ... or as patterns
   const T *V0;
   const T *V1;
   const T *V2;
@@ -125,6 +138,23 @@ inline cudaError_t launch_overlapped(F f, dim3 grid, unsigned threads, size_t sm
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, f, args...);
+}
+
+// the eight neighbours of element i: by its pattern, or from the table
+__device__ __forceinline__ void neighbours(const Connectivity &con, const int4 *__restrict__ table, int i, int s[8]) {
+  int4 lo, hi;
+  int b = 0;
+  if (con.pattern) {
+    const int p = con.pattern[i];
+    b = con.base[i];
+    lo = __ldg(con.offset + 2 * p);
+    hi = __ldg(con.offset + 2 * p + 1);
+  } else {
+    lo = table[2 * i];
+    hi = table[2 * i + 1];
+  }
+  s[0] = b + lo.x; s[1] = b + lo.y; s[2] = b + lo.z; s[3] = b + lo.w;
+  s[4] = b + hi.x; s[5] = b + hi.y; s[6] = b + hi.z; s[7] = b + hi.w;
 }
 
 // signal values of a step: the launch's own, or row min(step, sig_rows-1) of

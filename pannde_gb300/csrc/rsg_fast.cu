@@ -124,11 +124,11 @@ __device__ __forceinline__ void velocity_node(const VelArgs<typename Num<R>::S> 
                                               int step) {
   using N = Num<R>;
   const R cf = N::get(a.coef, n);
-  const int4 lo = a.ncc[2 * n], hi = a.ncc[2 * n + 1];
+  int s[8];
+  neighbours(a.con, a.ncc, n, s);
   if (OVERLAP) wait_previous();  // (tables only so far)
   R v0 = N::get(a.V0, n), v1 = N::get(a.V1, n), v2 = N::get(a.V2, n);
   if (!(cf == R())) {  // a zero coefficient marks a node owned by another partition
-    const int s[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
     R gx = N::val(a.gx), gy = N::val(a.gy), gz = N::val(a.gz);
     if (!UNIFORM) {
       gx = N::get(a.gnode, n);
@@ -232,8 +232,8 @@ template <typename R, bool UNIFORM, int SYM, bool OVERLAP = false>
 __device__ __forceinline__ void stress_cell(const StressArgs<typename Num<R>::S> &a, int c, int tile,
                                             int step) {
   using N = Num<R>;
-  const int4 lo = a.hex[2 * c], hi = a.hex[2 * c + 1];
-  const int s[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+  int s[8];
+  neighbours(a.con, a.hex, c, s);
   R gx = N::val(a.gx), gy = N::val(a.gy), gz = N::val(a.gz);
   if (!UNIFORM) {
     gx = N::get(a.gcell, c);
