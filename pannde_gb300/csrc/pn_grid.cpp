@@ -145,12 +145,15 @@ void upload_index(pn_solver *s, const std::vector<Keyed> &L, const std::vector<i
     }
     if (several) node.push_back(e1);
   }
-  out.id = s->alloc<int32_t>(id.size() * 4);
-  out.rows = s->alloc<uint2>(rows.size() * 4);
-  out.node = s->alloc<int32_t>(node.size() * 4);
-  s->upload_raw(out.id, id.data(), id.size() * 4);
-  s->upload_raw(out.rows, rows.data(), rows.size() * 4);
-  s->upload_raw(out.node, node.data(), node.size() * 4);
+  // rows (8-byte entries), then id, then node
+  std::vector<uint32_t> all(rows);
+  all.insert(all.end(), id.begin(), id.end());
+  all.insert(all.end(), node.begin(), node.end());
+  uint32_t *p = s->alloc<uint32_t>(all.size() * 4);
+  s->upload_raw(p, all.data(), all.size() * 4);
+  out.rows = (uint2 *)p;
+  out.id = (int32_t *)(p + rows.size());
+  out.node = out.id + id.size();
   ck(cudaStreamSynchronize(s->stream), "slot index upload");  // before the host lists go
 }
 
@@ -609,9 +612,11 @@ void grid_get_state(pn_solver *s, double *const *V, double *const *S) {
 }
 
 void grid_sources(pn_solver *s) {
-  std::vector<SourceEntry> fe, me;
-  const std::vector<const uint8_t *> masks = s->mask_ptrs();
-  build_source_entries(s->mesh, s->src, false, fe, me, &masks);
+  std::vector<SourceEntry> &fe = s->force_entries, &me = s->moment_entries;
+  if (s->src_dirty) {  // (re-tiling comes with the sources as they were)
+    const std::vector<const uint8_t *> masks = s->mask_ptrs();
+    build_source_entries(s->mesh, s->src, false, fe, me, &masks);
+  }
   ck(cudaStreamSynchronize(s->stream), "sources sync");
   s->release(s->d_frng); s->release(s->d_fkey); s->release(s->d_fsig); s->release(s->d_fw);
   s->release(s->d_mrng); s->release(s->d_mkey); s->release(s->d_msig); s->release(s->d_mw);

@@ -78,10 +78,11 @@ struct pn_solver {
   // table form
   int4 *d_hex = nullptr, *d_ncc = nullptr;
   // ... or the same as patterns (Connectivity): of the nodes' cells, of the cells' nodes
+  // (one allocation, held by offset)
   struct Patterns {
+    int4 *offset = nullptr;
     int32_t *base = nullptr;
     uint8_t *pattern = nullptr;
-    int4 *offset = nullptr;
   };
   Patterns n_con, c_con;
   void *d_gnode = nullptr, *d_gcell = nullptr;
@@ -137,6 +138,8 @@ struct pn_solver {
   std::vector<pn::Series> series;
   std::vector<std::vector<uint8_t>> src_mask;  // non-empty: window given by a caller's mask
   bool src_dirty = false;
+  // the sources' entries, kept for re-tiling (grid form; they do not depend on the tiles)
+  std::vector<pn::SourceEntry> force_entries, moment_entries;
   bool caller_signals = false;  // inside pn_solver_solve_signals
   // ... whose values each launch carries itself ([step of the call][source];
   // null: they are in the table)
@@ -161,10 +164,11 @@ struct pn_solver {
   int2 *d_frng = nullptr, *d_mrng = nullptr;
   int32_t *d_fkey = nullptr, *d_fsig = nullptr, *d_mkey = nullptr, *d_msig = nullptr;
   void *d_fw = nullptr, *d_mw = nullptr;
-  // ... and how a thread finds its own entries of a slot (SlotIndex)
+  // ... and how a thread finds its own entries of a slot (SlotIndex; one
+  // allocation, held by rows)
   struct SlotTables {
-    int32_t *id = nullptr;
     uint2 *rows = nullptr;
+    int32_t *id = nullptr;
     int32_t *node = nullptr;
   };
   SlotTables f_slots, m_slots, s_slots;
@@ -218,9 +222,8 @@ struct pn_solver {
   }
 
   void release(SlotTables &t) {
-    release(t.id);
     release(t.rows);
-    release(t.node);
+    t = SlotTables();
   }
 
   // upload a double host array in the storage type (double, float, or the

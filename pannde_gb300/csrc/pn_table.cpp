@@ -91,12 +91,12 @@ void upload_connectivity(pn_solver *s, const int32_t *list, int32_t n, int4 *&ta
   hvec<uint8_t> id;
   std::vector<int32_t> offsets;
   if (s->precision != PN_PREC_F64_EXACT && n > 0 && find_patterns(list, n, base, id, offsets)) {
-    con.base = s->alloc<int32_t>((size_t)n * 4);
-    con.pattern = s->alloc<uint8_t>((size_t)n);
-    con.offset = s->alloc<int4>(offsets.size() * 4);
+    con.offset = s->alloc<int4>(offsets.size() * 4 + (size_t)n * 5);
+    con.base = (int32_t *)con.offset + offsets.size();
+    con.pattern = (uint8_t *)(con.base + n);
+    s->upload_raw(con.offset, offsets.data(), offsets.size() * 4);
     s->upload_raw(con.base, base.data(), (size_t)n * 4);
     s->upload_raw(con.pattern, id.data(), (size_t)n);
-    s->upload_raw(con.offset, offsets.data(), offsets.size() * 4);
     ck(cudaStreamSynchronize(s->stream), "connectivity upload");  // before the host lists go
     return;
   }
