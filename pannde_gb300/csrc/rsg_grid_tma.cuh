@@ -403,6 +403,8 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
   const int64_t nidx0 = (int64_t)j * a.pnx + i;
   const int64_t cidx0 = (int64_t)j * a.pcx + i;
   const R gx = N::val(a.g[0]), gy = N::val(a.g[1]), gz = N::val(a.g[2]);
+  // (the FP64 form's kernel, short of registers, finds its row where it is used)
+  const St *sigrow = RANGE ? nullptr : signal_row(a, step);
   const int oc = i0 - 1 - cp.xs_c, on = i0 - cp.xs_n, om = i0 - cp.xs_m;  // offsets in the copies
   constexpr int ISSUER = Copies<St, TY, BATCH>::ISSUER;
   auto sslot = [&](int L) { return cp.sslot(L); };
@@ -552,7 +554,7 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
         const int2 fr = slot_entries<TY>(a.f_ix, sRf[k - k0 + 1], tx, ty);  // this node's force sources
         for (int e = fr.x; e < fr.y; e++) {
           const int key = __ldg(a.f_key + e);
-          const R w = N::val(a.f_w[e]), sg = N::val(signal_row(a, step)[__ldg(a.f_sig + e)]);
+          const R w = N::val(a.f_w[e]), sg = N::val((RANGE ? signal_row(a, step) : sigrow)[__ldg(a.f_sig + e)]);
           const int d = key >> 16;
           if (d == 0) ax = madd(w, sg, ax);
           else if (d == 1) ay = madd(w, sg, ay);
@@ -669,7 +671,7 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
         const int2 mr = slot_entries<TY>(a.m_ix, sRm[kc - k0], tx, ty);  // this cell's moments
         for (int ee = mr.x; ee < mr.y; ee++) {
           const int key = __ldg(a.m_key + ee);
-          const R w = N::val(a.m_w[ee]), sg = N::val(signal_row(a, step)[__ldg(a.m_sig + ee)]);
+          const R w = N::val(a.m_w[ee]), sg = N::val((RANGE ? signal_row(a, step) : sigrow)[__ldg(a.m_sig + ee)]);
           const int kk = key >> 16;
 #pragma unroll
           for (int f = 0; f < 6; f++)
