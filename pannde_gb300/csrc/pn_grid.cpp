@@ -549,7 +549,12 @@ int grid_put_state(pn_solver *s, const double *const *V, const double *const *S)
   // range, which puts every tile on the FP64 path for one step instead)
   const int64_t tiles = (int64_t)(g.nx / (kGridTileX - 1) + 1) * (g.ny / (kGridTileRows - 1) + 1);
   StateRangeFlags rv{}, rs{};
-  if (s->d_rflags) {  // staged: a refused state leaves the solver's flags as they were
+  if (s->d_rflags) {  // staged: a refused state leaves the current state's flags as they were
+    // (but not the idle half's: what is written there from here on, a refused
+    // state too, is no longer what the steps before left)
+    ck(cudaMemsetAsync(s->d_rflags + ((s->step + kFlagPhases - 1) % kFlagPhases) * tiles, (int)kFlagNonzero,
+                       (size_t)tiles * sizeof(uint32_t), s->stream),
+       "memset");
     if (!s->d_rflags_stage) s->d_rflags_stage = s->alloc<uint32_t>((size_t)tiles * sizeof(uint32_t));
     // (no tile is taken for quiet for two steps: kFlagNonzero in every byte)
     ck(cudaMemsetAsync(s->d_rflags_stage, (int)kFlagNonzero, (size_t)tiles * sizeof(uint32_t), s->stream), "memset");

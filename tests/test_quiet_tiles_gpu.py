@@ -104,3 +104,27 @@ def test_reused_buffers(cuda_device, monkeypatch, how, before):
             got.append(result(s))
     for a, b in zip(list(got[0][0]) + list(got[0][1]) + [got[0][2]], list(got[1][0]) + list(got[1][1]) + [got[1][2]]):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("before", [0, 1, 2])
+def test_refused_state_leaves_nothing_behind(cuda_device, monkeypatch, before):
+    """set_state writes the idle half before it can refuse: the next step must
+    not take what that left there for its own zeros."""
+    monkeypatch.setenv("PN_GRID_KCHUNK", "64")
+    c = problem(False)
+    V0, S0 = pulse(c)
+    V1, S1 = everywhere(c)
+    V1[2] = V1[2].copy()
+    V1[2][c.mesh.n_nodes // 2] = np.nan
+    got = []
+    for refused in (False, True):
+        with Solver.from_case(c, "f64", form="grid") as s:
+            s.set_state(V0, S0)
+            s.solve(4 + before)
+            if refused:
+                with pytest.raises(N.PnError):
+                    s.set_state(V1, S1)
+            s.solve(STEPS)
+            got.append(result(s))
+    for a, b in zip(list(got[0][0]) + list(got[0][1]) + [got[0][2]], list(got[1][0]) + list(got[1][1]) + [got[1][2]]):
+        assert np.array_equal(a, b)
