@@ -201,9 +201,7 @@ typedef struct pn_solver_info {
   double time;
   int32_t form;              /* PN_FORM_TABLE or PN_FORM_GRID */
   int32_t grid[3];           /* grid form: cells per axis */
-  int32_t grid_kernel;       /* grid form: 1 classic (register prefetch), 2 tensor-copy staging, 3
-                                tensor-copy staging in the FP64 form's two launches per step (its
-                                double-float and its FP64 blocks); 0 table */
+  int32_t grid_kernel;       /* grid form: 1 classic (register prefetch), 2 tensor-copy staging; 0 table */
 } pn_solver_info;
 
 /* What pn_solver_create would build, computed on the host only. */
@@ -212,7 +210,7 @@ typedef struct pn_plan {
   int32_t n_materials;
   int32_t uniform_spacing;
   double hx, hy, hz;                  /* the spacings when uniform_spacing */
-  int64_t device_bytes;               /* device memory pn_solver_create allocates */
+  int64_t device_bytes;               /* device memory pn_solver_create allocates (table form: at most) */
   int64_t algorithmic_bytes_per_step;
   int32_t form;                       /* the form PN_FORM_AUTO would pick */
   int32_t grid[3];                    /* grid form: cells per axis */

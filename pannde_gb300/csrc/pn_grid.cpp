@@ -149,7 +149,7 @@ void upload_index(pn_solver *s, const std::vector<Keyed> &L, const std::vector<i
   std::vector<uint32_t> all(rows);
   all.insert(all.end(), id.begin(), id.end());
   all.insert(all.end(), node.begin(), node.end());
-  uint32_t *p = s->alloc<uint32_t>(all.size() * 4);
+  uint32_t *p = s->alloc<uint32_t>(all.size() * 4, all.size() * 4);
   s->upload_raw(p, all.data(), all.size() * 4);
   out.rows = (uint2 *)p;
   out.id = (int32_t *)(p + rows.size());
@@ -426,7 +426,7 @@ void grid_create(pn_solver *s) {
                        std::max(s->r_cmax, s->r_cmax_s) > std::ldexp(1.0, 90);
   if (s->precision == PN_PREC_F64 && s->d_tmaps && s->r_elo <= s->r_ehi && s->r_elo_s <= s->r_ehi_s && !extreme) {
     const int64_t tiles = (int64_t)(g.nx / (kGridTileX - 1) + 1) * (g.ny / (kGridTileRows - 1) + 1);
-    s->d_rflags = s->alloc<uint32_t>((size_t)(kFlagPhases * tiles) * sizeof(uint32_t));
+    s->d_rflags = s->alloc<uint32_t>((size_t)(kFlagPhases * tiles) * sizeof(uint32_t), (size_t)tiles * sizeof(uint32_t));
     s->d_pathcnt = s->alloc<unsigned long long>(2 * sizeof(unsigned long long));
     ck(cudaMemsetAsync(s->d_pathcnt, 0, 2 * sizeof(unsigned long long), s->stream), "memset");
     grid_reset_range_flags(s);

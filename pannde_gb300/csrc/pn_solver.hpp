@@ -66,7 +66,8 @@ struct pn_solver {
   pn::MaterialTables mat;
 
   std::vector<void *> allocs;
-  int64_t dev_bytes = 0;
+  int64_t dev_bytes = 0;        // held, the uncounted ones not among them
+  int64_t uncounted_bytes = 0;
 
   // state: V[3] over nodes, S[6] over cells (grid form: buffer `cur` of two)
   void *V[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
@@ -195,21 +196,38 @@ struct pn_solver {
 
   bool is_df64() const { return precision == PN_PREC_DF64; }
 
+  // uncounted: bytes of it outside the budget (small indexes beside tables that
+  // a caller may have fitted to the byte)
   template <typename P>
-  P *alloc(size_t bytes) {
+  P *alloc(size_t bytes, size_t uncounted = 0) {
     if (bytes == 0) bytes = 16;
-    const int64_t budget = pn::hbm_budget();
-    if (budget >= 0 && dev_bytes + (int64_t)bytes > budget)
+    const int64_t budget = pn::hbm_budget(), counted = (int64_t)(bytes - uncounted);
+    if (budget >= 0 && dev_bytes + counted > budget && !(drop_reciprocals() && dev_bytes + counted <= budget))
       throw pn::SetupError{PN_ERR_ALLOC, "device allocation exceeds PN_HBM_BUDGET_BYTES"};
     void *p = nullptr;
-    const cudaError_t e = cudaMalloc(&p, bytes);
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation && drop_reciprocals()) {
+      (void)cudaGetLastError();
+      e = cudaMalloc(&p, bytes);
+    }
     if (e != cudaSuccess) {
       (void)cudaGetLastError();
       throw pn::SetupError{PN_ERR_ALLOC, std::string("cudaMalloc failed: ") + cudaGetErrorString(e)};
     }
     allocs.push_back(p);
-    dev_bytes += (int64_t)bytes;
+    dev_bytes += counted;
+    uncounted_bytes += (int64_t)uncounted;
     return (P *)p;
+  }
+
+  // the exact form's reciprocals are the first to go when something else needs
+  // the room (its kernels form them then); false: none held
+  bool drop_reciprocals() {
+    if (!d_rnode) return false;
+    dev_bytes -= 6 * (int64_t)sizeof(double) * ((int64_t)mesh.n_nodes + mesh.n_cells);
+    release(d_rnode);
+    d_rcell = nullptr;
+    return true;
   }
 
   template <typename P>

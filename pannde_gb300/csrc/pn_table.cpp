@@ -90,7 +90,8 @@ void upload_connectivity(pn_solver *s, const int32_t *list, int32_t n, int4 *&ta
   hvec<int32_t> base;
   hvec<uint8_t> id;
   std::vector<int32_t> offsets;
-  if (s->precision != PN_PREC_F64_EXACT && n > 0 && find_patterns(list, n, base, id, offsets)) {
+  if (s->precision != PN_PREC_F64_EXACT && n > 0 && find_patterns(list, n, base, id, offsets) &&
+      offsets.size() * 4 + (size_t)n * 5 <= (size_t)n * 32) {  // (a tiny mesh's many patterns may be the larger)
     con.offset = s->alloc<int4>(offsets.size() * 4 + (size_t)n * 5);
     con.base = (int32_t *)con.offset + offsets.size();
     con.pattern = (uint8_t *)(con.base + n);
@@ -145,11 +146,9 @@ void table_create(pn_solver *s) {
     s->upload_real(s->d_gcell, h.data(), h.size());
     if (exact) {
       try {  // two words of every element's reciprocals
-        s->d_rnode = s->alloc<void>(2 * g.size() * e);
-        s->d_rcell = s->alloc<void>(2 * h.size() * e);
+        s->d_rnode = s->alloc<void>(2 * (g.size() + h.size()) * e);
+        s->d_rcell = (double *)s->d_rnode + 2 * g.size();
       } catch (const SetupError &) {  // no room: the kernels form the reciprocals themselves
-        s->release(s->d_rnode);
-        s->release(s->d_rcell);
       }
       if (s->d_rcell) {
         ck(launch_exact_reciprocals((const double *)s->d_gnode, (int64_t)g.size(), (double *)s->d_rnode, s->stream),

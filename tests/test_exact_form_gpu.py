@@ -72,6 +72,27 @@ def test_bits(cuda_device, monkeypatch, mat, values, budget):
         assert same.all()
 
 
+@pytest.mark.parametrize("room", [0, 1], ids=["fitted", "reciprocals-fit"])
+def test_reciprocals_make_room(cuda_device, monkeypatch, room):
+    """Under a budget that holds the solver and its sensors' records but not the
+    reciprocals beside them, the records are what stays."""
+    c = cases.al_plate_case(nx=40, ny=33, nz=6, h=0.1e-3, nsteps=30, radius=0.5e-3, n_sensors=5)
+    recips = 48 * (c.mesh.n_nodes + c.mesh.n_cells)
+    capacity = recips // (5 * 3 * 8)  # the records take about as much
+    with Solver.from_case(c, "f64_exact", capacity=capacity) as s:
+        s.solve(30)
+        want = s.get_state()
+        full = s.info()["device_bytes"]  # (the first solve allocates too)
+    # without the reciprocals; or a little less than with them
+    monkeypatch.setenv("PN_HBM_BUDGET_BYTES", str(full - (1 if room else recips)))
+    with Solver.from_case(c, "f64_exact", capacity=capacity) as s:
+        s.solve(30)
+        got = s.get_state()
+        assert s.info()["device_bytes"] == full - recips
+    for a, b in zip(list(got[0]) + list(got[1]), list(want[0]) + list(want[1])):
+        assert np.array_equal(a, b)
+
+
 def test_plate_spacings(cuda_device):
     """i * h coordinates: spacings that differ in their last bits, and quiet material."""
     c = cases.al_plate_case(nx=40, ny=33, nz=6, h=0.1e-3, nsteps=30, radius=0.5e-3, n_sensors=5)
