@@ -271,8 +271,9 @@ constexpr int32_t kErrWait = 1;
 
 // A step's kernel may start while the one before it drains (launch_overlapped):
 // it loads the tables no step writes, then waits before it touches states,
-// path flags or traces.  A block lets the next kernel start when it reaches its last node layer: let at its
-// start, the next kernel's waiting blocks slowed the ones still marching
+// path flags or traces.  A block lets the next kernel start when it reaches its
+// last node layer: let at its start, the next kernel's waiting blocks slowed the
+// ones still marching
 // (laminate 400 x 400 x 40, FP32: 103.3 us per step without the overlap, 106.7
 // let at the start, 100.1 here; aluminium plate 64 x 64 x 8, FP32, one layer
 // per chunk: 8.2 / 5.6 / 5.2).
@@ -766,9 +767,10 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
 // has no source, no sensor to record and no split site (whose fix-up writes
 // outside the tiles' blocks).  Only launches of whole tall columns tell zeros
 // from values (a.fp64_chunk > 0); others mark every tile as holding values:
-// on small lattices the telling cost more (3%) than there is to save.  From rest a wave leaves most of a plate so for
-// the first hundreds of steps: laminate 400 x 400 x 40, an initial pulse of 80
-// cells' diameter, 20 steps with the state up- and downloaded 15.4 -> 14.3 ms.
+// on small lattices the telling cost more (3%) than there is to save.  From rest
+// a wave leaves most of a plate so for the first hundreds of steps: laminate
+// 400 x 400 x 40, an initial pulse of 80 cells' diameter, 20 steps with the state
+// up- and downloaded 15.4 -> 14.3 ms.
 template <int TY>
 __device__ __forceinline__ bool fp64_path(const GridArgs<double> &a, int bx, int by, int k0, int k1, int gxc,
                                           int step, bool clear, bool &quiet) {
