@@ -250,8 +250,10 @@ def roofline(case, info, kt, prec, peak, peak_kind):
     """HBM roofline of the dominant kernel from its CUDA-event average.
 
     Algorithmic bytes per launch:
-      table form  velocity: S read (6e/cell), V read+write, dt/rho, node slots (7e+32 /node)
-                  stress:   S read+write, material id, corner table (12e+36 /cell), V read (3e /node)
+      table form  velocity: S read (6e/cell), V read+write, dt/rho, connectivity (7e+5 /node)
+                  stress:   S read+write, material id, connectivity (12e+4+5 /cell), V read (3e /node)
+                  (connectivity as patterns; pn_solver_info counts the 32-byte tables
+                  that a mesh with many patterns keeps)
       grid form   fused step: S read+write + material byte (12e+1 /lattice cell),
                   V read+write + dt/rho (7e /lattice node) -- pn_solver_info
     with e the bytes per value (4 FP32, 8 FP64 and double-float)."""
@@ -261,8 +263,8 @@ def roofline(case, info, kt, prec, peak, peak_kind):
     if info.get("form_name") == "grid":
         alg = {"grid_step": info["algorithmic_bytes_per_step"]}
     else:
-        alg = {"velocity": nc * 6 * e + nn * (7 * e + 32),
-               "stress": nc * (12 * e + 36) + nn * 3 * e}
+        alg = {"velocity": nc * 6 * e + nn * (7 * e + 5),
+               "stress": nc * (12 * e + 9) + nn * 3 * e}
     dom = max(avg, key=lambda k: avg[k])
     achieved = alg[dom] / (avg[dom] * 1e-3) / 1e9
     form = info.get("form_name", "table")
