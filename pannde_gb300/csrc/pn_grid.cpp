@@ -426,7 +426,8 @@ void grid_create(pn_solver *s) {
                        std::max(s->r_cmax, s->r_cmax_s) > std::ldexp(1.0, 90);
   if (s->precision == PN_PREC_F64 && s->d_tmaps && s->r_elo <= s->r_ehi && s->r_elo_s <= s->r_ehi_s && !extreme) {
     const int64_t tiles = (int64_t)(g.nx / (kGridTileX - 1) + 1) * (g.ny / (kGridTileRows - 1) + 1);
-    s->d_rflags = s->alloc<uint32_t>((size_t)(kFlagPhases * tiles) * sizeof(uint32_t), (size_t)tiles * sizeof(uint32_t));
+    s->d_rflags = s->alloc<uint32_t>((size_t)(kFlagPhases * (tiles + 1)) * sizeof(uint32_t),
+                                       (size_t)(tiles + kFlagPhases) * sizeof(uint32_t));
     s->d_pathcnt = s->alloc<unsigned long long>(2 * sizeof(unsigned long long));
     ck(cudaMemsetAsync(s->d_pathcnt, 0, 2 * sizeof(unsigned long long), s->stream), "memset");
     grid_reset_range_flags(s);
@@ -439,7 +440,7 @@ void grid_reset_range_flags(pn_solver *s) {
   if (!s->d_rflags) return;
   const GridMap &g = s->grid;
   const int64_t tiles = (int64_t)(g.nx / (kGridTileX - 1) + 1) * (g.ny / (kGridTileRows - 1) + 1);
-  ck(cudaMemsetAsync(s->d_rflags, 0, (size_t)(kFlagPhases * tiles) * sizeof(uint32_t), s->stream), "memset");
+  ck(cudaMemsetAsync(s->d_rflags, 0, (size_t)(kFlagPhases * (tiles + 1)) * sizeof(uint32_t), s->stream), "memset");
   // every bit: every tile on the FP64 path, and none taken for quiet for two
   // steps (nothing is known of either buffer half)
   for (int64_t p : {s->step, s->step + kFlagPhases - 1})
@@ -595,7 +596,7 @@ int grid_put_state(pn_solver *s, const double *const *V, const double *const *S)
     if (bad[2]) {
       grid_reset_range_flags(s);  // a split-site copy out of range: FP64 for one step
     } else {
-      ck(cudaMemsetAsync(s->d_rflags, 0, (size_t)(kFlagPhases * tiles) * sizeof(uint32_t), s->stream), "memset");
+      ck(cudaMemsetAsync(s->d_rflags, 0, (size_t)(kFlagPhases * (tiles + 1)) * sizeof(uint32_t), s->stream), "memset");
       ck(cudaMemsetAsync(s->d_rflags + ((s->step + kFlagPhases - 1) % kFlagPhases) * tiles, (int)kFlagNonzero,
                          (size_t)tiles * sizeof(uint32_t), s->stream),
          "memset");

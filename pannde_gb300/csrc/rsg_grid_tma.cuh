@@ -828,6 +828,24 @@ __device__ __forceinline__ bool fp64_path(const GridArgs<double> &a, int bx, int
   return fp64;
 }
 
+// The columns on the FP64 path in the previous step, counted behind the flag
+// words (four words rotating like them): columns are cut into pieces while at
+// most three quarters of the launch's are on it.  With all of them there the
+// pieces' re-marched layers cost more than their balance gives (laminate 400 x
+// 400 x 40: 1.258 ms per step against 1.228 uncut; with half of them 0.767
+// against 0.844).
+__device__ __forceinline__ bool cut_columns(const GridArgs<double> &a, int bx, int by, int gxc, int step, bool fp64,
+                                            bool first) {
+  const int gyc = a.ny / 7 + 1, nt = gxc * gyc, phase = (a.flag_phase + step) % kFlagPhases;
+  uint32_t *count = a.rflags + kFlagPhases * nt;
+  if (first && threadIdx.x == 0) {
+    if (fp64) atomicAdd(count + (phase + 1) % kFlagPhases, 1u);
+    if (bx == 0 && by == 0) count[(phase + 2) % kFlagPhases] = 0;
+  }
+  const uint32_t cols = (uint32_t)(a.tail_chunk > 0 ? a.tail_from : nt);
+  return 4 * __ldcg(count + phase) <= 3 * cols;
+}
+
 // tile (bx, by) and layer range [k0, k0 + kc) of this block of a single
 // solver's launch: the 3D grid (x, y, chunk of kchunk layers), or with a
 // tail split (tail_chunk > 0) the 1D grid of whole columns, then the
@@ -886,6 +904,7 @@ __device__ __forceinline__ void f64h_block(const GridArgs<double> &a, unsigned c
   // launch's last wave (tail split) each
   if (threadIdx.x == 0 && first && (k0 == 0 || a.tail_chunk > 0) && a.path_count)
     atomicAdd(a.path_count + (fp64 ? 0 : 1), 1ull);
+  const bool cut = column && cut_columns(a, bx, by, gxc, step, fp64, first) && fp64;
   if (!work) return;
   if (quiet) {  // (the copies already under way land before the block ends)
     if (first && threadIdx.x == cp.ISSUER) {
@@ -897,8 +916,8 @@ __device__ __forceinline__ void f64h_block(const GridArgs<double> &a, unsigned c
     return;
   }
   if (column) {
-    if (!fp64 && !first) return;
-    if (fp64) {
+    if (!cut && !first) return;
+    if (cut) {
       cp.k0 = piece * a.fp64_chunk;
       cp.k1 = min(ktop, cp.k0 + a.fp64_chunk);
       if (cp.k0 >= ktop) return;

@@ -128,3 +128,27 @@ def test_refused_state_leaves_nothing_behind(cuda_device, monkeypatch, before):
             got.append(result(s))
     for a, b in zip(list(got[0][0]) + list(got[0][1]) + [got[0][2]], list(got[1][0]) + list(got[1][1]) + [got[1][2]]):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("share", [0.3, 0.74, 0.78, 1.0])
+def test_columns_cut_or_whole(cuda_device, monkeypatch, share):
+    """Columns on the FP64 path are cut into pieces while at most three
+    quarters of them are: the bits are those of equal chunks on either side of
+    the line, and the counts do not depend on it."""
+    c = problem(True)
+    rng = np.random.default_rng(6)
+    x = c.mesh.x / c.mesh.x.max()
+    V0 = [rng.normal(size=c.mesh.n_nodes) * np.where(x <= share, 1e-200, 1e-3) for _ in range(3)]
+    cx = np.asarray(x)[c.mesh.hexes.reshape(-1, 8)].mean(axis=1)
+    S0 = [rng.normal(size=c.mesh.n_cells) * np.where(cx <= share, 1e-195, 1e4) for _ in range(6)]
+    got = []
+    for kchunk in ("64", "5"):
+        monkeypatch.setenv("PN_GRID_KCHUNK", kchunk)
+        with Solver.from_case(c, "f64", form="grid") as s:
+            s.set_state(V0, S0)
+            s.solve(STEPS)
+            got.append((result(s), s.path_counts()))
+    (a, na), (b, nb) = got
+    for u, v in zip(list(a[0]) + list(a[1]) + [a[2]], list(b[0]) + list(b[1]) + [b[2]]):
+        assert np.array_equal(u, v)
+    assert na[0] > 0 and sum(na) == sum(nb)
