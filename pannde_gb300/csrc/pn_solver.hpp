@@ -221,9 +221,11 @@ struct pn_solver {
   }
 
   // the exact form's reciprocals are the first to go when something else needs
-  // the room (its kernels form them then); false: none held
+  // the room (its kernels form them then); false: none held.  Argument blocks
+  // are filled after the last allocation before their launch.
   bool drop_reciprocals() {
     if (!d_rnode) return false;
+    pn::ck(cudaStreamSynchronize(stream), "reciprocals sync");  // steps in flight read them
     dev_bytes -= 6 * (int64_t)sizeof(double) * ((int64_t)mesh.n_nodes + mesh.n_cells);
     release(d_rnode);
     d_rcell = nullptr;

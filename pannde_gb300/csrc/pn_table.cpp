@@ -300,12 +300,13 @@ template <typename T>
 void run(pn_solver *s, int32_t nsteps) {
   VelArgs<T> va;
   StressArgs<T> sa;
-  table_args<T>(s, va, sa);
   const int64_t nsig = (int64_t)s->src.size();
   int32_t done = 0;
   while (done < nsteps) {
     int32_t chunk = nsteps - done;
     ensure_signal_rows(s, chunk);
+    // (after it: the table's room may have come from the exact form's reciprocals)
+    table_args<T>(s, va, sa);
     if (nsig > 0 && !s->sig_hold)
       chunk = (int32_t)std::min<int64_t>(chunk, s->sig_step0 + s->sig_rows - s->step);
     va.rec_base = s->rec_count;

@@ -1,0 +1,77 @@
+"""Device memory as the host code keeps it, without a device: the library's
+host sources over tests/cxx/fake_cuda.cpp, whose allocations are host memory
+with every copy, fill and launch argument checked against them."""
+import ctypes
+import shutil
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+from pannde_gb300 import _native as N
+from pannde_gb300 import cases
+from pannde_gb300.build import _cuda_home
+from pannde_gb300.solver import Batch, Solver
+
+ROOT = Path(__file__).resolve().parent.parent
+CSRC = ROOT / "pannde_gb300" / "csrc"
+
+
+@pytest.fixture(scope="module")
+def fake_lib(tmp_path_factory):
+    if not shutil.which("g++") or not (_cuda_home() / "include" / "cuda_runtime.h").exists():
+        pytest.skip("no g++ or no CUDA headers")
+    out = tmp_path_factory.mktemp("fake")
+    inc = ["-I", str(_cuda_home() / "include"), "-I", str(CSRC), "-I", str(ROOT / "include")]
+    srcs = [ROOT / "tests" / "cxx" / "fake_cuda.cpp"] + [CSRC / f"pn_{n}.cpp" for n in
+            ("setup", "table", "grid", "capi", "batch", "energy", "partition")]
+    jobs = [subprocess.Popen(["g++", "-std=c++17", "-O1", "-fPIC", "-fopenmp", *inc, "-c", str(s), "-o",
+                              str(out / (s.stem + ".o"))], stderr=subprocess.PIPE, text=True) for s in srcs]
+    for j in jobs:
+        err = j.communicate()[1]
+        assert j.returncode == 0, err
+    so = out / "libfake.so"
+    r = subprocess.run(["g++", "-shared", "-fopenmp", "-o", str(so)] + [str(out / (s.stem + ".o")) for s in srcs] +
+                       ["-Wl,--no-undefined", "-Wl,-Bsymbolic"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    return so
+
+
+@pytest.fixture
+def fake(fake_lib, monkeypatch):
+    lib = N.load(fake_lib)
+    lib.fake_first_fault.restype = ctypes.c_char_p
+    for f in ("fake_held", "fake_launches", "fake_launches_without_reciprocals"):
+        getattr(lib, f).restype = ctypes.c_int64
+    lib.fake_set_room.argtypes = [ctypes.c_int64]
+    monkeypatch.setattr(N, "_lib", lib)
+    monkeypatch.delenv("PN_HBM_BUDGET_BYTES", raising=False)
+    lib.fake_reset()
+    yield lib
+    assert lib.fake_faults() == 0, lib.fake_first_fault().decode()
+
+
+def plate(**kw):
+    return cases.al_plate_case(**dict(dict(nx=14, ny=11, nz=6, h=0.1e-3, nsteps=30, radius=0.5e-3, n_sensors=5), **kw))
+
+
+@pytest.mark.parametrize("how", ["budget", "device"])
+def test_launches_after_the_reciprocals_made_room(fake, monkeypatch, how):
+    """Exact form: the first solve's signal table takes the room that the
+    reciprocals held; that solve's launches, and the later ones, are given none."""
+    c = plate()
+    with Solver.from_case(c, "f64_exact") as s:
+        s.solve(3)
+        full, held = s.info()["device_bytes"], fake.fake_held()
+    assert fake.fake_launches() == 6 and fake.fake_launches_without_reciprocals() == 0
+    if how == "budget":
+        monkeypatch.setenv("PN_HBM_BUDGET_BYTES", str(full - 1))
+    else:
+        fake.fake_set_room(held - 1)
+    with Solver.from_case(c, "f64_exact") as s:
+        s.solve(3)
+        assert s.info()["device_bytes"] == full - 48 * (c.mesh.n_nodes + c.mesh.n_cells)
+        assert fake.fake_launches_without_reciprocals() == 6
+        s.solve(2)
+    assert fake.fake_launches_without_reciprocals() == 10
