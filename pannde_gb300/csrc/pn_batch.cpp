@@ -699,7 +699,7 @@ int pn_batch_solve_noalloc(pn_batch *b, int32_t nsteps) {
     for (size_t m = 0; m < b->members.size(); m++) {
       pn_solver *s = b->members[m];
       if (s->has_mask_sources()) return berr(PN_ERR_INVALID, "window-mask sources need pn_solver_solve_signals");
-      if (s->src_dirty || (!s->src.empty() && s->sig_alloc_rows == 0))
+      if (s->src_dirty || (!s->src.empty() && s->sig_room() == 0))
         return berr(PN_ERR_INVALID, "pn_batch_solve_noalloc: member " + std::to_string(m) +
                                         " has sources whose device tables are not built yet; one pn_batch_solve "
                                         "or pn_solver_solve step builds them");

@@ -15,6 +15,16 @@
 
 namespace pn {
 
+// room for `rows` rows of the present sources' values (no step in flight reads the table)
+static void reserve_signal_rows(pn_solver *s, int64_t rows) {
+  const int64_t nsig = (int64_t)s->src.size();
+  if (rows <= s->sig_room()) return;
+  s->release(s->d_sig);
+  s->sig_alloc_values = 0;
+  s->d_sig = s->alloc<void>((size_t)rows * nsig * s->esz);
+  s->sig_alloc_values = rows * nsig;
+}
+
 void ensure_signal_rows(pn_solver *s, int64_t nsteps, bool may_alloc) {
   const int64_t nsig = (int64_t)s->src.size();
   if (nsig == 0 || s->caller_signals) return;  // caller rows cover the whole call
@@ -27,8 +37,8 @@ void ensure_signal_rows(pn_solver *s, int64_t nsteps, bool may_alloc) {
   // without allocation, at most the rows the table already has
   int64_t want = std::min<int64_t>(std::max<int64_t>(nsteps, 1024), kSigRowsCap);
   if (!may_alloc) {
-    if (s->sig_alloc_rows <= 0) throw SetupError{PN_ERR_INVALID, "signal table not resident"};
-    want = std::min<int64_t>(want, s->sig_alloc_rows);
+    if (s->sig_room() <= 0) throw SetupError{PN_ERR_INVALID, "signal table not resident"};
+    want = std::min<int64_t>(want, s->sig_room());
   }
   std::vector<double> rows;
   rows.reserve((size_t)want * nsig);
@@ -46,11 +56,7 @@ void ensure_signal_rows(pn_solver *s, int64_t nsteps, bool may_alloc) {
     t += s->dt;  // the same accumulation as solve(): time += dt
   }
   ck(cudaStreamSynchronize(s->stream), "signal sync");
-  if (r > s->sig_alloc_rows) {
-    s->release(s->d_sig);
-    s->d_sig = s->alloc<void>((size_t)r * nsig * s->esz);
-    s->sig_alloc_rows = r;
-  }
+  reserve_signal_rows(s, r);
   s->upload_real(s->d_sig, rows.data(), rows.size());
   ck(cudaStreamSynchronize(s->stream), "signal upload");
   s->sig_step0 = s->step;
@@ -452,11 +458,7 @@ int pn_solver_solve_signals(pn_solver *s, int32_t nsteps, const double *values, 
         s->call_values = values;
       } else {
         pn::ck(cudaStreamSynchronize(s->stream), "signal sync");
-        if (nsteps > s->sig_alloc_rows) {
-          s->release(s->d_sig);
-          s->d_sig = s->alloc<void>((size_t)nsteps * nsig * s->esz);
-          s->sig_alloc_rows = nsteps;
-        }
+        pn::reserve_signal_rows(s, nsteps);
         s->upload_real(s->d_sig, values, (size_t)nsteps * nsig);
         pn::ck(cudaStreamSynchronize(s->stream), "signal upload");
       }

@@ -176,7 +176,11 @@ struct pn_solver {
   // signal table: rows [sig_step0, sig_step0 + sig_rows) of [n_sig] values;
   // sig_hold: the last row holds for every later step
   void *d_sig = nullptr;
-  int64_t sig_step0 = 0, sig_rows = 0, sig_alloc_rows = 0;
+  int64_t sig_step0 = 0, sig_rows = 0;
+  int64_t sig_alloc_values = 0;  // values d_sig has room for
+  int64_t sig_room() const {     // ... rows of the present sources
+    return src.empty() ? 0 : sig_alloc_values / (int64_t)src.size();
+  }
   bool sig_hold = false, sig_valid = false;
 
   // sensors

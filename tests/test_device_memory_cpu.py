@@ -75,3 +75,25 @@ def test_launches_after_the_reciprocals_made_room(fake, monkeypatch, how):
         assert fake.fake_launches_without_reciprocals() == 6
         s.solve(2)
     assert fake.fake_launches_without_reciprocals() == 10
+
+
+@pytest.mark.parametrize("form, prec", [("grid", "f32"), ("grid", "f64"), ("table", "f64"), ("table", "f64_exact")])
+@pytest.mark.parametrize("how", ["solve", "signals", "batch"])
+def test_signal_rows_of_sources_added_later(fake, form, prec, how):
+    """The signal table was sized for fewer sources: rows of more need a larger one."""
+    if how == "batch" and prec == "f64_exact":
+        pytest.skip("not batched")
+    c = plate()
+    more = [cases.WindowSource(N.PN_SOURCE_FORCE, g, d, c.sources[0].center, c.sources[0].radius, c.sources[0].ds,
+                               c.sources[0].times, c.sources[0].values) for g in range(1, 5) for d in range(3)]
+    with Solver.from_case(c, prec, form=form) as s, Batch() as b:
+        s.solve(2)
+        s.add_sources(more)
+        if how == "solve":
+            s.solve(2)
+        elif how == "signals":
+            s.solve_signals(np.zeros((1000, 13)))
+        else:
+            b.add(s)
+            b.solve(2)
+            b.solve_noalloc(2)
