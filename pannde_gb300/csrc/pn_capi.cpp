@@ -454,11 +454,14 @@ int pn_solver_solve_signals(pn_solver *s, int32_t nsteps, const double *values, 
       return set_err(PN_ERR_NOT_FINITE, "non-finite signal value");
     refresh_sources(s);
     if (nsig > 0 && nsteps > 0) {
+      if (nsteps > s->sig_room()) {  // (the allocation-free batch solve refills these rows)
+        pn::ck(cudaStreamSynchronize(s->stream), "signal sync");
+        pn::reserve_signal_rows(s, nsteps);
+      }
       if (nsig <= pn::kSignalsHere) {  // few sources: each launch carries its step's values
         s->call_values = values;
       } else {
         pn::ck(cudaStreamSynchronize(s->stream), "signal sync");
-        pn::reserve_signal_rows(s, nsteps);
         s->upload_real(s->d_sig, values, (size_t)nsteps * nsig);
         pn::ck(cudaStreamSynchronize(s->stream), "signal upload");
       }

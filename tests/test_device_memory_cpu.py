@@ -97,3 +97,20 @@ def test_signal_rows_of_sources_added_later(fake, form, prec, how):
             b.add(s)
             b.solve(2)
             b.solve_noalloc(2)
+
+
+@pytest.mark.parametrize("n_sources", [1, 9])
+@pytest.mark.parametrize("form", ["grid", "table"])
+def test_caller_signals_leave_rows_for_the_allocation_free_batch(fake, form, n_sources):
+    """A solver advanced by solve_signals alone is taken by solve_noalloc,
+    whether its launches carry the values (few sources) or a table does."""
+    c = plate()
+    c.sources = [cases.WindowSource(N.PN_SOURCE_FORCE, g // 3, g % 3, c.sources[0].center, c.sources[0].radius,
+                                    c.sources[0].ds, c.sources[0].times, c.sources[0].values)
+                 for g in range(n_sources)]
+    with Solver.from_case(c, "f32", form=form) as s, Batch() as b:
+        s.solve_signals(np.zeros((3, n_sources)))
+        b.add(s)
+        held = fake.fake_held()
+        b.solve_noalloc(7)
+        assert fake.fake_held() == held or held + 262144 == fake.fake_held()  # (the fixed scratch, once)
