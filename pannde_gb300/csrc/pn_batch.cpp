@@ -579,11 +579,11 @@ void solve_grid(pn_batch *b, int32_t nsteps, int precision, const Stage &stage, 
                 }
               });
     pn::ck(cudaStreamSynchronize(b->stream), "batch chunk");
-    if (!range_flags)  // members stepped without their flags: FP64 path first when next alone
-      for (pn_solver *s : b->members) pn::grid_reset_range_flags(s);
     b->last_rows = shapes[staged_shape].first;
     b->last_shape = shapes[staged_shape].second;
     advance(b, chunk);
+    if (!range_flags)  // members stepped without their flags: FP64 path first when next alone
+      for (pn_solver *s : b->members) pn::grid_reset_range_flags(s);  // (the step count is the next step's)
     done += chunk;
   }
 }
