@@ -273,7 +273,7 @@ void solve_table(pn_batch *b, int32_t nsteps, int precision, const Stage &stage,
     const int32_t chunk = common_chunk(b, nsteps - done, may_alloc);
     for (int m = 0; m < n; m++) {
       pn_solver *s = b->members[m];
-      pn::table_args<T>(s, va[m], sa[m]);
+      pn::table_args(s, va[m], sa[m]);
       const int64_t nsig = (int64_t)s->src.size();
       if (nsig > 0) {
         const int64_t row0 = pn::sig_row(s, 0);
@@ -433,7 +433,7 @@ void solve_grid(pn_batch *b, int32_t nsteps, int precision, const Stage &stage, 
       for (int m = 0; m < n; m++) {
         pn_solver *s = b->members[m];
         pn::GridArgs<T> a;
-        pn::grid_args<T>(s, a);
+        pn::grid_args(s, a);
         const int64_t nsig = (int64_t)s->src.size();
         if (nsig > 0) {
           const int64_t row0 = pn::sig_row(s, 0);

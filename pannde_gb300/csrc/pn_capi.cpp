@@ -378,7 +378,6 @@ int pn_solver_set_sensors(pn_solver *s, const int32_t *nodes, int32_t n, int32_t
     pn::ck(cudaStreamSynchronize(s->stream), "sensors sync");
     s->release(s->d_stile); s->release(s->d_snode); s->release(s->d_sidx);
     s->release(s->d_srng); s->release(s->d_skey); s->release(s->d_traces);
-    s->release(s->s_slots);
     s->n_sens = 0;
     s->rec_cap = 0;
     s->rec_count = 0;

@@ -99,7 +99,7 @@ struct Keyed {
 };
 
 // entries sorted by (slot, local index), stably: a thread finds its own
-// entries of a slot by its place in it (SlotIndex) or a binary search
+// entries of a slot by its place in it (upload_ranges) or a binary search
 // (first_local, the classic kernel), and one node's entries keep their order
 // (the order their terms are added in)
 void ranges_of(std::vector<Keyed> &L, int64_t n_slots, std::vector<int32_t> &rng) {
@@ -115,49 +115,43 @@ void ranges_of(std::vector<Keyed> &L, int64_t n_slots, std::vector<int32_t> &rng
   }
 }
 
-// the slots' index (SlotIndex, rsg_grid.cuh) over sorted entries and their
-// ranges, on the device; empty lists have none
-void upload_index(pn_solver *s, const std::vector<Keyed> &L, const std::vector<int32_t> &rng, int tile_rows,
-                  pn_solver::SlotTables &out) {
+// the slots' ranges on the device, with places, rows and lists behind them
+// (rsg_grid.cuh slot_entries) for the tensor-copy kernel
+void upload_ranges(pn_solver *s, const std::vector<Keyed> &L, const std::vector<int32_t> &rng, int tile_rows,
+                   int2 *&out) {
   const size_t n_slots = rng.size() / 2;
-  std::vector<int32_t> id(n_slots, -1), node;
-  std::vector<uint32_t> rows;
-  int32_t slots = 0;
+  std::vector<int32_t> all(2 * n_slots + (n_slots + 1) / 2 * 2, 0), node;  // (rows start on 8 bytes)
+  std::vector<size_t> listed;  // rows' words that are places in node
   for (size_t sl = 0; sl < n_slots; sl++) {
-    const int32_t e0 = rng[2 * sl], e1 = rng[2 * sl + 1];
-    if (e0 == e1) continue;
-    id[sl] = slots++;
+    const int32_t e0 = all[2 * sl] = rng[2 * sl], e1 = all[2 * sl + 1] = rng[2 * sl + 1];
+    all[2 * n_slots + sl] = -1;
+    if (e0 == e1 || !s->d_tmaps) continue;
     bool several = false;  // entries at one node of the slot
     for (int32_t e = e0 + 1; e < e1; e++) several = several || (L[e].key & 0xffff) == (L[e - 1].key & 0xffff);
-    const size_t at = rows.size();
-    rows.resize(at + 2 * (size_t)tile_rows, 0);
+    const size_t at = all.size();
+    all[2 * n_slots + sl] = (int32_t)(at / 2);
+    all.resize(at + 2 * (size_t)tile_rows, 0);
     std::vector<bool> begun((size_t)tile_rows, false);
     for (int32_t e = e0; e < e1; e++) {
       if (e > e0 && (L[e].key & 0xffff) == (L[e - 1].key & 0xffff)) continue;
       const int t = L[e].key & 0xffff, ty = t / kGridTileX, tx = t % kGridTileX;
-      uint32_t *r = &rows[at + 2 * (size_t)ty];
+      const size_t r = at + 2 * (size_t)ty;
       if (!begun[(size_t)ty]) {
         begun[(size_t)ty] = true;
-        r[1] = several ? (uint32_t)node.size() | 0x80000000u : (uint32_t)e;
+        all[r + 1] = several ? (int32_t)node.size() : e;
+        if (several) listed.push_back(r + 1);
       }
-      r[0] |= 1u << tx;
+      all[r] |= (int32_t)(1u << tx);
       if (several) node.push_back(e);
     }
     if (several) node.push_back(e1);
   }
-  // rows (8-byte entries), then id, then node
-  std::vector<uint32_t> all(rows);
-  all.insert(all.end(), id.begin(), id.end());
+  for (size_t q : listed) all[q] = (int32_t)((uint32_t)((size_t)all[q] + all.size()) | 0x80000000u);
   all.insert(all.end(), node.begin(), node.end());
-  uint32_t *p = s->alloc<uint32_t>(all.size() * 4, all.size() * 4);
-  s->upload_raw(p, all.data(), all.size() * 4);
-  out.rows = (uint2 *)p;
-  out.id = (int32_t *)(p + rows.size());
-  out.node = out.id + id.size();
-  ck(cudaStreamSynchronize(s->stream), "slot index upload");  // before the host lists go
+  out = s->alloc<int2>(all.size() * 4, (all.size() - rng.size()) * 4);
+  s->upload_raw(out, all.data(), all.size() * 4);
+  ck(cudaStreamSynchronize(s->stream), "ranges upload");  // before the host list goes
 }
-
-SlotIndex index_of(const pn_solver::SlotTables &t) { return SlotIndex{t.id, t.rows, t.node}; }
 
 }  // namespace
 
@@ -322,7 +316,6 @@ bool grid_set_tile_rows(pn_solver *s, int rows) {
   if (!s->src.empty() && !s->src_dirty) grid_sources(s);
   if (s->n_sens > 0) {
     s->release(s->d_srng); s->release(s->d_skey); s->release(s->d_sidx);
-    s->release(s->s_slots);
     grid_sensors(s, s->sensor_pairs);
   }
   ck(cudaStreamSynchronize(s->stream), "retile upload");
@@ -626,19 +619,16 @@ void grid_sources(pn_solver *s) {
   ck(cudaStreamSynchronize(s->stream), "sources sync");
   s->release(s->d_frng); s->release(s->d_fkey); s->release(s->d_fsig); s->release(s->d_fw);
   s->release(s->d_mrng); s->release(s->d_mkey); s->release(s->d_msig); s->release(s->d_mw);
-  s->release(s->f_slots);
-  s->release(s->m_slots);
   const GridMap &g = s->grid;
   const Tiles T = tiles_of(g, s->tile_rows);
   s->n_force = (int32_t)fe.size();
   s->n_moment = (int32_t)me.size();
   s->n_src_nodes = s->n_src_cells = 0;
   auto upload = [&](std::vector<Keyed> &L, int64_t layers, int2 *&rng, int32_t *&key, int32_t *&sig,
-                    void *&w, pn_solver::SlotTables &index) {
+                    void *&w) {
     if (L.empty()) return;
     std::vector<int32_t> r;
     ranges_of(L, T.blocks() * layers, r);
-    if (s->d_tmaps) upload_index(s, L, r, s->tile_rows, index);
     std::vector<int32_t> k(L.size()), sg(L.size());
     std::vector<double> wt(L.size());
     for (size_t q = 0; q < L.size(); q++) {
@@ -646,11 +636,10 @@ void grid_sources(pn_solver *s) {
       sg[q] = L[q].sig;
       wt[q] = L[q].w;
     }
-    rng = s->alloc<int2>(r.size() * 4);
+    upload_ranges(s, L, r, s->tile_rows, rng);
     key = s->alloc<int32_t>(k.size() * 4);
     sig = s->alloc<int32_t>(sg.size() * 4);
     w = s->alloc<void>(wt.size() * s->esz);
-    s->upload_raw(rng, r.data(), r.size() * 4);
     s->upload_raw(key, k.data(), k.size() * 4);
     s->upload_raw(sig, sg.data(), sg.size() * 4);
     s->upload_real(w, wt.data(), wt.size());
@@ -684,8 +673,8 @@ void grid_sources(pn_solver *s) {
     const int32_t fx = g.fix_of_cell.empty() ? -1 : g.fix_of_cell[(size_t)me[q].elem];
     if (fx >= 0) s->fix_moments.push_back({fx, me[q].comp, me[q].sig, s->dt * me[q].w});
   }
-  upload(F, g.nz + 1, s->d_frng, s->d_fkey, s->d_fsig, s->d_fw, s->f_slots);
-  upload(M, g.nz, s->d_mrng, s->d_mkey, s->d_msig, s->d_mw, s->m_slots);
+  upload(F, g.nz + 1, s->d_frng, s->d_fkey, s->d_fsig, s->d_fw);
+  upload(M, g.nz, s->d_mrng, s->d_mkey, s->d_msig, s->d_mw);
   if (s->d_rflags) {  // the stresses' double-float range also covers the source weights
     double cmin = s->r_cmin_s, cmax = s->r_cmax_s;
     for (const std::vector<Keyed> *L : {&F, &M})
@@ -724,23 +713,21 @@ void grid_sensors(pn_solver *s, const std::vector<std::pair<int32_t, int32_t>> &
   }
   std::vector<int32_t> r;
   ranges_of(L, T.blocks() * (g.nz + 1), r);
-  if (s->d_tmaps) upload_index(s, L, r, s->tile_rows, s->s_slots);
   std::vector<int32_t> key(L.size()), idx(L.size());
   for (size_t q = 0; q < L.size(); q++) {
     key[q] = L[q].key;
     idx[q] = L[q].idx;
   }
-  s->d_srng = s->alloc<int2>(r.size() * 4);
+  upload_ranges(s, L, r, s->tile_rows, s->d_srng);
   s->d_skey = s->alloc<int32_t>(key.size() * 4);
   s->d_sidx = s->alloc<int32_t>(idx.size() * 4);
-  s->upload_raw(s->d_srng, r.data(), r.size() * 4);
   s->upload_raw(s->d_skey, key.data(), key.size() * 4);
   s->upload_raw(s->d_sidx, idx.data(), idx.size() * 4);
   grid_split_upload(s);
 }
 
-template <typename T>
-void grid_args(pn_solver *s, GridArgs<T> &a) {
+template <typename T, bool OWN>
+void grid_args(pn_solver *s, GridArgs<T, OWN> &a) {
   const GridMap &g = s->grid;
   std::memset(&a, 0, sizeof(a));
   a.nx = g.nx;
@@ -757,17 +744,14 @@ void grid_args(pn_solver *s, GridArgs<T> &a) {
   a.g[2] = to_store<T>(folded ? 1.0 : 0.25 / s->mesh.hz);
   if (s->n_force > 0) {
     a.f_rng = s->d_frng; a.f_key = s->d_fkey; a.f_sig = s->d_fsig; a.f_w = (const T *)s->d_fw;
-    a.f_ix = index_of(s->f_slots);
   }
   if (s->n_moment > 0) {
     a.m_rng = s->d_mrng; a.m_key = s->d_mkey; a.m_sig = s->d_msig; a.m_w = (const T *)s->d_mw;
-    a.m_ix = index_of(s->m_slots);
   }
   a.n_sens = s->n_sens;
   a.traces = s->d_traces;
   a.rec_cap = s->rec_cap;
   a.s_rng = s->n_sens > 0 ? s->d_srng : nullptr;
-  if (s->n_sens > 0) a.s_ix = index_of(s->s_slots);
   a.s_key = s->d_skey;
   a.s_idx = s->d_sidx;
   a.sig_stride = 0;
@@ -812,16 +796,17 @@ const void *grid_maps_for(const pn_solver *s, int in) {
   return s->d_tmaps ? (const void *)((const unsigned char *)s->d_tmaps + (size_t)in * grid_tma_maps_bytes())
                     : nullptr;
 }
-template void grid_args<double>(pn_solver *, GridArgs<double> &);
-template void grid_args<float>(pn_solver *, GridArgs<float> &);
-template void grid_args<float2>(pn_solver *, GridArgs<float2> &);
+template void grid_args<double, false>(pn_solver *, GridArgs<double> &);
+template void grid_args<float, false>(pn_solver *, GridArgs<float> &);
+template void grid_args<float2, false>(pn_solver *, GridArgs<float2> &);
 
 namespace {
 
 template <typename T>
 void run(pn_solver *s, int32_t nsteps) {
-  GridArgs<T> a;
-  grid_args<T>(s, a);
+  GridLaunch<T> a{};
+  grid_args(s, a);
+  if (s->d_tmaps) a.places = slot_places(a, s->tile_rows);
   const int64_t nsig = (int64_t)s->src.size();
   int32_t done = 0;
   while (done < nsteps) {

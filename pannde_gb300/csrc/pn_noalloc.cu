@@ -14,8 +14,8 @@
 namespace pn {
 namespace {
 
-// argument blocks + tile prefixes of one batch call (about 270 grid-form or
-// 550 table-form members)
+// argument blocks + tile prefixes of one batch call (about 250 grid-form or
+// 540 table-form members)
 static __device__ __align__(256) unsigned char g_batch_scratch[kNoAllocScratchBytes];
 
 std::mutex g_setup;

@@ -110,7 +110,7 @@ void stage(pn_partitioned *q, pn::BatchLaunch &L) {
   std::vector<int> vs((size_t)n + 1, 0), ss((size_t)n + 1, 0);
   for (int m = 0; m < n; m++) {
     pn_solver *s = q->parts[(size_t)m];
-    pn::table_args<T>(s, va[(size_t)m], sa[(size_t)m]);
+    pn::table_args(s, va[(size_t)m], sa[(size_t)m]);
     const int64_t nsig = (int64_t)s->src.size();
     if (nsig > 0) {
       const int64_t row0 = pn::sig_row(s, 0);

@@ -77,15 +77,8 @@ struct pn_solver {
   void *d_coef = nullptr, *d_ctab = nullptr;
 
   // table form
-  int4 *d_hex = nullptr, *d_ncc = nullptr;
-  // ... or the same as patterns (Connectivity): of the nodes' cells, of the cells' nodes
-  // (one allocation, held by offset)
-  struct Patterns {
-    int4 *offset = nullptr;
-    int32_t *base = nullptr;
-    uint8_t *pattern = nullptr;
-  };
-  Patterns n_con, c_con;
+  int4 *d_hex = nullptr, *d_ncc = nullptr;      // the cells' nodes, the nodes' cells
+  int32_t hex_patterns = 0, ncc_patterns = 0;  // ... as so many patterns (0: tables)
   void *d_gnode = nullptr, *d_gcell = nullptr;
   void *d_rnode = nullptr, *d_rcell = nullptr;  // exact form: reciprocals of the spacings, or null
   int32_t *d_mat = nullptr;
@@ -162,17 +155,9 @@ struct pn_solver {
   int2 *d_ftile = nullptr, *d_mtile = nullptr;
   int32_t *d_felem = nullptr, *d_fcode = nullptr, *d_melem = nullptr, *d_mcode = nullptr;
   // grid-form lists: per (block, layer) ranges, key, signal
-  int2 *d_frng = nullptr, *d_mrng = nullptr;
+  int2 *d_frng = nullptr, *d_mrng = nullptr;  // slots' ranges, places and rows behind them (rsg_grid.cuh slot_entries)
   int32_t *d_fkey = nullptr, *d_fsig = nullptr, *d_mkey = nullptr, *d_msig = nullptr;
   void *d_fw = nullptr, *d_mw = nullptr;
-  // ... and how a thread finds its own entries of a slot (SlotIndex; one
-  // allocation, held by rows)
-  struct SlotTables {
-    uint2 *rows = nullptr;
-    int32_t *id = nullptr;
-    int32_t *node = nullptr;
-  };
-  SlotTables f_slots, m_slots, s_slots;
   // signal table: rows [sig_step0, sig_step0 + sig_rows) of [n_sig] values;
   // sig_hold: the last row holds for every later step
   void *d_sig = nullptr;
@@ -243,11 +228,6 @@ struct pn_solver {
     if (it != allocs.end()) allocs.erase(it);
     cudaFree((void *)p);
     p = nullptr;
-  }
-
-  void release(SlotTables &t) {
-    release(t.rows);
-    t = SlotTables();
   }
 
   // upload a double host array in the storage type (double, float, or the
@@ -402,8 +382,8 @@ int64_t step_bytes(const pn_solver *s);
 
 // argument blocks of one solver (pointers, tables, constants; the per-step
 // fields -- signal row, record, buffers -- are the caller's to set)
-template <typename T> void table_args(pn_solver *s, VelArgs<T> &va, StressArgs<T> &sa);
-template <typename T> void grid_args(pn_solver *s, GridArgs<T> &a);
+template <typename T, bool OWN> void table_args(pn_solver *s, VelArgs<T, OWN> &va, StressArgs<T, OWN> &sa);
+template <typename T, bool OWN> void grid_args(pn_solver *s, GridArgs<T, OWN> &a);
 // tensor maps of input buffer `in` (0/1) for the tensor-copy kernel, or null
 const void *grid_maps_for(const pn_solver *s, int in);
 

@@ -86,26 +86,24 @@ bool find_patterns(const int32_t *list, int32_t n, hvec<int32_t> &base, hvec<uin
 
 // the device's connectivity of one kind: patterns for the fast forms where they
 // suffice, else the table
-void upload_connectivity(pn_solver *s, const int32_t *list, int32_t n, int4 *&table, pn_solver::Patterns &con) {
+void upload_connectivity(pn_solver *s, const int32_t *list, int32_t n, int4 *&table, int32_t &n_patterns) {
   hvec<int32_t> base;
   hvec<uint8_t> id;
   std::vector<int32_t> offsets;
   if (s->precision != PN_PREC_F64_EXACT && n > 0 && find_patterns(list, n, base, id, offsets) &&
       offsets.size() * 4 + (size_t)n * 5 <= (size_t)n * 32) {  // (a tiny mesh's many patterns may be the larger)
-    con.offset = s->alloc<int4>(offsets.size() * 4 + (size_t)n * 5);
-    con.base = (int32_t *)con.offset + offsets.size();
-    con.pattern = (uint8_t *)(con.base + n);
-    s->upload_raw(con.offset, offsets.data(), offsets.size() * 4);
-    s->upload_raw(con.base, base.data(), (size_t)n * 4);
-    s->upload_raw(con.pattern, id.data(), (size_t)n);
+    n_patterns = (int32_t)(offsets.size() / 8);
+    table = s->alloc<int4>(offsets.size() * 4 + (size_t)n * 5);
+    int32_t *d_base = (int32_t *)table + offsets.size();
+    s->upload_raw(table, offsets.data(), offsets.size() * 4);
+    s->upload_raw(d_base, base.data(), (size_t)n * 4);
+    s->upload_raw(d_base + n, id.data(), (size_t)n);
     ck(cudaStreamSynchronize(s->stream), "connectivity upload");  // before the host lists go
     return;
   }
   table = s->alloc<int4>((size_t)n * 32);
   s->upload_raw(table, list, (size_t)n * 32);
 }
-
-Connectivity connectivity(const pn_solver::Patterns &p) { return Connectivity{p.base, p.pattern, p.offset}; }
 
 }  // namespace
 
@@ -121,8 +119,8 @@ void table_create(pn_solver *s) {
   s->d_ctab = s->alloc<void>((size_t)s->mat.n_mat * 36 * e);
   for (int k = 0; k < 3; k++) ck(cudaMemsetAsync(s->V[0][k], 0, (size_t)nn * e, s->stream), "memset");
   for (int k = 0; k < 6; k++) ck(cudaMemsetAsync(s->S[0][k], 0, (size_t)nc * e, s->stream), "memset");
-  upload_connectivity(s, s->mesh.hex.data(), nc, s->d_hex, s->c_con);
-  upload_connectivity(s, s->mesh.ncc.data(), nn, s->d_ncc, s->n_con);
+  upload_connectivity(s, s->mesh.hex.data(), nc, s->d_hex, s->hex_patterns);
+  upload_connectivity(s, s->mesh.ncc.data(), nn, s->d_ncc, s->ncc_patterns);
   s->upload_real(s->d_coef, s->mat.coef.data(), nn);
   s->upload_raw(s->d_mat, s->mat.cell_mat.data(), (size_t)nc * 4);
   s->sym = symmetry_class(s->mat);
@@ -241,13 +239,13 @@ void table_sensors(pn_solver *s, const std::vector<std::pair<int32_t, int32_t>> 
   s->upload_raw(s->d_sidx, ix.data(), ix.size() * 4);
 }
 
-template <typename T>
-void table_args(pn_solver *s, VelArgs<T> &va, StressArgs<T> &sa) {
+template <typename T, bool OWN>
+void table_args(pn_solver *s, VelArgs<T, OWN> &va, StressArgs<T, OWN> &sa) {
   std::memset(&va, 0, sizeof(va));
   std::memset(&sa, 0, sizeof(sa));
   va.n_nodes = s->mesh.n_nodes;
   va.ncc = s->d_ncc;
-  va.con = connectivity(s->n_con);
+  va.n_patterns = s->ncc_patterns;
   T *const *V = (T *const *)s->V[0];
   T *const *S = (T *const *)s->S[0];
   va.V0 = V[0]; va.V1 = V[1]; va.V2 = V[2];
@@ -257,7 +255,6 @@ void table_args(pn_solver *s, VelArgs<T> &va, StressArgs<T> &sa) {
   va.gy = to_store<T>(0.25 / s->mesh.hy);
   va.gz = to_store<T>(0.25 / s->mesh.hz);
   va.gnode = (const T *)s->d_gnode;
-  va.rnode = (const T *)s->d_rnode;
   if (s->n_force > 0) {
     va.tile_src = s->d_ftile; va.src_elem = s->d_felem; va.src_code = s->d_fcode;
     va.src_w = (const T *)s->d_fw;
@@ -271,14 +268,13 @@ void table_args(pn_solver *s, VelArgs<T> &va, StressArgs<T> &sa) {
   }
   sa.n_cells = s->mesh.n_cells;
   sa.hex = s->d_hex;
-  sa.con = connectivity(s->c_con);
+  sa.n_patterns = s->hex_patterns;
   sa.V0 = V[0]; sa.V1 = V[1]; sa.V2 = V[2];
   sa.S0 = S[0]; sa.S1 = S[1]; sa.S2 = S[2]; sa.S3 = S[3]; sa.S4 = S[4]; sa.S5 = S[5];
   sa.mat = s->d_mat;
   sa.ctab = (const T *)s->d_ctab;
   sa.gx = va.gx; sa.gy = va.gy; sa.gz = va.gz;
   sa.gcell = (const T *)s->d_gcell;
-  sa.rcell = (const T *)s->d_rcell;
   sa.dt = to_store<T>(s->dt);
   if (s->n_moment > 0) {
     sa.tile_src = s->d_mtile; sa.src_elem = s->d_melem; sa.src_code = s->d_mcode;
@@ -290,23 +286,25 @@ void table_args(pn_solver *s, VelArgs<T> &va, StressArgs<T> &sa) {
   sa.has_moments = s->has_moments ? 1 : 0;
   sa.sym = s->sym;
 }
-template void table_args<double>(pn_solver *, VelArgs<double> &, StressArgs<double> &);
-template void table_args<float>(pn_solver *, VelArgs<float> &, StressArgs<float> &);
-template void table_args<float2>(pn_solver *, VelArgs<float2> &, StressArgs<float2> &);
+template void table_args<double, false>(pn_solver *, VelArgs<double> &, StressArgs<double> &);
+template void table_args<float, false>(pn_solver *, VelArgs<float> &, StressArgs<float> &);
+template void table_args<float2, false>(pn_solver *, VelArgs<float2> &, StressArgs<float2> &);
 
 namespace {
 
 template <typename T>
 void run(pn_solver *s, int32_t nsteps) {
-  VelArgs<T> va;
-  StressArgs<T> sa;
+  VelLaunch<T> va{};
+  StressLaunch<T> sa{};
   const int64_t nsig = (int64_t)s->src.size();
   int32_t done = 0;
   while (done < nsteps) {
     int32_t chunk = nsteps - done;
     ensure_signal_rows(s, chunk);
     // (after it: the table's room may have come from the exact form's reciprocals)
-    table_args<T>(s, va, sa);
+    table_args(s, va, sa);
+    va.recips = (const T *)s->d_rnode;
+    sa.recips = (const T *)s->d_rcell;
     if (nsig > 0 && !s->sig_hold)
       chunk = (int32_t)std::min<int64_t>(chunk, s->sig_step0 + s->sig_rows - s->step);
     va.rec_base = s->rec_count;

@@ -28,22 +28,33 @@ constexpr int kTile = 256;  // elements per tile == threads per block
 // so neither a copy nor a wait for the steps in flight
 constexpr int kSignalsHere = 8;
 
+// What only a solver's own launches take (VelLaunch, StressLaunch, GridLaunch).
+// The blocks that a batch's kernels read (VelArgs, StressArgs, GridArgs) are
+// staged on the device, one per member, in the allocation-free call in a scratch
+// of fixed size, and hold nothing that a batch does not use.
+template <typename T, bool OWN>
+struct OwnLaunch {};
+template <typename T>
+struct OwnLaunch<T, true> {
+  int32_t sig_here;    // 1: this step's values are sig_vals
+  T sig_vals[kSignalsHere];
+  const T *recips;     // exact form: the reciprocals of the spacings in two words (k_reciprocals), or null
+};
+
 // Connectivity as patterns (fast forms): an element's eight neighbours are its
 // base plus the offsets of its pattern.  Meshes numbered along lattice lines,
 // graded, holed or cracked ones too, have a few dozen patterns (interior, faces,
 // edges, rims), so an element takes 5 bytes instead of 32; a mesh with more than
 // 256 keeps the tables.  A missing cell's offset is INT32_MIN (base + it < 0).
-struct Connectivity {
-  const int32_t *__restrict__ base;     // [elements]
-  const uint8_t *__restrict__ pattern;  // [elements], null: the table
-  const int4 *__restrict__ offset;      // [patterns * 2]
-};
+// In one allocation: the patterns' offsets (two int4 each), the elements' bases
+// (int32), their pattern numbers (uint8); n_patterns 0: the table, two int4 an
+// element.
 
-template <typename T>
-struct VelArgs {
+template <typename T, bool OWN = false>
+struct VelArgs : OwnLaunch<T, OWN> {
   int32_t n_nodes;
-  const int4 *__restrict__ ncc;  // [n_nodes*2]
-  Connectivity con;              // ... or, when con.pattern is set, as patterns
+  int32_t n_patterns;
+  const int4 *__restrict__ ncc;  // the nodes' cells: table or patterns
   T *V0;
   T *V1;
   T *V2;
@@ -58,7 +69,6 @@ struct VelArgs {
   // (fast forms: 0.25/d; exact form: d)
   T gx, gy, gz;
   const T *__restrict__ gnode;
-  const T *__restrict__ rnode;  // exact form only: reciprocal spacings [3][n_nodes] (exact_reciprocal)
   // force sources
   const int2 *__restrict__ tile_src;  // [n_tiles] or null
   const int32_t *__restrict__ src_elem;
@@ -68,8 +78,6 @@ struct VelArgs {
   int32_t n_sig;
   int32_t sig_stride;            // 0 when sigval already points at this step's row
   int32_t sig_rows;
-  int32_t sig_here;              // 1: this step's values are sig_vals
-  T sig_vals[kSignalsHere];
   // sensors
   const int2 *__restrict__ tile_sens;  // [n_tiles] or null
   const int32_t *__restrict__ sens_node;
@@ -80,11 +88,10 @@ struct VelArgs {
   int64_t rec_cap;
 };
 
-template <typename T>
-struct StressArgs {
+template <typename T, bool OWN = false>
+struct StressArgs : OwnLaunch<T, OWN> {
   int32_t n_cells;
-  const int4 *__restrict__ hex;  // [n_cells*2]
-  Connectivity con;              // ... or as patterns
+  int32_t n_patterns;
   const T *V0;
   const T *V1;
   const T *V2;
@@ -94,11 +101,13 @@ struct StressArgs {
   T *S3;
   T *S4;
   T *S5;
+  // the cells' nodes: table or patterns (ahead of V0 it leaves the pointers on 16
+  // bytes, and FP32 k_stress spills: graded plate 200 x 200 x 40 1.19 instead of 1.15 ms)
+  const int4 *__restrict__ hex;
   const int32_t *__restrict__ mat;
   const T *__restrict__ ctab;
   T gx, gy, gz;
   const T *__restrict__ gcell;  // per cell [3][n_cells] or null
-  const T *__restrict__ rcell;  // exact form only: reciprocal spacings [3][n_cells]
   T dt;                          // exact form only (fast forms fold dt into ctab)
   // moment sources
   const int2 *__restrict__ tile_src;
@@ -109,12 +118,19 @@ struct StressArgs {
   int32_t n_sig;
   int32_t sig_stride;
   int32_t sig_rows;
-  int32_t sig_here;
-  T sig_vals[kSignalsHere];
   int32_t has_moments;
   int32_t sym;  // symmetry class of the whole stiffness table (symmetry_class): 0 general, 1 monoclinic
                 // about z, 2 orthotropic
 };
+
+template <typename T> using VelLaunch = VelArgs<T, true>;
+template <typename T> using StressLaunch = StressArgs<T, true>;
+
+// whether an argument block is a solver's own launch's
+template <typename A, typename = void>
+struct is_launch : std::false_type {};
+template <typename A>
+struct is_launch<A, std::void_t<decltype(A::sig_here)>> : std::true_type {};
 
 #ifdef __CUDACC__
 // Programmatic dependent launch between the kernels of consecutive half
@@ -140,15 +156,16 @@ inline cudaError_t launch_overlapped(F f, dim3 grid, unsigned threads, size_t sm
   return cudaLaunchKernelEx(&cfg, f, args...);
 }
 
-// the eight neighbours of element i: by its pattern, or from the table
-__device__ __forceinline__ void neighbours(const Connectivity &con, const int4 *__restrict__ table, int i, int s[8]) {
+// the eight neighbours of element i of n: by its pattern, or from the table
+__device__ __forceinline__ void neighbours(const int4 *__restrict__ table, int n_patterns, int n, int i, int s[8]) {
   int4 lo, hi;
   int b = 0;
-  if (con.pattern) {
-    const int p = con.pattern[i];
-    b = con.base[i];
-    lo = __ldg(con.offset + 2 * p);
-    hi = __ldg(con.offset + 2 * p + 1);
+  if (n_patterns > 0) {
+    const int32_t *__restrict__ base = reinterpret_cast<const int32_t *>(table + 2 * n_patterns);
+    const int p = (reinterpret_cast<const uint8_t *>(base + n))[i];
+    b = base[i];
+    lo = __ldg(table + 2 * p);
+    hi = __ldg(table + 2 * p + 1);
   } else {
     lo = table[2 * i];
     hi = table[2 * i + 1];
@@ -161,19 +178,21 @@ __device__ __forceinline__ void neighbours(const Connectivity &con, const int4 *
 // the table (null: no sources)
 template <typename A>
 __device__ __forceinline__ auto signal_row(const A &a, int step) -> decltype(a.sigval) {
-  if (a.sig_here) return a.sig_vals;
+  if constexpr (is_launch<A>::value) {
+    if (a.sig_here) return a.sig_vals;
+  }
   return a.sigval ? a.sigval + (int64_t)min(step, a.sig_rows - 1) * a.sig_stride : nullptr;
 }
 #endif
 
 // Launchers (defined in rsg_fast.cu / rsg_exact.cu).  step = index of this
 // step inside the current solve() call (selects the signal row).
-cudaError_t launch_velocity_f64(const VelArgs<double> &a, int step, bool uniform, cudaStream_t st);
-cudaError_t launch_stress_f64(const StressArgs<double> &a, int step, bool uniform, cudaStream_t st);
-cudaError_t launch_velocity_f32(const VelArgs<float> &a, int step, bool uniform, cudaStream_t st);
-cudaError_t launch_stress_f32(const StressArgs<float> &a, int step, bool uniform, cudaStream_t st);
-cudaError_t launch_velocity_df64(const VelArgs<float2> &a, int step, bool uniform, cudaStream_t st);
-cudaError_t launch_stress_df64(const StressArgs<float2> &a, int step, bool uniform, cudaStream_t st);
+cudaError_t launch_velocity_f64(const VelLaunch<double> &a, int step, bool uniform, cudaStream_t st);
+cudaError_t launch_stress_f64(const StressLaunch<double> &a, int step, bool uniform, cudaStream_t st);
+cudaError_t launch_velocity_f32(const VelLaunch<float> &a, int step, bool uniform, cudaStream_t st);
+cudaError_t launch_stress_f32(const StressLaunch<float> &a, int step, bool uniform, cudaStream_t st);
+cudaError_t launch_velocity_df64(const VelLaunch<float2> &a, int step, bool uniform, cudaStream_t st);
+cudaError_t launch_stress_df64(const StressLaunch<float2> &a, int step, bool uniform, cudaStream_t st);
 // a batch of table-form members: device arrays of their argument blocks and
 // the prefix sums of their tile counts (members own consecutive tiles)
 struct BatchLaunch {
@@ -193,7 +212,7 @@ cudaError_t launch_table_batch_halves(const BatchLaunch &b, int precision, int s
 // rec[i], rec[i + n]: the two words of the reciprocal of spacing d[i] as the
 // exact kernels take it (rsg_exact.cu)
 cudaError_t launch_exact_reciprocals(const double *d, int64_t n, double *rec, cudaStream_t st);
-cudaError_t launch_velocity_exact(const VelArgs<double> &a, int step, cudaStream_t st);
-cudaError_t launch_stress_exact(const StressArgs<double> &a, int step, cudaStream_t st);
+cudaError_t launch_velocity_exact(const VelLaunch<double> &a, int step, cudaStream_t st);
+cudaError_t launch_stress_exact(const StressLaunch<double> &a, int step, cudaStream_t st);
 
 }  // namespace pn

@@ -223,7 +223,7 @@ __host__ __device__ constexpr bool c_used(int sym, int k, int j) {  // as in rsg
 }
 
 // sensor traces: V after this step at the sensors of this tile
-__device__ __forceinline__ void record(const VelArgs<double> &a, int n, int step, double v0,
+__device__ __forceinline__ void record(const VelLaunch<double> &a, int n, int step, double v0,
                                        double v1, double v2) {
   if (!a.tile_sens) return;
   const int2 r = a.tile_sens[blockIdx.x];
@@ -238,7 +238,7 @@ __device__ __forceinline__ void record(const VelArgs<double> &a, int n, int step
   }
 }
 
-__global__ void __launch_bounds__(kTile) k_velocity_exact(const __grid_constant__ VelArgs<double> a, int step) {
+__global__ void __launch_bounds__(kTile) k_velocity_exact(const __grid_constant__ VelLaunch<double> a, int step) {
   let_next_start();
   const int n = blockIdx.x * kTile + threadIdx.x;
   if (n >= a.n_nodes) return;
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(kTile) k_velocity_exact(const __grid_constant_
   }
   const int s[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
   const int64_t ny = (int64_t)a.n_nodes + n, nz = 2 * (int64_t)a.n_nodes + n, n3 = 3 * (int64_t)a.n_nodes;
-  Divisor dx(a.gnode[n], a.rnode, n, n3), dy(a.gnode[ny], a.rnode, ny, n3), dz(a.gnode[nz], a.rnode, nz, n3);
+  Divisor dx(a.gnode[n], a.recips, n, n3), dy(a.gnode[ny], a.recips, ny, n3), dz(a.gnode[nz], a.recips, nz, n3);
   double xd[3] = {0., 0., 0.};
   bool sourced = false;
   if (a.tile_src) {
@@ -296,14 +296,14 @@ __global__ void __launch_bounds__(kTile) k_velocity_exact(const __grid_constant_
 }
 
 template <int SYM, bool MOMENTS>
-__global__ void __launch_bounds__(kTile) k_stress_exact(const __grid_constant__ StressArgs<double> a, int step) {
+__global__ void __launch_bounds__(kTile) k_stress_exact(const __grid_constant__ StressLaunch<double> a, int step) {
   let_next_start();
   const int c = blockIdx.x * kTile + threadIdx.x;
   if (c >= a.n_cells) return;
   const int4 lo = a.hex[2 * c], hi = a.hex[2 * c + 1];
   const int s[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
   const int64_t cy = (int64_t)a.n_cells + c, cz = 2 * (int64_t)a.n_cells + c, n3 = 3 * (int64_t)a.n_cells;
-  Divisor dx(a.gcell[c], a.rcell, c, n3), dy(a.gcell[cy], a.rcell, cy, n3), dz(a.gcell[cz], a.rcell, cz, n3);
+  Divisor dx(a.gcell[c], a.recips, c, n3), dy(a.gcell[cy], a.recips, cy, n3), dz(a.gcell[cz], a.recips, cz, n3);
   const double *V[3] = {a.V0, a.V1, a.V2};
   wait_previous();  // (tables only so far)
   // v[j][i], d[j][i]: velocity component j along axis i
@@ -377,13 +377,13 @@ cudaError_t launch_exact_reciprocals(const double *d, int64_t n, double *rec, cu
   return cudaGetLastError();
 }
 
-cudaError_t launch_velocity_exact(const VelArgs<double> &a, int step, cudaStream_t st) {
+cudaError_t launch_velocity_exact(const VelLaunch<double> &a, int step, cudaStream_t st) {
   if (a.n_nodes <= 0) return cudaSuccess;
   const unsigned grid = (unsigned)((a.n_nodes + kTile - 1) / kTile);
   return launch_overlapped(k_velocity_exact, dim3(grid), kTile, 0, st, a, step);
 }
 
-cudaError_t launch_stress_exact(const StressArgs<double> &a, int step, cudaStream_t st) {
+cudaError_t launch_stress_exact(const StressLaunch<double> &a, int step, cudaStream_t st) {
   if (a.n_cells <= 0) return cudaSuccess;
   const unsigned grid = (unsigned)((a.n_cells + kTile - 1) / kTile);
   auto run = [&](auto kernel) { return launch_overlapped(kernel, dim3(grid), kTile, 0, st, a, step); };

@@ -119,13 +119,12 @@ __device__ __forceinline__ void gather_nodes(const typename Num<R>::S *f, const 
 }
 
 // velocity update of node n (tile = n / kTile, step within the call)
-template <typename R, bool UNIFORM, bool OVERLAP = false>
-__device__ __forceinline__ void velocity_node(const VelArgs<typename Num<R>::S> &a, int n, int tile,
-                                              int step) {
+template <typename R, bool UNIFORM, bool OVERLAP = false, typename A>
+__device__ __forceinline__ void velocity_node(const A &a, int n, int tile, int step) {
   using N = Num<R>;
   const R cf = N::get(a.coef, n);
   int s[8];
-  neighbours(a.con, a.ncc, n, s);
+  neighbours(a.ncc, a.n_patterns, a.n_nodes, n, s);
   if (OVERLAP) wait_previous();  // (tables only so far)
   R v0 = N::get(a.V0, n), v1 = N::get(a.V1, n), v2 = N::get(a.V2, n);
   if (!(cf == R())) {  // a zero coefficient marks a node owned by another partition
@@ -228,12 +227,11 @@ __host__ __device__ constexpr bool c_used(int sym, int k, int j) {
 }
 
 // stress update of cell c
-template <typename R, bool UNIFORM, int SYM, bool OVERLAP = false>
-__device__ __forceinline__ void stress_cell(const StressArgs<typename Num<R>::S> &a, int c, int tile,
-                                            int step) {
+template <typename R, bool UNIFORM, int SYM, bool OVERLAP = false, typename A>
+__device__ __forceinline__ void stress_cell(const A &a, int c, int tile, int step) {
   using N = Num<R>;
   int s[8];
-  neighbours(a.con, a.hex, c, s);
+  neighbours(a.hex, a.n_patterns, a.n_cells, c, s);
   R gx = N::val(a.gx), gy = N::val(a.gy), gz = N::val(a.gz);
   if (!UNIFORM) {
     gx = N::get(a.gcell, c);
@@ -287,14 +285,14 @@ __device__ __forceinline__ void stress_cell(const StressArgs<typename Num<R>::S>
 }
 
 template <typename R, bool UNIFORM>
-__global__ void __launch_bounds__(kTile) k_velocity(const __grid_constant__ VelArgs<typename Num<R>::S> a, int step) {
+__global__ void __launch_bounds__(kTile) k_velocity(const __grid_constant__ VelLaunch<typename Num<R>::S> a, int step) {
   let_next_start();
   const int n = blockIdx.x * kTile + threadIdx.x;
   if (n < a.n_nodes) velocity_node<R, UNIFORM, true>(a, n, blockIdx.x, step);
 }
 
 template <typename R, bool UNIFORM, int SYM>
-__global__ void __launch_bounds__(kTile) k_stress(const __grid_constant__ StressArgs<typename Num<R>::S> a, int step) {
+__global__ void __launch_bounds__(kTile) k_stress(const __grid_constant__ StressLaunch<typename Num<R>::S> a, int step) {
   let_next_start();
   const int c = blockIdx.x * kTile + threadIdx.x;
   if (c < a.n_cells) stress_cell<R, UNIFORM, SYM, true>(a, c, blockIdx.x, step);
@@ -388,7 +386,7 @@ __global__ void __launch_bounds__(kTile) k_stress_batch(const StressArgs<typenam
 }
 
 template <typename R>
-cudaError_t launch_vel(const VelArgs<typename Num<R>::S> &a, int step, bool uniform, cudaStream_t st) {
+cudaError_t launch_vel(const VelLaunch<typename Num<R>::S> &a, int step, bool uniform, cudaStream_t st) {
   if (a.n_nodes <= 0) return cudaSuccess;
   const unsigned grid = (unsigned)((a.n_nodes + kTile - 1) / kTile);
   return uniform ? launch_overlapped(k_velocity<R, true>, dim3(grid), kTile, 0, st, a, step)
@@ -396,14 +394,14 @@ cudaError_t launch_vel(const VelArgs<typename Num<R>::S> &a, int step, bool unif
 }
 
 template <typename R, int SYM>
-cudaError_t launch_str_sym(const StressArgs<typename Num<R>::S> &a, int step, bool uniform, cudaStream_t st) {
+cudaError_t launch_str_sym(const StressLaunch<typename Num<R>::S> &a, int step, bool uniform, cudaStream_t st) {
   const unsigned grid = (unsigned)((a.n_cells + kTile - 1) / kTile);
   return uniform ? launch_overlapped(k_stress<R, true, SYM>, dim3(grid), kTile, 0, st, a, step)
                  : launch_overlapped(k_stress<R, false, SYM>, dim3(grid), kTile, 0, st, a, step);
 }
 
 template <typename R>
-cudaError_t launch_str(const StressArgs<typename Num<R>::S> &a, int step, bool uniform, cudaStream_t st) {
+cudaError_t launch_str(const StressLaunch<typename Num<R>::S> &a, int step, bool uniform, cudaStream_t st) {
   if (a.n_cells <= 0) return cudaSuccess;
   if (a.sym == 2) return launch_str_sym<R, 2>(a, step, uniform, st);
   if (a.sym == 1) return launch_str_sym<R, 1>(a, step, uniform, st);
@@ -445,22 +443,22 @@ cudaError_t launch_batch(const BatchLaunch &b, int step, int halves, cudaStream_
 
 }  // namespace
 
-cudaError_t launch_velocity_f64(const VelArgs<double> &a, int step, bool uniform, cudaStream_t st) {
+cudaError_t launch_velocity_f64(const VelLaunch<double> &a, int step, bool uniform, cudaStream_t st) {
   return launch_vel<double>(a, step, uniform, st);
 }
-cudaError_t launch_stress_f64(const StressArgs<double> &a, int step, bool uniform, cudaStream_t st) {
+cudaError_t launch_stress_f64(const StressLaunch<double> &a, int step, bool uniform, cudaStream_t st) {
   return launch_str<double>(a, step, uniform, st);
 }
-cudaError_t launch_velocity_f32(const VelArgs<float> &a, int step, bool uniform, cudaStream_t st) {
+cudaError_t launch_velocity_f32(const VelLaunch<float> &a, int step, bool uniform, cudaStream_t st) {
   return launch_vel<float>(a, step, uniform, st);
 }
-cudaError_t launch_stress_f32(const StressArgs<float> &a, int step, bool uniform, cudaStream_t st) {
+cudaError_t launch_stress_f32(const StressLaunch<float> &a, int step, bool uniform, cudaStream_t st) {
   return launch_str<float>(a, step, uniform, st);
 }
-cudaError_t launch_velocity_df64(const VelArgs<float2> &a, int step, bool uniform, cudaStream_t st) {
+cudaError_t launch_velocity_df64(const VelLaunch<float2> &a, int step, bool uniform, cudaStream_t st) {
   return launch_vel<df64>(a, step, uniform, st);
 }
-cudaError_t launch_stress_df64(const StressArgs<float2> &a, int step, bool uniform, cudaStream_t st) {
+cudaError_t launch_stress_df64(const StressLaunch<float2> &a, int step, bool uniform, cudaStream_t st) {
   return launch_str<df64>(a, step, uniform, st);
 }
 cudaError_t launch_table_batch(const BatchLaunch &b, int precision, int step, cudaStream_t st) {

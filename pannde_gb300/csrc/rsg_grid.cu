@@ -78,8 +78,8 @@ __host__ __device__ constexpr bool c_used(int sym, int k, int j) {
 }
 
 // one block's work: tile (bx, by) of a grid with gxc tiles along x, z chunk bz
-template <typename R, int TX, int TY, int SYM>
-__device__ __forceinline__ void grid_block(const GridArgs<typename GNum<R>::S> &a, int bx, int by, int bz,
+template <typename R, int TX, int TY, int SYM, typename A>
+__device__ __forceinline__ void grid_block(const A &a, int bx, int by, int bz,
                                            int gxc, int step) {
   using N = GNum<R>;
   using St = typename N::S;
@@ -306,7 +306,7 @@ __device__ __forceinline__ void grid_block(const GridArgs<typename GNum<R>::S> &
 }
 
 template <typename R, int TX, int TY, int SYM>
-__global__ void __launch_bounds__(TX *TY) k_grid_step(const __grid_constant__ GridArgs<typename GNum<R>::S> a,
+__global__ void __launch_bounds__(TX *TY) k_grid_step(const __grid_constant__ GridLaunch<typename GNum<R>::S> a,
                                                         int step) {
   grid_block<R, TX, TY, SYM>(a, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x, step);
 }
@@ -364,12 +364,12 @@ struct Setup {
 };
 
 template <typename R, int TX, int TY, int SYM>
-cudaError_t launch_t(const GridArgs<typename GNum<R>::S> &a, cudaStream_t st) {
+cudaError_t launch_t(const GridLaunch<typename GNum<R>::S> &a, cudaStream_t st) {
   using S = Setup<R, TX, TY, SYM>;
   int sms = 0, per_sm = 0;
   cudaError_t e = S::ensure(sms, per_sm);
   if (e != cudaSuccess) return e;
-  GridArgs<typename GNum<R>::S> b = a;
+  GridLaunch<typename GNum<R>::S> b = a;
   const unsigned gx = (unsigned)(a.nx / (TX - 1) + 1), gy = (unsigned)(a.ny / (TY - 1) + 1);
   if (b.kchunk <= 0) b.kchunk = grid_chunk_for(a.nz, (long long)gx * gy, sms, per_sm);
   const dim3 grid(gx, gy, (unsigned)((a.nz + b.kchunk - 1) / b.kchunk));
@@ -390,7 +390,7 @@ cudaError_t launch_batch_t(const GridBatchLaunch &b, int step, cudaStream_t st) 
 }
 
 template <typename R>
-cudaError_t launch_sym(const GridArgs<typename GNum<R>::S> &a, int sym, cudaStream_t st) {
+cudaError_t launch_sym(const GridLaunch<typename GNum<R>::S> &a, int sym, cudaStream_t st) {
   if (a.nx <= 0 || a.ny <= 0 || a.nz <= 0) return cudaSuccess;
   if (sym == 2) return launch_t<R, 32, 8, 2>(a, st);
   if (sym == 1) return launch_t<R, 32, 8, 1>(a, st);
@@ -527,13 +527,13 @@ int grid_chunk_layers(int precision, const std::map<int, long long> &tops, bool 
   return grid_chunk_for(tops, sms, per_sm);
 }
 
-cudaError_t launch_grid_f32(const GridArgs<float> &a, int sym, cudaStream_t st) {
+cudaError_t launch_grid_f32(const GridLaunch<float> &a, int sym, cudaStream_t st) {
   return launch_sym<float>(a, sym, st);
 }
-cudaError_t launch_grid_f64(const GridArgs<double> &a, int sym, cudaStream_t st) {
+cudaError_t launch_grid_f64(const GridLaunch<double> &a, int sym, cudaStream_t st) {
   return launch_sym<double>(a, sym, st);
 }
-cudaError_t launch_grid_df64(const GridArgs<float2> &a, int sym, cudaStream_t st) {
+cudaError_t launch_grid_df64(const GridLaunch<float2> &a, int sym, cudaStream_t st) {
   return launch_sym<df64>(a, sym, st);
 }
 cudaError_t launch_grid_batch(const GridBatchLaunch &b, int precision, int step, cudaStream_t st) {

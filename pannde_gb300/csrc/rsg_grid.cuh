@@ -32,23 +32,23 @@ struct FixCell {
   int32_t m0, m1;     // its moment entries [m0, m1)
 };
 
-// A thread's own entries of its (block, layer) slot without a search
-// (tensor-copy kernel): id gives a non-empty slot its number (-1: empty); rows
-// holds per slot and tile row one bit per lane with entries and where the
-// row's first entry lies, so a lane's own is found by counting bits.  With
-// more than one entry at some node of the slot (bit 31 of the second word)
-// that place counts the slot's nodes instead, and node[] holds where each
-// one's entries begin (and the slot's end).  Every lane reading through a
-// slot of a few hundred entries, or searching it, was the longest serial
-// chain of a small lattice's step: a dependent load per probe.
-struct SlotIndex {
-  const int32_t *id;    // [blocks][layers]
-  const uint2 *rows;    // [slots][tile rows]
-  const int32_t *node;
+// where the slots' rows lie: int32 per slot, behind the ranges (slot_entries)
+struct SlotPlaces {
+  const int32_t *f, *m, *s;
 };
 
+template <typename T, bool OWN>
+struct OwnGridLaunch {};
 template <typename T>
-struct GridArgs {
+struct OwnGridLaunch<T, true> : OwnLaunch<T, true> {
+  int32_t fp64_chunk;  // FP64 form: layers per piece of a column on the FP64 path (0: not cut)
+  // (found from the ranges' addresses by every block, a 64 x 64 x 8 plate's FP32
+  // step took 5.20 us instead of 5.16, a 400 x 400 x 40 laminate's 98.7 instead of 98.3)
+  SlotPlaces places;
+};
+
+template <typename T, bool OWN = false>
+struct GridArgs : OwnGridLaunch<T, OWN> {
   int32_t nx, ny, nz;  // cells per axis
   int32_t pnx, pcx;    // row pitch (sites) of node / cell buffers
   int32_t kchunk;      // cell layers per block along z (set by the launcher when 0)
@@ -65,23 +65,18 @@ struct GridArgs {
   const int32_t *f_key;  // local node | direction << 16
   const int32_t *f_sig;
   const T *f_w;
-  SlotIndex f_ix;
   // moment sources, ranges per (block, cell layer): [blocks][nz]
   const int2 *m_rng;
   const int32_t *m_key;  // local cell | Voigt component << 16
   const int32_t *m_sig;
   const T *m_w;          // weights carry dt
-  SlotIndex m_ix;
   const T *sigval;       // signal rows: row min(step, sig_rows-1) at stride sig_stride
   int32_t sig_stride;    // 0 when sigval already points at the step's row
   int32_t sig_rows;
-  int32_t sig_here;      // 1: this step's values are sig_vals
-  T sig_vals[kSignalsHere];
   // sensors, ranges per (block, node layer)
   const int2 *s_rng;
   const int32_t *s_key;  // local node
   const int32_t *s_idx;  // sensor number
-  SlotIndex s_ix;
   double *traces;        // [records][n_sens][3]
   int32_t n_sens;
   int64_t rec;           // record written by step 0 of the launch (rec + step later)
@@ -121,8 +116,25 @@ struct GridArgs {
   // column into chunks of tail_chunk layers, chunk-major (the last partial wave
   // of whole columns would leave most SMs idle); 0: the 3D grid of kchunk chunks
   int32_t tail_from, tail_chunk;
-  int32_t fp64_chunk;  // FP64 form: layers per piece of a column on the FP64 path (0: not cut)
 };
+
+// a solver's own launch
+template <typename T> using GridLaunch = GridArgs<T, true>;
+
+// the places of a block's own launch, or found from the ranges (null: no list)
+template <typename T>
+#ifdef __CUDACC__
+__host__ __device__ __forceinline__
+#else
+inline
+#endif
+SlotPlaces slot_places(const T &a, int tile_rows) {
+  const int64_t tiles = (int64_t)(a.nx / 31 + 1) * (a.ny / (tile_rows - 1) + 1);
+  auto of = [&](const int2 *rng, int64_t slots) {
+    return rng ? reinterpret_cast<const int32_t *>(rng + slots) : nullptr;
+  };
+  return SlotPlaces{of(a.f_rng, tiles * (a.nz + 1)), of(a.m_rng, tiles * a.nz), of(a.s_rng, tiles * (a.nz + 1))};
+}
 
 // where a thread's scan of its (block, layer) slot starts (classic kernel): the entries are
 // sorted by local index (key & 0xffff), so in a long slot (a transducer patch
@@ -131,6 +143,12 @@ struct GridArgs {
 // is scanned from its start.  The scan skips entries of smaller local index
 // and stops at the first larger one.
 #ifdef __CUDACC__
+template <typename Args>
+__device__ __forceinline__ SlotPlaces places_of(const Args &a, int tile_rows) {
+  if constexpr (is_launch<Args>::value) return a.places;
+  else return slot_places(a, tile_rows);
+}
+
 __device__ __forceinline__ int first_local(const int32_t *__restrict__ key, int lo, int hi, int t) {
   if (hi - lo <= 32) return lo;  // a short slot: scanned from its start (independent loads)
   while (lo < hi) {
@@ -141,14 +159,23 @@ __device__ __forceinline__ int first_local(const int32_t *__restrict__ key, int 
   return lo;
 }
 
-// entries [x, y) of lane tx of tile row ty (TY rows) in slot `id`
-template <int TY>
-__device__ __forceinline__ int2 slot_entries(const SlotIndex &ix, int id, int tx, int ty) {
-  if (id < 0) return make_int2(0, 0);
-  const uint2 r = __ldg(ix.rows + (int64_t)id * TY + ty);
+// A thread's own entries of its (block, layer) slot without a search
+// (tensor-copy kernel).  Behind the ranges of a list lie, in the same allocation,
+// per slot the place of its rows (SlotPlaces; -1: no entry), counted in 8-byte
+// words from the ranges' start; the rows, per tile row one bit per lane with
+// entries and where the row's first entry lies, so a lane's own is found by
+// counting bits; and lists: with more than one entry at some node of the slot (bit
+// 31 of the second word) that place is one in 4-byte words from the ranges' start,
+// where a list says where each node's entries begin (and the slot's end).  Every
+// lane reading through a slot of a few hundred entries, or searching it, was the
+// longest serial chain of a small lattice's step: a dependent load per probe.
+__device__ __forceinline__ int2 slot_entries(const int2 *rng, int at, int tx, int ty) {
+  if (at < 0) return make_int2(0, 0);
+  const uint2 r = __ldg(reinterpret_cast<const uint2 *>(rng) + at + ty);
   if (!((r.x >> tx) & 1u)) return make_int2(0, 0);
   const int n = (int)(r.y & 0x7fffffffu) + __popc(r.x & ((1u << tx) - 1u));
-  if (r.y >> 31) return make_int2(__ldg(ix.node + n), __ldg(ix.node + n + 1));
+  const int32_t *words = reinterpret_cast<const int32_t *>(rng);
+  if (r.y >> 31) return make_int2(__ldg(words + n), __ldg(words + n + 1));
   return make_int2(n, n + 1);
 }
 #endif
@@ -198,9 +225,9 @@ struct GridBatchLaunch {
   const int *order = nullptr;
 };
 cudaError_t launch_grid_batch(const GridBatchLaunch &b, int precision, int step, cudaStream_t st);
-cudaError_t launch_grid_f32(const GridArgs<float> &a, int sym, cudaStream_t st);
-cudaError_t launch_grid_f64(const GridArgs<double> &a, int sym, cudaStream_t st);
-cudaError_t launch_grid_df64(const GridArgs<float2> &a, int sym, cudaStream_t st);
+cudaError_t launch_grid_f32(const GridLaunch<float> &a, int sym, cudaStream_t st);
+cudaError_t launch_grid_f64(const GridLaunch<double> &a, int sym, cudaStream_t st);
+cudaError_t launch_grid_df64(const GridLaunch<float2> &a, int sym, cudaStream_t st);
 
 // tensor-copy kernel (rsg_grid_tma.cu): maps of one input parity occupy
 // grid_tma_maps_bytes(); encoding fails (false) when a buffer or pitch does not
@@ -212,13 +239,13 @@ bool grid_tma_encode(int precision, int tile_rows, int nx, int ny, int nz, int p
                      const void *const V[3], const void *const S[6], const void *coef, const uint8_t *mat,
                      void *out);
 int grid_tma_blocks_per_sm(int precision, int tile_rows = kGridTileRows);
-cudaError_t launch_grid_tma(const void *args /* GridArgs<storage type> */, int precision, int sym,
+cudaError_t launch_grid_tma(const void *args /* GridLaunch<storage type> */, int precision, int sym,
                             cudaStream_t st);
 cudaError_t launch_grid_tma_batch(const GridBatchLaunch &b, int precision, int step, cudaStream_t st);
 
 // fix-up of split sites after a step launch (rsg_split.cu): the copies'
 // velocities, then the fix cells' stresses, from the step's input buffers
-cudaError_t launch_grid_split(const void *args /* GridArgs<storage type> */, int precision, cudaStream_t st);
+cudaError_t launch_grid_split(const void *args /* GridLaunch<storage type> */, int precision, cudaStream_t st);
 struct GridSplitBatch {
   int n_members;
   const void *args;         // GridArgs<S>[n_members] (device)

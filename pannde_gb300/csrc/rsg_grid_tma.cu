@@ -7,11 +7,11 @@
 namespace pn {
 
 // rsg_grid_tma16.cu
-cudaError_t launch_grid_tma_f32_rows16(const GridArgs<float> &a, int sym, cudaStream_t st);
+cudaError_t launch_grid_tma_f32_rows16(const GridLaunch<float> &a, int sym, cudaStream_t st);
 cudaError_t launch_grid_tma_batch_f32_rows16(const GridBatchLaunch &b, int step, cudaStream_t st);
 int grid_tma_blocks_per_sm_f32_rows16();
 // rsg_grid_tma_f64.cu
-cudaError_t launch_grid_tma_f64h(const GridArgs<double> &a, int sym, cudaStream_t st);
+cudaError_t launch_grid_tma_f64h(const GridLaunch<double> &a, int sym, cudaStream_t st);
 cudaError_t launch_grid_tma_batch_f64h(const GridBatchLaunch &b, int step, cudaStream_t st);
 
 namespace {
@@ -108,17 +108,17 @@ int grid_tma_blocks_per_sm(int precision, int tile_rows) {
 
 cudaError_t launch_grid_tma(const void *args, int precision, int sym, cudaStream_t st) {
   if (precision == 2) {
-    const GridArgs<float> &a = *(const GridArgs<float> *)args;
+    const GridLaunch<float> &a = *(const GridLaunch<float> *)args;
     if (a.tile_rows == 16) return launch_grid_tma_f32_rows16(a, sym, st);
     if (a.tile_rows != 8) return cudaErrorInvalidValue;
     return launch_sym<float, 8>(a, sym, st);
   }
   if (precision == 3) {
-    const GridArgs<float2> &a = *(const GridArgs<float2> *)args;
+    const GridLaunch<float2> &a = *(const GridLaunch<float2> *)args;
     if (a.tile_rows != 8) return cudaErrorInvalidValue;
     return launch_sym<df64, 8>(a, sym, st);
   }
-  const GridArgs<double> &a = *(const GridArgs<double> *)args;
+  const GridLaunch<double> &a = *(const GridLaunch<double> *)args;
   if (a.tile_rows != 8) return cudaErrorInvalidValue;
   if (a.rflags) return launch_grid_tma_f64h(a, sym, st);  // the FP64 form: per-block double-float / FP64 path
   return launch_sym<double, 8>(a, sym, st);

@@ -280,7 +280,7 @@ constexpr int32_t kErrWait = 1;
 
 // The block's tile copies: ring slots, barriers and the issue of one layer's
 // copies (layers [k0 - 1, k1] of tile (bx, by)).
-template <typename St, int TY, bool BATCH>
+template <typename St, int TY>
 struct Copies {
   using G = Geo<(int)sizeof(St), TY>;
   const GridMaps *M;
@@ -290,7 +290,8 @@ struct Copies {
   // the copies are issued (and, on failure, drained) by the first thread of
   // the last warp: its row is the tile's apron, which has no stress half
   static constexpr int ISSUER = (TY - 1) * TX;
-  __device__ __forceinline__ Copies(const GridArgs<St> &a, unsigned char *smem, int bx, int by, int k0_, int k1_)
+  template <typename Args>
+  __device__ __forceinline__ Copies(const Args &a, unsigned char *smem, int bx, int by, int k0_, int k1_)
       : M(reinterpret_cast<const GridMaps *>(a.tmaps)), k0(k0_), k1(k1_), skip(a.test_skip_layer) {
     // 128-byte aligned base, by an offset from the shared array, so that every
     // tile pointer stays in the shared state space (shared loads and stores,
@@ -360,17 +361,23 @@ struct Copies {
 
 // the tile's columns (and their apron) hold no solid cell at or above its top:
 // the march ends there, and a chunk above it has nothing to do
-template <typename T>
-__device__ __forceinline__ int tile_top(const GridArgs<T> &a, int blk) {
+template <typename Args>
+__device__ __forceinline__ int tile_top(const Args &a, int blk) {
   return a.ktop ? min(a.nz, __ldg(a.ktop + blk)) : a.nz;
+}
+
+// the FP64 form's layers per piece of a column (a batch's launches cut none)
+template <typename Args>
+__device__ __forceinline__ int fp64_chunk_of(const Args &a) {
+  if constexpr (is_launch<Args>::value) return a.fp64_chunk;
+  else return 0;
 }
 
 // RANGE (the FP64 form's kernel): every V and S value the block stores is
 // tested against the double-float range, and a block that stored one outside
 // it marks its tile for the FP64 path in the next step (range_flags_write).
-template <typename K, int SYM, int TY, bool BATCH = false, bool RANGE = false>
-__device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::S> &a,
-                                               const Copies<typename GNum<K>::S, TY, BATCH> &cp, int bx, int by,
+template <typename K, int SYM, int TY, bool RANGE = false, typename Args>
+__device__ __forceinline__ void grid_block_tma(const Args &a, const Copies<typename GNum<K>::S, TY> &cp, int bx, int by,
                                                bool last_chunk, int gxc, int step) {
   using N = GNum<K>;
   using R = typename N::R;
@@ -407,7 +414,7 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
   // (the FP64 form's kernel, short of registers, finds its row where it is used)
   const St *sigrow = RANGE ? nullptr : signal_row(a, step);
   const int oc = i0 - 1 - cp.xs_c, on = i0 - cp.xs_n, om = i0 - cp.xs_m;  // offsets in the copies
-  constexpr int ISSUER = Copies<St, TY, BATCH>::ISSUER;
+  constexpr int ISSUER = Copies<St, TY>::ISSUER;
   auto sslot = [&](int L) { return cp.sslot(L); };
   auto vslot = [&](int L) { return cp.vslot(L); };
   auto mslot = [&](int L) { return cp.mslot(L); };
@@ -417,13 +424,15 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
   // per-chunk tables: stiffness rows, source and sensor ranges
   for (int q = t; q < a.n_rows * 36; q += NT) sC[q] = N::tsto(N::val(a.ctab[q]));
   const int nL = k1 - k0 + 2;  // node layers k0-1 .. k1
+  const SlotPlaces sp = places_of(a, TY);
   for (int q = t; q < nL; q += NT) {
     const int k = k0 - 1 + q;
     const bool ok = k >= 0 && k <= nz;
-    sRf[q] = (a.f_ix.id && ok) ? __ldg(a.f_ix.id + (int64_t)blk * (nz + 1) + k) : -1;
-    sRs[q] = (a.s_ix.id && ok) ? __ldg(a.s_ix.id + (int64_t)blk * (nz + 1) + k) : -1;
+    const int64_t sl = (int64_t)blk * (nz + 1) + k;
+    sRf[q] = (sp.f && ok) ? __ldg(sp.f + sl) : -1;
+    sRs[q] = (sp.s && ok) ? __ldg(sp.s + sl) : -1;
   }
-  for (int q = t; q < k1 - k0; q += NT) sRm[q] = a.m_ix.id ? __ldg(a.m_ix.id + (int64_t)blk * nz + k0 + q) : -1;
+  for (int q = t; q < k1 - k0; q += NT) sRm[q] = sp.m ? __ldg(sp.m + (int64_t)blk * nz + k0 + q) : -1;
   if (!RANGE) wait_previous();  // (the FP64 form's blocks have waited to choose their path)
   __syncthreads();
   // split the stress slot of layer L in place (df64d): each stored double
@@ -552,7 +561,7 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
         ax = add_uu(axu, to_u(blx));
         ay = add_uu(ayu, to_u(bly));
         az = add_uu(azu, to_u(blz));
-        const int2 fr = slot_entries<TY>(a.f_ix, sRf[k - k0 + 1], tx, ty);  // this node's force sources
+        const int2 fr = slot_entries(a.f_rng, sRf[k - k0 + 1], tx, ty);  // this node's force sources
         for (int e = fr.x; e < fr.y; e++) {
           const int key = __ldg(a.f_key + e);
           const R w = N::val(a.f_w[e]), sg = N::val((RANGE ? signal_row(a, step) : sigrow)[__ldg(a.f_sig + e)]);
@@ -604,7 +613,7 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
           }
           const int64_t rec = a.rec + step;
           if (rec < a.rec_cap) {
-            const int2 sr = slot_entries<TY>(a.s_ix, sRs[k - k0 + 1], tx, ty);
+            const int2 sr = slot_entries(a.s_rng, sRs[k - k0 + 1], tx, ty);
             for (int e = sr.x; e < sr.y; e++) {  // sensor traces
               double *tr = a.traces + (rec * a.n_sens + __ldg(a.s_idx + e)) * 3;
               tr[0] = out(0);
@@ -669,7 +678,7 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
 #pragma unroll
           for (int f = 0; f < 6; f++) acc[f] = N::ld(a.S_in[f], cg);
         }
-        const int2 mr = slot_entries<TY>(a.m_ix, sRm[kc - k0], tx, ty);  // this cell's moments
+        const int2 mr = slot_entries(a.m_rng, sRm[kc - k0], tx, ty);  // this cell's moments
         for (int ee = mr.x; ee < mr.y; ee++) {
           const int key = __ldg(a.m_key + ee);
           const R w = N::val(a.m_w[ee]), sg = N::val((RANGE ? signal_row(a, step) : sigrow)[__ldg(a.m_sig + ee)]);
@@ -737,7 +746,7 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
     }
   }
   if constexpr (RANGE) {  // values left the double-float range: mark the tile (and its edges)
-    if (a.fp64_chunk > 0) {  // values other than zero are told from zeros (fp64_path)
+    if (fp64_chunk_of(a) > 0) {  // values other than zero are told from zeros (fp64_path)
       oorb = __reduce_or_sync(0xffffffffu, oorb | (nonzero ? kFlagNonzero : 0u));
       if (tx != 0) oorb = 0;
     }
@@ -771,15 +780,15 @@ __device__ __forceinline__ void grid_block_tma(const GridArgs<typename GNum<K>::
 // a wave leaves most of a plate so for the first hundreds of steps: laminate
 // 400 x 400 x 40, an initial pulse of 80 cells' diameter, 20 steps with the state
 // up- and downloaded 15.4 -> 14.3 ms.
-template <int TY>
-__device__ __forceinline__ bool fp64_path(const GridArgs<double> &a, int bx, int by, int k0, int k1, int gxc,
+template <int TY, typename Args>
+__device__ __forceinline__ bool fp64_path(const Args &a, int bx, int by, int k0, int k1, int gxc,
                                           int step, bool clear, bool &quiet) {
   constexpr int NT = TX * TY;
   const int t = threadIdx.x;
   const int gyc = a.ny / (TY - 1) + 1, nt = gxc * gyc;
   const int blk = by * gxc + bx;
   const int phase = (a.flag_phase + step) % kFlagPhases;
-  const bool track = a.fp64_chunk > 0;
+  const bool track = fp64_chunk_of(a) > 0;
   if (clear && t == 0) {
     a.rflags[((phase + 2) % kFlagPhases) * nt + blk] = 0;
     if (!track) atomicOr(a.rflags + ((phase + 1) % kFlagPhases) * nt + blk, kFlagNonzero);
@@ -834,7 +843,8 @@ __device__ __forceinline__ bool fp64_path(const GridArgs<double> &a, int bx, int
 // pieces' re-marched layers cost more than their balance gives (laminate 400 x
 // 400 x 40: 1.258 ms per step against 1.228 uncut; with half of them 0.767
 // against 0.844).
-__device__ __forceinline__ bool cut_columns(const GridArgs<double> &a, int bx, int by, int gxc, int step, bool fp64,
+template <typename Args>
+__device__ __forceinline__ bool cut_columns(const Args &a, int bx, int by, int gxc, int step, bool fp64,
                                             bool first) {
   const int gyc = a.ny / 7 + 1, nt = gxc * gyc, phase = (a.flag_phase + step) % kFlagPhases;
   uint32_t *count = a.rflags + kFlagPhases * nt;
@@ -851,7 +861,7 @@ __device__ __forceinline__ bool cut_columns(const GridArgs<double> &a, int bx, i
 // tail split (tail_chunk > 0) the 1D grid of whole columns, then the
 // remaining tiles' chunks of tail_chunk layers, chunk-major
 template <int TY, typename T>
-__device__ __forceinline__ void block_coords(const GridArgs<T> &a, int &bx, int &by, int &k0, int &kc, int &gxc) {
+__device__ __forceinline__ void block_coords(const GridLaunch<T> &a, int &bx, int &by, int &k0, int &kc, int &gxc) {
   gxc = a.nx / (TX - 1) + 1;
   if (a.tail_chunk > 0) {
     const int id = blockIdx.x, tiles = gxc * (a.ny / (TY - 1) + 1);
@@ -888,12 +898,12 @@ __device__ __forceinline__ void block_coords(const GridArgs<T> &a, int &bx, int 
 // each; on the double-float path piece 0 marches the column and the other
 // pieces' blocks end.  Every piece's block decides alike, over the column.
 // piece < 0: a chunk [k0, k0 + kc) of its own.
-template <int SYM, bool BATCH>
-__device__ __forceinline__ void f64h_block(const GridArgs<double> &a, unsigned char *smem, int bx, int by, int k0,
+template <int SYM, typename Args>
+__device__ __forceinline__ void f64h_block(const Args &a, unsigned char *smem, int bx, int by, int k0,
                                            int kc, int piece, int gxc, int step) {
   const int ktop = tile_top(a, by * gxc + bx);
   const bool column = piece >= 0;
-  Copies<double, 8, BATCH> cp(a, smem, bx, by, column ? 0 : k0, column ? ktop : min(ktop, k0 + kc));
+  Copies<double, 8> cp(a, smem, bx, by, column ? 0 : k0, column ? ktop : min(ktop, k0 + kc));
   // both paths read the same tiles: the copies start before the path is chosen
   const bool work = cp.k0 < cp.k1, first = piece <= 0;
   if (work && first && threadIdx.x == cp.ISSUER) cp.start();
@@ -918,14 +928,14 @@ __device__ __forceinline__ void f64h_block(const GridArgs<double> &a, unsigned c
   if (column) {
     if (!cut && !first) return;
     if (cut) {
-      cp.k0 = piece * a.fp64_chunk;
-      cp.k1 = min(ktop, cp.k0 + a.fp64_chunk);
+      cp.k0 = piece * fp64_chunk_of(a);
+      cp.k1 = min(ktop, cp.k0 + fp64_chunk_of(a));
       if (cp.k0 >= ktop) return;
     }
     if (!first && threadIdx.x == cp.ISSUER) cp.start();
   }
-  if (fp64) grid_block_tma<double, SYM, 8, BATCH, true>(a, cp, bx, by, cp.k1 == ktop, gxc, step);
-  else grid_block_tma<df64d, SYM, 8, BATCH, true>(a, cp, bx, by, cp.k1 == ktop, gxc, step);
+  if (fp64) grid_block_tma<double, SYM, 8, true>(a, cp, bx, by, cp.k1 == ktop, gxc, step);
+  else grid_block_tma<df64d, SYM, 8, true>(a, cp, bx, by, cp.k1 == ktop, gxc, step);
 }
 
 // resident blocks per SM the FP64 form's kernel is compiled for (its register
@@ -935,17 +945,17 @@ __device__ __forceinline__ void f64h_block(const GridArgs<double> &a, unsigned c
 #endif
 
 // an argument block copied to shared memory by the whole block
-template <typename A>
-__device__ __forceinline__ void load_block(unsigned char *dst, const A *src) {
-  static_assert(sizeof(A) % 8 == 0, "argument blocks are copied in 8-byte words");
-  for (int w = threadIdx.x; w < (int)(sizeof(A) / 8); w += blockDim.x)
+template <typename Args>
+__device__ __forceinline__ void load_block(unsigned char *dst, const Args *src) {
+  static_assert(sizeof(Args) % 8 == 0, "argument blocks are copied in 8-byte words");
+  for (int w = threadIdx.x; w < (int)(sizeof(Args) / 8); w += blockDim.x)
     reinterpret_cast<unsigned long long *>(dst)[w] = __ldg(reinterpret_cast<const unsigned long long *>(src) + w);
   __syncthreads();
 }
 
 template <int SYM>
 __global__ void __launch_bounds__(TX * 8, PN_F64H_MIN_BLOCKS)
-    k_grid_tma_f64h(const __grid_constant__ GridArgs<double> a, int step) {
+    k_grid_tma_f64h(const __grid_constant__ GridLaunch<double> a, int step) {
   extern __shared__ unsigned char smem_raw[];
   int bx, by, k0, kc, piece = -1, gxc;
   if (a.fp64_chunk > 0) {
@@ -971,7 +981,7 @@ __global__ void __launch_bounds__(TX * 8, PN_F64H_MIN_BLOCKS)
   } else {
     block_coords<8>(a, bx, by, k0, kc, gxc);
   }
-  f64h_block<SYM, false>(a, smem_raw, bx, by, k0, kc, piece, gxc, step);
+  f64h_block<SYM>(a, smem_raw, bx, by, k0, kc, piece, gxc, step);
 }
 
 template <int SYM>
@@ -991,7 +1001,7 @@ __global__ void __launch_bounds__(TX * 8, PN_F64H_MIN_BLOCKS)
   const GridArgs<double> &a = *reinterpret_cast<const GridArgs<double> *>(sargs);
   const int local = id - __ldg(block_start + lo);
   const int gxc = a.nx / (TX - 1) + 1, gyc = a.ny / 7 + 1;
-  f64h_block<SYM, true>(a, smem_raw, local % gxc, (local / gxc) % gyc, local / (gxc * gyc) * a.kchunk, a.kchunk, -1, gxc,
+  f64h_block<SYM>(a, smem_raw, local % gxc, (local / gxc) % gyc, local / (gxc * gyc) * a.kchunk, a.kchunk, -1, gxc,
                         step);
 }
 
@@ -1003,23 +1013,23 @@ __global__ void __launch_bounds__(TX * 8, PN_F64H_MIN_BLOCKS)
 template <typename R, int TY> struct GMinBlocks { static constexpr int v = TY == 8 ? 3 : 1; };
 template <int TY> struct GMinBlocks<float, TY> { static constexpr int v = PN_GRID_F32_MIN_BLOCKS; };
 
-template <typename R, int SYM, int TY, bool BATCH>
-__device__ __forceinline__ void run_block(const GridArgs<typename GNum<R>::S> &a, unsigned char *smem, int bx, int by,
-                                          int k0, int kc, int gxc, int step) {
+template <typename R, int SYM, int TY, typename Args>
+__device__ __forceinline__ void run_block(const Args &a, unsigned char *smem, int bx, int by, int k0, int kc, int gxc,
+                                          int step) {
   const int ktop = tile_top(a, by * gxc + bx), k1 = min(ktop, k0 + kc);
   if (k0 >= k1) return;
-  const Copies<typename GNum<R>::S, TY, BATCH> cp(a, smem, bx, by, k0, k1);
+  const Copies<typename GNum<R>::S, TY> cp(a, smem, bx, by, k0, k1);
   if (threadIdx.x == cp.ISSUER) cp.start();
-  grid_block_tma<R, SYM, TY, BATCH>(a, cp, bx, by, k1 == ktop, gxc, step);
+  grid_block_tma<R, SYM, TY>(a, cp, bx, by, k1 == ktop, gxc, step);
 }
 
 template <typename R, int SYM, int TY>
 __global__ void __launch_bounds__(TX *TY, GMinBlocks<R, TY>::v)
-    k_grid_tma(const __grid_constant__ GridArgs<typename GNum<R>::S> a, int step) {
+    k_grid_tma(const __grid_constant__ GridLaunch<typename GNum<R>::S> a, int step) {
   extern __shared__ unsigned char smem_raw[];
   int bx, by, k0, kc, gxc;
   block_coords<TY>(a, bx, by, k0, kc, gxc);
-  run_block<R, SYM, TY, false>(a, smem_raw, bx, by, k0, kc, gxc, step);
+  run_block<R, SYM, TY>(a, smem_raw, bx, by, k0, kc, gxc, step);
 }
 
 template <typename R, int SYM, int TY>
@@ -1042,7 +1052,7 @@ __global__ void __launch_bounds__(TX *TY, GMinBlocks<R, TY>::v)
   const GridArgs<typename GNum<R>::S> &a = *reinterpret_cast<const GridArgs<typename GNum<R>::S> *>(sargs);
   const int local = id - __ldg(block_start + lo);
   const int gxc = a.nx / (TX - 1) + 1, gyc = a.ny / (TY - 1) + 1;
-  run_block<R, SYM, TY, true>(a, smem_raw, local % gxc, (local / gxc) % gyc, local / (gxc * gyc) * a.kchunk, a.kchunk,
+  run_block<R, SYM, TY>(a, smem_raw, local % gxc, (local / gxc) % gyc, local / (gxc * gyc) * a.kchunk, a.kchunk,
                               gxc, step);
 }
 
@@ -1078,7 +1088,7 @@ struct SetupT {
 // grid of a single solver's launch: chunks (kchunk, when the caller left it
 // 0) and the tail split; grid.x == 0: a chunk longer than the kernel stages
 template <int TY, typename T>
-dim3 single_grid(GridArgs<T> &b, int sms, int per_sm) {
+dim3 single_grid(GridLaunch<T> &b, int sms, int per_sm) {
   const unsigned gx = (unsigned)(b.nx / (TX - 1) + 1), gy = (unsigned)(b.ny / (TY - 1) + 1);
   if (b.kchunk <= 0) b.kchunk = grid_chunk_for(b.nz, (long long)gx * gy, sms, per_sm);
   if (b.kchunk > KC_MAX) return dim3(0, 1, 1);
@@ -1091,12 +1101,12 @@ dim3 single_grid(GridArgs<T> &b, int sms, int per_sm) {
 }
 
 template <typename R, int SYM, int TY>
-cudaError_t launch_t(const GridArgs<typename GNum<R>::S> &a, cudaStream_t st) {
+cudaError_t launch_t(const GridLaunch<typename GNum<R>::S> &a, cudaStream_t st) {
   using S = SetupT<R, SYM, TY>;
   int sms = 0, per_sm = 0;
   cudaError_t e = S::ensure(sms, per_sm);
   if (e != cudaSuccess) return e;
-  GridArgs<typename GNum<R>::S> b = a;
+  GridLaunch<typename GNum<R>::S> b = a;
   const dim3 grid = single_grid<TY>(b, sms, per_sm);
   if (grid.x == 0) return cudaErrorInvalidValue;
   return launch_overlapped(k_grid_tma<R, SYM, TY>, grid, TX * TY, S::smem, st, b, 0);
@@ -1142,12 +1152,12 @@ struct SetupH {
 // downloaded: 14.0 ms uncut, 12.5 / 11.4 / 11.8 in 2 / 3 / 5 pieces; a state that
 // is all double-float pays 1% for the further pieces' blocks.
 template <int SYM>
-cudaError_t launch_h(const GridArgs<double> &a, cudaStream_t st) {
+cudaError_t launch_h(const GridLaunch<double> &a, cudaStream_t st) {
   int sms = 0, per_sm = 0;
   cudaError_t e = SetupT<double, SYM, 8>::ensure(sms, per_sm);
   if (e == cudaSuccess) e = SetupH<SYM>::ensure();
   if (e != cudaSuccess) return e;
-  GridArgs<double> b = a;
+  GridLaunch<double> b = a;
   dim3 grid = single_grid<8>(b, sms, per_sm);
   if (grid.x == 0) return cudaErrorInvalidValue;
   b.fp64_chunk = 0;
@@ -1173,7 +1183,7 @@ template <typename T> inline bool is_one(T v) { return v == T(1); }
 template <> inline bool is_one<float2>(float2 v) { return v.x == 1.0f && v.y == 0.0f; }
 
 template <typename R, int TY>
-cudaError_t launch_sym(const GridArgs<typename GNum<R>::S> &a, int sym, cudaStream_t st) {
+cudaError_t launch_sym(const GridLaunch<typename GNum<R>::S> &a, int sym, cudaStream_t st) {
   if (a.nx <= 0 || a.ny <= 0 || a.nz <= 0) return cudaSuccess;
   if (!a.tmaps || a.n_rows > ROWS_MAX) return cudaErrorInvalidValue;
   const bool cubic = is_one(a.g[0]) && is_one(a.g[1]) && is_one(a.g[2]);
@@ -1187,7 +1197,7 @@ cudaError_t launch_sym(const GridArgs<typename GNum<R>::S> &a, int sym, cudaStre
   }
 }
 
-inline cudaError_t launch_sym_h(const GridArgs<double> &a, int sym, cudaStream_t st) {
+inline cudaError_t launch_sym_h(const GridLaunch<double> &a, int sym, cudaStream_t st) {
   if (a.nx <= 0 || a.ny <= 0 || a.nz <= 0) return cudaSuccess;
   if (!a.tmaps || a.n_rows > ROWS_MAX || !a.rflags) return cudaErrorInvalidValue;
   const bool cubic = is_one(a.g[0]) && is_one(a.g[1]) && is_one(a.g[2]);

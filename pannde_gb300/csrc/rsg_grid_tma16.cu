@@ -7,7 +7,7 @@
 
 namespace pn {
 
-cudaError_t launch_grid_tma_f32_rows16(const GridArgs<float> &a, int sym, cudaStream_t st) {
+cudaError_t launch_grid_tma_f32_rows16(const GridLaunch<float> &a, int sym, cudaStream_t st) {
   return launch_sym<float, 16>(a, sym, st);
 }
 

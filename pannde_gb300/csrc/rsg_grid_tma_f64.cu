@@ -7,7 +7,7 @@
 
 namespace pn {
 
-cudaError_t launch_grid_tma_f64h(const GridArgs<double> &a, int sym, cudaStream_t st) {
+cudaError_t launch_grid_tma_f64h(const GridLaunch<double> &a, int sym, cudaStream_t st) {
   return launch_sym_h(a, sym, st);
 }
 

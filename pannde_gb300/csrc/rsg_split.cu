@@ -56,8 +56,8 @@ constexpr int TPB = 128;
 // FP64 form (a.rflags set): a stored value outside the double-float range
 // puts the tile of lattice column (i, j) on the FP64 path for the next step
 // (the tensor-copy kernel's flags, rsg_grid_tma.cuh fp64_path)
-template <typename S>
-__device__ __forceinline__ void flag_range(const GridArgs<S> &a, double v, int64_t i, int64_t j, int step,
+template <typename S, typename A>
+__device__ __forceinline__ void flag_range(const A &a, double v, int64_t i, int64_t j, int step,
                                            bool stress) {
   if (!a.rflags || in_df64_range(v, (uint32_t)(stress ? a.r_elo_s : a.r_elo), (uint32_t)(stress ? a.r_ehi_s : a.r_ehi)))
     return;
@@ -69,8 +69,8 @@ __device__ __forceinline__ void flag_range(const GridArgs<S> &a, double v, int64
 // velocity of copy q: x differences of Sxx, Sxy, Sxz; y of Sxy, Syy, Syz; z of
 // Sxz, Syz, Szz over the cells the copy joins (a cell's sign along an axis is
 // + on the site's upper side)
-template <typename S>
-__device__ void copy_velocity(const GridArgs<S> &a, int q, int step) {
+template <typename S, typename A>
+__device__ void copy_velocity(const A &a, int q, int step) {
   using N = SN<S>;
   using R = typename N::R;
   const SplitCopy cp = a.copies[q];
@@ -123,7 +123,7 @@ __device__ void copy_velocity(const GridArgs<S> &a, int q, int step) {
     vn[c] = N::val(vold[c]);
     if (!(cf == R())) vn[c] = madd(cf, acc[c], vn[c]);
     a.V_out[c][cp.v] = N::sto(vn[c]);
-    flag_range(a, N::dbl(vn[c]), cp.i, cp.j, step, false);
+    flag_range<S>(a, N::dbl(vn[c]), cp.i, cp.j, step, false);
   }
   const int64_t rec = a.rec + step;
   if (rec < a.rec_cap)
@@ -136,8 +136,8 @@ __device__ void copy_velocity(const GridArgs<S> &a, int q, int step) {
 }
 
 // stress of fix cell q from its corners' new velocities
-template <typename S>
-__device__ void fix_stress(const GridArgs<S> &a, int q, int step) {
+template <typename S, typename A>
+__device__ void fix_stress(const A &a, int q, int step) {
   using N = SN<S>;
   using R = typename N::R;
   const FixCell fc = a.fix[q];
@@ -189,22 +189,22 @@ __device__ void fix_stress(const GridArgs<S> &a, int q, int step) {
 #pragma unroll
     for (int j = 0; j < 6; j++) acc[k] = madd(N::val(Cm[6 * k + j]), e[j], acc[k]);
     a.S_out[k][fc.cell] = N::sto(acc[k]);
-    flag_range(a, N::dbl(acc[k]), fc.cell % a.pcx, (fc.cell / a.pcx) % a.ny, step, true);
+    flag_range<S>(a, N::dbl(acc[k]), fc.cell % a.pcx, (fc.cell / a.pcx) % a.ny, step, true);
   }
 }
 
 template <typename S>
-__global__ void __launch_bounds__(TPB) k_split_copies(const __grid_constant__ GridArgs<S> a) {
+__global__ void __launch_bounds__(TPB) k_split_copies(const __grid_constant__ GridLaunch<S> a) {
   let_next_start();
   const int q = blockIdx.x * TPB + threadIdx.x;
-  if (q < a.n_copies) copy_velocity(a, q, 0);
+  if (q < a.n_copies) copy_velocity<S>(a, q, 0);
 }
 
 template <typename S>
-__global__ void __launch_bounds__(TPB) k_split_cells(const __grid_constant__ GridArgs<S> a) {
+__global__ void __launch_bounds__(TPB) k_split_cells(const __grid_constant__ GridLaunch<S> a) {
   let_next_start();
   const int q = blockIdx.x * TPB + threadIdx.x;
-  if (q < a.n_fix) fix_stress(a, q, 0);
+  if (q < a.n_fix) fix_stress<S>(a, q, 0);
 }
 
 // member of flat item id: start[m] <= id < start[m + 1]
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(TPB)
   const int id = blockIdx.x * TPB + threadIdx.x;
   if (id >= total) return;
   const int m = member_of(start, n, id);
-  copy_velocity(args[m], id - __ldg(start + m), step);
+  copy_velocity<S>(args[m], id - __ldg(start + m), step);
 }
 
 template <typename S>
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(TPB)
   const int id = blockIdx.x * TPB + threadIdx.x;
   if (id >= total) return;
   const int m = member_of(start, n, id);
-  fix_stress(args[m], id - __ldg(start + m), step);
+  fix_stress<S>(args[m], id - __ldg(start + m), step);
 }
 
 template <typename F, typename... A>
@@ -246,7 +246,7 @@ cudaError_t launch(F f, int items, cudaStream_t st, A... args) {
 }
 
 template <typename S>
-cudaError_t split_one(const GridArgs<S> &a, cudaStream_t st) {
+cudaError_t split_one(const GridLaunch<S> &a, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
   if (a.n_copies > 0) e = launch(k_split_copies<S>, a.n_copies, st, a);
   if (e == cudaSuccess && a.n_fix > 0) e = launch(k_split_cells<S>, a.n_fix, st, a);
@@ -267,9 +267,9 @@ cudaError_t split_batch(const GridSplitBatch &b, int step, cudaStream_t st) {
 }  // namespace
 
 cudaError_t launch_grid_split(const void *args, int precision, cudaStream_t st) {
-  if (precision == 2) return split_one<float>(*(const GridArgs<float> *)args, st);
-  if (precision == 3) return split_one<float2>(*(const GridArgs<float2> *)args, st);
-  return split_one<double>(*(const GridArgs<double> *)args, st);
+  if (precision == 2) return split_one<float>(*(const GridLaunch<float> *)args, st);
+  if (precision == 3) return split_one<float2>(*(const GridLaunch<float2> *)args, st);
+  return split_one<double>(*(const GridLaunch<double> *)args, st);
 }
 
 cudaError_t launch_grid_split_batch(const GridSplitBatch &b, int precision, int step, cudaStream_t st) {

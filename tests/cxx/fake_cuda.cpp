@@ -55,7 +55,7 @@ void table(const void *p, const char *what) {  // a table a launch reads: none, 
 }
 
 template <typename T>
-void velocity(const pn::VelArgs<T> &a) {
+void velocity(const pn::VelLaunch<T> &a) {
   g_launches++;
   for (const void *p : {(const void *)a.V0, (const void *)a.S0, (const void *)a.S5, (const void *)a.coef,
                         (const void *)a.gnode, (const void *)a.tile_src, (const void *)a.tile_sens})
@@ -64,7 +64,7 @@ void velocity(const pn::VelArgs<T> &a) {
 }
 
 template <typename T>
-void stress(const pn::StressArgs<T> &a) {
+void stress(const pn::StressLaunch<T> &a) {
   g_launches++;
   for (const void *p : {(const void *)a.V0, (const void *)a.S0, (const void *)a.S5, (const void *)a.mat,
                         (const void *)a.gcell, (const void *)a.tile_src})
@@ -145,24 +145,24 @@ cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaErrorNot
 
 namespace pn {
 
-cudaError_t launch_velocity_exact(const VelArgs<double> &a, int, cudaStream_t) {
+cudaError_t launch_velocity_exact(const VelLaunch<double> &a, int, cudaStream_t) {
   velocity(a);
-  table(a.rnode, "velocity launch's reciprocals");
-  if (!a.rnode) g_null_reciprocals++;
+  table(a.recips, "velocity launch's reciprocals");
+  if (!a.recips) g_null_reciprocals++;
   return cudaSuccess;
 }
-cudaError_t launch_stress_exact(const StressArgs<double> &a, int, cudaStream_t) {
+cudaError_t launch_stress_exact(const StressLaunch<double> &a, int, cudaStream_t) {
   stress(a);
-  table(a.rcell, "stress launch's reciprocals");
-  if (!a.rcell) g_null_reciprocals++;
+  table(a.recips, "stress launch's reciprocals");
+  if (!a.recips) g_null_reciprocals++;
   return cudaSuccess;
 }
-cudaError_t launch_velocity_f64(const VelArgs<double> &a, int, bool, cudaStream_t) { return velocity(a), cudaSuccess; }
-cudaError_t launch_velocity_f32(const VelArgs<float> &a, int, bool, cudaStream_t) { return velocity(a), cudaSuccess; }
-cudaError_t launch_velocity_df64(const VelArgs<float2> &a, int, bool, cudaStream_t) { return velocity(a), cudaSuccess; }
-cudaError_t launch_stress_f64(const StressArgs<double> &a, int, bool, cudaStream_t) { return stress(a), cudaSuccess; }
-cudaError_t launch_stress_f32(const StressArgs<float> &a, int, bool, cudaStream_t) { return stress(a), cudaSuccess; }
-cudaError_t launch_stress_df64(const StressArgs<float2> &a, int, bool, cudaStream_t) { return stress(a), cudaSuccess; }
+cudaError_t launch_velocity_f64(const VelLaunch<double> &a, int, bool, cudaStream_t) { return velocity(a), cudaSuccess; }
+cudaError_t launch_velocity_f32(const VelLaunch<float> &a, int, bool, cudaStream_t) { return velocity(a), cudaSuccess; }
+cudaError_t launch_velocity_df64(const VelLaunch<float2> &a, int, bool, cudaStream_t) { return velocity(a), cudaSuccess; }
+cudaError_t launch_stress_f64(const StressLaunch<double> &a, int, bool, cudaStream_t) { return stress(a), cudaSuccess; }
+cudaError_t launch_stress_f32(const StressLaunch<float> &a, int, bool, cudaStream_t) { return stress(a), cudaSuccess; }
+cudaError_t launch_stress_df64(const StressLaunch<float2> &a, int, bool, cudaStream_t) { return stress(a), cudaSuccess; }
 cudaError_t launch_exact_reciprocals(const double *d, int64_t n, double *rec, cudaStream_t) {
   device(d, (size_t)n * 8, "spacings");
   device(rec, (size_t)n * 16, "reciprocals");
@@ -181,9 +181,9 @@ cudaError_t grid_step(const A &a) {
     table(p, "grid launch");
   return cudaSuccess;
 }
-cudaError_t launch_grid_f32(const GridArgs<float> &a, int, cudaStream_t) { return grid_step(a); }
-cudaError_t launch_grid_f64(const GridArgs<double> &a, int, cudaStream_t) { return grid_step(a); }
-cudaError_t launch_grid_df64(const GridArgs<float2> &a, int, cudaStream_t) { return grid_step(a); }
+cudaError_t launch_grid_f32(const GridLaunch<float> &a, int, cudaStream_t) { return grid_step(a); }
+cudaError_t launch_grid_f64(const GridLaunch<double> &a, int, cudaStream_t) { return grid_step(a); }
+cudaError_t launch_grid_df64(const GridLaunch<float2> &a, int, cudaStream_t) { return grid_step(a); }
 cudaError_t launch_grid_tma(const void *, int, int, cudaStream_t) { return g_launches++, cudaSuccess; }
 cudaError_t launch_grid_batch(const GridBatchLaunch &, int, int, cudaStream_t) { return g_launches++, cudaSuccess; }
 cudaError_t launch_grid_tma_batch(const GridBatchLaunch &, int, int, cudaStream_t) { return g_launches++, cudaSuccess; }

@@ -114,3 +114,28 @@ def test_caller_signals_leave_rows_for_the_allocation_free_batch(fake, form, n_s
         held = fake.fake_held()
         b.solve_noalloc(7)
         assert fake.fake_held() == held or held + 262144 == fake.fake_held()  # (the fixed scratch, once)
+
+
+@pytest.mark.parametrize("form, prec, block", [("grid", "f32", 512), ("grid", "f64", 520), ("grid", "df64", 520),
+                                               ("table", "f32", 232), ("table", "f64", 240), ("table", "df64", 240)])
+def test_members_the_fixed_scratch_takes(fake, form, prec, block):
+    """A member's argument block keeps its size: the allocation-free batch
+    solve takes as many members as its 256 KiB hold, and no more."""
+    def room(n):
+        starts = 2 * (n + 1) if form == "grid" else n + 1
+        return 2 * (-(-block * n // 256) * 256) + 2 * (-(-starts * 4 // 256) * 256)
+    most = max(n for n in range(1, 1000) if room(n) <= 256 * 1024)
+    m = cases.voxel_mesh(np.ones((2, 2, 2), dtype=bool), 1e-4)
+    c = cases.Case("tiny", m, np.array([2700.0]), cases.c21_from_6x6(cases.isotropic(70e9, 0.33))[None],
+                   np.zeros(m.n_cells, np.int32), 1e-9)
+    sv = [Solver(m, c, c.dt, prec, form) for _ in range(most + 1)]
+    with Batch() as b:
+        for s in sv[:most]:
+            b.add(s)
+        b.solve_noalloc(1)
+        b.add(sv[most])
+        with pytest.raises(N.PnError) as e:
+            b.solve_noalloc(1)
+        assert f"{most + 1} members need {room(most + 1)} bytes" in e.value.msg
+    for s in sv:
+        s.close()
