@@ -1009,9 +1009,11 @@ __global__ void __launch_bounds__(TX * 8, PN_F64H_MIN_BLOCKS)
 // follows): 3 for 8-byte storage (80 registers; shared memory holds 3 blocks);
 // 4 for 4-byte storage (56-64 registers; left to itself the compiler takes 80
 // and 3 blocks fit: laminate FP32 107.8 us per step against 105.8)
-// (32 x 16 tiles with 8-byte storage: shared memory holds one block per SM)
+// (32 x 16 tiles: half as many, the same threads; four of them left 32 registers
+// and 300 bytes of spills, laminate FP32 238.9 us per step against 100.8, uncapped
+// 102.6.  With 8-byte storage shared memory holds one block per SM)
 template <typename R, int TY> struct GMinBlocks { static constexpr int v = TY == 8 ? 3 : 1; };
-template <int TY> struct GMinBlocks<float, TY> { static constexpr int v = PN_GRID_F32_MIN_BLOCKS; };
+template <int TY> struct GMinBlocks<float, TY> { static constexpr int v = TY == 8 ? PN_GRID_F32_MIN_BLOCKS : PN_GRID_F32_MIN_BLOCKS / 2; };
 
 template <typename R, int SYM, int TY, typename Args>
 __device__ __forceinline__ void run_block(const Args &a, unsigned char *smem, int bx, int by, int k0, int kc, int gxc,
