@@ -58,6 +58,9 @@ struct pn_batch {
     std::vector<int> ids;
   };
   std::vector<Order> orders;
+  // ... and the chunk lengths chosen for them, by (tile rows, tensor-copy kernel,
+  // PN_GRID_KCHUNK): a call of a few dozen steps is short beside the members' tile tops
+  std::map<std::tuple<int, bool, std::string>, int> chunk_len;
 
   ~pn_batch() {
     if (exec) cudaGraphExecDestroy(exec);
@@ -389,19 +392,21 @@ void solve_grid(pn_batch *b, int32_t nsteps, int precision, const Stage &stage, 
     size_t start_ints = 2 * (n + 1);
     // chunk length of shape c for a member: the batch's own choice over all
     // members' columns (0), or so many chunks per column
-    std::map<int, int> own_len;  // by tile rows
+    const char *kchunk_env = std::getenv("PN_GRID_KCHUNK");
+    const std::string kchunk_set = kchunk_env ? kchunk_env : "";
     auto chunk_layers = [&](int c, const pn_solver *s) {
       const int rows = shapes[c].first, per = shapes[c].second, nz = s->grid.nz;
       if (per != 0) return std::min(pn::kGridChunkMax, std::max(1, (nz + per - 1) / per));
-      auto it = own_len.find(rows);
-      if (it == own_len.end()) {
+      const auto key = std::make_tuple(rows, tma, kchunk_set);
+      auto it = b->chunk_len.find(key);
+      if (it == b->chunk_len.end()) {
         std::map<int, long long> tops;
         for (pn_solver *q : b->members)
           if (tma)
-            for (int32_t top : pn::grid_tile_tops(q->grid, rows)) tops[std::min(top, q->grid.nz)]++;
+            for (const auto &t : pn::grid_top_counts(q, rows)) tops[t.first] += t.second;
           else tops[q->grid.nz] += (long long)(q->grid.nx / (tx - 1) + 1) * (q->grid.ny / (rows - 1) + 1);
         tops.erase(0);
-        it = own_len.emplace(rows, pn::grid_chunk_layers(precision, tops, tma, rows)).first;
+        it = b->chunk_len.emplace(key, pn::grid_chunk_layers(precision, tops, tma, rows)).first;
       }
       return std::max(1, std::min(it->second, nz));
     };
@@ -643,6 +648,7 @@ int pn_batch_add(pn_batch *b, pn_solver *m) {
   if (m->has_mask_sources()) return berr(PN_ERR_INVALID, "window-mask sources need pn_solver_solve_signals");
   b->members.push_back(m);
   b->orders.clear();
+  b->chunk_len.clear();
   return PN_OK;
 }
 
@@ -652,6 +658,7 @@ int pn_batch_remove(pn_batch *b, pn_solver *m) {
   if (it == b->members.end()) return berr(PN_ERR_INVALID, "solver not in the batch");
   b->members.erase(it);
   b->orders.clear();
+  b->chunk_len.clear();
   return PN_OK;
 }
 

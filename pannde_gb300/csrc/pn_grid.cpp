@@ -170,6 +170,16 @@ std::vector<int32_t> grid_tile_tops(const GridMap &g, int tile_rows) {
   return top;
 }
 
+const std::map<int, long long> &grid_top_counts(pn_solver *s, int tile_rows) {
+  auto it = s->top_counts.find(tile_rows);
+  if (it == s->top_counts.end()) {
+    std::map<int, long long> n;
+    for (int32_t top : grid_tile_tops(s->grid, tile_rows)) n[std::min(top, s->grid.nz)]++;
+    it = s->top_counts.emplace(tile_rows, std::move(n)).first;
+  }
+  return it->second;
+}
+
 // The tensor-copy kernel (rsg_grid_tma.cu) runs when the stiffness table fits
 // its shared-memory rows and every buffer meets the copy rules; otherwise the
 // classic kernel (rsg_grid.cu).  PN_GRID_KERNEL=classic selects the classic

@@ -86,6 +86,7 @@ struct pn_solver {
   // grid form
   pn::GridMap grid;
   int sym = 0;             // material symmetry class of the stiffness table (both forms)
+  std::map<int, std::map<int, long long>> top_counts;  // by tile rows (grid_top_counts)
   uint8_t *d_gmat = nullptr;
   void *d_tmaps = nullptr;   // tensor maps [2 input parities] (null: classic kernel)
   int32_t *d_ktop = nullptr; // [tiles] cell layers the tensor-copy kernel marches per tile
@@ -354,6 +355,8 @@ bool grid_eligible(const MeshTables &m, const MaterialTables &mt, int precision,
 // per tile: 1 + the highest solid cell layer in the columns of its cell box
 // with the apron, i.e. the cell layers the tensor-copy kernel marches
 std::vector<int32_t> grid_tile_tops(const GridMap &g, int tile_rows = kGridTileRows);
+// number of tile columns per height in cell layers (kept with the solver)
+const std::map<int, long long> &grid_top_counts(pn_solver *s, int tile_rows);
 // tile rows a new solver's tensor-copy kernel starts with
 int grid_default_tile_rows(int precision, const GridMap &g);
 // re-tile a solver's tensor-copy kernel (maps, tile tops, source and sensor

@@ -26,7 +26,7 @@ std::map<uintptr_t, Block> g_blocks;
 int64_t g_held = 0, g_room = -1;  // bytes held; most that may be (-1: any)
 int g_faults = 0;
 std::string g_first;
-int64_t g_launches = 0, g_null_reciprocals = 0;
+int64_t g_launches = 0, g_null_reciprocals = 0, g_chunk_choices = 0;
 
 void fault(const std::string &what) {
   if (g_faults++ == 0) g_first = what;
@@ -80,12 +80,13 @@ int fake_faults() { return g_faults; }
 const char *fake_first_fault() { return g_first.c_str(); }
 int64_t fake_launches() { return g_launches; }
 int64_t fake_launches_without_reciprocals() { return g_null_reciprocals; }
+int64_t fake_chunk_choices() { return g_chunk_choices; }
 int64_t fake_held() { return g_held; }
 void fake_set_room(int64_t bytes) { g_room = bytes; }
 void fake_reset() {
   g_faults = 0;
   g_first.clear();
-  g_launches = g_null_reciprocals = 0;
+  g_launches = g_null_reciprocals = g_chunk_choices = 0;
   g_room = -1;
 }
 
@@ -196,6 +197,7 @@ bool grid_tma_encode(int, int, int, int, int, int, int, const void *const[3], co
   return true;
 }
 int grid_chunk_layers(int, const std::map<int, long long> &tops, bool, int) {
+  g_chunk_choices++;
   return tops.empty() ? 1 : tops.rbegin()->first;
 }
 cudaError_t launch_state_store(int, const double *, int64_t, const int64_t *, void *, cudaStream_t, int32_t *,

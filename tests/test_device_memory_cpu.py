@@ -42,7 +42,7 @@ def fake_lib(tmp_path_factory):
 def fake(fake_lib, monkeypatch):
     lib = N.load(fake_lib)
     lib.fake_first_fault.restype = ctypes.c_char_p
-    for f in ("fake_held", "fake_launches", "fake_launches_without_reciprocals"):
+    for f in ("fake_held", "fake_launches", "fake_chunk_choices", "fake_launches_without_reciprocals"):
         getattr(lib, f).restype = ctypes.c_int64
     lib.fake_set_room.argtypes = [ctypes.c_int64]
     monkeypatch.setattr(N, "_lib", lib)
@@ -139,3 +139,20 @@ def test_members_the_fixed_scratch_takes(fake, form, prec, block):
         assert f"{most + 1} members need {room(most + 1)} bytes" in e.value.msg
     for s in sv:
         s.close()
+
+
+def test_batch_calls_keep_the_chosen_chunk_length(fake):
+    """A batch chooses its chunk length once per set of members and tile rows,
+    not from every member's lattice in every call."""
+    c = plate()
+    with Solver.from_case(c, "f32", form="grid") as s, Solver.from_case(c, "f32", form="grid") as t, Batch() as b:
+        b.add(s)
+        b.solve(5)
+        first = fake.fake_chunk_choices()
+        for _ in range(3):
+            b.solve(5)
+        b.solve_noalloc(5)
+        assert first > 0 and fake.fake_chunk_choices() == first
+        b.add(t)
+        b.solve(5)
+        assert fake.fake_chunk_choices() == 2 * first
