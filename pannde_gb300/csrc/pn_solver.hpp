@@ -65,7 +65,11 @@ struct pn_solver {
   pn::MeshTables mesh;
   pn::MaterialTables mat;
 
-  std::vector<void *> allocs;
+  struct Held {
+    void *p;
+    int64_t counted, uncounted;  // bytes (uncounted: see alloc)
+  };
+  std::vector<Held> held;
   int64_t dev_bytes = 0;        // held, the uncounted ones not among them
   int64_t uncounted_bytes = 0;
 
@@ -204,7 +208,7 @@ struct pn_solver {
       (void)cudaGetLastError();
       throw pn::SetupError{PN_ERR_ALLOC, std::string("cudaMalloc failed: ") + cudaGetErrorString(e)};
     }
-    allocs.push_back(p);
+    held.push_back({p, counted, (int64_t)uncounted});
     dev_bytes += counted;
     uncounted_bytes += (int64_t)uncounted;
     return (P *)p;
@@ -216,7 +220,6 @@ struct pn_solver {
   bool drop_reciprocals() {
     if (!d_rnode) return false;
     pn::ck(cudaStreamSynchronize(stream), "reciprocals sync");  // steps in flight read them
-    dev_bytes -= 6 * (int64_t)sizeof(double) * ((int64_t)mesh.n_nodes + mesh.n_cells);
     release(d_rnode);
     d_rcell = nullptr;
     return true;
@@ -225,8 +228,12 @@ struct pn_solver {
   template <typename P>
   void release(P *&p) {
     if (!p) return;
-    auto it = std::find(allocs.begin(), allocs.end(), (void *)p);
-    if (it != allocs.end()) allocs.erase(it);
+    auto it = std::find_if(held.begin(), held.end(), [&](const Held &h) { return h.p == (void *)p; });
+    if (it != held.end()) {
+      dev_bytes -= it->counted;
+      uncounted_bytes -= it->uncounted;
+      held.erase(it);
+    }
     cudaFree((void *)p);
     p = nullptr;
   }
@@ -322,8 +329,8 @@ struct pn_solver {
 
   ~pn_solver() {
     clear_marks();
-    for (void *p : allocs) cudaFree(p);
-    allocs.clear();
+    for (const Held &h : held) cudaFree(h.p);
+    held.clear();
   }
 };
 

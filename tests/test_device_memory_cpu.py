@@ -156,3 +156,23 @@ def test_batch_calls_keep_the_chosen_chunk_length(fake):
         b.add(t)
         b.solve(5)
         assert fake.fake_chunk_choices() == 2 * first
+
+
+@pytest.mark.parametrize("form, prec", [("grid", "f64"), ("grid", "f32"), ("table", "f32"), ("table", "f64_exact")])
+def test_device_bytes_are_what_is_held(fake, form, prec):
+    """Sensors set again, sources added, a longer signal table: what was given
+    back is not counted."""
+    c = plate()
+    with Solver.from_case(c, prec, form=form) as s:
+        before = fake.fake_held() - s.info()["device_bytes"]
+        s.solve(2)
+        once = s.info()["device_bytes"]
+        for _ in range(3):
+            s.set_sensors(c.sensors, 30)
+        assert s.info()["device_bytes"] == once
+        s.add_sources([cases.WindowSource(N.PN_SOURCE_FORCE, 1, 0, c.sources[0].center, c.sources[0].radius,
+                                          c.sources[0].ds, c.sources[0].times, c.sources[0].values)])
+        s.solve(2)
+        s.get_state()
+        s.energy()
+        assert fake.fake_held() - s.info()["device_bytes"] == before == 0
