@@ -429,8 +429,7 @@ void grid_create(pn_solver *s) {
                        std::max(s->r_cmax, s->r_cmax_s) > std::ldexp(1.0, 90);
   if (s->precision == PN_PREC_F64 && s->d_tmaps && s->r_elo <= s->r_ehi && s->r_elo_s <= s->r_ehi_s && !extreme) {
     const int64_t tiles = (int64_t)(g.nx / (kGridTileX - 1) + 1) * (g.ny / (kGridTileRows - 1) + 1);
-    s->d_rflags = s->alloc<uint32_t>((size_t)(kFlagPhases * (tiles + 1)) * sizeof(uint32_t),
-                                       (size_t)(tiles + kFlagPhases) * sizeof(uint32_t));
+    s->d_rflags = s->alloc<uint8_t>((size_t)(kFlagPhases * tiles));  // (whole words: kFlagPhases is 4)
     s->d_pathcnt = s->alloc<unsigned long long>(2 * sizeof(unsigned long long));
     ck(cudaMemsetAsync(s->d_pathcnt, 0, 2 * sizeof(unsigned long long), s->stream), "memset");
     grid_reset_range_flags(s);
@@ -439,16 +438,21 @@ void grid_create(pn_solver *s) {
   ck(cudaStreamSynchronize(s->stream), "create sync");
 }
 
+// no flag set, no column counted (the counts, three words behind the error word)
+static void clear_flags(pn_solver *s, int64_t tiles) {
+  ck(cudaMemsetAsync(s->d_rflags, 0, (size_t)(kFlagPhases * tiles), s->stream), "memset");
+  ck(cudaMemsetAsync(s->d_err + 1, 0, 3 * sizeof(uint32_t), s->stream), "memset");
+}
+
 void grid_reset_range_flags(pn_solver *s) {
   if (!s->d_rflags) return;
   const GridMap &g = s->grid;
   const int64_t tiles = (int64_t)(g.nx / (kGridTileX - 1) + 1) * (g.ny / (kGridTileRows - 1) + 1);
-  ck(cudaMemsetAsync(s->d_rflags, 0, (size_t)(kFlagPhases * (tiles + 1)) * sizeof(uint32_t), s->stream), "memset");
+  clear_flags(s, tiles);
   // every bit: every tile on the FP64 path, and none taken for quiet for two
   // steps (nothing is known of either buffer half)
   for (int64_t p : {s->step, s->step + kFlagPhases - 1})
-    ck(cudaMemsetAsync(s->d_rflags + (p % kFlagPhases) * tiles, 0xff, (size_t)tiles * sizeof(uint32_t), s->stream),
-       "memset");
+    ck(cudaMemsetAsync(s->d_rflags + (p % kFlagPhases) * tiles, 0xff, (size_t)tiles, s->stream), "memset");
 }
 
 void grid_split_upload(pn_solver *s) {
@@ -557,11 +561,11 @@ int grid_put_state(pn_solver *s, const double *const *V, const double *const *S)
     // (but not the idle half's: what is written there from here on, a refused
     // state too, is no longer what the steps before left)
     ck(cudaMemsetAsync(s->d_rflags + ((s->step + kFlagPhases - 1) % kFlagPhases) * tiles, (int)kFlagNonzero,
-                       (size_t)tiles * sizeof(uint32_t), s->stream),
+                       (size_t)tiles, s->stream),
        "memset");
-    if (!s->d_rflags_stage) s->d_rflags_stage = s->alloc<uint32_t>((size_t)tiles * sizeof(uint32_t));
-    // (no tile is taken for quiet for two steps: kFlagNonzero in every byte)
-    ck(cudaMemsetAsync(s->d_rflags_stage, (int)kFlagNonzero, (size_t)tiles * sizeof(uint32_t), s->stream), "memset");
+    if (!s->d_rflags_stage) s->d_rflags_stage = s->alloc<uint8_t>((size_t)(tiles + 3) / 4 * 4);
+    // (no tile is taken for quiet for two steps)
+    ck(cudaMemsetAsync(s->d_rflags_stage, (int)kFlagNonzero, (size_t)tiles, s->stream), "memset");
     rv.flags = s->d_rflags_stage;
     rv.unplaced = s->d_nonfinite + 2;
     rv.gxc = g.nx / (kGridTileX - 1) + 1;
@@ -599,11 +603,11 @@ int grid_put_state(pn_solver *s, const double *const *V, const double *const *S)
     if (bad[2]) {
       grid_reset_range_flags(s);  // a split-site copy out of range: FP64 for one step
     } else {
-      ck(cudaMemsetAsync(s->d_rflags, 0, (size_t)(kFlagPhases * (tiles + 1)) * sizeof(uint32_t), s->stream), "memset");
+      clear_flags(s, tiles);
       ck(cudaMemsetAsync(s->d_rflags + ((s->step + kFlagPhases - 1) % kFlagPhases) * tiles, (int)kFlagNonzero,
-                         (size_t)tiles * sizeof(uint32_t), s->stream),
+                         (size_t)tiles, s->stream),
          "memset");
-      ck(cudaMemcpyAsync(s->d_rflags + (s->step % kFlagPhases) * tiles, s->d_rflags_stage, (size_t)tiles * sizeof(uint32_t),
+      ck(cudaMemcpyAsync(s->d_rflags + (s->step % kFlagPhases) * tiles, s->d_rflags_stage, (size_t)tiles,
                          cudaMemcpyDeviceToDevice, s->stream),
          "range flags");
     }
@@ -817,6 +821,7 @@ void run(pn_solver *s, int32_t nsteps) {
   GridLaunch<T> a{};
   grid_args(s, a);
   if (s->d_tmaps) a.places = slot_places(a, s->tile_rows);
+  a.fp64_cols = (uint32_t *)s->d_err + 1;
   const int64_t nsig = (int64_t)s->src.size();
   int32_t done = 0;
   while (done < nsteps) {
@@ -836,6 +841,7 @@ void run(pn_solver *s, int32_t nsteps) {
       }
       a.tmaps = grid_maps_for(s, in);
       a.flag_phase = (int32_t)((s->step + k) % kFlagPhases);
+      a.cols_phase = (int32_t)((s->step + k) % 3);
       a.sig_here = s->call_values ? 1 : 0;
       if (s->call_values)
         for (int64_t q = 0; q < nsig; q++) a.sig_vals[q] = to_store<T>(s->call_values[(done + k) * nsig + q]);

@@ -101,7 +101,7 @@ struct pn_solver {
   // stresses, from the magnitudes of the coefficients each is multiplied by
   // (velocities: dt*C*g and g; stresses: dt/rho*g, g and source weights);
   // block counts of the two paths [fp64, df64]
-  uint32_t *d_rflags = nullptr;
+  uint8_t *d_rflags = nullptr;
   int32_t r_elo = 1, r_ehi = 0, r_elo_s = 1, r_ehi_s = 0;
   double r_cmin = 1.0, r_cmax = 1.0, r_cmin_s = 1.0, r_cmax_s = 1.0;
   unsigned long long *d_pathcnt = nullptr;
@@ -110,7 +110,7 @@ struct pn_solver {
   // and the force weights (the kernel's g is then 1); 1.0 when not folded
   double gfold = 1.0;
   int32_t *d_err = nullptr;  // device error word of the grid kernels
-  uint32_t *d_rflags_stage = nullptr;  // FP64 form: set_state's tile flags before the state is accepted
+  uint8_t *d_rflags_stage = nullptr;  // FP64 form: set_state's tile flags before the state is accepted
   int32_t *d_nonfinite = nullptr;  // [4] set_state's NaN / infinity flags (velocity, stress), and
                                    // (FP64 form) an out-of-range value at a split site's copy
   // split sites (grid.copy_node / fix_cell): the step's fix-up tables, rebuilt

@@ -156,6 +156,15 @@ inline cudaError_t launch_overlapped(F f, dim3 grid, unsigned threads, size_t sm
   return cudaLaunchKernelEx(&cfg, f, args...);
 }
 
+// or bits into a byte of an array of flags, or clear it (the array's words are
+// only ever written by atomics while a kernel runs)
+__device__ __forceinline__ void flag_or(uint8_t *flags, int64_t i, uint32_t bits) {
+  atomicOr(reinterpret_cast<uint32_t *>(flags + (i & ~(int64_t)3)), bits << (8 * (int)(i & 3)));
+}
+__device__ __forceinline__ void flag_clear(uint8_t *flags, int64_t i) {
+  atomicAnd(reinterpret_cast<uint32_t *>(flags + (i & ~(int64_t)3)), ~(0xffu << (8 * (int)(i & 3))));
+}
+
 // the eight neighbours of element i of n: by its pattern, or from the table
 __device__ __forceinline__ void neighbours(const int4 *__restrict__ table, int n_patterns, int n, int i, int s[8]) {
   int4 lo, hi;

@@ -42,6 +42,8 @@ struct OwnGridLaunch {};
 template <typename T>
 struct OwnGridLaunch<T, true> : OwnLaunch<T, true> {
   int32_t fp64_chunk;  // FP64 form: layers per piece of a column on the FP64 path (0: not cut)
+  int32_t cols_phase;  // ... this step's number modulo 3,
+  uint32_t *fp64_cols;  // and the columns on that path in a step, three rotating counts (cut_columns)
   // (found from the ranges' addresses by every block, a 64 x 64 x 8 plate's FP32
   // step took 5.20 us instead of 5.16, a 400 x 400 x 40 laminate's 98.7 instead of 98.3)
   SlotPlaces places;
@@ -101,11 +103,11 @@ struct GridArgs : OwnGridLaunch<T, OWN> {
   const T *cm_w;
   int32_t test_skip_layer;  // failure-path test: the layer whose copies are never issued (kNoLayer: none)
   int32_t tile_rows;        // rows TY of the 32 x TY block tile (8, or 16 with the tensor-copy kernel)
-  // FP64 form with the tensor-copy kernel: per-tile path flag words [kFlagPhases][tiles]
+  // FP64 form with the tensor-copy kernel: per-tile path flags, bytes [kFlagPhases][tiles]
   // (rsg_grid_tma.cuh fp64_path) and the double-float ranges as biased double
   // exponents, [r_elo, r_ehi] for velocities and [r_elo_s, r_ehi_s] for
   // stresses and source terms; rflags null: no path choice (the other forms)
-  uint32_t *rflags;
+  uint8_t *rflags;
   int32_t flag_phase;       // (step of this launch's step 0) % kFlagPhases
   int32_t r_elo, r_ehi;
   int32_t r_elo_s, r_ehi_s;
@@ -180,7 +182,7 @@ __device__ __forceinline__ int2 slot_entries(const int2 *rng, int at, int tx, in
 }
 #endif
 
-// the FP64 form's flag words rotate: read (the previous step's), written by this
+// the FP64 form's flags rotate: read (the previous step's), written by this
 // step, being cleared for the next, and the step before the previous one's
 constexpr int kFlagPhases = 4;
 constexpr uint32_t kFlagNonzero = 0x20u;  // the tile stored a value other than zero

@@ -752,7 +752,7 @@ __device__ __forceinline__ void grid_block_tma(const Args &a, const Copies<typen
     }
     if (oorb) {
       const int nt = gxc * (a.ny / (TY - 1) + 1);
-      atomicOr(a.rflags + ((a.flag_phase + step + 1) % kFlagPhases) * nt + blk, oorb);
+      flag_or(a.rflags, ((a.flag_phase + step + 1) % kFlagPhases) * nt + blk, oorb);
     }
   }
 }
@@ -764,7 +764,7 @@ __device__ __forceinline__ void grid_block_tma(const Args &a, const Copies<typen
 // its first node and cell column for the tile on its left, rows likewise, and
 // a corner for a diagonal neighbour: both edge bits), or when one of this
 // step's source terms of its layers lies outside the range; the double-float
-// path (df64d) otherwise.  Flags rotate through four per-tile words: read
+// path (df64d) otherwise.  Flags rotate through four bytes per tile: read
 // (flag_phase + step) % 4, or-ed by this step's blocks (+1), cleared for the
 // step after next by each tile's first chunk (+2), and the step before the
 // previous one's (+3).  Block-uniform.
@@ -790,8 +790,8 @@ __device__ __forceinline__ bool fp64_path(const Args &a, int bx, int by, int k0,
   const int phase = (a.flag_phase + step) % kFlagPhases;
   const bool track = fp64_chunk_of(a) > 0;
   if (clear && t == 0) {
-    a.rflags[((phase + 2) % kFlagPhases) * nt + blk] = 0;
-    if (!track) atomicOr(a.rflags + ((phase + 1) % kFlagPhases) * nt + blk, kFlagNonzero);
+    flag_clear(a.rflags, ((phase + 2) % kFlagPhases) * nt + blk);
+    if (!track) flag_or(a.rflags, ((phase + 1) % kFlagPhases) * nt + blk, kFlagNonzero);
   }
   bool f = false, active = !track || a.n_copies > 0 || a.n_fix > 0;
   if (t < 9) {
@@ -837,23 +837,20 @@ __device__ __forceinline__ bool fp64_path(const Args &a, int bx, int by, int k0,
   return fp64;
 }
 
-// The columns on the FP64 path in the previous step, counted behind the flag
-// words (four words rotating like them): columns are cut into pieces while at
-// most three quarters of the launch's are on it.  With all of them there the
-// pieces' re-marched layers cost more than their balance gives (laminate 400 x
-// 400 x 40: 1.258 ms per step against 1.228 uncut; with half of them 0.767
-// against 0.844).
-template <typename Args>
-__device__ __forceinline__ bool cut_columns(const Args &a, int bx, int by, int gxc, int step, bool fp64,
+// The columns on the FP64 path in the previous step (three counts rotating like
+// the flags): columns are cut into pieces while at most three quarters of the
+// launch's are on it.  With all of them there the pieces' re-marched layers cost
+// more than their balance gives (laminate 400 x 400 x 40: 1.258 ms per step
+// against 1.228 uncut; with half of them 0.767 against 0.844).
+__device__ __forceinline__ bool cut_columns(const GridLaunch<double> &a, int bx, int by, int gxc, bool fp64,
                                             bool first) {
-  const int gyc = a.ny / 7 + 1, nt = gxc * gyc, phase = (a.flag_phase + step) % kFlagPhases;
-  uint32_t *count = a.rflags + kFlagPhases * nt;
+  const int gyc = a.ny / 7 + 1, nt = gxc * gyc, phase = a.cols_phase;
   if (first && threadIdx.x == 0) {
-    if (fp64) atomicAdd(count + (phase + 1) % kFlagPhases, 1u);
-    if (bx == 0 && by == 0) count[(phase + 2) % kFlagPhases] = 0;
+    if (fp64) atomicAdd(a.fp64_cols + (phase + 1) % 3, 1u);
+    if (bx == 0 && by == 0) a.fp64_cols[(phase + 2) % 3] = 0;
   }
   const uint32_t cols = (uint32_t)(a.tail_chunk > 0 ? a.tail_from : nt);
-  return 4 * __ldcg(count + phase) <= 3 * cols;
+  return 4 * __ldcg(a.fp64_cols + phase) <= 3 * cols;
 }
 
 // tile (bx, by) and layer range [k0, k0 + kc) of this block of a single
@@ -914,7 +911,8 @@ __device__ __forceinline__ void f64h_block(const Args &a, unsigned char *smem, i
   // launch's last wave (tail split) each
   if (threadIdx.x == 0 && first && (k0 == 0 || a.tail_chunk > 0) && a.path_count)
     atomicAdd(a.path_count + (fp64 ? 0 : 1), 1ull);
-  const bool cut = column && cut_columns(a, bx, by, gxc, step, fp64, first) && fp64;
+  bool cut = false;
+  if constexpr (is_launch<Args>::value) cut = column && cut_columns(a, bx, by, gxc, fp64, first) && fp64;
   if (!work) return;
   if (quiet) {  // (the copies already under way land before the block ends)
     if (first && threadIdx.x == cp.ISSUER) {

@@ -63,7 +63,7 @@ __device__ __forceinline__ void flag_range(const A &a, double v, int64_t i, int6
     return;
   const int gxc = a.nx / (kGridTileX - 1) + 1, gyc = a.ny / (a.tile_rows - 1) + 1;
   const int64_t blk = (j / (a.tile_rows - 1)) * gxc + i / (kGridTileX - 1);
-  atomicOr(a.rflags + ((a.flag_phase + step + 1) % kFlagPhases) * (int64_t)gxc * gyc + blk, 0x1fu);  // the tile, every edge
+  flag_or(a.rflags, ((a.flag_phase + step + 1) % kFlagPhases) * (int64_t)gxc * gyc + blk, 0x1fu);  // the tile, every edge
 }
 
 // velocity of copy q: x differences of Sxx, Sxy, Sxz; y of Sxy, Syy, Syz; z of

@@ -16,6 +16,7 @@
 
 #include "../../include/pannde_gb300.h"
 #include "df64.cuh"
+#include "rsg_common.cuh"
 #include "rsg_state.cuh"
 
 namespace {
@@ -45,7 +46,7 @@ __device__ __forceinline__ void flag_value(const pn::StateRangeFlags &rf, int64_
   const int bx = x / 31, tx = x - 31 * bx, by = y / rf.ty_own, ty = y - rf.ty_own * by;
   uint32_t bits = 1u | (tx == 0 ? 2u : 0u) | (ty == 0 ? 8u : 0u);
   if (rf.cell) bits |= (tx == 30 ? 4u : 0u) | (ty == rf.ty_own - 1 ? 16u : 0u);
-  atomicOr(rf.flags + (int64_t)by * rf.gxc + bx, bits);
+  pn::flag_or(rf.flags, (int64_t)by * rf.gxc + bx, bits);
 }
 
 // dst[map ? map[i] : i] = cvt(src[i]), i < n

@@ -8,13 +8,13 @@ namespace pn {
 
 // The FP64 form's tile flags for a state written into the voxel lattice:
 // each value outside [2^(e_lo-1023), 2^(e_hi-1022)) (zero aside) or-s the bits
-// the step kernel would record for it into its tile's word, flags[tile] (1
+// the step kernel would record for it into its tile's byte, flags[tile] (1
 // any; 2 / 4 the tile's first / last owned column; 8 / 16 its first / last
 // owned row; the last two for cells only).  Lattice index j = (layer * rows
 // + y) * pitch + x, tiles of 31 x ty_own owned sites, gxc tiles along x; an
 // index at or past lattice_len (a split site's copy) sets *unplaced instead.
 struct StateRangeFlags {
-  uint32_t *flags;
+  uint8_t *flags;
   int32_t *unplaced;
   int64_t lattice_len;
   int32_t pitch, rows, gxc, ty_own;

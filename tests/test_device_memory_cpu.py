@@ -176,3 +176,16 @@ def test_device_bytes_are_what_is_held(fake, form, prec):
         s.get_state()
         s.energy()
         assert fake.fake_held() - s.info()["device_bytes"] == before  # (what others hold)
+
+
+@pytest.mark.parametrize("nx, ny", [(5, 4), (62, 4), (70, 40)])
+def test_path_flags_take_no_more_than_three_words_a_tile(fake, monkeypatch, nx, ny):
+    """The FP64 form's flags keep to the room that three words per tile took."""
+    c = plate(nx=nx, ny=ny, radius=0.1e-3)
+    got = {}
+    for path in ("fp64", ""):  # (fp64: the form without flags)
+        monkeypatch.setenv("PN_F64_PATH", path)
+        with Solver.from_case(c, "f64", form="grid") as s:
+            got[path] = s.info()["device_bytes"]
+    tiles = (nx // 31 + 1) * (ny // 7 + 1)
+    assert got[""] - got["fp64"] <= 16 + 12 * tiles  # 16: the path counts
