@@ -536,7 +536,7 @@ int pn_solver_get_info(pn_solver *s, pn_solver_info *info) {
   info->n_source_cells = s->n_src_cells;
   info->n_sensors = s->n_sens;
   info->algorithmic_bytes_per_step = pn::step_bytes(s);
-  info->device_bytes = s->dev_bytes + s->uncounted_bytes;
+  info->device_bytes = s->dev_bytes;
   info->dt = s->dt;
   info->time = s->time;
   info->form = s->form;

@@ -120,12 +120,12 @@ void ranges_of(std::vector<Keyed> &L, int64_t n_slots, std::vector<int32_t> &rng
 void upload_ranges(pn_solver *s, const std::vector<Keyed> &L, const std::vector<int32_t> &rng, int tile_rows,
                    int2 *&out) {
   const size_t n_slots = rng.size() / 2;
-  std::vector<int32_t> all(2 * n_slots + (n_slots + 1) / 2 * 2, 0), node;  // (rows start on 8 bytes)
+  std::vector<int32_t> all(rng), node;
   std::vector<size_t> listed;  // rows' words that are places in node
-  for (size_t sl = 0; sl < n_slots; sl++) {
-    const int32_t e0 = all[2 * sl] = rng[2 * sl], e1 = all[2 * sl + 1] = rng[2 * sl + 1];
-    all[2 * n_slots + sl] = -1;
-    if (e0 == e1 || !s->d_tmaps) continue;
+  if (s->d_tmaps) all.resize(2 * n_slots + (n_slots + 1) / 2 * 2, -1);  // the places (rows start on 8 bytes)
+  for (size_t sl = 0; sl < n_slots && s->d_tmaps; sl++) {
+    const int32_t e0 = rng[2 * sl], e1 = rng[2 * sl + 1];
+    if (e0 == e1) continue;
     bool several = false;  // entries at one node of the slot
     for (int32_t e = e0 + 1; e < e1; e++) several = several || (L[e].key & 0xffff) == (L[e - 1].key & 0xffff);
     const size_t at = all.size();
@@ -148,7 +148,11 @@ void upload_ranges(pn_solver *s, const std::vector<Keyed> &L, const std::vector<
   }
   for (size_t q : listed) all[q] = (int32_t)((uint32_t)((size_t)all[q] + all.size()) | 0x80000000u);
   all.insert(all.end(), node.begin(), node.end());
-  out = s->alloc<int2>(all.size() * 4, (all.size() - rng.size()) * 4);
+  out = s->alloc_ranges(all.size() * 4, rng.size() * 4);
+  if (void *page = s->page_of(out)) {
+    std::memcpy(page, all.data(), all.size() * 4);
+    return;
+  }
   s->upload_raw(out, all.data(), all.size() * 4);
   ck(cudaStreamSynchronize(s->stream), "ranges upload");  // before the host list goes
 }
@@ -819,14 +823,15 @@ namespace {
 template <typename T>
 void run(pn_solver *s, int32_t nsteps) {
   GridLaunch<T> a{};
-  grid_args(s, a);
-  if (s->d_tmaps) a.places = slot_places(a, s->tile_rows);
-  a.fp64_cols = (uint32_t *)s->d_err + 1;
   const int64_t nsig = (int64_t)s->src.size();
   int32_t done = 0;
   while (done < nsteps) {
     int32_t chunk = nsteps - done;
     ensure_signal_rows(s, chunk);
+    // (after it: the table's room may have come from the slots' ranges)
+    grid_args(s, a);
+    if (s->d_tmaps) a.places = slot_places(a, s->tile_rows);
+    a.fp64_cols = (uint32_t *)s->d_err + 1;
     if (nsig > 0 && !s->sig_hold)
       chunk = (int32_t)std::min<int64_t>(chunk, s->sig_step0 + s->sig_rows - s->step);
     for (int32_t k = 0; k < chunk; k++) {

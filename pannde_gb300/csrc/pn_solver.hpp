@@ -65,13 +65,17 @@ struct pn_solver {
   pn::MeshTables mesh;
   pn::MaterialTables mat;
 
+  // memory of the solver; page: held in page-locked host memory instead (ranges
+  // that found no room for what lies behind them), counted as the part that counts
+  // either way
   struct Held {
     void *p;
-    int64_t counted, uncounted;  // bytes (uncounted: see alloc)
+    int64_t bytes, least;
+    void *page;
+    int64_t counted() const { return page ? least : bytes; }
   };
   std::vector<Held> held;
-  int64_t dev_bytes = 0;        // held, the uncounted ones not among them
-  int64_t uncounted_bytes = 0;
+  int64_t dev_bytes = 0;  // the budget's count of them
 
   // state: V[3] over nodes, S[6] over cells (grid form: buffer `cur` of two)
   void *V[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
@@ -190,33 +194,37 @@ struct pn_solver {
 
   bool is_df64() const { return precision == PN_PREC_DF64; }
 
-  // uncounted: bytes of it outside the budget (small indexes beside tables that
-  // a caller may have fitted to the byte)
+  bool fits(int64_t bytes) const {
+    const int64_t budget = pn::hbm_budget();
+    return budget < 0 || dev_bytes + bytes <= budget;
+  }
+
+  void hold(void *p, int64_t bytes, int64_t least, void *page = nullptr) {
+    held.push_back({p, bytes, least, page});
+    dev_bytes += held.back().counted();
+  }
+
   template <typename P>
-  P *alloc(size_t bytes, size_t uncounted = 0) {
+  P *alloc(size_t bytes) {
     if (bytes == 0) bytes = 16;
-    const int64_t budget = pn::hbm_budget(), counted = (int64_t)(bytes - uncounted);
-    if (budget >= 0 && dev_bytes + counted > budget && !(drop_reciprocals() && dev_bytes + counted <= budget))
-      throw pn::SetupError{PN_ERR_ALLOC, "device allocation exceeds PN_HBM_BUDGET_BYTES"};
+    while (!fits((int64_t)bytes))
+      if (!make_room()) throw pn::SetupError{PN_ERR_ALLOC, "device allocation exceeds PN_HBM_BUDGET_BYTES"};
     void *p = nullptr;
-    cudaError_t e = cudaMalloc(&p, bytes);
-    if (e == cudaErrorMemoryAllocation && drop_reciprocals()) {
-      (void)cudaGetLastError();
-      e = cudaMalloc(&p, bytes);
-    }
+    cudaError_t e;
+    while ((e = cudaMalloc(&p, bytes)) == cudaErrorMemoryAllocation && make_room()) (void)cudaGetLastError();
     if (e != cudaSuccess) {
       (void)cudaGetLastError();
       throw pn::SetupError{PN_ERR_ALLOC, std::string("cudaMalloc failed: ") + cudaGetErrorString(e)};
     }
-    held.push_back({p, counted, (int64_t)uncounted});
-    dev_bytes += counted;
-    uncounted_bytes += (int64_t)uncounted;
+    hold(p, (int64_t)bytes, (int64_t)bytes);
     return (P *)p;
   }
 
-  // the exact form's reciprocals are the first to go when something else needs
-  // the room (its kernels form them then); false: none held.  Argument blocks
-  // are filled after the last allocation before their launch.
+  // Tables kept for speed give way when something else needs the room; false: none
+  // left.  Argument blocks are filled after the last allocation before their launch.
+  bool make_room() { return drop_reciprocals() || ranges_to_host(); }
+
+  // the exact form's reciprocals (its kernels form them then)
   bool drop_reciprocals() {
     if (!d_rnode) return false;
     pn::ck(cudaStreamSynchronize(stream), "reciprocals sync");  // steps in flight read them
@@ -225,17 +233,73 @@ struct pn_solver {
     return true;
   }
 
+  // Ranges with the slots' rows behind them (grid form): in device memory where the
+  // whole fits, else in page-locked host memory that the kernels read, where the
+  // ranges alone fit.  (A step then reads a few of them over the CPU-GPU link.)
+  int2 *alloc_ranges(size_t bytes, size_t least) {
+    if (fits((int64_t)bytes)) {
+      void *p = nullptr;
+      if (cudaMalloc(&p, bytes) == cudaSuccess) {
+        hold(p, (int64_t)bytes, (int64_t)least);
+        return (int2 *)p;
+      }
+      (void)cudaGetLastError();
+    }
+    while (!fits((int64_t)least))
+      if (!make_room()) throw pn::SetupError{PN_ERR_ALLOC, "device allocation exceeds PN_HBM_BUDGET_BYTES"};
+    void *page = nullptr;
+    int2 *d = page_memory(bytes, page);
+    hold(d, (int64_t)bytes, (int64_t)least, page);
+    return d;
+  }
+  static int2 *page_memory(size_t bytes, void *&page) {
+    void *d = nullptr;
+    cudaError_t e = cudaHostAlloc(&page, bytes, cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(&d, page, 0);
+    if (e != cudaSuccess) {
+      (void)cudaGetLastError();
+      throw pn::SetupError{PN_ERR_ALLOC, std::string("page-locked memory: ") + cudaGetErrorString(e)};
+    }
+    return (int2 *)d;
+  }
+  void *page_of(const void *p) const {
+    for (const Held &h : held)
+      if (h.p == p) return h.page;
+    return nullptr;
+  }
+  bool ranges_to_host() {
+    bool moved = false;
+    for (int2 **r : {&d_frng, &d_mrng, &d_srng}) {
+      auto it = std::find_if(held.begin(), held.end(), [&](const Held &h) { return *r && h.p == (void *)*r; });
+      if (it == held.end() || it->page || it->least >= it->bytes) continue;
+      pn::ck(cudaStreamSynchronize(stream), "ranges sync");  // steps in flight read them
+      void *page = nullptr;
+      int2 *d = page_memory((size_t)it->bytes, page);
+      pn::ck(cudaMemcpy(page, *r, (size_t)it->bytes, cudaMemcpyDeviceToHost), "ranges");
+      cudaFree(*r);
+      dev_bytes -= it->counted();
+      it->p = *r = d;
+      it->page = page;
+      dev_bytes += it->counted();
+      moved = true;
+    }
+    return moved;
+  }
+
   template <typename P>
   void release(P *&p) {
     if (!p) return;
     auto it = std::find_if(held.begin(), held.end(), [&](const Held &h) { return h.p == (void *)p; });
     if (it != held.end()) {
-      dev_bytes -= it->counted;
-      uncounted_bytes -= it->uncounted;
+      dev_bytes -= it->counted();
+      free_held(*it);
       held.erase(it);
     }
-    cudaFree((void *)p);
     p = nullptr;
+  }
+  static void free_held(const Held &h) {
+    if (h.page) cudaFreeHost(h.page);
+    else cudaFree(h.p);
   }
 
   // upload a double host array in the storage type (double, float, or the
@@ -329,7 +393,7 @@ struct pn_solver {
 
   ~pn_solver() {
     clear_marks();
-    for (const Held &h : held) cudaFree(h.p);
+    for (const Held &h : held) free_held(h);
     held.clear();
   }
 };

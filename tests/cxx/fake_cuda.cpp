@@ -110,6 +110,16 @@ cudaError_t cudaFree(void *p) {
   g_held -= (int64_t)it->second.bytes;
   return cudaSuccess;
 }
+cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {  // (a device may read it)
+  *p = std::aligned_alloc(256, (n + 255) / 256 * 256);
+  g_blocks[(uintptr_t)*p] = Block{n, true};
+  return cudaSuccess;
+}
+cudaError_t cudaHostGetDevicePointer(void **d, void *h, unsigned) { return *d = h, cudaSuccess; }
+cudaError_t cudaFreeHost(void *p) {
+  g_held += (int64_t)g_blocks[(uintptr_t)p].bytes;
+  return cudaFree(p);
+}
 cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind k) {
   bool ok = true;
   if (k != cudaMemcpyDeviceToHost) ok = device(d, n, "copy to the device") && ok;
@@ -178,14 +188,19 @@ cudaError_t grid_step(const A &a) {
   g_launches++;
   for (const void *p : {(const void *)a.V_in[0], (const void *)a.V_out[2], (const void *)a.S_in[0],
                         (const void *)a.S_out[5], (const void *)a.coef, (const void *)a.mat, (const void *)a.f_rng,
-                        (const void *)a.m_rng, (const void *)a.s_rng})
+                        (const void *)a.m_rng, (const void *)a.s_rng, (const void *)a.places.f,
+                        (const void *)a.places.m, (const void *)a.places.s, (const void *)a.f_key})
     table(p, "grid launch");
   return cudaSuccess;
 }
 cudaError_t launch_grid_f32(const GridLaunch<float> &a, int, cudaStream_t) { return grid_step(a); }
 cudaError_t launch_grid_f64(const GridLaunch<double> &a, int, cudaStream_t) { return grid_step(a); }
 cudaError_t launch_grid_df64(const GridLaunch<float2> &a, int, cudaStream_t) { return grid_step(a); }
-cudaError_t launch_grid_tma(const void *, int, int, cudaStream_t) { return g_launches++, cudaSuccess; }
+cudaError_t launch_grid_tma(const void *a, int precision, int, cudaStream_t) {
+  return precision == PN_PREC_F32 ? grid_step(*(const GridLaunch<float> *)a)
+       : precision == PN_PREC_DF64 ? grid_step(*(const GridLaunch<float2> *)a)
+                                   : grid_step(*(const GridLaunch<double> *)a);
+}
 cudaError_t launch_grid_batch(const GridBatchLaunch &, int, int, cudaStream_t) { return g_launches++, cudaSuccess; }
 cudaError_t launch_grid_tma_batch(const GridBatchLaunch &, int, int, cudaStream_t) { return g_launches++, cudaSuccess; }
 cudaError_t launch_grid_split(const void *, int, cudaStream_t) { return cudaSuccess; }

@@ -189,3 +189,39 @@ def test_path_flags_take_no_more_than_three_words_a_tile(fake, monkeypatch, nx, 
             got[path] = s.info()["device_bytes"]
     tiles = (nx // 31 + 1) * (ny // 7 + 1)
     assert got[""] - got["fp64"] <= 16 + 12 * tiles  # 16: the path counts
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+def test_slots_rows_give_way_to_a_budget(fake, monkeypatch, prec):
+    """Grid form: what lies behind the slots' ranges takes no room that a
+    budget does not have.  The least budget is that of the form without it (the
+    classic kernel's, the tensor maps and tile tops beside it); up to the full
+    size the solver holds no more than the budget, and its launches read live
+    memory."""
+    c = plate(nx=70, ny=30)
+
+    def run(budget=None):
+        if budget is None:
+            monkeypatch.delenv("PN_HBM_BUDGET_BYTES", raising=False)
+        else:
+            monkeypatch.setenv("PN_HBM_BUDGET_BYTES", str(budget))
+        others = fake.fake_held()
+        with Solver.from_case(c, prec, form="grid") as s:
+            s.solve(2)
+            s.get_state()  # (staging and index maps)
+            s.solve(2)
+            assert budget is None or fake.fake_held() - others <= s.info()["device_bytes"] <= budget
+            return s.info()["device_bytes"]
+
+    full = run()
+    monkeypatch.setenv("PN_GRID_KERNEL", "classic")
+    classic = run()
+    monkeypatch.delenv("PN_GRID_KERNEL")
+    tiles = (70 // 31 + 1) * (30 // 7 + 1)
+    least = classic + 2 * 11 * 128 + 4 * tiles + (16 + 4 * tiles if prec == "f64" else 0)
+    assert least < full
+    for budget in {full, full - 1, (full + least) // 2, least + 1, least}:
+        run(budget)
+    with pytest.raises(N.PnError) as e:
+        run(least - 1)
+    assert e.value.code == N.PN_ERR_ALLOC
