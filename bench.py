@@ -626,6 +626,9 @@ def main():
         # form leaves tiles that hold nothing but zeros alone, so the whole
         # lattice's bytes are not what those steps move
         paths = line["roofline"].get("f64_paths")
+        if rd.get("f64_paths"):  # as many blocks as every launch of a developed state counts
+            paths["left_alone_blocks"] = (rd["f64_paths"]["fp64_blocks"] + rd["f64_paths"]["double_float_blocks"] -
+                                          paths["fp64_blocks"] - paths["double_float_blocks"])
         line["roofline"] = dict(rd, f64_paths_from_rest=paths,
                                 state="developed (f64_developed_state); the headline's window from rest leaves tiles "
                                       "of zeros alone and has no byte count of its own")

@@ -460,7 +460,8 @@ int pn_partitioned_destroy(pn_partitioned *p);
 
 /* Blocks of the FP64 grid form's step kernel that took the FP64 path and the
    double-float path since the solver was created (both 0 in other forms); a
-   tile column that a launch cuts into equal z chunks counts as one.
+   tile column that a launch cuts into equal z chunks counts as one, and one
+   that it leaves alone, holding nothing but zeros, as none.
    No counterpart in the reference: the FP64 form computes each tile in
    double-float arithmetic (48-bit significand, |error| well inside the
    1e-10 contract) unless the tile or a neighbour holds values outside

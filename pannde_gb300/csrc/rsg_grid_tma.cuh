@@ -908,8 +908,8 @@ __device__ __forceinline__ void f64h_block(const Args &a, unsigned char *smem, i
   bool quiet;
   const bool fp64 = fp64_path<8>(a, bx, by, cp.k0, cp.k1, gxc, step, first && k0 == 0, quiet);
   // a column cut into equal chunks or FP64 pieces counts once, the chunks of a
-  // launch's last wave (tail split) each
-  if (threadIdx.x == 0 && first && (k0 == 0 || a.tail_chunk > 0) && a.path_count)
+  // launch's last wave (tail split) each; one left alone took neither path
+  if (threadIdx.x == 0 && first && (k0 == 0 || a.tail_chunk > 0) && !(work && quiet) && a.path_count)
     atomicAdd(a.path_count + (fp64 ? 0 : 1), 1ull);
   bool cut = false;
   if constexpr (is_launch<Args>::value) cut = column && cut_columns(a, bx, by, gxc, fp64, first) && fp64;
