@@ -333,11 +333,17 @@ int pn_solver_get_info(pn_solver *s, pn_solver_info *info);
    S[6] receive the pointers.  Element type by precision (double, float, or
    float2 (hi, lo) for PN_PREC_DF64); order by form: the caller's node / cell
    numbering in the table form, the lattice numbering (x fastest) in the grid
-   form.  The FP64 grid form chooses per tile between FP64 and double-float
+   form.  The grid form keeps two halves of the state and swaps them every
+   step: the pointers are the current state's after an even number of further
+   steps and the other half's after an odd one, which the next step overwrites.
+   The FP64 grid form chooses per tile between FP64 and double-float
    arithmetic from the values its last step stored; this call puts every tile
    on the FP64 path for the next step, so values written through the pointers
    after this call and before the next solve are taken exactly -- call it
-   again after writing between later steps. */
+   again after writing between later steps: values written through pointers of
+   an earlier call are taken too, but by the arithmetic that the last step's
+   values chose.  (From this call on, every solve computes all tiles for two
+   steps before it again leaves those alone that hold nothing but zeros.) */
 int pn_solver_device_state(pn_solver *s, void **V, void **S);
 
 /* Energy audit of the current state, formed and summed in FP64 whatever the

@@ -554,7 +554,10 @@ int pn_solver_device_state(pn_solver *s, void **V, void **S) {
     if (!s || !V || !S) return set_err(PN_ERR_INVALID, "null argument");
     for (int k = 0; k < 3; k++) V[k] = s->V[s->cur][k];
     for (int k = 0; k < 6; k++) S[k] = s->S[s->cur][k];
-    if (s->form == PN_FORM_GRID) pn::grid_reset_range_flags(s);  // the caller may write through them
+    if (s->form == PN_FORM_GRID) {  // the caller may write through them, now and later (grid_run)
+      pn::grid_reset_range_flags(s);
+      s->pointers_out = true;
+    }
     return PN_OK;
   });
 }

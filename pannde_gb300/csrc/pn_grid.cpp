@@ -823,6 +823,13 @@ namespace {
 template <typename T>
 void run(pn_solver *s, int32_t nsteps) {
   GridLaunch<T> a{};
+  if (s->pointers_out && s->d_rflags && nsteps > 0) {  // no tile is taken for zeros by what the steps before stored
+    const GridMap &g = s->grid;
+    const int64_t tiles = (int64_t)(g.nx / (kGridTileX - 1) + 1) * (g.ny / (kGridTileRows - 1) + 1);
+    ck(launch_mark_tiles(s->d_rflags, tiles, (int)(s->step % kFlagPhases), (int)((s->step + kFlagPhases - 1) % kFlagPhases),
+                         s->stream),
+       "tile marks");
+  }
   const int64_t nsig = (int64_t)s->src.size();
   int32_t done = 0;
   while (done < nsteps) {

@@ -105,6 +105,7 @@ struct pn_solver {
   // stresses, from the magnitudes of the coefficients each is multiplied by
   // (velocities: dt*C*g and g; stresses: dt/rho*g, g and source weights);
   // block counts of the two paths [fp64, df64]
+  bool pointers_out = false;  // the caller has the state's addresses (pn_solver_device_state)
   uint8_t *d_rflags = nullptr;
   int32_t r_elo = 1, r_ehi = 0, r_elo_s = 1, r_ehi_s = 0;
   double r_cmin = 1.0, r_cmax = 1.0, r_cmin_s = 1.0, r_cmax_s = 1.0;

@@ -17,6 +17,7 @@
 #include "../../include/pannde_gb300.h"
 #include "df64.cuh"
 #include "rsg_common.cuh"
+#include "rsg_grid.cuh"
 #include "rsg_state.cuh"
 
 namespace {
@@ -47,6 +48,13 @@ __device__ __forceinline__ void flag_value(const pn::StateRangeFlags &rf, int64_
   uint32_t bits = 1u | (tx == 0 ? 2u : 0u) | (ty == 0 ? 8u : 0u);
   if (rf.cell) bits |= (tx == 30 ? 4u : 0u) | (ty == rf.ty_own - 1 ? 16u : 0u);
   pn::flag_or(rf.flags, (int64_t)by * rf.gxc + bx, bits);
+}
+
+__global__ void __launch_bounds__(256) k_mark_tiles(uint8_t *flags, int64_t tiles, int p0, int p1) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= tiles) return;
+  pn::flag_or(flags, p0 * tiles + i, pn::kFlagNonzero);
+  pn::flag_or(flags, p1 * tiles + i, pn::kFlagNonzero);
 }
 
 // dst[map ? map[i] : i] = cvt(src[i]), i < n
@@ -118,6 +126,12 @@ cudaError_t launch_state_store(int precision, const double *src, int64_t n, cons
     case PN_PREC_DF64: k_state_store<float2><<<nb, 256, 0, st>>>(src, n, map, (float2 *)dst, nonfinite, StateRangeFlags{}); break;
     default: k_state_store<double><<<nb, 256, 0, st>>>(src, n, map, (double *)dst, nonfinite, f); break;
   }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mark_tiles(uint8_t *flags, int64_t tiles, int p0, int p1, cudaStream_t st) {
+  if (tiles <= 0) return cudaSuccess;
+  k_mark_tiles<<<(unsigned)((tiles + 255) / 256), 256, 0, st>>>(flags, tiles, p0, p1);
   return cudaGetLastError();
 }
 

@@ -30,6 +30,10 @@ cudaError_t launch_state_store(int precision, const double *src, int64_t n, cons
                                void *dst, cudaStream_t st, int32_t *nonfinite = nullptr,
                                const StateRangeFlags *rf = nullptr);
 
+// The FP64 form's flags of a state that may have been written from outside: every
+// tile holds values, in both buffer halves (phases p0 and p1 of flags [.][tiles]).
+cudaError_t launch_mark_tiles(uint8_t *flags, int64_t tiles, int p0, int p1, cudaStream_t st);
+
 // Read src[map[i]] (src[i] when map is null) in the storage type of
 // `precision` and write it as FP64 to dst[i] (device), i < n.
 cudaError_t launch_state_load(int precision, const void *src, int64_t n, const int64_t *map,

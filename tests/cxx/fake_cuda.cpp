@@ -222,6 +222,10 @@ cudaError_t launch_state_store(int, const double *, int64_t, const int64_t *, vo
 cudaError_t launch_state_load(int, const void *, int64_t, const int64_t *, double *, cudaStream_t) {
   return cudaSuccess;
 }
+cudaError_t launch_mark_tiles(uint8_t *flags, int64_t tiles, int p0, int p1, cudaStream_t) {
+  device(flags + (p0 > p1 ? p0 : p1) * tiles, (size_t)tiles, "tile marks");
+  return cudaSuccess;
+}
 int energy_blocks(int64_t) { return 1; }
 cudaError_t launch_energy_nodes(int, const void *const[3], const double *, int64_t, double *, int, cudaStream_t) {
   return cudaSuccess;
