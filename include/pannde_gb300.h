@@ -210,7 +210,8 @@ typedef struct pn_plan {
   int32_t n_materials;
   int32_t uniform_spacing;
   double hx, hy, hz;                  /* the spacings when uniform_spacing */
-  int64_t device_bytes;               /* device memory pn_solver_create allocates (table form: at most) */
+  int64_t device_bytes;               /* device memory pn_solver_create needs (table form: at most; the
+                                         exact form keeps more where there is room, and gives it up) */
   int64_t algorithmic_bytes_per_step;
   int32_t form;                       /* the form PN_FORM_AUTO would pick */
   int32_t grid[3];                    /* grid form: cells per axis */

@@ -156,7 +156,7 @@ int create_common(const pn_mesh *mesh, double dt, int32_t mode, pn_solver **out,
     s->form = choose_form(s->mesh, s->mat, precision, form, s->grid);
     // size everything first so that a budget failure allocates nothing
     const int64_t need = s->form == PN_FORM_GRID ? pn::grid_footprint(s->grid, s->mat, precision)
-                                                 : pn::table_footprint(s->mesh, s->mat, precision, false);
+                                                 : pn::table_footprint(s->mesh, s->mat, precision);
     const int64_t budget = pn::hbm_budget();
     if (budget >= 0 && need > budget)
       return set_err(PN_ERR_ALLOC, "solver needs " + std::to_string(need) +
@@ -536,7 +536,10 @@ int pn_solver_get_info(pn_solver *s, pn_solver_info *info) {
   info->n_source_cells = s->n_src_cells;
   info->n_sensors = s->n_sens;
   info->algorithmic_bytes_per_step = pn::step_bytes(s);
-  info->device_bytes = s->dev_bytes;
+  {
+    const auto lock = s->hold_spares();
+    info->device_bytes = s->dev_bytes;
+  }
   info->dt = s->dt;
   info->time = s->time;
   info->form = s->form;

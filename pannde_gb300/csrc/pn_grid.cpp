@@ -823,6 +823,7 @@ namespace {
 template <typename T>
 void run(pn_solver *s, int32_t nsteps) {
   GridLaunch<T> a{};
+  s->note_capture();
   if (s->pointers_out && s->d_rflags && nsteps > 0) {  // no tile is taken for zeros by what the steps before stored
     const GridMap &g = s->grid;
     const int64_t tiles = (int64_t)(g.nx / (kGridTileX - 1) + 1) * (g.ny / (kGridTileRows - 1) + 1);

@@ -9,8 +9,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <cstdlib>
+#include <mutex>
+#include <shared_mutex>
 #include <string>
 #include <vector>
 
@@ -64,6 +67,30 @@ struct pn_solver {
 
   pn::MeshTables mesh;
   pn::MaterialTables mat;
+
+  // Solvers (exact form, of the whole process) that hold reciprocals, and the lock
+  // under which they are given up: by their own next allocation, or by another
+  // solver's that the device has no memory for.  Held shared while a solve's launches
+  // are given their addresses and while an exact solver's list of allocations changes.
+  struct Spares {
+    std::shared_mutex use;
+    std::vector<pn_solver *> of;
+  };
+  static Spares &spares() {
+    static Spares s;
+    return s;
+  }
+  std::shared_lock<std::shared_mutex> hold_spares() const {
+    return precision == PN_PREC_F64_EXACT ? std::shared_lock<std::shared_mutex>(spares().use)
+                                          : std::shared_lock<std::shared_mutex>();
+  }
+  // a stream capture has recorded launches of this solver: what they read stays
+  std::atomic<bool> captured{false};
+  void note_capture() {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &st) != cudaSuccess) (void)cudaGetLastError();
+    if (st == cudaStreamCaptureStatusActive) captured = true;
+  }
 
   // memory of the solver; page: held in page-locked host memory instead (ranges
   // that found no room for what lies behind them), counted as the part that counts
@@ -201,6 +228,7 @@ struct pn_solver {
   }
 
   void hold(void *p, int64_t bytes, int64_t least, void *page = nullptr) {
+    const auto lock = hold_spares();
     held.push_back({p, bytes, least, page});
     dev_bytes += held.back().counted();
   }
@@ -212,7 +240,8 @@ struct pn_solver {
       if (!make_room()) throw pn::SetupError{PN_ERR_ALLOC, "device allocation exceeds PN_HBM_BUDGET_BYTES"};
     void *p = nullptr;
     cudaError_t e;
-    while ((e = cudaMalloc(&p, bytes)) == cudaErrorMemoryAllocation && make_room()) (void)cudaGetLastError();
+    while ((e = cudaMalloc(&p, bytes)) == cudaErrorMemoryAllocation && (make_room() || drop_others(device)))
+      (void)cudaGetLastError();
     if (e != cudaSuccess) {
       (void)cudaGetLastError();
       throw pn::SetupError{PN_ERR_ALLOC, std::string("cudaMalloc failed: ") + cudaGetErrorString(e)};
@@ -227,11 +256,32 @@ struct pn_solver {
 
   // the exact form's reciprocals (its kernels form them then)
   bool drop_reciprocals() {
-    if (!d_rnode) return false;
+    if (precision != PN_PREC_F64_EXACT) return false;
+    std::unique_lock<std::shared_mutex> lock(spares().use);
+    if (!d_rnode || captured) return false;
     pn::ck(cudaStreamSynchronize(stream), "reciprocals sync");  // steps in flight read them
-    release(d_rnode);
-    d_rcell = nullptr;
+    give_up_reciprocals();
     return true;
+  }
+  void give_up_reciprocals() {  // (under the lock)
+    release_held(d_rnode);
+    d_rnode = d_rcell = nullptr;
+    auto &of = spares().of;
+    of.erase(std::remove(of.begin(), of.end(), this), of.end());
+  }
+  // another solver's reciprocals on this device; false: none
+  static bool drop_others(int device) {
+    std::unique_lock<std::shared_mutex> lock(spares().use);
+    for (pn_solver *s : spares().of) {
+      if (s->device != device || s->captured) continue;
+      if (cudaDeviceSynchronize() != cudaSuccess) {  // its steps in flight read them
+        (void)cudaGetLastError();
+        return false;
+      }
+      s->give_up_reciprocals();
+      return true;
+    }
+    return false;
   }
 
   // Ranges with the slots' rows behind them (grid form): in device memory where the
@@ -270,6 +320,7 @@ struct pn_solver {
   }
   bool ranges_to_host() {
     bool moved = false;
+    if (captured) return false;
     for (int2 **r : {&d_frng, &d_mrng, &d_srng}) {
       auto it = std::find_if(held.begin(), held.end(), [&](const Held &h) { return *r && h.p == (void *)*r; });
       if (it == held.end() || it->page || it->least >= it->bytes) continue;
@@ -290,13 +341,16 @@ struct pn_solver {
   template <typename P>
   void release(P *&p) {
     if (!p) return;
-    auto it = std::find_if(held.begin(), held.end(), [&](const Held &h) { return h.p == (void *)p; });
-    if (it != held.end()) {
-      dev_bytes -= it->counted();
-      free_held(*it);
-      held.erase(it);
-    }
+    const auto lock = hold_spares();
+    release_held(p);
     p = nullptr;
+  }
+  void release_held(const void *p) {
+    auto it = std::find_if(held.begin(), held.end(), [&](const Held &h) { return h.p == p; });
+    if (it == held.end()) return;
+    dev_bytes -= it->counted();
+    free_held(*it);
+    held.erase(it);
   }
   static void free_held(const Held &h) {
     if (h.page) cudaFreeHost(h.page);
@@ -394,6 +448,11 @@ struct pn_solver {
 
   ~pn_solver() {
     clear_marks();
+    if (precision == PN_PREC_F64_EXACT) {
+      std::unique_lock<std::shared_mutex> lock(spares().use);
+      auto &of = spares().of;
+      of.erase(std::remove(of.begin(), of.end(), this), of.end());
+    }
     for (const Held &h : held) free_held(h);
     held.clear();
   }
@@ -411,8 +470,7 @@ int64_t sig_row(const pn_solver *s, int64_t step_in_call);  // row of this step
 int symmetry_class(const MaterialTables &mt);
 
 // table form (pn_table.cpp)
-// (reciprocals: with the exact form's reciprocal spacings, which it can do without)
-int64_t table_footprint(const MeshTables &m, const MaterialTables &mt, int precision, bool reciprocals = true);
+int64_t table_footprint(const MeshTables &m, const MaterialTables &mt, int precision);
 void table_create(pn_solver *s);
 void table_sources(pn_solver *s);
 void table_sensors(pn_solver *s, const std::vector<std::pair<int32_t, int32_t>> &sorted);

@@ -11,14 +11,13 @@
 
 namespace pn {
 
-int64_t table_footprint(const MeshTables &m, const MaterialTables &mt, int precision, bool reciprocals) {
+int64_t table_footprint(const MeshTables &m, const MaterialTables &mt, int precision) {
   const int64_t nn = m.n_nodes, nc = m.n_cells;
   const int64_t e = precision == PN_PREC_F32 ? 4 : 8;
   const bool per_elem = precision == PN_PREC_F64_EXACT || !m.uniform;
   int64_t need = nn * 3 * e + nc * 6 * e + nc * 32 + nn * 32 + nn * e + nc * 4 +
                  (int64_t)mt.n_mat * 36 * e;
   if (per_elem) need += nn * 3 * e + nc * 3 * e;
-  if (precision == PN_PREC_F64_EXACT && reciprocals) need += nn * 6 * e + nc * 6 * e;
   return need;
 }
 
@@ -143,12 +142,22 @@ void table_create(pn_solver *s) {
     s->upload_real(s->d_gnode, g.data(), g.size());
     s->upload_real(s->d_gcell, h.data(), h.size());
     if (exact) {
-      try {  // two words of every element's reciprocals
-        s->d_rnode = s->alloc<void>(2 * (g.size() + h.size()) * e);
-        s->d_rcell = (double *)s->d_rnode + 2 * g.size();
-      } catch (const SetupError &) {  // no room: the kernels form the reciprocals themselves
+      // two words of every element's reciprocals, where that is a small part (an
+      // eighth) of what is free: other solvers get them back when they need the memory
+      // (drop_others), other libraries' allocations cannot; without them the kernels
+      // form them
+      const size_t bytes = 2 * (g.size() + h.size()) * e;
+      size_t free = 0, total = 0;
+      if (cudaMemGetInfo(&free, &total) != cudaSuccess) (void)cudaGetLastError();
+      void *rec = nullptr;
+      if (s->fits((int64_t)bytes) && bytes <= free / 8 && cudaMalloc(&rec, bytes) != cudaSuccess) {
+        (void)cudaGetLastError();
+        rec = nullptr;
       }
-      if (s->d_rcell) {
+      if (rec) {
+        s->hold(rec, (int64_t)bytes, (int64_t)bytes);
+        s->d_rnode = rec;
+        s->d_rcell = (double *)rec + 2 * g.size();
         ck(launch_exact_reciprocals((const double *)s->d_gnode, (int64_t)g.size(), (double *)s->d_rnode, s->stream),
            "reciprocals");
         ck(launch_exact_reciprocals((const double *)s->d_gcell, (int64_t)h.size(), (double *)s->d_rcell, s->stream),
@@ -158,6 +167,10 @@ void table_create(pn_solver *s) {
     ck(cudaStreamSynchronize(s->stream), "create sync");  // before the arrays go
   }
   ck(cudaStreamSynchronize(s->stream), "create sync");
+  if (s->d_rnode) {
+    std::unique_lock<std::shared_mutex> lock(pn_solver::spares().use);
+    pn_solver::spares().of.push_back(s);
+  }
 }
 
 void table_put_state(pn_solver *s, const double *const *V, const double *const *S) {
@@ -296,12 +309,14 @@ template <typename T>
 void run(pn_solver *s, int32_t nsteps) {
   VelLaunch<T> va{};
   StressLaunch<T> sa{};
+  s->note_capture();
   const int64_t nsig = (int64_t)s->src.size();
   int32_t done = 0;
   while (done < nsteps) {
     int32_t chunk = nsteps - done;
     ensure_signal_rows(s, chunk);
     // (after it: the table's room may have come from the exact form's reciprocals)
+    const auto lock = s->hold_spares();  // until the chunk's launches are enqueued
     table_args(s, va, sa);
     va.recips = (const T *)s->d_rnode;
     sa.recips = (const T *)s->d_rcell;

@@ -25,6 +25,7 @@ struct Block {
 std::map<uintptr_t, Block> g_blocks;
 int64_t g_held = 0, g_room = -1;  // bytes held; most that may be (-1: any)
 int g_faults = 0;
+bool g_capturing = false;
 std::string g_first;
 int64_t g_launches = 0, g_null_reciprocals = 0, g_chunk_choices = 0;
 
@@ -83,7 +84,9 @@ int64_t fake_launches_without_reciprocals() { return g_null_reciprocals; }
 int64_t fake_chunk_choices() { return g_chunk_choices; }
 int64_t fake_held() { return g_held; }
 void fake_set_room(int64_t bytes) { g_room = bytes; }
+void fake_set_capturing(int on) { g_capturing = on != 0; }
 void fake_reset() {
+  g_capturing = false;
   g_faults = 0;
   g_first.clear();
   g_launches = g_null_reciprocals = g_chunk_choices = 0;
@@ -139,6 +142,15 @@ cudaError_t cudaGetDevice(int *d) { return *d = 0, cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr, int) { return *v = 152, cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t) { return "fake"; }
+cudaError_t cudaMemGetInfo(size_t *f, size_t *t) {
+  *t = (size_t)1 << 38;
+  *f = g_room >= 0 ? (size_t)(g_room - g_held) : *t;
+  return cudaSuccess;
+}
+cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
+cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus *st) {
+  return *st = g_capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone, cudaSuccess;
+}
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *, const void *) { return cudaErrorInvalidValue; }
 cudaError_t cudaEventCreate(cudaEvent_t *e) { return *e = nullptr, cudaSuccess; }

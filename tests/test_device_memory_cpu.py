@@ -225,3 +225,57 @@ def test_slots_rows_give_way_to_a_budget(fake, monkeypatch, prec):
     with pytest.raises(N.PnError) as e:
         run(least - 1)
     assert e.value.code == N.PN_ERR_ALLOC
+
+
+def test_another_solver_takes_the_reciprocals_room(fake):
+    """Device memory that holds one exact solver's reciprocals or another
+    solver, not both: the other solver is created, and the first goes on
+    without; one whose launches a stream capture recorded keeps them."""
+    c = plate(nx=30, ny=30)
+    base = fake.fake_held()
+    with Solver.from_case(c, "f64_exact") as a:
+        a.solve(2)
+        one = fake.fake_held() - base
+        recips = 48 * (c.mesh.n_nodes + c.mesh.n_cells)
+        with Solver.from_case(c, "f32", form="table") as b:
+            b.solve(2)
+            two = fake.fake_held() - base - one
+    for captured in (False, True):
+        fake.fake_reset()
+        with Solver.from_case(c, "f64_exact") as a:
+            fake.fake_set_capturing(captured)
+            a.solve(2)
+            fake.fake_set_capturing(False)
+            assert fake.fake_launches_without_reciprocals() == 0
+            fake.fake_set_room(base + one + two - recips)
+            if captured:
+                with pytest.raises(N.PnError):
+                    Solver.from_case(c, "f32", form="table").solve(2)
+                a.solve(1)
+                assert fake.fake_launches_without_reciprocals() == 0
+                continue
+            with Solver.from_case(c, "f32", form="table") as b:
+                b.solve(2)
+                a.solve(2)
+                assert fake.fake_launches_without_reciprocals() == 4
+                assert a.info()["device_bytes"] == one - recips
+
+
+def test_reciprocals_leave_most_of_the_memory_free(fake):
+    """They are taken only as a small part of what is free (other libraries
+    cannot get them back), and a plan does not count them."""
+    import ctypes as ct
+    c = plate()
+    base = fake.fake_held()
+    recips = 48 * (c.mesh.n_nodes + c.mesh.n_cells)
+    m, k1 = c.mesh.as_struct()
+    tab, k2 = c.material_table()
+    plan = N.PnPlan()
+    N.check(fake.pn_plan_solver(ct.byref(m), None, ct.byref(tab), c.dt, N.PN_PREC_F64_EXACT, ct.byref(plan)))
+    for room, without in ((plan.device_bytes + 9 * recips, False), (plan.device_bytes + 7 * recips, True)):
+        fake.fake_reset()
+        fake.fake_set_room(base + room)
+        with Solver(c.mesh, c, c.dt, "f64_exact") as s:
+            assert s.info()["device_bytes"] == plan.device_bytes + (0 if without else recips)
+            s.solve(1)
+            assert fake.fake_launches_without_reciprocals() == (2 if without else 0)
