@@ -239,6 +239,7 @@ def time_device(case, prec, steps, warmup, torch, dist, energy=False, state=None
     s.solve(steps)
     kt = s.kernel_times()
     info = s.info()
+    info["table_bytes"] = s.table_bytes()
     info["path_counts"] = (p1[0] - p0[0], p1[1] - p0[1])
     if energy:  # FP64 energy audit of the final state
         info["energy"] = s.energy()
@@ -250,10 +251,10 @@ def roofline(case, info, kt, prec, peak, peak_kind):
     """HBM roofline of the dominant kernel from its CUDA-event average.
 
     Algorithmic bytes per launch:
-      table form  velocity: S read (6e/cell), V read+write, dt/rho, connectivity (7e+5 /node)
-                  stress:   S read+write, material id, connectivity (12e+4+5 /cell), V read (3e /node)
-                  (connectivity as patterns; pn_solver_info counts the 32-byte tables
-                  that a mesh with many patterns keeps)
+      table form  velocity: S read (6e/cell), V read+write, dt/rho, tables (7e+tn /node)
+                  stress:   S read+write, material id, tables (12e+4+tc /cell), V read (3e /node)
+                  (tn, tc: pn_solver_table_bytes -- connectivity, spacings, reciprocals as held;
+                  pn_solver_info counts the 32-byte connectivity tables)
       grid form   fused step: S read+write + material byte (12e+1 /lattice cell),
                   V read+write + dt/rho (7e /lattice node) -- pn_solver_info
     with e the bytes per value (4 FP32, 8 FP64 and double-float)."""
@@ -263,8 +264,9 @@ def roofline(case, info, kt, prec, peak, peak_kind):
     if info.get("form_name") == "grid":
         alg = {"grid_step": info["algorithmic_bytes_per_step"]}
     else:
-        alg = {"velocity": nc * 6 * e + nn * (7 * e + 5),
-               "stress": nc * (12 * e + 9) + nn * 3 * e}
+        tn, tc = info["table_bytes"]
+        alg = {"velocity": nc * 6 * e + nn * (7 * e + tn),
+               "stress": nc * (12 * e + 4 + tc) + nn * 3 * e}
     dom = max(avg, key=lambda k: avg[k])
     achieved = alg[dom] / (avg[dom] * 1e-3) / 1e9
     form = info.get("form_name", "table")

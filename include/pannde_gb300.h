@@ -476,6 +476,13 @@ int pn_partitioned_destroy(pn_partitioned *p);
    double. */
 int pn_solver_path_counts(pn_solver *s, int64_t *fp64_blocks, int64_t *df64_blocks);
 
+/* Table form: bytes of tables that a step reads per node (velocity half) and
+   per cell (stress half) beside the state, dt/rho and the material id:
+   connectivity (32 as a table, 5 as patterns of relative neighbours), spacings
+   where each element has its own, the exact form's reciprocals while held.  (A
+   measurement aid; 0 in the grid form.) */
+int pn_solver_table_bytes(pn_solver *s, int32_t *per_node, int32_t *per_cell);
+
 /* ---- diagnostics -------------------------------------------------------------
    Issue rates of the arithmetic pipes the step kernels lean on, measured on
    the current device (no counterpart in the reference; a measurement aid for

@@ -589,6 +589,17 @@ int pn_solver_path_counts(pn_solver *s, int64_t *fp64_blocks, int64_t *df64_bloc
   });
 }
 
+int pn_solver_table_bytes(pn_solver *s, int32_t *per_node, int32_t *per_cell) {
+  if (!s || !per_node || !per_cell) return set_err(PN_ERR_INVALID, "null argument");
+  *per_node = *per_cell = 0;
+  if (s->form != PN_FORM_TABLE) return PN_OK;
+  const auto lock = s->hold_spares();
+  const int32_t own = (s->d_gnode ? 3 * (int32_t)s->esz : 0) + (s->d_rnode ? 48 : 0);
+  *per_node = (s->ncc_patterns > 0 ? 5 : 32) + own;
+  *per_cell = (s->hex_patterns > 0 ? 5 : 32) + own;
+  return PN_OK;
+}
+
 int pn_measure_pipe_rates(double *rates, int32_t n) {
   return guarded([&]() -> int {
     if (!rates || n < 0) return set_err(PN_ERR_INVALID, "null rates or negative count");

@@ -188,6 +188,13 @@ class Solver:
     def synchronize(self):
         N.check(self._lib.pn_solver_synchronize(self._h))
 
+    def table_bytes(self) -> tuple[int, int]:
+        """Bytes of tables a step of the table form reads per node and per cell
+        beside the state (pn_solver_table_bytes)."""
+        n, c = ctypes.c_int32(0), ctypes.c_int32(0)
+        N.check(self._lib.pn_solver_table_bytes(self._h, ctypes.byref(n), ctypes.byref(c)))
+        return n.value, c.value
+
     def path_counts(self) -> tuple[int, int]:
         """(FP64-path blocks, double-float-path blocks) of the FP64 grid
         form's steps so far (pn_solver_path_counts)."""

@@ -279,3 +279,20 @@ def test_reciprocals_leave_most_of_the_memory_free(fake):
             assert s.info()["device_bytes"] == plan.device_bytes + (0 if without else recips)
             s.solve(1)
             assert fake.fake_launches_without_reciprocals() == (2 if without else 0)
+
+
+def test_table_bytes_are_of_what_the_solver_holds(fake, monkeypatch):
+    c = plate()
+    shuffled = np.random.default_rng(3).permutation(c.mesh.n_cells)
+    many = cases.Case("m", cases.HexMesh(c.mesh.x, c.mesh.y, c.mesh.z, c.mesh.hexes[shuffled]), c.density, c.cij,
+                      c.cell_material[shuffled], c.dt)
+
+    def of(case, prec, form="table"):
+        with Solver(case.mesh, case, case.dt, prec, form) as s:
+            return s.table_bytes()
+    assert of(c, "f32", "grid") == (0, 0)
+    assert of(c, "f32") == (5, 5)  # a plate: patterns, one spacing
+    assert of(many, "f64") == (32, 5)  # the nodes' cells in no order: a table
+    assert of(c, "f64_exact") == (32 + 24 + 48, 32 + 24 + 48)
+    fake.fake_set_room(fake.fake_held() + 3000000)
+    assert of(plate(nx=40, ny=40), "f64_exact") == (32 + 24, 32 + 24)  # no reciprocals held
