@@ -13,24 +13,15 @@
 
 namespace pn {
 
-// 2: only the C11..C33 block and the shear diagonal; 1: monoclinic about z;
-// 0: general (see c_used in rsg_grid.cu and rsg_fast.cu)
+// the least general class (c_used) that holds every entry of the table other than zero
 int symmetry_class(const MaterialTables &mt) {
-  bool ortho = true, mono = true;
-  for (int32_t m = 0; m < mt.n_mat; m++) {
-    const double *c = &mt.c36[(size_t)m * 36];
+  int sym = 2;
+  for (int32_t m = 0; m < mt.n_mat; m++)
     for (int k = 0; k < 6; k++)
-      for (int j = 0; j < 6; j++) {
-        const double v = c[k * 6 + j];
-        if (v == 0.0) continue;
-        const bool in_ortho = (k < 3 && j < 3) || k == j;
-        const bool in_mono = in_ortho || (k == 5 && j < 3) || (j == 5 && k < 3) || (k == 3 && j == 4) ||
-                             (k == 4 && j == 3);
-        ortho = ortho && in_ortho;
-        mono = mono && in_mono;
-      }
-  }
-  return ortho ? 2 : mono ? 1 : 0;
+      for (int j = 0; j < 6; j++)
+        if (mt.c36[(size_t)m * 36 + k * 6 + j] != 0.0)
+          while (!c_used(sym, k, j)) sym--;
+  return sym;
 }
 
 namespace {
@@ -782,7 +773,7 @@ void grid_args(pn_solver *s, GridArgs<T, OWN> &a) {
     bool ortho = true;
     for (int k = 0; k < 6 && ortho && r < s->mat.n_mat; k++)
       for (int j = 0; j < 6; j++)
-        if (!((k < 3 && j < 3) || k == j) && s->mat.c36[(size_t)r * 36 + k * 6 + j] != 0.0) ortho = false;
+        if (!c_used(2, k, j) && s->mat.c36[(size_t)r * 36 + k * 6 + j] != 0.0) ortho = false;
     if (ortho) a.ortho_rows |= 1u << r;
   }
   a.n_copies = (int32_t)g.copy_node.size();

@@ -132,6 +132,19 @@ struct is_launch : std::false_type {};
 template <typename A>
 struct is_launch<A, std::void_t<decltype(A::sig_here)>> : std::true_type {};
 
+// Entries (k, j) of the stiffness product by symmetry class (symmetry_class): 0
+// general, 1 monoclinic about z, 2 orthotropic in the axes; the others are zero, so
+// 36 / 20 / 12 terms remain
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr bool c_used(int sym, int k, int j) {
+  return sym == 0 ? true
+       : sym == 2 ? ((k < 3 && j < 3) || k == j)
+                  : ((k < 3 && j < 3) || k == j || (k == 5 && j < 3) || (j == 5 && k < 3) ||
+                     (k == 3 && j == 4) || (k == 4 && j == 3));
+}
+
 #ifdef __CUDACC__
 // Programmatic dependent launch between the kernels of consecutive half
 // steps: launch_overlapped marks a launch that may start while the kernel

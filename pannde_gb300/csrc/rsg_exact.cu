@@ -118,8 +118,9 @@ struct Divisor {
 // System/6000 processor", 1990): q is within half an ulp and a term of 2^-52
 // ulp, so the value before the last rounding is off by less than 2^-53 times
 // that, below the least distance ulp/2 * ulp(c)/c of v / c from a boundary.  Both
-// need every intermediate to be a normal number: |v| in [2^-850, 2^850] and c in
-// [2^-100, 2^100] (or r = 0); ok says so.  A zero v gives +0 whatever its sign,
+// need quotients and remainders to be normal numbers: |v| in [2^-850, 2^850] and c in
+// [2^-100, 2^100] (or r = 0); ok says so.  (v rl may be subnormal, rl lies down to
+// about 2^-205: its rounding is then off by 2^-1075 at most, 2^-125 of the quotient.)  A zero v gives +0 whatever its sign,
 // as (0 + v) * 0.25 / d does.
 template <bool LONG>
 __device__ __forceinline__ double div_spacing(double v, const Divisor &d, bool &ok) {
@@ -213,13 +214,6 @@ __device__ __forceinline__ void divide9(const double v[3][3], Divisor &dx, Divis
       for (int j = 0; j < 9; j++) q[j / 3][j % 3] = i == j ? w : q[j / 3][j % 3];
     }
   }
-}
-
-__host__ __device__ constexpr bool c_used(int sym, int k, int j) {  // as in rsg_fast.cu
-  return sym == 0 ? true
-       : sym == 2 ? ((k < 3 && j < 3) || k == j)
-                  : ((k < 3 && j < 3) || k == j || (k == 5 && j < 3) || (j == 5 && k < 3) ||
-                     (k == 3 && j == 4) || (k == 4 && j == 3));
 }
 
 // sensor traces: V after this step at the sensors of this tile

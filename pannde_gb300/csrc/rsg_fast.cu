@@ -216,16 +216,6 @@ __device__ __forceinline__ void velocity_node(const A &a, int n, int tile, int s
   }
 }
 
-// entries of the stiffness product by the material table's symmetry class (0
-// general, 1 monoclinic about z, 2 orthotropic in the axes): the others are
-// zero, 36 / 20 / 12 terms
-__host__ __device__ constexpr bool c_used(int sym, int k, int j) {
-  return sym == 0 ? true
-       : sym == 2 ? ((k < 3 && j < 3) || k == j)
-                  : ((k < 3 && j < 3) || k == j || (k == 5 && j < 3) || (j == 5 && k < 3) ||
-                     (k == 3 && j == 4) || (k == 4 && j == 3));
-}
-
 // stress update of cell c
 template <typename R, bool UNIFORM, int SYM, bool OVERLAP = false, typename A>
 __device__ __forceinline__ void stress_cell(const A &a, int c, int tile, int step) {

@@ -67,16 +67,6 @@ template <> struct GNum<df64> {
   static __device__ __forceinline__ double dbl(df64 v) { return (double)v.hi + (double)v.lo; }
 };
 
-// stiffness entries kept by material symmetry class (all others are zero):
-// 0 general, 1 monoclinic about z (no C14 C15 C24 C25 C34 C35 C46 C56),
-// 2 orthotropic in the axes (C11..C33 block and the three shear diagonals)
-__host__ __device__ constexpr bool c_used(int sym, int k, int j) {
-  return sym == 0 ? true
-       : sym == 2 ? ((k < 3 && j < 3) || k == j)
-                  : ((k < 3 && j < 3) || k == j || (k == 5 && j < 3) || (j == 5 && k < 3) ||
-                     (k == 3 && j == 4) || (k == 4 && j == 3));
-}
-
 // one block's work: tile (bx, by) of a grid with gxc tiles along x, z chunk bz
 template <typename R, int TX, int TY, int SYM, typename A>
 __device__ __forceinline__ void grid_block(const A &a, int bx, int by, int bz,
@@ -435,14 +425,15 @@ static double chunk_time(const std::map<int, long long> &tops, int len, int sms,
   return std::max(share + uncovered * last * latency, last * std::max(latency, (double)per_sm));
 }
 
-int grid_chunk_for(const std::map<int, long long> &tops, int sms, int per_sm) {
+// tuning override: PN_GRID_KCHUNK cell layers per chunk (0: not set)
+static int kchunk_set() {
+  const char *v = std::getenv("PN_GRID_KCHUNK");
+  return v ? std::max(std::atoi(v), 0) : 0;
+}
+
+static int chunk_by_model(const std::map<int, long long> &tops, int sms, int per_sm) {
   const int nz = tops.empty() ? 0 : tops.rbegin()->first;
   if (nz <= 0) return 1;
-  // tuning override: PN_GRID_KCHUNK cell layers per chunk
-  if (const char *v = std::getenv("PN_GRID_KCHUNK")) {
-    const int k = std::atoi(v);
-    if (k > 0) return std::min(std::min(k, kGridChunkMax), nz);
-  }
   int best = 0;
   double best_t = 0.0;
   for (int chunks = (nz + kGridChunkMax - 1) / kGridChunkMax, last = 0; chunks <= nz; chunks++) {
@@ -458,25 +449,30 @@ int grid_chunk_for(const std::map<int, long long> &tops, int sms, int per_sm) {
   return best;
 }
 
+int grid_chunk_for(const std::map<int, long long> &tops, int sms, int per_sm) {
+  const int set = kchunk_set(), nz = tops.empty() ? 0 : tops.rbegin()->first;
+  return nz > 0 && set > 0 ? std::min(std::min(set, kGridChunkMax), nz) : chunk_by_model(tops, sms, per_sm);
+}
+
+// (called once per launch)
 int grid_chunk_for(int nz, long long xy_blocks, int sms, int per_sm) {
   if (nz <= 0) return 1;
+  if (const int set = kchunk_set()) return std::min(std::min(set, kGridChunkMax), nz);
   // as many columns as resident blocks or more: whole columns (each cut costs
   // two re-marched layers), the last wave's cut by grid_tail_split
-  if (xy_blocks >= (long long)sms * per_sm && !std::getenv("PN_GRID_KCHUNK")) {
+  if (xy_blocks >= (long long)sms * per_sm) {
     const int chunks = (nz + kGridChunkMax - 1) / kGridChunkMax;
     return (nz + chunks - 1) / chunks;
   }
-  // (called once per launch: the last answer of the thread is kept with what it depends on)
+  // the last answer of the thread is kept with what it depends on
   struct Last {
     int nz, sms, per_sm, len;
     long long xy;
   };
   static thread_local Last last{0, 0, 0, 0, 0};
-  const bool fixed = std::getenv("PN_GRID_KCHUNK") != nullptr;
-  if (!fixed && last.nz == nz && last.xy == xy_blocks && last.sms == sms && last.per_sm == per_sm) return last.len;
-  const int len = grid_chunk_for(std::map<int, long long>{{nz, xy_blocks}}, sms, per_sm);
-  if (!fixed) last = Last{nz, sms, per_sm, len, xy_blocks};
-  return len;
+  if (last.nz != nz || last.xy != xy_blocks || last.sms != sms || last.per_sm != per_sm)
+    last = Last{nz, sms, per_sm, chunk_by_model({{nz, xy_blocks}}, sms, per_sm), xy_blocks};
+  return last.len;
 }
 
 // The blocks of a one-chunk launch run in waves of `slots`; whole columns in

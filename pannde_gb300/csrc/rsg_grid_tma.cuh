@@ -201,13 +201,6 @@ template <> struct GNum<df64d> {
   static __device__ __forceinline__ double dbl(df64 v) { return join(v); }
 };
 
-__host__ __device__ constexpr bool c_used(int sym, int k, int j) {
-  return sym == 0 ? true
-       : sym == 2 ? ((k < 3 && j < 3) || k == j)
-                  : ((k < 3 && j < 3) || k == j || (k == 5 && j < 3) || (j == 5 && k < 3) ||
-                     (k == 3 && j == 4) || (k == 4 && j == 3));
-}
-
 // ---- PTX wrappers: mbarrier, tensor copy, timer -------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
