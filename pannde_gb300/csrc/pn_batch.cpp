@@ -95,7 +95,7 @@ void ensure_capacity(pn_batch *b, size_t args_bytes, size_t start_ints) {
     for (int k = 0; k < 2; k++) {
       if (b->d_args[k]) cudaFree(b->d_args[k]);
       b->d_args[k] = nullptr;
-      pn::ck(cudaMalloc(&b->d_args[k], args_bytes), "batch args");
+      pn::ck(pn_solver::malloc_beside((void **)&b->d_args[k], args_bytes), "batch args");
     }
     b->cap_args = args_bytes;
   }
@@ -103,7 +103,7 @@ void ensure_capacity(pn_batch *b, size_t args_bytes, size_t start_ints) {
     for (int k = 0; k < 2; k++) {
       if (b->d_start[k]) cudaFree(b->d_start[k]);
       b->d_start[k] = nullptr;
-      pn::ck(cudaMalloc(&b->d_start[k], start_ints * sizeof(int)), "batch tiles");
+      pn::ck(pn_solver::malloc_beside((void **)&b->d_start[k], start_ints * sizeof(int)), "batch tiles");
     }
     b->cap_start = start_ints;
   }

@@ -272,18 +272,18 @@ int pn_partitioned_create(const pn_mesh *mesh, const pn_material_table *material
       }
     }
     q->n_halo = (int64_t)ex.size();
-    pn::ck(cudaMalloc(&q->d_ex, std::max<size_t>(ex.size(), 1) * sizeof(int4)), "halo list");
+    pn::ck(pn_solver::malloc_beside((void **)&q->d_ex, std::max<size_t>(ex.size(), 1) * sizeof(int4)), "halo list");
     if (!ex.empty())
       pn::ck(cudaMemcpy(q->d_ex, ex.data(), ex.size() * sizeof(int4), cudaMemcpyHostToDevice), "halo list");
     std::vector<void *> vp((size_t)n_parts * 3);
     for (int p = 0; p < n_parts; p++)
       for (int c = 0; c < 3; c++) vp[(size_t)p * 3 + c] = q->parts[(size_t)p]->V[0][c];
-    pn::ck(cudaMalloc((void **)&q->d_vptr, vp.size() * sizeof(void *)), "halo pointers");
+    pn::ck(pn_solver::malloc_beside((void **)&q->d_vptr, vp.size() * sizeof(void *)), "halo pointers");
     pn::ck(cudaMemcpy(q->d_vptr, vp.data(), vp.size() * sizeof(void *), cudaMemcpyHostToDevice), "halo pointers");
     const size_t abytes = std::max(sizeof(pn::VelArgs<double>), sizeof(pn::StressArgs<double>)) * n_parts;
     for (int k = 0; k < 2; k++) {
-      pn::ck(cudaMalloc(&q->d_args[k], abytes), "partition args");
-      pn::ck(cudaMalloc((void **)&q->d_start[k], sizeof(int) * (n_parts + 1)), "partition tiles");
+      pn::ck(pn_solver::malloc_beside((void **)&q->d_args[k], abytes), "partition args");
+      pn::ck(pn_solver::malloc_beside((void **)&q->d_start[k], sizeof(int) * (n_parts + 1)), "partition tiles");
     }
     *out = q.release();
     return PN_OK;

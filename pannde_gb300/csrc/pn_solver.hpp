@@ -77,8 +77,8 @@ struct pn_solver {
     std::vector<pn_solver *> of;
   };
   static Spares &spares() {
-    static Spares s;
-    return s;
+    static Spares *s = new Spares;  // (outlives every solver)
+    return *s;
   }
   std::shared_lock<std::shared_mutex> hold_spares() const {
     return precision == PN_PREC_F64_EXACT ? std::shared_lock<std::shared_mutex>(spares().use)
@@ -231,6 +231,15 @@ struct pn_solver {
     const auto lock = hold_spares();
     held.push_back({p, bytes, least, page});
     dev_bytes += held.back().counted();
+  }
+
+  // device memory beside the solvers' own (a batch's staging, a partition's lists)
+  static cudaError_t malloc_beside(void **p, size_t bytes) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    while ((e = cudaMalloc(p, bytes)) == cudaErrorMemoryAllocation && drop_others(dev)) (void)cudaGetLastError();
+    return e;
   }
 
   template <typename P>

@@ -296,3 +296,15 @@ def test_table_bytes_are_of_what_the_solver_holds(fake, monkeypatch):
     assert of(c, "f64_exact") == (32 + 24 + 48, 32 + 24 + 48)
     fake.fake_set_room(fake.fake_held() + 3000000)
     assert of(plate(nx=40, ny=40), "f64_exact") == (32 + 24, 32 + 24)  # no reciprocals held
+
+
+def test_a_batch_takes_the_reciprocals_room(fake):
+    c = plate(nx=30, ny=30)
+    with Solver.from_case(c, "f64_exact") as a, Solver.from_case(c, "f32", form="table") as s, Batch() as b:
+        a.solve(1)
+        s.solve(1)
+        b.add(s)
+        fake.fake_set_room(fake.fake_held() + 16)
+        b.solve(2)  # its staging
+        a.solve(1)
+        assert fake.fake_launches_without_reciprocals() == 2
