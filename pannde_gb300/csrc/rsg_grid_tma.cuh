@@ -834,7 +834,12 @@ __device__ __forceinline__ bool fp64_path(const Args &a, int bx, int by, int k0,
 // the flags): columns are cut into pieces while at most three quarters of the
 // launch's are on it.  With all of them there the pieces' re-marched layers cost
 // more than their balance gives (laminate 400 x 400 x 40: 1.258 ms per step
-// against 1.228 uncut; with half of them 0.767 against 0.844).
+// against 1.228 uncut; with half of them 0.767 against 0.844).  The line lies
+// between runs from rest, whose other columns are quiet, and states with all
+// columns at work: there cutting pays without a tail split (400 x 400 x 16, half
+// the columns: 388 us against 452; 600 x 300 x 24, 70%: 716 against 795) and costs
+// 2-5% with one (400 x 400 x 24, a quarter: 462 against 439; 400 x 400 x 40: 721
+// against 701).
 __device__ __forceinline__ bool cut_columns(const GridLaunch<double> &a, int bx, int by, int gxc, bool fp64,
                                             bool first) {
   const int gyc = a.ny / 7 + 1, nt = gxc * gyc, phase = a.cols_phase;
@@ -1143,7 +1148,11 @@ struct SetupH {
 // own copies), where the launch has whole columns.  Laminate 400 x 400 x 40,
 // an initial pulse and a transducer, 20 steps with the state up- and
 // downloaded: 14.0 ms uncut, 12.5 / 11.4 / 11.8 in 2 / 3 / 5 pieces; a state that
-// is all double-float pays 1% for the further pieces' blocks.
+// is all double-float pays 1% for the further pieces' blocks.  On 400 x 400 columns
+// of other heights, us per step uncut / 2 / 3 / 4 pieces, from a pulse of 80 cells'
+// diameter: 16 layers 155 / 150 / 147 / 146, 20 197 / 179 / 152 / 152, 24 238 / 211 / 160
+// / 162, 32 314 / 271 / 212 / 192; of 200 cells: 255 / 180 / 183 / 183, 267 / 208 / 211 /
+// 214, 320 / 241 / 251 / 250, 425 / 324 / 316 / 320.
 template <int SYM>
 cudaError_t launch_h(const GridLaunch<double> &a, cudaStream_t st) {
   int sms = 0, per_sm = 0;
