@@ -154,6 +154,19 @@ constexpr bool c_used(int sym, int k, int j) {
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// The half-step kernels of the table form let the next one start when a thread
+// has formed its results, a launch of many blocks already when it begins: blocks of
+// the next kernel that start beside the first wave of a small one gather on the SMs
+// that it leaves free, and run there one after the other.  Us per step, at the
+// beginning / when formed (no overlap, older kernels): plate 64 x 64 x 8 (149 blocks)
+// FP64 35.3 / 17.8 (25.8), exact 64.6 / 41.0 (53.5); 96 x 96 x 16 (625 blocks) in
+// random numbering FP32 63.7 / 42.1 (49.5), FP64 41.8 / 40.3; 131 x 97 x 21 (1112) FP64
+// 64.2 / 64.6; 200 x 200 x 40 (6471) FP32 54.7 / 55.4, FP64 345 / 346.
+constexpr unsigned kManyBlocks = 1024;
+__device__ __forceinline__ void let_next_start_if_many() {
+  if (gridDim.x >= kManyBlocks) let_next_start();
+}
+
 template <typename F, typename... A>
 inline cudaError_t launch_overlapped(F f, dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchConfig_t cfg{};

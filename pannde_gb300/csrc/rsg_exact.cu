@@ -233,7 +233,7 @@ __device__ __forceinline__ void record(const VelLaunch<double> &a, int n, int st
 }
 
 __global__ void __launch_bounds__(kTile) k_velocity_exact(const __grid_constant__ VelLaunch<double> a, int step) {
-  let_next_start();
+  let_next_start_if_many();
   const int n = blockIdx.x * kTile + threadIdx.x;
   if (n >= a.n_nodes) return;
   const double cf = a.coef[n];
@@ -281,6 +281,7 @@ __global__ void __launch_bounds__(kTile) k_velocity_exact(const __grid_constant_
       for (int q = 0; q < 3; q++) v0[q] = q == d ? w : v0[q];
     }
   }
+  let_next_start();
 #pragma unroll
   for (int d = 0; d < 3; d++) vn[d] = vn[d] + cf * v0[d];
   a.V0[n] = vn[0];
@@ -291,7 +292,7 @@ __global__ void __launch_bounds__(kTile) k_velocity_exact(const __grid_constant_
 
 template <int SYM, bool MOMENTS>
 __global__ void __launch_bounds__(kTile) k_stress_exact(const __grid_constant__ StressLaunch<double> a, int step) {
-  let_next_start();
+  let_next_start_if_many();
   const int c = blockIdx.x * kTile + threadIdx.x;
   if (c >= a.n_cells) return;
   const int4 lo = a.hex[2 * c], hi = a.hex[2 * c + 1];
@@ -359,6 +360,7 @@ __global__ void __launch_bounds__(kTile) k_stress_exact(const __grid_constant__ 
 #pragma unroll
     for (int ks = 0; ks < 6; ks++) acc[ks] = acc[ks] + mom[ks];
   }
+  let_next_start();
 #pragma unroll
   for (int ks = 0; ks < 6; ks++) S[ks][c] = S[ks][c] + a.dt * acc[ks];
 }

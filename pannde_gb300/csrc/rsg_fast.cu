@@ -194,6 +194,7 @@ __device__ __forceinline__ void velocity_node(const A &a, int n, int tile, int s
         else az = az + v;
       }
     }
+    if (OVERLAP) let_next_start();
     v0 = madd(cf, ax, v0);
     v1 = madd(cf, ay, v1);
     v2 = madd(cf, az, v2);
@@ -265,6 +266,7 @@ __device__ __forceinline__ void stress_cell(const A &a, int c, int tile, int ste
         if (q == k) acc[q] = acc[q] + v;
     }
   }
+  if (OVERLAP) let_next_start();
 #pragma unroll
   for (int k = 0; k < 6; k++) {
 #pragma unroll
@@ -276,14 +278,14 @@ __device__ __forceinline__ void stress_cell(const A &a, int c, int tile, int ste
 
 template <typename R, bool UNIFORM>
 __global__ void __launch_bounds__(kTile) k_velocity(const __grid_constant__ VelLaunch<typename Num<R>::S> a, int step) {
-  let_next_start();
+  let_next_start_if_many();
   const int n = blockIdx.x * kTile + threadIdx.x;
   if (n < a.n_nodes) velocity_node<R, UNIFORM, true>(a, n, blockIdx.x, step);
 }
 
 template <typename R, bool UNIFORM, int SYM>
 __global__ void __launch_bounds__(kTile) k_stress(const __grid_constant__ StressLaunch<typename Num<R>::S> a, int step) {
-  let_next_start();
+  let_next_start_if_many();
   const int c = blockIdx.x * kTile + threadIdx.x;
   if (c < a.n_cells) stress_cell<R, UNIFORM, SYM, true>(a, c, blockIdx.x, step);
 }
