@@ -372,7 +372,7 @@ struct pn_solver {
     if (n == 0) return;
     if (is_df64()) {
       pn::hvec<float> tmp(2 * n);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (n > 16384)  // (as in all_finite)
       for (int64_t i = 0; i < (int64_t)n; i++) pn::split_df(src_[i], tmp[2 * i], tmp[2 * i + 1]);
       pn::ck(cudaMemcpyAsync(dst, tmp.data(), n * 8, cudaMemcpyHostToDevice, stream), "upload");
       pn::ck(cudaStreamSynchronize(stream), "upload sync");
@@ -380,7 +380,7 @@ struct pn_solver {
       pn::ck(cudaMemcpyAsync(dst, src_, n * 8, cudaMemcpyHostToDevice, stream), "upload");
     } else {
       pn::hvec<float> tmp(n);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (n > 16384)  // (as in all_finite)
       for (int64_t i = 0; i < (int64_t)n; i++) tmp[i] = (float)src_[i];
       pn::ck(cudaMemcpyAsync(dst, tmp.data(), n * 4, cudaMemcpyHostToDevice, stream), "upload");
       pn::ck(cudaStreamSynchronize(stream), "upload sync");
