@@ -301,6 +301,14 @@ __device__ __forceinline__ int member_of(const int *__restrict__ tile_start, int
   return lo;
 }
 
+// resident blocks per SM the batch kernels are compiled for: left to itself the
+// compiler took 64 registers in FP32 and 72-80 in the others' stress halves, one
+// block fewer.  Us per step: four plates of 0.8 M cells FP32 133 -> 123 (six blocks
+// 138), double-float 258 -> 240; eight of 14,000-90,000 cells FP32 26.8 -> 24.3, FP64
+// 91.2 -> 87.5; forty of 480 cells FP32 13.5 -> 14.1
+template <typename R> struct BatchBlocks { static constexpr int v = 4; };
+template <> struct BatchBlocks<float> { static constexpr int v = 5; };
+
 // batches: block b takes the contiguous share [b*T/B, (b+1)*T/B) of the T
 // tiles of all members (members' tiles in member order).  The argument block
 // of the member being worked on sits in shared memory, copied in once when
@@ -320,7 +328,7 @@ __device__ __forceinline__ void share_of_tiles(int total, int &t0, int &t1) {
 }
 
 template <typename R>
-__global__ void __launch_bounds__(kTile) k_velocity_batch(const VelArgs<typename Num<R>::S> *__restrict__ args,
+__global__ void __launch_bounds__(kTile, BatchBlocks<R>::v) k_velocity_batch(const VelArgs<typename Num<R>::S> *__restrict__ args,
                                                           const int *__restrict__ tile_start, int n_members,
                                                           int step) {
   __shared__ __align__(16) VelArgs<typename Num<R>::S> a;
@@ -346,7 +354,7 @@ __global__ void __launch_bounds__(kTile) k_velocity_batch(const VelArgs<typename
 }
 
 template <typename R>
-__global__ void __launch_bounds__(kTile) k_stress_batch(const StressArgs<typename Num<R>::S> *__restrict__ args,
+__global__ void __launch_bounds__(kTile, BatchBlocks<R>::v) k_stress_batch(const StressArgs<typename Num<R>::S> *__restrict__ args,
                                                         const int *__restrict__ tile_start, int n_members,
                                                         int step) {
   __shared__ __align__(16) StressArgs<typename Num<R>::S> a;
