@@ -389,6 +389,7 @@ int pn_solver_set_sensors(pn_solver *s, const int32_t *nodes, int32_t n, int32_t
     else pn::table_sensors(s, pr);
     s->d_traces = s->alloc<double>((size_t)std::max(capacity_steps, 1) * n * 3 * 8);
     pn::ck(cudaStreamSynchronize(s->stream), "sensors upload");
+    s->uploading.clear();
     s->n_sens = n;
     s->rec_cap = capacity_steps;
     return PN_OK;

@@ -145,7 +145,7 @@ void upload_ranges(pn_solver *s, const std::vector<Keyed> &L, const std::vector<
     return;
   }
   s->upload_raw(out, all.data(), all.size() * 4);
-  ck(cudaStreamSynchronize(s->stream), "ranges upload");  // before the host list goes
+  s->uploading.push_back(std::move(all));  // until the caller has waited
 }
 
 }  // namespace
@@ -324,6 +324,7 @@ bool grid_set_tile_rows(pn_solver *s, int rows) {
     grid_sensors(s, s->sensor_pairs);
   }
   ck(cudaStreamSynchronize(s->stream), "retile upload");
+  s->uploading.clear();
   return true;
 }
 
@@ -700,6 +701,7 @@ void grid_sources(pn_solver *s) {
   }
   grid_split_upload(s);
   ck(cudaStreamSynchronize(s->stream), "sources upload");
+  s->uploading.clear();
 }
 
 void grid_sensors(pn_solver *s, const std::vector<std::pair<int32_t, int32_t>> &pr) {

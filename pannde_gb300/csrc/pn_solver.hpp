@@ -102,6 +102,7 @@ struct pn_solver {
     int64_t counted() const { return page ? least : bytes; }
   };
   std::vector<Held> held;
+  std::vector<std::vector<int32_t>> uploading;  // host lists on their way to the device
   int64_t dev_bytes = 0;  // the budget's count of them
 
   // state: V[3] over nodes, S[6] over cells (grid form: buffer `cur` of two)

@@ -35,7 +35,8 @@ bool find_patterns(const int32_t *list, int32_t n, hvec<int32_t> &base, hvec<uin
   std::vector<std::vector<Row>> found((size_t)team);
   for (auto &rows : found) rows.reserve(kMost);  // nothing is allocated inside the region
   std::vector<char> many((size_t)team, 0);
-#pragma omp parallel for schedule(static) num_threads(team)
+  // (the process's whole team: one of another size would be built anew for the region)
+#pragma omp parallel for schedule(static, 1) if (team > 1)
   for (int r = 0; r < team; r++) {
     const int32_t e0 = (int32_t)((int64_t)n * r / team), e1 = (int32_t)((int64_t)n * (r + 1) / team);
     std::vector<Row> &rows = found[(size_t)r];
@@ -74,8 +75,11 @@ bool find_patterns(const int32_t *list, int32_t n, hvec<int32_t> &base, hvec<uin
       to[(size_t)r].push_back((uint8_t)at);
     }
   }
-#pragma omp parallel for schedule(static) num_threads(team)
-  for (int r = 0; r < team; r++)
+  bool renumbered = false;
+  for (auto &numbers : to)
+    for (size_t q = 0; q < numbers.size(); q++) renumbered = renumbered || numbers[q] != q;
+#pragma omp parallel for schedule(static, 1) if (team > 1)
+  for (int r = 0; r < (renumbered ? team : 0); r++)
     for (int32_t e = (int32_t)((int64_t)n * r / team); e < (int32_t)((int64_t)n * (r + 1) / team); e++)
       id[e] = to[(size_t)r][id[e]];
   offsets.clear();
@@ -84,11 +88,17 @@ bool find_patterns(const int32_t *list, int32_t n, hvec<int32_t> &base, hvec<uin
 }
 
 // the device's connectivity of one kind: patterns for the fast forms where they
-// suffice, else the table
-void upload_connectivity(pn_solver *s, const int32_t *list, int32_t n, int4 *&table, int32_t &n_patterns) {
+// suffice, else the table (the lists are the caller's: they live until it has waited)
+struct PatternLists {
   hvec<int32_t> base;
   hvec<uint8_t> id;
   std::vector<int32_t> offsets;
+};
+void upload_connectivity(pn_solver *s, const int32_t *list, int32_t n, int4 *&table, int32_t &n_patterns,
+                         PatternLists &lists) {
+  hvec<int32_t> &base = lists.base;
+  hvec<uint8_t> &id = lists.id;
+  std::vector<int32_t> &offsets = lists.offsets;
   if (s->precision != PN_PREC_F64_EXACT && n > 0 && find_patterns(list, n, base, id, offsets) &&
       offsets.size() * 4 + (size_t)n * 5 <= (size_t)n * 32) {  // (a tiny mesh's many patterns may be the larger)
     n_patterns = (int32_t)(offsets.size() / 8);
@@ -97,7 +107,6 @@ void upload_connectivity(pn_solver *s, const int32_t *list, int32_t n, int4 *&ta
     s->upload_raw(table, offsets.data(), offsets.size() * 4);
     s->upload_raw(d_base, base.data(), (size_t)n * 4);
     s->upload_raw(d_base + n, id.data(), (size_t)n);
-    ck(cudaStreamSynchronize(s->stream), "connectivity upload");  // before the host lists go
     return;
   }
   table = s->alloc<int4>((size_t)n * 32);
@@ -118,8 +127,9 @@ void table_create(pn_solver *s) {
   s->d_ctab = s->alloc<void>((size_t)s->mat.n_mat * 36 * e);
   for (int k = 0; k < 3; k++) ck(cudaMemsetAsync(s->V[0][k], 0, (size_t)nn * e, s->stream), "memset");
   for (int k = 0; k < 6; k++) ck(cudaMemsetAsync(s->S[0][k], 0, (size_t)nc * e, s->stream), "memset");
-  upload_connectivity(s, s->mesh.hex.data(), nc, s->d_hex, s->hex_patterns);
-  upload_connectivity(s, s->mesh.ncc.data(), nn, s->d_ncc, s->ncc_patterns);
+  PatternLists hex_lists, ncc_lists;
+  upload_connectivity(s, s->mesh.hex.data(), nc, s->d_hex, s->hex_patterns, hex_lists);
+  upload_connectivity(s, s->mesh.ncc.data(), nn, s->d_ncc, s->ncc_patterns, ncc_lists);
   s->upload_real(s->d_coef, s->mat.coef.data(), nn);
   s->upload_raw(s->d_mat, s->mat.cell_mat.data(), (size_t)nc * 4);
   s->sym = symmetry_class(s->mat);
