@@ -81,6 +81,10 @@ void cell_ijk(const GridMap &g, int64_t q, int64_t &i, int64_t &j, int64_t &k) {
   k = q / ((int64_t)g.pcx * g.ny);
 }
 
+// tiles from which on the FP64 form's columns are cut (their counts take room, a
+// few columns are no launch of whole ones)
+constexpr int64_t kCutTiles = 8;
+
 // (block, layer, local, payload) rows sorted by (block, layer) with the
 // per (block, layer) ranges
 struct Keyed {
@@ -425,7 +429,10 @@ void grid_create(pn_solver *s) {
                        std::max(s->r_cmax, s->r_cmax_s) > std::ldexp(1.0, 90);
   if (s->precision == PN_PREC_F64 && s->d_tmaps && s->r_elo <= s->r_ehi && s->r_elo_s <= s->r_ehi_s && !extreme) {
     const int64_t tiles = (int64_t)(g.nx / (kGridTileX - 1) + 1) * (g.ny / (kGridTileRows - 1) + 1);
-    s->d_rflags = s->alloc<uint8_t>((size_t)(kFlagPhases * tiles));  // (whole words: kFlagPhases is 4)
+    // the flags (kFlagPhases whole words per four tiles), then the column counts
+    const size_t flags = (size_t)((kFlagPhases * tiles + 7) / 8 * 8);
+    s->d_rflags = s->alloc<uint8_t>(flags + (tiles >= kCutTiles ? 3 * sizeof(unsigned long long) : 0));
+    if (tiles >= kCutTiles) s->d_fp64_cols = (unsigned long long *)(s->d_rflags + flags);
     s->d_pathcnt = s->alloc<unsigned long long>(2 * sizeof(unsigned long long));
     ck(cudaMemsetAsync(s->d_pathcnt, 0, 2 * sizeof(unsigned long long), s->stream), "memset");
     grid_reset_range_flags(s);
@@ -434,10 +441,11 @@ void grid_create(pn_solver *s) {
   ck(cudaStreamSynchronize(s->stream), "create sync");
 }
 
-// no flag set, no column counted (the counts, three words behind the error word)
+// no flag set, no column counted
 static void clear_flags(pn_solver *s, int64_t tiles) {
+  s->flags_step = s->step;
   ck(cudaMemsetAsync(s->d_rflags, 0, (size_t)(kFlagPhases * tiles), s->stream), "memset");
-  ck(cudaMemsetAsync(s->d_err + 1, 0, 3 * sizeof(uint32_t), s->stream), "memset");
+  if (s->d_fp64_cols) ck(cudaMemsetAsync(s->d_fp64_cols, 0, 3 * sizeof(unsigned long long), s->stream), "memset");
 }
 
 void grid_reset_range_flags(pn_solver *s) {
@@ -832,7 +840,7 @@ void run(pn_solver *s, int32_t nsteps) {
     // (after it: the table's room may have come from the slots' ranges)
     grid_args(s, a);
     if (s->d_tmaps) a.places = slot_places(a, s->tile_rows);
-    a.fp64_cols = (uint32_t *)s->d_err + 1;
+    a.fp64_cols = s->d_fp64_cols;
     if (nsig > 0 && !s->sig_hold)
       chunk = (int32_t)std::min<int64_t>(chunk, s->sig_step0 + s->sig_rows - s->step);
     for (int32_t k = 0; k < chunk; k++) {
@@ -847,7 +855,7 @@ void run(pn_solver *s, int32_t nsteps) {
       }
       a.tmaps = grid_maps_for(s, in);
       a.flag_phase = (int32_t)((s->step + k) % kFlagPhases);
-      a.cols_phase = (int32_t)((s->step + k) % 3);
+      a.cols_phase = (int32_t)((s->step + k) % 3) | (s->step + k < s->flags_step + 3 ? 4 : 0);
       a.sig_here = s->call_values ? 1 : 0;
       if (s->call_values)
         for (int64_t q = 0; q < nsig; q++) a.sig_vals[q] = to_store<T>(s->call_values[(done + k) * nsig + q]);

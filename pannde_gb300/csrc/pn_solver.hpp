@@ -135,6 +135,8 @@ struct pn_solver {
   // block counts of the two paths [fp64, df64]
   bool pointers_out = false;  // the caller has the state's addresses (pn_solver_device_state)
   uint8_t *d_rflags = nullptr;
+  unsigned long long *d_fp64_cols = nullptr;  // behind them
+  int64_t flags_step = 0;                      // step at which they were set anew
   int32_t r_elo = 1, r_ehi = 0, r_elo_s = 1, r_ehi_s = 0;
   double r_cmin = 1.0, r_cmax = 1.0, r_cmin_s = 1.0, r_cmax_s = 1.0;
   unsigned long long *d_pathcnt = nullptr;

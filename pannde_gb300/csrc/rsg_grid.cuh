@@ -42,8 +42,9 @@ struct OwnGridLaunch {};
 template <typename T>
 struct OwnGridLaunch<T, true> : OwnLaunch<T, true> {
   int32_t fp64_chunk;  // FP64 form: layers per piece of a column on the FP64 path (0: not cut)
-  int32_t cols_phase;  // ... this step's number modulo 3,
-  uint32_t *fp64_cols;  // and the columns on that path in a step, three rotating counts (cut_columns)
+  int32_t cols_phase;  // ... this step's number modulo 3 | 4 in the first three steps with new flags,
+  unsigned long long *fp64_cols;  // and the columns at work and on that path in a step, three rotating counts
+                                  // (cut_columns; null: columns are not cut)
   // (found from the ranges' addresses by every block, a 64 x 64 x 8 plate's FP32
   // step took 5.20 us instead of 5.16, a 400 x 400 x 40 laminate's 98.7 instead of 98.3)
   SlotPlaces places;

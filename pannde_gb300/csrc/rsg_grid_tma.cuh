@@ -830,25 +830,28 @@ __device__ __forceinline__ bool fp64_path(const Args &a, int bx, int by, int k0,
   return fp64;
 }
 
-// The columns on the FP64 path in the previous step (three counts rotating like
-// the flags): columns are cut into pieces while at most three quarters of the
-// launch's are on it.  With all of them there the pieces' re-marched layers cost
-// more than their balance gives (laminate 400 x 400 x 40: 1.258 ms per step
-// against 1.228 uncut; with half of them 0.767 against 0.844).  The line lies
-// between runs from rest, whose other columns are quiet, and states with all
-// columns at work: there cutting pays without a tail split (400 x 400 x 16, half
-// the columns: 388 us against 452; 600 x 300 x 24, 70%: 716 against 795) and costs
-// 2-5% with one (400 x 400 x 24, a quarter: 462 against 439; 400 x 400 x 40: 721
-// against 701).
+// The columns at work in the previous step and those of them on the FP64 path
+// (low and high half of three counts that rotate like the flags): columns are cut
+// into pieces while at most three quarters of the launch's are on that path.  With
+// all of them there the pieces' re-marched layers cost more than their balance
+// gives (laminate 400 x 400 x 40: 1.258 ms per step against 1.228 uncut; with half
+// of them 0.767 against 0.844).  A launch with a tail split cuts only while a
+// quarter of its columns is quiet: its whole columns fill the SMs once, and where
+// all work, the pieces come after (400 x 400 x 24, half the columns: 574 us against
+// 555; 400 x 400 x 40: 717 against 702); for three steps after the flags were set
+// anew every column works, and says nothing of that.  Without a split cutting pays there too
+// (400 x 400 x 16, half: 385 against 453; 600 x 300 x 24, three quarters: 750
+// against 795).
 __device__ __forceinline__ bool cut_columns(const GridLaunch<double> &a, int bx, int by, int gxc, bool fp64,
-                                            bool first) {
-  const int gyc = a.ny / 7 + 1, nt = gxc * gyc, phase = a.cols_phase;
+                                            bool quiet, bool first) {
+  const int gyc = a.ny / 7 + 1, nt = gxc * gyc, phase = a.cols_phase & 3;
   if (first && threadIdx.x == 0) {
-    if (fp64) atomicAdd(a.fp64_cols + (phase + 1) % 3, 1u);
+    if (fp64 || !quiet) atomicAdd(a.fp64_cols + (phase + 1) % 3, (fp64 ? 1ull << 32 : 0ull) + 1ull);
     if (bx == 0 && by == 0) a.fp64_cols[(phase + 2) % 3] = 0;
   }
-  const uint32_t cols = (uint32_t)(a.tail_chunk > 0 ? a.tail_from : nt);
-  return 4 * __ldcg(a.fp64_cols + phase) <= 3 * cols;
+  const unsigned long long n = __ldcg(a.fp64_cols + phase);
+  const uint32_t cols = (uint32_t)(a.tail_chunk > 0 ? a.tail_from : nt), working = (uint32_t)n;
+  return 4 * (uint32_t)(n >> 32) <= 3 * cols && (a.tail_chunk == 0 || (a.cols_phase & 4) != 0 || 4 * working <= 3 * cols);
 }
 
 // tile (bx, by) and layer range [k0, k0 + kc) of this block of a single
@@ -910,7 +913,7 @@ __device__ __forceinline__ void f64h_block(const Args &a, unsigned char *smem, i
   if (threadIdx.x == 0 && first && (k0 == 0 || a.tail_chunk > 0) && !(work && quiet) && a.path_count)
     atomicAdd(a.path_count + (fp64 ? 0 : 1), 1ull);
   bool cut = false;
-  if constexpr (is_launch<Args>::value) cut = column && cut_columns(a, bx, by, gxc, fp64, first) && fp64;
+  if constexpr (is_launch<Args>::value) cut = column && cut_columns(a, bx, by, gxc, fp64, quiet, first) && fp64;
   if (!work) return;
   if (quiet) {  // (the copies already under way land before the block ends)
     if (first && threadIdx.x == cp.ISSUER) {
@@ -1163,7 +1166,7 @@ cudaError_t launch_h(const GridLaunch<double> &a, cudaStream_t st) {
   dim3 grid = single_grid<8>(b, sms, per_sm);
   if (grid.x == 0) return cudaErrorInvalidValue;
   b.fp64_chunk = 0;
-  if (b.kchunk >= b.nz && b.nz >= 16) {
+  if (b.kchunk >= b.nz && b.nz >= 16 && b.fp64_cols) {
     b.fp64_chunk = std::max(8, (b.nz + 2) / 3);
     const unsigned pieces = (unsigned)((b.nz + b.fp64_chunk - 1) / b.fp64_chunk);
     const unsigned cols = b.tail_chunk > 0 ? (unsigned)b.tail_from : grid.x * grid.y;

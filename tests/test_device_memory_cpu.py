@@ -218,7 +218,8 @@ def test_slots_rows_give_way_to_a_budget(fake, monkeypatch, prec):
     classic = run()
     monkeypatch.delenv("PN_GRID_KERNEL")
     tiles = (70 // 31 + 1) * (30 // 7 + 1)
-    least = classic + 2 * 11 * 128 + 4 * tiles + (16 + 4 * tiles if prec == "f64" else 0)
+    flags = 16 + (4 * tiles + 7) // 8 * 8 + 24 if prec == "f64" else 0  # path counts, flags, column counts
+    least = classic + 2 * 11 * 128 + 4 * tiles + flags
     assert least < full
     for budget in {full, full - 1, (full + least) // 2, least + 1, least}:
         run(budget)

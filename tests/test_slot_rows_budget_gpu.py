@@ -36,7 +36,8 @@ def test_rows_in_host_memory(cuda_device, monkeypatch, how, prec):
     _, classic = run()
     monkeypatch.delenv("PN_GRID_KERNEL")
     tiles = (130 // 31 + 1) * (60 // 7 + 1)
-    least = classic + 2 * 11 * 128 + 4 * tiles + (16 + 4 * tiles if prec == "f64" else 0)
+    flags = 16 + (4 * tiles + 7) // 8 * 8 + 24 if prec == "f64" else 0  # path counts, flags, column counts
+    least = classic + 2 * 11 * 128 + 4 * tiles + flags
     assert least < full
     for budget in (full - 1, least):
         got, held = run(budget)
